@@ -9,6 +9,8 @@
 // tile to the next; tcgen05.commit releases a stage.  Two accumulator buffers in TMEM let the
 // epilogue of one tile overlap the main loop of the next.
 //
+// More than 128 rows go to the kernel on pairs of SMs (gemm_pair.cu); this one runs 65..128 rows, expert tiles and, where there is
+// no workspace for the stream-K kernel, fewer.
 // The 128-row operand of the instruction is the activation tile for prefill-sized m; for
 // m <= 64 the operands are swapped (weights take the 128 rows, tokens the N side) so that
 // small decode batches do not waste seven eighths of the tensor-core tile.
@@ -17,8 +19,7 @@
 // error in a device status word, stops waiting everywhere, frees its TMEM and returns.
 #include <cstdlib>
 
-#include "linear.cuh"
-#include "tcgen05.cuh"
+#include "gemm_tile.cuh"
 
 namespace lri {
 namespace {
@@ -26,37 +27,6 @@ namespace {
 using namespace tc;
 
 __device__ int g_gemm_status = 0;  // 0 ok, else the code of the first wait that gave up
-
-struct GemmShape {
-  int m, n, k;
-};
-
-// One unit of work of a persistent CTA: an output tile and a slice of K.
-struct WorkItem {
-  int tile_p, tile_q;
-};
-struct GemmGrid {
-  int tiles_p, tiles_q;
-  int group;  // P tiles per panel
-  // expert tiles: the number of P tiles in use and the weight matrix of each are read from the device
-  const int* tiles;
-  int matrix_rows;
-};
-// Order of the output tiles.  The P tiles are taken in panels of `group`; inside a panel the
-// Q tile is the slow index.  The CTAs that run at the same time then share one panel of P
-// (a few MB, stays in L2) and a handful of Q tiles, each of which all of them use at once, so
-// that both operands come from DRAM about once per panel instead of once per P tile.
-__device__ __forceinline__ WorkItem work_item(int item, const GemmGrid& g) {
-  WorkItem w;
-  const int panel_items = g.group * g.tiles_q;
-  const int panel = item / panel_items;
-  const int r = item - panel * panel_items;
-  const int p0 = panel * g.group;
-  const int gm = min(g.group, g.tiles_p - p0);
-  w.tile_q = r / gm;
-  w.tile_p = p0 + (r - w.tile_q * gm);
-  return w;
-}
 
 // P = operand with 128 rows per tile, Q = operand with BN rows per tile.
 // SWAP == false: P = A (tokens), Q = W;  D[i, j] -> C[tile_p*128 + i, tile_q*BN + j]
@@ -66,19 +36,11 @@ __device__ __forceinline__ WorkItem work_item(int item, const GemmGrid& g) {
 // ring keeps running across items (the producer is already fetching the next item's operands
 // while the last MMAs of the current one execute) and the accumulator is double-buffered in
 // TMEM, so the epilogue of item i overlaps the main loop of item i + 1.
-//
-// EPI (SWAP == false only) fuses the projection's epilogue into the store of the tile:
-//   EPI_SWIGLU  the Q tile is BN/2 up rows followed by the BN/2 matching gate rows of w1, so that a
-//               thread finds up_j and gate_j of its token in the same accumulator row; it stores
-//               silu(gate) * up to h [m, I] (lin.y, lin.n = I)
-//   EPI_GLU     as SWIGLU with the clamped unit, on fp32 accumulators (scaled per row for experts)
-//   EPI_F32     stores the fp32 accumulators
-//   EPI_QKV     a thread rotates the 16 adjacent pairs of each 32-column chunk of its token with the
-//               table row of the token's position and stores them to q_out / k-cache / v-cache
+// EPI (SWAP == false only) fuses the projection's epilogue into the store of the tile (store_row, gemm_tile.cuh).
 template <typename T, int BN, bool SWAP, int EPI>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constant__ CUtensorMap tmap_q,
-                    T* __restrict__ c, GemmShape shape, GemmGrid grid, int stages, const LinearParams lin) {
+                    T* __restrict__ c, GemmShape shape, GemmGrid grid, uint32_t stages, const LinearParams lin) {
   constexpr bool kGlu = EPI == EPI_SWIGLU || EPI == EPI_GLU;
   extern __shared__ uint8_t smem_raw[];
   constexpr uint32_t kTileP = kBM * kBK * 2;
@@ -92,7 +54,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_con
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // uniform for the compiler too
   const int lane = threadIdx.x & 31;
   const int num_kt = (shape.k + kBK - 1) / kBK;
 
@@ -103,7 +65,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_con
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
-    for (int s = 0; s < stages; ++s) {
+    for (uint32_t s = 0; s < stages; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
     }
@@ -123,7 +85,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_con
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = tmem_base_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
   // everything above overlaps the tail of the preceding kernel when launched as its programmatic dependent
   pdl_wait();
   pdl_launch_dependents();
@@ -133,19 +95,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_con
   }
   const int items = grid.tiles_p * grid.tiles_q;
 
+  // Fetching and issuing are serial work of one warp, and with it what a step costs unless it is short: the loops are
+  // warp-uniform (one elected lane issues), so that addresses and descriptors stay in uniform registers, and the place in the
+  // ring is counted, not divided out (see gemm_pair.cu).
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t g = 0;  // K tiles loaded so far, over all items: position in the ring
-      bool ok = true;
-      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-        const WorkItem w = work_item(item, grid);
-        const int row0 = grid.tiles ? grid.tiles[1 + w.tile_p] * grid.matrix_rows : 0;  // first weight row of the tile's matrix
-        for (int kt = 0; kt < num_kt; ++kt, ++g) {
-          const uint32_t s = g % static_cast<uint32_t>(stages);
-          const uint32_t round = g / static_cast<uint32_t>(stages);
-          // a fresh barrier passes a wait on parity 1, so the first round does not block
-          ok = mbar_wait(empty0 + 8 * s, (round & 1u) ^ 1u, &abort_flag, 1, &g_gemm_status);
-          if (!ok) break;
+    uint32_t s = 0, parity = 1;  // a fresh barrier passes a wait on parity 1, so the first round does not block
+    bool ok = true;
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+      const WorkItem w = work_item(item, grid);
+      const int row0 = grid.tiles ? grid.tiles[1 + w.tile_p] * grid.matrix_rows : 0;  // first weight row of the tile's matrix
+      for (int kt = 0; kt < num_kt; ++kt) {
+        ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, parity, &abort_flag, 1, &g_gemm_status));
+        if (!ok) break;
+        if (elect_one()) {
           mbar_expect_tx(full0 + 8 * s, kStageBytes);
           const uint32_t dst = base + s * kStageBytes;
           const int kx = kt * kBK;
@@ -157,43 +119,40 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_con
             tma_load_2d(dst + kTileP, &tmap_q, full0 + 8 * s, kx, row0 + w.tile_q * BN);
           }
         }
+        if (++s == stages) s = 0, parity ^= 1u;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // fp32 accumulate, A and B of type T, both K-major, N = BN, M = 128
-      constexpr uint32_t kFmt = sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-      constexpr uint32_t idesc = (1u << 4) | (kFmt << 7) | (kFmt << 10) | (static_cast<uint32_t>(BN >> 3) << 17) |
-                                 (static_cast<uint32_t>(kBM >> 4) << 24);
-      uint32_t g = 0;
-      bool ok = true;
-      int it = 0;
-      for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
-        const WorkItem w = work_item(item, grid);
-        const uint32_t a = it & 1;
-        const uint32_t use = static_cast<uint32_t>(it) >> 1;
-        // the epilogue must have drained this accumulator buffer (its first use does not block)
-        ok = mbar_wait(acc_empty0 + 8 * a, (use & 1u) ^ 1u, &abort_flag, 4, &g_gemm_status);
+    // fp32 accumulate, A and B of type T, both K-major, N = BN, M = 128
+    constexpr uint32_t idesc = umma_idesc<T>(BN);
+    uint32_t s = 0, parity = 0;
+    bool ok = true;
+    int it = 0;
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
+      const uint32_t a = it & 1;
+      const uint32_t use = static_cast<uint32_t>(it) >> 1;
+      // the epilogue must have drained this accumulator buffer (its first use does not block)
+      ok = __all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * a, (use & 1u) ^ 1u, &abort_flag, 4, &g_gemm_status));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t d_tmem = tmem_base + a * kAccCols;
+      for (int kt = 0; kt < num_kt; ++kt) {
+        ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, parity, &abort_flag, 2, &g_gemm_status));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d_tmem = tmem_base + a * kAccCols;
-        for (int kt = 0; kt < num_kt; ++kt, ++g) {
-          const uint32_t s = g % static_cast<uint32_t>(stages);
-          const uint32_t round = g / static_cast<uint32_t>(stages);
-          ok = mbar_wait(full0 + 8 * s, round & 1u, &abort_flag, 2, &g_gemm_status);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t pa = base + s * kStageBytes;
-          const uint64_t pdesc = smem_desc_sw128(pa);
-          const uint64_t qdesc = smem_desc_sw128(pa + kTileP);
+        if (elect_one()) {
+          const uint64_t pdesc = smem_desc_sw128(base + s * kStageBytes);
+          const uint64_t qdesc = smem_desc_sw128(base + s * kStageBytes + kTileP);
 #pragma unroll
           for (int kk = 0; kk < kBK / kUmmaK; ++kk) {
             // 16 K-elements = 32 bytes further along the swizzled row: +2 in 16-byte units
             umma_f16(d_tmem, pdesc + 2 * kk, qdesc + 2 * kk, idesc, (kt > 0 || kk > 0) ? 1u : 0u);
           }
           umma_commit(empty0 + 8 * s);  // the stage is free once these MMAs have read it
+          if (kt == num_kt - 1) umma_commit(acc_full0 + 8 * a);  // arrives when every MMA issued so far has completed
         }
-        if (ok) umma_commit(acc_full0 + 8 * a);  // arrives when every MMA issued so far has completed
+        __syncwarp();
+        if (++s == stages) s = 0, parity ^= 1u;
       }
     }
   } else {
@@ -209,136 +168,24 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_con
       if (!__all_sync(0xffffffffu, ready)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tacc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * kAccCols;
-      if (!SWAP && kGlu) {
-        const int64_t row = static_cast<int64_t>(w.tile_p) * kBM + i;
-        const float sc = EPI == EPI_GLU && lin.ex.row_scale && row < shape.m ? lin.ex.row_scale[row] : 1.f;
-#pragma unroll 1
-        for (int cc = 0; cc < BN / 2; cc += 32) {
-          uint32_t up[32], gate[32];
-          tmem_ld32(tacc + cc, up);
-          tmem_ld32(tacc + BN / 2 + cc, gate);
-          const int64_t j0 = static_cast<int64_t>(w.tile_q) * (BN / 2) + cc;
-          if (row >= shape.m || j0 >= lin.n) continue;
-          T* dst = static_cast<T*>(lin.y) + row * lin.n + j0;
-          __align__(16) T out[32];
-#pragma unroll
-          for (int e = 0; e < 32; ++e)
-            out[e] = EPI == EPI_GLU
-                         ? Num<T>::from_f(clamped_glu(sc * __uint_as_float(gate[e]), sc * __uint_as_float(up[e]), lin.ex.glu))
-                         : swiglu_rounded<T>(rnd<T>(__uint_as_float(up[e])), rnd<T>(__uint_as_float(gate[e])));
-          if (j0 + 32 <= lin.n && (lin.n & 7) == 0) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) reinterpret_cast<uint4*>(dst)[v] = reinterpret_cast<const uint4*>(out)[v];
-          } else {
-#pragma unroll
-            for (int e = 0; e < 32; ++e)
-              if (j0 + e < lin.n) dst[e] = out[e];
-          }
-        }
-      } else if (!SWAP && EPI == EPI_QKV) {
-        const int64_t row = static_cast<int64_t>(w.tile_p) * kBM + i;
-        const int hd = lin.head_dim;
-        const int64_t nq = static_cast<int64_t>(lin.n_head) * hd, nk = static_cast<int64_t>(lin.n_kv) * hd;
-        const int64_t b = row / lin.S, sq = row - b * lin.S;
-        int64_t pos = 0, trow = 0;
-        bool live = row < shape.m;
-        if (live) {
-          pos = load_pos(lin.input_pos, lin.pos_is_i64, sq);
-          trow = lin.table_gathered ? sq : pos;
-          live = pos >= 0 && pos < lin.smax && trow < lin.table_rows;
-        }
-#pragma unroll 1
-        for (int cc = 0; cc < BN; cc += 32) {
-          uint32_t r[32];
-          tmem_ld32(tacc + cc, r);
-          const int64_t n = static_cast<int64_t>(w.tile_q) * BN + cc;  // a 32-column chunk never straddles a head
-          if (!live || n >= shape.n) continue;
-          float f[32];
-#pragma unroll
-          for (int e = 0; e < 32; ++e) f[e] = rnd<T>(__uint_as_float(r[e]));
-          T* dst;
-          if (n < nq + nk) {
-            const int64_t nn = n < nq ? n : n - nq;
-            const int e0 = static_cast<int>(nn % hd);
-            const uint4* cs = reinterpret_cast<const uint4*>(static_cast<const T*>(lin.rope_table) +
-                                                             (trow * (hd >> 1) + (e0 >> 1)) * 2);
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              float t[8];
-              unpack8<T>(cs[v], t);  // (cos, sin) of 4 pairs
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                float o0, o1;
-                rope_pair(f[v * 8 + 2 * q], f[v * 8 + 2 * q + 1], t[2 * q], t[2 * q + 1], o0, o1);
-                f[v * 8 + 2 * q] = o0;
-                f[v * 8 + 2 * q + 1] = o1;
-              }
-            }
-            dst = n < nq ? static_cast<T*>(lin.q_out) + row * nq + n
-                         : static_cast<T*>(lin.k_cache) + ((b * lin.n_kv + nn / hd) * lin.smax + pos) * hd + e0;
-          } else {
-            const int64_t nn = n - nq - nk;
-            dst = static_cast<T*>(lin.v_cache) + ((b * lin.n_kv + nn / hd) * lin.smax + pos) * hd + nn % hd;
-          }
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            float g8[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) g8[e] = f[v * 8 + e];
-            reinterpret_cast<uint4*>(dst)[v] = pack8<T>(g8);
-          }
-        }
+      if (!SWAP) {
+        store_row<T, EPI>(lin, c, shape, static_cast<int64_t>(w.tile_p) * kBM + i, w.tile_q, BN, tacc);
       } else
 #pragma unroll 1
       for (int cc = 0; cc < BN; cc += 32) {
         uint32_t r[32];
-        const uint32_t taddr = tacc + cc;
-        tmem_ld32(taddr, r);  // BN == 16: only the first 16 columns are valid (32 are allocated)
+        tmem_ld32(tacc + cc, r);  // BN == 16: only the first 16 columns are valid (32 are allocated)
         constexpr int kValid = BN < 32 ? BN : 32;
-        if (!SWAP) {
-          const int64_t row = static_cast<int64_t>(w.tile_p) * kBM + i;
-          const int64_t col0 = static_cast<int64_t>(w.tile_q) * BN + cc;
-          if (EPI == EPI_F32) {
-            float* dst = static_cast<float*>(lin.y) + row * shape.n + col0;
-            if (row < shape.m) {
-              if (col0 + kValid <= shape.n) {
+        const int64_t n = static_cast<int64_t>(w.tile_p) * kBM + i;
+        const int64_t tok0 = static_cast<int64_t>(w.tile_q) * BN + cc;
+        if (n < shape.n) {
 #pragma unroll
-                for (int v = 0; v < kValid / 4; ++v)
-                  reinterpret_cast<uint4*>(dst)[v] = make_uint4(r[v * 4], r[v * 4 + 1], r[v * 4 + 2], r[v * 4 + 3]);
-              } else {
-#pragma unroll
-                for (int e = 0; e < kValid; ++e)
-                  if (col0 + e < shape.n) dst[e] = __uint_as_float(r[e]);
-              }
-            }
-          } else if (row < shape.m) {
-            T* dst = c + row * shape.n + col0;
-            if (col0 + kValid <= shape.n) {
-#pragma unroll
-              for (int v = 0; v < kValid / 8; ++v) {
-                float f[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[v * 8 + e]);
-                reinterpret_cast<uint4*>(dst)[v] = pack8<T>(f);
-              }
-            } else {
-#pragma unroll
-              for (int e = 0; e < kValid; ++e)
-                if (col0 + e < shape.n) dst[e] = Num<T>::from_f(__uint_as_float(r[e]));
-            }
-          }
-        } else {
-          const int64_t n = static_cast<int64_t>(w.tile_p) * kBM + i;
-          const int64_t tok0 = static_cast<int64_t>(w.tile_q) * BN + cc;
-          if (n < shape.n) {
-#pragma unroll
-            for (int e = 0; e < kValid; ++e) {
-              if (tok0 + e >= shape.m) continue;
-              if (EPI == EPI_F32)
-                static_cast<float*>(lin.y)[(tok0 + e) * shape.n + n] = __uint_as_float(r[e]);
-              else
-                c[(tok0 + e) * shape.n + n] = Num<T>::from_f(__uint_as_float(r[e]));
-            }
+          for (int e = 0; e < kValid; ++e) {
+            if (tok0 + e >= shape.m) continue;
+            if (EPI == EPI_F32)
+              static_cast<float*>(lin.y)[(tok0 + e) * shape.n + n] = __uint_as_float(r[e]);
+            else
+              c[(tok0 + e) * shape.n + n] = Num<T>::from_f(__uint_as_float(r[e]));
           }
         }
       }
@@ -469,7 +316,7 @@ int launch_tile(int dtype, const void* a, const void* w, void* c, int64_t m, int
   usable = usable < 1 ? 1 : usable;
   const int ctas = static_cast<int>(items < usable ? items : usable);
   LRI_CUDA(launch_pdl(kern, dim3(static_cast<unsigned>(ctas)), dim3(kGemmThreads), static_cast<size_t>(smem), st, tp, tq,
-                      static_cast<T*>(c), shape, grid, stages, lin ? *lin : LinearParams{}));
+                      static_cast<T*>(c), shape, grid, static_cast<uint32_t>(stages), lin ? *lin : LinearParams{}));
   LRI_LAUNCH_CHECK("gemm_tcgen05_kernel");
   return LRI_OK;
 }
@@ -479,6 +326,11 @@ int launch_typed(int dtype, const void* a, const void* w, void* c, int64_t m, in
   if (m <= 16) return launch_tile<T, 16, true>(dtype, a, w, c, m, n, k, st);
   if (m <= 32) return launch_tile<T, 32, true>(dtype, a, w, c, m, n, k, st);
   if (m <= 64) return launch_tile<T, 64, true>(dtype, a, w, c, m, n, k, st);
+  if (const int bn = gemm_pair_bn(m, n)) {
+    LinearParams p{};
+    p.x = a, p.w = w, p.y = c, p.n = n, p.k = k;
+    return gemm_pair_launch(dtype, EPI_PLAIN, p, m, n, bn, st);
+  }
   // prefill: pick the N tile that leaves fewer idle SMs in the last wave
   const int sms = sm_count();
   const int64_t mt = (m + kBM - 1) / kBM;
@@ -496,6 +348,10 @@ int launch_f32(int dtype, const void* a, const void* w, float* c, int64_t m, int
   if (m <= 16) return launch_tile<T, 16, true, EPI_F32>(dtype, a, w, nullptr, m, n, k, st, &p);
   if (m <= 32) return launch_tile<T, 32, true, EPI_F32>(dtype, a, w, nullptr, m, n, k, st, &p);
   if (m <= 64) return launch_tile<T, 64, true, EPI_F32>(dtype, a, w, nullptr, m, n, k, st, &p);
+  if (const int bn = gemm_pair_bn(m, n)) {
+    p.x = a, p.w = w, p.n = n, p.k = k;
+    return gemm_pair_launch(dtype, EPI_F32, p, m, n, bn, st);
+  }
   const int sms = sm_count();
   const int64_t mt = (m + kBM - 1) / kBM;
   const int64_t t256 = mt * ((n + 255) / 256), t128 = mt * ((n + 127) / 128);
@@ -522,6 +378,7 @@ template <typename T, int EPI>
 int launch_fused(int dtype, const LinearParams& p, int64_t m, cudaStream_t st) {
   constexpr bool kGlu = EPI == EPI_SWIGLU || EPI == EPI_GLU;
   const int n_rows = kGlu ? 2 * p.n : p.n;       // rows of the weight
+  if (const int bn = gemm_pair_bn(m, n_rows)) return gemm_pair_launch(dtype, EPI, p, m, n_rows, bn, st);
   const int64_t mt = (m + kBM - 1) / kBM;
   const int w256 = kGlu ? 128 : 256, w128 = kGlu ? 64 : 128;  // outputs per Q tile
   const int64_t t256 = mt * ((p.n + w256 - 1) / w256), t128 = mt * ((p.n + w128 - 1) / w128);

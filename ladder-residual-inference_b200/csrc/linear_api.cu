@@ -15,6 +15,7 @@ namespace lri {
 bool gemm_tcgen05_supports(int64_t m, int n, int k);
 int gemm_tcgen05_launch(int dtype, const void* a, const void* w, void* c, int64_t m, int n, int k, cudaStream_t st);
 int gemm_tcgen05_status_read_and_clear(int* status_out);
+int gemm_pair_status_read_and_clear(int* status_out);
 int attn_prefill_tc_status_read_and_clear(int* status_out);
 int window_attention_tc_status_read_and_clear(int* status_out);
 int state_scan_status_read_and_clear(int* status_out);
@@ -46,6 +47,7 @@ const OptionSpec kOptionSpecs[OPT_COUNT] = {
     {"decode_splits", "LRI_DECODE_SPLITS", 0, 0, 64},
     {"attn_prefill_tc", "LRI_ATTN_PREFILL_TC", 1, 0, 1},
     {"gemm_reserve_sms", "LRI_GEMM_RESERVE_SMS", 0, 0, 64},
+    {"gemm_pair", "LRI_GEMM_PAIR", 1, 0, 256},
     {"attn_head_tile", "LRI_ATTN_HEAD_TILE", 0, 0, 4},
     {"moe_stream_pairs", "LRI_MOE_STREAM_PAIRS", 10, 0, 65535},
     {"window_tc", "LRI_WINDOW_TC", 1, 0, 1},
@@ -62,6 +64,7 @@ bool option_value_ok(int which, int v) {
   if (which == OPT_GEMV_U) return v == 0 || v == 2;
   if (which == OPT_GEMV_MT) return v == 0 || v == 1 || v == 2 || v == 4;
   if (which == OPT_ATTN_HEAD_TILE || which == OPT_SCAN_COLUMNS || which == OPT_SCAN_WARPS) return v == 0 || v == 1 || v == 2 || v == 4;
+  if (which == OPT_GEMM_PAIR) return v <= 1 || (v >= 64 && v % 32 == 0);
   if (which == OPT_SCAN_LANES) return v == 0 || v == 8 || v == 16;
   return true;
 }
@@ -336,6 +339,10 @@ extern "C" int lri_gemm_status(void) {
   if (rc != LRI_OK) return rc;
   rc = gemm_streamk_status_read_and_clear(&v2);
   if (rc != LRI_OK) return rc;
+  int v5 = 0;
+  rc = gemm_pair_status_read_and_clear(&v5);
+  if (rc != LRI_OK) return rc;
+  v = v != 0 ? v : v5;
   rc = attn_prefill_tc_status_read_and_clear(&v3);
   if (rc != LRI_OK) return rc;
   if (v != 0 || v2 != 0)
