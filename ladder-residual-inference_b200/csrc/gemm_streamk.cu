@@ -79,9 +79,9 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // uniform for the compiler too
   const int lane = threadIdx.x & 31;
-  const int stages = p.stages;
+  const uint32_t stages = static_cast<uint32_t>(p.stages);
   const int64_t units = static_cast<int64_t>(p.tiles) * p.total_kt;
   const int u_begin = unit_start(blockIdx.x, units, p.ctas);
   const int u_end = unit_start(blockIdx.x + 1, units, p.ctas);
@@ -93,7 +93,7 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
-    for (int s = 0; s < stages; ++s) {
+    for (uint32_t s = 0; s < stages; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
     }
@@ -113,50 +113,65 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = tmem_base_slot;
-  pdl_wait();
-  pdl_launch_dependents();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
 
+  // warp-uniform loops, one elected lane issues (see gemm_pair.cu)
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t g = 0;
-      bool ok = true;
-      for (int u = u_begin; u < u_end && ok; ++u, ++g) {
-        const int tile = u / p.total_kt;
-        const int kt = u - tile * p.total_kt;
-        const uint32_t s = g % static_cast<uint32_t>(stages);
-        const uint32_t round = g / static_cast<uint32_t>(stages);
-        ok = mbar_wait(empty0 + 8 * s, (round & 1u) ^ 1u, &abort_flag, 11, &g_streamk_status);
-        if (!ok) break;
-        mbar_expect_tx(full0 + 8 * s, kStageBytes);
-        const uint32_t dst = base + s * kStageBytes;
-        tma_load_2d(dst, &tmap_w, full0 + 8 * s, kt * kBK, tile * kBM);
-        if (kAcc == 2) tma_load_2d(dst + kTileW, &tmap_w, full0 + 8 * s, kt * kBK, p.lin.n + tile * kBM);  // gate rows
-        tma_load_2d(dst + kAcc * kTileW, &tmap_x, full0 + 8 * s, kt * kBK, 0);
+    uint32_t s = 0, parity = 0;
+    const int tile0 = u_begin / p.total_kt, kt0 = u_begin - tile0 * p.total_kt;
+    int tile = tile0, kt = kt0;
+    auto fetch_weights = [&]() {
+      mbar_expect_tx(full0 + 8 * s, kStageBytes);
+      const uint32_t dst = base + s * kStageBytes;
+      tma_load_2d(dst, &tmap_w, full0 + 8 * s, kt * kBK, tile * kBM);
+      if (kAcc == 2) tma_load_2d(dst + kTileW, &tmap_w, full0 + 8 * s, kt * kBK, p.lin.n + tile * kBM);  // gate rows
+    };
+    // The weights do not depend on the preceding kernel: fill the ring with them while it still runs (147 KB per SM, 3.3 us of HBM
+    // time), the token rows follow once it is complete.
+    const int ahead = min(static_cast<int>(stages), u_end - u_begin);
+    for (int u = 0; u < ahead; ++u, ++s) {
+      if (elect_one()) fetch_weights();
+      if (++kt == p.total_kt) kt = 0, ++tile;
+    }
+    __syncwarp();
+    pdl_wait();
+    pdl_launch_dependents();
+    for (int u = 0; u < ahead; ++u)
+      if (elect_one()) tma_load_2d(base + u * kStageBytes + kAcc * kTileW, &tmap_x, full0 + 8 * u, (kt0 + u) % p.total_kt * kBK, 0);
+    __syncwarp();
+    if (s == stages) s = 0;
+    for (int u = u_begin + ahead; u < u_end; ++u) {
+      if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, parity, &abort_flag, 11, &g_streamk_status))) break;
+      if (elect_one()) {
+        fetch_weights();
+        tma_load_2d(base + s * kStageBytes + kAcc * kTileW, &tmap_x, full0 + 8 * s, kt * kBK, 0);
       }
+      __syncwarp();
+      if (++s == stages) s = 0, parity ^= 1u;
+      if (++kt == p.total_kt) kt = 0, ++tile;
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc<T>(BN);
-      uint32_t g = 0;
-      bool ok = true;
-      int seg = 0;
-      for (int u = u_begin; u < u_end && ok; ++seg) {
-        const int tile = u / p.total_kt;
-        const int kt0 = u - tile * p.total_kt;
-        const int nk = min(p.total_kt - kt0, u_end - u);
-        const uint32_t a = seg & 1;
-        const uint32_t use = static_cast<uint32_t>(seg) >> 1;
-        ok = mbar_wait(acc_empty0 + 8 * a, (use & 1u) ^ 1u, &abort_flag, 14, &g_streamk_status);
+    pdl_wait();
+    pdl_launch_dependents();
+    constexpr uint32_t idesc = umma_idesc<T>(BN);
+    uint32_t s = 0, parity = 0;
+    bool ok = true;
+    int seg = 0;
+    for (int u = u_begin; u < u_end && ok; ++seg) {
+      const int tile = u / p.total_kt;
+      const int kt0 = u - tile * p.total_kt;
+      const int nk = min(p.total_kt - kt0, u_end - u);
+      const uint32_t a = seg & 1;
+      const uint32_t use = static_cast<uint32_t>(seg) >> 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * a, (use & 1u) ^ 1u, &abort_flag, 14, &g_streamk_status));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t d_tmem = tmem_base + a * kBufCols;
+      for (int kt = 0; kt < nk; ++kt) {
+        ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, parity, &abort_flag, 12, &g_streamk_status));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d_tmem = tmem_base + a * kBufCols;
-        for (int kt = 0; kt < nk; ++kt, ++g) {
-          const uint32_t s = g % static_cast<uint32_t>(stages);
-          const uint32_t round = g / static_cast<uint32_t>(stages);
-          ok = mbar_wait(full0 + 8 * s, round & 1u, &abort_flag, 12, &g_streamk_status);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (elect_one()) {
           const uint32_t pa = base + s * kStageBytes;
           const uint64_t xdesc = smem_desc_sw128(pa + kAcc * kTileW);
 #pragma unroll
@@ -167,12 +182,16 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
               umma_f16(d_tmem + h * kAccCols, wdesc + 2 * kk, xdesc + 2 * kk, idesc, (kt > 0 || kk > 0) ? 1u : 0u);
           }
           umma_commit(empty0 + 8 * s);
+          if (kt == nk - 1) umma_commit(acc_full0 + 8 * a);
         }
-        if (ok) umma_commit(acc_full0 + 8 * a);
-        u += nk;
+        __syncwarp();
+        if (++s == stages) s = 0, parity ^= 1u;
       }
+      u += nk;
     }
   } else {
+    pdl_wait();  // a preceding kernel may still read what the stores below overwrite
+    pdl_launch_dependents();
     const int quarter = warp & 3;
     const int i = quarter * 32 + lane;  // row of the accumulator = output within the tile
     const int m = p.lin.m;
