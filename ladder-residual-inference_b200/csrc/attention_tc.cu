@@ -69,7 +69,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // uniform for the compiler too
+  const int lane = threadIdx.x & 31;
   const int q_tile = gridDim.x - 1 - blockIdx.x;  // long (late) tiles first
   const int q0 = q_tile * kFaM;
   const int head = blockIdx.y, b = blockIdx.z;
@@ -106,7 +107,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = tmem_base_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
 
   int64_t pos0 = load_pos(p.input_pos, p.pos_is_i64, 0);
   pos0 = pos0 < 0 ? 0 : pos0;
@@ -116,15 +117,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   const int n_tiles = static_cast<int>((kv_end + kFaN - 1) / kFaN);  // >= 1
   const int kv_row0_hi = static_cast<int>((static_cast<int64_t>(b) * p.n_kv + kvh) * p.smax);  // row of key 0 in the [rows, HD] view
 
+  // warp-uniform loops, one elected lane issues: a loop run by one lane takes 74 cycles a product (see gemm_pair.cu), and a tile
+  // has HD / 16 + 4 of them
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, kQBytes);
 #pragma unroll
       for (int c = 0; c < kChunks; ++c)
         tma_load_2d(q_smem + c * kQChunkBytes, &tmap_q, q_full, head * HD + c * 64, b * p.S + q0);
-      for (int j = 0; j < n_tiles; ++j) {
-        const uint32_t s = j % kFaStages, round = j / kFaStages;
-        if (!mbar_wait(kv_empty0 + 8 * s, (round & 1u) ^ 1u, &abort_flag, 1, &g_attn_tc_status)) break;
+    }
+    __syncwarp();
+    for (int j = 0; j < n_tiles; ++j) {
+      const uint32_t s = j % kFaStages, round = j / kFaStages;
+      if (!__all_sync(0xffffffffu, mbar_wait(kv_empty0 + 8 * s, (round & 1u) ^ 1u, &abort_flag, 1, &g_attn_tc_status))) break;
+      if (elect_one()) {
         mbar_expect_tx(kv_full0 + 8 * s, kStageBytes);
         const uint32_t dst = kv_smem + s * kStageBytes;
         const int row = kv_row0_hi + j * kFaN;
@@ -134,24 +140,24 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
           tma_load_2d(dst + kTileBytes + c * kKvChunkBytes, &tmap_v, kv_full0 + 8 * s, c * 64, row);
         }
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-      // S = Q K^T: both operands K-major, N = 64
-      constexpr uint32_t idesc_qk = (1u << 4) | (kFmt << 7) | (kFmt << 10) | (static_cast<uint32_t>(kFaN >> 3) << 17) |
-                                    (static_cast<uint32_t>(kFaM >> 4) << 24);
-      // O += P V: A from TMEM (K-major), B MN-major (bit 16), N = HD
-      constexpr uint32_t idesc_pv = (1u << 4) | (kFmt << 7) | (kFmt << 10) | (1u << 16) |
-                                    (static_cast<uint32_t>(HD >> 3) << 17) | (static_cast<uint32_t>(kFaM >> 4) << 24);
-      constexpr uint32_t v_lbo = kKvChunkBytes;  // between the 64-column chunks of head_dim
-      constexpr uint32_t v_sbo = 1024u;           // between groups of 8 keys
-      bool ok = mbar_wait(q_full, 0, &abort_flag, 2, &g_attn_tc_status);
+    constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+    // S = Q K^T: both operands K-major, N = 64
+    constexpr uint32_t idesc_qk = umma_idesc<T>(kFaN);
+    // O += P V: A from TMEM (K-major), B MN-major (bit 16), N = HD
+    constexpr uint32_t idesc_pv = (1u << 4) | (kFmt << 7) | (kFmt << 10) | (1u << 16) |
+                                  (static_cast<uint32_t>(HD >> 3) << 17) | (static_cast<uint32_t>(kFaM >> 4) << 24);
+    constexpr uint32_t v_lbo = kKvChunkBytes;  // between the 64-column chunks of head_dim
+    constexpr uint32_t v_sbo = 1024u;           // between groups of 8 keys
+    bool ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0, &abort_flag, 2, &g_attn_tc_status));
 
-      auto issue_qk = [&](int j) {
-        const uint32_t s = j % kFaStages, round = j / kFaStages;
-        if (!mbar_wait(kv_full0 + 8 * s, round & 1u, &abort_flag, 3, &g_attn_tc_status)) return false;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    auto issue_qk = [&](int j) {
+      const uint32_t s = j % kFaStages, round = j / kFaStages;
+      if (!__all_sync(0xffffffffu, mbar_wait(kv_full0 + 8 * s, round & 1u, &abort_flag, 3, &g_attn_tc_status))) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (elect_one()) {
         const uint32_t k_smem = kv_smem + s * kStageBytes;
         const uint32_t d = tmem_base + static_cast<uint32_t>(j & 1) * kSCols;
 #pragma unroll
@@ -161,13 +167,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
           umma_f16(d, qd, kd, idesc_qk, kk > 0 ? 1u : 0u);
         }
         umma_commit(s_full0 + 8 * (j & 1));
-        return true;
-      };
-      auto issue_pv = [&](int j) {
-        const uint32_t s = j % kFaStages;
-        if (!mbar_wait(p_full0 + 8 * (j & 1), (static_cast<uint32_t>(j) >> 1) & 1u, &abort_flag, 4, &g_attn_tc_status))
-          return false;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      __syncwarp();
+      return true;
+    };
+    auto issue_pv = [&](int j) {
+      const uint32_t s = j % kFaStages;
+      if (!__all_sync(0xffffffffu, mbar_wait(p_full0 + 8 * (j & 1), (static_cast<uint32_t>(j) >> 1) & 1u, &abort_flag, 4, &g_attn_tc_status)))
+        return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (elect_one()) {
         const uint32_t v_smem = kv_smem + s * kStageBytes + kTileBytes;
         const uint32_t pa = tmem_base + static_cast<uint32_t>(j & 1) * kSCols;  // P over the first 32 columns of S
 #pragma unroll
@@ -178,13 +187,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         }
         umma_commit(kv_empty0 + 8 * s);      // K and V of this stage have been read
         umma_commit(o_done0 + 8 * (j & 1));  // O holds tiles 0..j
-        return true;
-      };
-      if (ok) ok = issue_qk(0);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        if (j + 1 < n_tiles) ok = issue_qk(j + 1);
-        if (ok) ok = issue_pv(j);
       }
+      __syncwarp();
+      return true;
+    };
+    if (ok) ok = issue_qk(0);
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      if (j + 1 < n_tiles) ok = issue_qk(j + 1);
+      if (ok) ok = issue_pv(j);
     }
   } else {
     const int quarter = warp & 3;       // TMEM lanes a warp may touch: 32 * (warp id mod 4)

@@ -94,7 +94,8 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap tq1, const __grid
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // uniform for the compiler too
+  const int lane = threadIdx.x & 31;
   const int q_tile = gridDim.x - 1 - blockIdx.x;  // long (late) tiles first
   const int q0 = q_tile * kRows * kGroups;
   const int head = blockIdx.y, b = blockIdx.z;
@@ -131,7 +132,7 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap tq1, const __grid
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = tmem_base_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
   pdl_wait();
   pdl_launch_dependents();
 
@@ -155,8 +156,9 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap tq1, const __grid
   all.n = gt[groups - 1].lo + gt[groups - 1].n - all.lo;  // the groups' ranges overlap or follow one another
   auto active = [&](int g, int t) { return t >= gt[g].lo && t < gt[g].lo + gt[g].n; };
 
+  // warp-uniform loops, one elected lane issues: a loop run by one lane takes 74 cycles a product (see gemm_pair.cu)
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, kGroups * Z::kQBytes);
 #pragma unroll
       for (int g = 0; g < kGroups; ++g) {
@@ -168,13 +170,16 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap tq1, const __grid
         for (int c = 0; c < C2; ++c)
           tma_load_3d(base + g * Z::kQBytes + (C1 + c) * kQChunk, &tq2, q_full, c * 64, head, row);
       }
-      for (int j = 0; j < all.n; ++j) {
-        const uint32_t s = j % kStages, round = j / kStages;
-        if (!mbar_wait(kv_empty0 + 8 * s, (round & 1u) ^ 1u, &abort_flag, 1, &g_window_tc_status)) break;
+    }
+    __syncwarp();
+    const int kv_head = static_cast<int>(b * p.batch_heads) + head / p.group;
+    for (int j = 0; j < all.n; ++j) {
+      const uint32_t s = j % kStages, round = j / kStages;
+      if (!__all_sync(0xffffffffu, mbar_wait(kv_empty0 + 8 * s, (round & 1u) ^ 1u, &abort_flag, 1, &g_window_tc_status))) break;
+      if (elect_one()) {
         mbar_expect_tx(kv_full0 + 8 * s, Z::kStage);
         const uint32_t dst = kv_smem + s * Z::kStage;
         const int row = static_cast<int>(b * p.batch_rows) + (all.lo + j) * kKeys;
-        const int kv_head = static_cast<int>(b * p.batch_heads) + head / p.group;
 #pragma unroll
         for (int c = 0; c < C1; ++c) tma_load_3d(dst + c * kKvChunk, &tk1, kv_full0 + 8 * s, c * 64, kv_head, row);
 #pragma unroll
@@ -182,16 +187,17 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap tq1, const __grid
 #pragma unroll
         for (int c = 0; c < CV; ++c) tma_load_3d(dst + (kQk + c) * kKvChunk, &tv, kv_full0 + 8 * s, c * 64, kv_head, row);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-      constexpr uint32_t idesc_qk = umma_idesc<T>(kKeys);
-      // A from TMEM (K-major), B MN-major (bit 16), N = value columns
-      constexpr uint32_t idesc_pv = (1u << 4) | (kFmt << 7) | (kFmt << 10) | (1u << 16) |
-                                    (static_cast<uint32_t>(CV * 64 >> 3) << 17) | (static_cast<uint32_t>(kRows >> 4) << 24);
-      bool ok = mbar_wait(q_full, 0, &abort_flag, 2, &g_window_tc_status);
-      auto issue_qk = [&](int g, int t) {
+    constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+    constexpr uint32_t idesc_qk = umma_idesc<T>(kKeys);
+    // A from TMEM (K-major), B MN-major (bit 16), N = value columns
+    constexpr uint32_t idesc_pv = (1u << 4) | (kFmt << 7) | (kFmt << 10) | (1u << 16) |
+                                  (static_cast<uint32_t>(CV * 64 >> 3) << 17) | (static_cast<uint32_t>(kRows >> 4) << 24);
+    bool ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0, &abort_flag, 2, &g_window_tc_status));
+    auto issue_qk = [&](int g, int t) {
+      if (elect_one()) {
         const uint32_t k_smem = kv_smem + ((t - all.lo) % kStages) * Z::kStage;
         const uint32_t d = tmem_base + g * kGroupCols + ((t - gt[g].lo) & 1) * kKeys;
 #pragma unroll
@@ -201,11 +207,15 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap tq1, const __grid
           umma_f16(d, qd, kd, idesc_qk, kk > 0 ? 1u : 0u);
         }
         umma_commit(s_full(g, (t - gt[g].lo) & 1));
-      };
-      auto issue_pv = [&](int g, int t) {
-        const int jg = t - gt[g].lo;
-        if (!mbar_wait(p_full(g, jg & 1), (static_cast<uint32_t>(jg) >> 1) & 1u, &abort_flag, 4, &g_window_tc_status)) return false;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      __syncwarp();
+    };
+    auto issue_pv = [&](int g, int t) {
+      const int jg = t - gt[g].lo;
+      if (!__all_sync(0xffffffffu, mbar_wait(p_full(g, jg & 1), (static_cast<uint32_t>(jg) >> 1) & 1u, &abort_flag, 4, &g_window_tc_status)))
+        return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (elect_one()) {
         const uint32_t v_smem = kv_smem + ((t - all.lo) % kStages) * Z::kStage + kQk * kKvChunk;
         const uint32_t pa = tmem_base + g * kGroupCols + (jg & 1) * kKeys;
 #pragma unroll
@@ -213,25 +223,27 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap tq1, const __grid
           umma_ts_f16(tmem_base + g * kGroupCols + 2 * kKeys, pa + kk * 8,
                       smem_desc_mn_sw128(v_smem + kk * 2048u, kKvChunk, 1024u), idesc_pv, (jg > 0 || kk > 0) ? 1u : 0u);
         umma_commit(o_done(g, jg & 1));
-        return true;
-      };
-      // S of tile t is issued before P of tile t - 1 is awaited, so the tensor pipe works while the softmax warps do
-      for (int j = 0; j <= all.n && ok; ++j) {
-        const int t = all.lo + j;
-        if (j < all.n) {
-          ok = mbar_wait(kv_full0 + 8 * (j % kStages), (j / kStages) & 1u, &abort_flag, 3, &g_window_tc_status);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      __syncwarp();
+      return true;
+    };
+    // S of tile t is issued before P of tile t - 1 is awaited, so the tensor pipe works while the softmax warps do
+    for (int j = 0; j <= all.n && ok; ++j) {
+      const int t = all.lo + j;
+      if (j < all.n) {
+        ok = __all_sync(0xffffffffu, mbar_wait(kv_full0 + 8 * (j % kStages), (j / kStages) & 1u, &abort_flag, 3, &g_window_tc_status));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-          for (int g = 0; g < kGroups; ++g)
-            if (active(g, t)) issue_qk(g, t);
-        }
-        if (j > 0) {
+        for (int g = 0; g < kGroups; ++g)
+          if (active(g, t)) issue_qk(g, t);
+      }
+      if (j > 0) {
 #pragma unroll
-          for (int g = 0; g < kGroups; ++g)
-            if (ok && active(g, t - 1)) ok = issue_pv(g, t - 1);
-          if (ok) umma_commit(kv_empty0 + 8 * ((j - 1) % kStages));
-        }
+        for (int g = 0; g < kGroups; ++g)
+          if (ok && active(g, t - 1)) ok = issue_pv(g, t - 1);
+        if (ok && elect_one()) umma_commit(kv_empty0 + 8 * ((j - 1) % kStages));
+        __syncwarp();
       }
     }
   } else {
