@@ -14,6 +14,11 @@ int attn_decode_cluster_head_tile(int B, int n_kv, int g);
 int attn_decode_cluster_launch(int dtype, const void* q, const void* k_cache, const void* v_cache,
                                const void* input_pos, int pos_is_i64, void* out, int B, int n_head, int n_kv,
                                int head_dim, int64_t smax, int num_splits, float scale_log2, cudaStream_t st);
+// form for many sequences (attention_stream.cu)
+bool attn_decode_stream_supports(int64_t pairs, int group, int64_t smax);
+int attn_decode_stream_launch(int dtype, const void* q, const void* k_cache, const void* v_cache, const void* input_pos, int pos_is_i64,
+                              void* out, int B, int n_head, int n_kv, int head_dim, int64_t smax, float scale_log2, unsigned int* counters,
+                              float* parts, int64_t part_slots, cudaStream_t st);
 // tcgen05 / TMEM form of the prefill kernel (attention_tc.cu)
 bool attn_prefill_tc_supports(int B, int S, int n_head, int n_kv, int head_dim, int64_t smax);
 int attn_prefill_tc_launch(int dtype, const void* q, const void* k_cache, const void* v_cache, const void* input_pos,
@@ -485,318 +490,6 @@ __global__ void __launch_bounds__(kPfThreads) attn_prefill_kernel(const PrefillP
   }
 }
 
-// =====================================================================================================
-// F3, large batches: the query heads of one KV head as the rows of tensor-core tiles
-// =====================================================================================================
-// With 16 or more sequences the K/V bytes of a layer are tens to hundreds of MB and the kernel
-// above, built for the latency of a single sequence (every K row costs shuffle-reduced dot
-// products for each query head), cannot issue fast enough to stream them.  Here a CTA takes one
-// (sequence, KV head, range of positions) and treats the g <= 16 query heads that share the KV head
-// as the 16 rows of mma.sync tiles: S = Q K^T and O += P V run on the tensor cores exactly as in
-// the prefill kernel, with a "query tile" that is the head group instead of 16 positions.  Each of
-// the 4 warps walks its own tiles of 16 positions (tile w, w + 4, ...) through a private 3-stage
-// cp.async ring (8.5 KB per stage: about 100 KB in flight per CTA, two CTAs per SM), keeps its
-// own online-softmax state, and the warps, then the ranges, are merged as in the kernel above.
-constexpr int kMmaDecWarps = 4;
-constexpr int kMmaDecThreads = kMmaDecWarps * 32;
-constexpr int kMmaDecStages = 3;
-constexpr int kMmaDecTile = 16;   // positions per warp tile
-constexpr int kMmaDecMaxGroup = 16;
-
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-template <typename T, int HD>
-__global__ void __launch_bounds__(kMmaDecThreads, 2) attn_decode_mma_kernel(const DecodeParams p) {
-  constexpr int LDS = HD + 8;  // padded row length in elements (bank-conflict-free ldmatrix)
-  constexpr int KB = HD / 16;  // k blocks of Q K^T
-  constexpr int OB = HD / 8;   // 8-column blocks of the output
-  constexpr int CPR = HD / 8;  // 16-byte chunks per row
-  constexpr int kTileElems = kMmaDecTile * LDS;
-  constexpr int kStageElems = 2 * kTileElems;  // K tile, V tile
-  extern __shared__ __align__(16) uint8_t dm_smem[];
-  T* sq = reinterpret_cast<T*>(dm_smem);                      // [16][LDS]
-  T* ring = sq + kMmaDecTile * LDS;                            // [warps][stages][K | V]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
-  const int g = p.n_head / p.n_kv;
-  const int head0 = kvh * g;
-
-  pdl_launch_dependents();
-  pdl_wait();  // q and the newest cache row were written by the preceding kernel
-  int64_t ctx = load_pos(p.input_pos, p.pos_is_i64, 0) + 1;
-  ctx = ctx < 0 ? 0 : (ctx > p.smax ? p.smax : ctx);
-  const int64_t chunk = (ctx + p.num_splits - 1) / p.num_splits;
-  const int64_t p0 = split * chunk;
-  const int64_t p1 = (p0 + chunk < ctx) ? p0 + chunk : ctx;
-  const int n_tiles = p1 > p0 ? static_cast<int>((p1 - p0 + kMmaDecTile - 1) / kMmaDecTile) : 0;
-
-  const T* kg = static_cast<const T*>(p.k_cache) + (static_cast<int64_t>(b) * p.n_kv + kvh) * p.smax * HD;
-  const T* vg = static_cast<const T*>(p.v_cache) + (static_cast<int64_t>(b) * p.n_kv + kvh) * p.smax * HD;
-  T* my_ring = ring + warp * (kMmaDecStages * kStageElems);
-
-  // tile `t` (positions p0 + 16 t ...) of this range into stage `st` of the warp's ring
-  auto issue = [&](int t, int st) {
-    if (t < n_tiles) {
-      T* dk = my_ring + st * kStageElems;
-      T* dv = dk + kTileElems;
-      const int64_t j0 = p0 + static_cast<int64_t>(t) * kMmaDecTile;
-#pragma unroll
-      for (int c = lane; c < kMmaDecTile * CPR; c += 32) {
-        const int r = c / CPR, cc = c % CPR;
-        const int64_t j = j0 + r;
-        const bool ok = j < p1;
-        const int64_t jc = ok ? j : 0;
-        cp_async16(static_cast<uint32_t>(__cvta_generic_to_shared(dk + r * LDS + cc * 8)), kg + jc * HD + cc * 8, ok);
-        cp_async16(static_cast<uint32_t>(__cvta_generic_to_shared(dv + r * LDS + cc * 8)), vg + jc * HD + cc * 8, ok);
-      }
-    }
-    cp_async_commit();  // always: the group count per thread stays the same on every path
-  };
-  // start the K/V stream, then fetch Q behind it
-#pragma unroll
-  for (int s = 0; s < kMmaDecStages - 1; ++s) issue(warp + s * kMmaDecWarps, s);
-
-  // ---- Q: head h of the group is row h; rows from g up are zero -----------------------------------
-  const T* qg = static_cast<const T*>(p.q) + (static_cast<int64_t>(b) * p.n_head + head0) * HD;
-  for (int c = threadIdx.x; c < kMmaDecTile * CPR; c += kMmaDecThreads) {
-    const int r = c / CPR, cc = c % CPR;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (r < g) v = *reinterpret_cast<const uint4*>(qg + static_cast<int64_t>(r) * HD + cc * 8);
-    *reinterpret_cast<uint4*>(sq + r * LDS + cc * 8) = v;
-  }
-  __syncthreads();
-  uint32_t qa[KB][4];
-  {
-    const int row = (lane & 7) + ((lane >> 3) & 1) * 8;
-    const int col = (lane >> 4) * 8;
-#pragma unroll
-    for (int kb = 0; kb < KB; ++kb)
-      ldmatrix_x4(static_cast<uint32_t>(__cvta_generic_to_shared(sq + row * LDS + kb * 16 + col)), qa[kb]);
-  }
-
-  float o[OB][4];
-#pragma unroll
-  for (int i = 0; i < OB; ++i)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
-  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-
-  int it = 0;
-  for (int t = warp; t < n_tiles; t += kMmaDecWarps, ++it) {
-    // keep kMmaDecStages - 1 tiles in flight beyond the one being consumed
-    issue(t + (kMmaDecStages - 1) * kMmaDecWarps, (it + kMmaDecStages - 1) % kMmaDecStages);
-    cp_async_wait_group<kMmaDecStages - 1>();
-    __syncwarp();
-    const T* sk = my_ring + (it % kMmaDecStages) * kStageElems;
-    const T* sv = sk + kTileElems;
-    const int64_t kv0 = p0 + static_cast<int64_t>(t) * kMmaDecTile;
-
-    // ---- scores 16 heads x 16 positions -----------------------------------------------------------
-    float sc[2][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) sc[i][e] = 0.f;
-#pragma unroll
-    for (int kb = 0; kb < KB; ++kb) {
-      const int krow = (lane & 7) + (lane >> 4) * 8;
-      const int kcol = kb * 16 + ((lane >> 3) & 1) * 8;
-      uint32_t bf[4];
-      ldmatrix_x4(static_cast<uint32_t>(__cvta_generic_to_shared(sk + krow * LDS + kcol)), bf);
-      mma16816<T>(sc[0], qa[kb], bf[0], bf[1]);
-      mma16816<T>(sc[1], qa[kb], bf[2], bf[3]);
-    }
-    // ---- scale, mask the positions past the range, online softmax ------------------------------------
-    float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-    for (int nb = 0; nb < 2; ++nb) {
-      const int64_t key = kv0 + nb * 8 + (lane & 3) * 2;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float v = (key + (e & 1) < p1) ? sc[nb][e] * p.scale_log2 : -INFINITY;
-        sc[nb][e] = v;
-        mx[e >> 1] = fmaxf(mx[e >> 1], v);
-      }
-    }
-    float corr[2];
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-      const float m_new = fmaxf(m_run[r], mx[r]);
-      const float m_use = m_new == -INFINITY ? 0.f : m_new;
-      corr[r] = exp2f(m_run[r] - m_use);
-      m_run[r] = m_new;
-      mx[r] = m_use;
-      l_run[r] *= corr[r];
-    }
-    uint32_t pa[4];
-#pragma unroll
-    for (int nb = 0; nb < 2; ++nb) {
-      float pv[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        pv[e] = exp2f(sc[nb][e] - mx[e >> 1]);
-        l_run[e >> 1] += pv[e];
-      }
-      pa[nb * 2 + 0] = pack2<T>(pv[0], pv[1]);
-      pa[nb * 2 + 1] = pack2<T>(pv[2], pv[3]);
-    }
-#pragma unroll
-    for (int i = 0; i < OB; ++i) {
-      o[i][0] *= corr[0];
-      o[i][1] *= corr[0];
-      o[i][2] *= corr[1];
-      o[i][3] *= corr[1];
-    }
-    // ---- O += P V (16 positions = one k block) ------------------------------------------------------------
-#pragma unroll
-    for (int ob2 = 0; ob2 < OB / 2; ++ob2) {
-      const int vrow = (lane & 7) + ((lane >> 3) & 1) * 8;
-      const int vcol = ob2 * 16 + (lane >> 4) * 8;
-      uint32_t bf[4];
-      ldmatrix_x4_trans(static_cast<uint32_t>(__cvta_generic_to_shared(sv + vrow * LDS + vcol)), bf);
-      mma16816<T>(o[2 * ob2], pa, bf[0], bf[1]);
-      mma16816<T>(o[2 * ob2 + 1], pa, bf[2], bf[3]);
-    }
-    __syncwarp();  // every lane is done with this stage before a later issue() overwrites it
-  }
-  cp_async_wait_all();
-  __syncthreads();  // the rings are free: they now hold the warps' results
-
-  // ---- the warps' (max, sum, values) per head, then the CTA's ---------------------------------------------
-  float* sm_o = reinterpret_cast<float*>(ring);                       // [warps][16][HD]
-  float* sm_m = sm_o + kMmaDecWarps * kMmaDecTile * HD;               // [warps][16]
-  float* sm_l = sm_m + kMmaDecWarps * kMmaDecTile;                    // [warps][16]
-  __shared__ unsigned int ticket_s;
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
-    l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
-  }
-  {
-    const int r0 = lane >> 2, r1 = r0 + 8;
-    if ((lane & 3) == 0) {
-      sm_m[warp * kMmaDecTile + r0] = m_run[0];
-      sm_m[warp * kMmaDecTile + r1] = m_run[1];
-      sm_l[warp * kMmaDecTile + r0] = l_run[0];
-      sm_l[warp * kMmaDecTile + r1] = l_run[1];
-    }
-#pragma unroll
-    for (int i = 0; i < OB; ++i) {
-      const int e = i * 8 + (lane & 3) * 2;
-      float* d0 = sm_o + (warp * kMmaDecTile + r0) * HD + e;
-      float* d1 = sm_o + (warp * kMmaDecTile + r1) * HD + e;
-      d0[0] = o[i][0];
-      d0[1] = o[i][1];
-      d1[0] = o[i][2];
-      d1[1] = o[i][3];
-    }
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < g * HD; idx += kMmaDecThreads) {
-    const int h = idx / HD, e = idx % HD;
-    float mm = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kMmaDecWarps; ++w) mm = fmaxf(mm, sm_m[w * kMmaDecTile + h]);
-    float ll = 0.f, oo = 0.f;
-    if (mm > -INFINITY) {
-#pragma unroll
-      for (int w = 0; w < kMmaDecWarps; ++w) {
-        const float wt = exp2f(sm_m[w * kMmaDecTile + h] - mm);  // 0 for warps that saw no position
-        ll += sm_l[w * kMmaDecTile + h] * wt;
-        oo += sm_o[(w * kMmaDecTile + h) * HD + e] * wt;
-      }
-    }
-    const int64_t slot = (static_cast<int64_t>(b) * p.n_head + head0 + h) * p.num_splits + split;
-    p.part_o[slot * HD + e] = oo;
-    if (e == 0) {
-      p.part_ml[slot * 2] = mm;
-      p.part_ml[slot * 2 + 1] = ll;
-    }
-  }
-
-  // ---- the last CTA of this (sequence, KV head) merges the ranges ---------------------------------------------
-  __threadfence();
-  __syncthreads();
-  unsigned int* counter = p.counters + static_cast<int64_t>(b) * gridDim.y + blockIdx.y;
-  if (threadIdx.x == 0) ticket_s = atomicAdd(counter, 1u);
-  __syncthreads();
-  if (ticket_s != static_cast<unsigned int>(p.num_splits - 1)) return;
-  __threadfence();
-  float* wgt = sm_o;                                  // [g][kMaxSplits]
-  float* inv = wgt + kMmaDecMaxGroup * kMaxSplits;    // [g]
-  const int ns = p.num_splits;
-  for (int h = warp; h < g; h += kMmaDecWarps) {
-    const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + (static_cast<int64_t>(b) * p.n_head + head0 + h) * ns;
-    float2 v[kMaxSplits / 32];
-    float mm = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < kMaxSplits / 32; ++i) {
-      const int sp = lane + 32 * i;
-      v[i] = sp < ns ? __ldcg(ml + sp) : make_float2(-INFINITY, 0.f);
-      mm = fmaxf(mm, v[i].x);
-    }
-    mm = warp_max(mm);
-    float ll = 0.f;
-#pragma unroll
-    for (int i = 0; i < kMaxSplits / 32; ++i) {
-      const int sp = lane + 32 * i;
-      const float w = mm == -INFINITY ? 0.f : exp2f(v[i].x - mm);
-      ll += v[i].y * w;
-      if (sp < ns) wgt[h * kMaxSplits + sp] = w;
-    }
-    ll = warp_sum(ll);
-    if (lane == 0) inv[h] = ll > 0.f ? 1.f / ll : 0.f;
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < g * (HD / 4); idx += kMmaDecThreads) {
-    const int h = idx / (HD / 4), e4 = idx % (HD / 4);
-    const float4* po = reinterpret_cast<const float4*>(p.part_o) +
-                       ((static_cast<int64_t>(b) * p.n_head + head0 + h) * ns) * (HD / 4) + e4;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int sp = 0; sp < ns; ++sp) {
-      const float4 ov = __ldcg(po + static_cast<int64_t>(sp) * (HD / 4));
-      const float w = wgt[h * kMaxSplits + sp];
-      acc.x = fmaf(ov.x, w, acc.x);
-      acc.y = fmaf(ov.y, w, acc.y);
-      acc.z = fmaf(ov.z, w, acc.z);
-      acc.w = fmaf(ov.w, w, acc.w);
-    }
-    const float s = inv[h];
-    T* dst = static_cast<T*>(p.out) + (static_cast<int64_t>(b) * p.n_head + head0 + h) * HD + e4 * 4;
-    uint2 packed;
-    packed.x = pack2<T>(acc.x * s, acc.y * s);
-    packed.y = pack2<T>(acc.z * s, acc.w * s);
-    *reinterpret_cast<uint2*>(dst) = packed;
-  }
-  if (threadIdx.x == 0) *counter = 0u;  // ready for the next call
-}
-
-template <int HD>
-constexpr int mma_decode_smem() {
-  return (kMmaDecTile + kMmaDecWarps * kMmaDecStages * 2 * kMmaDecTile) * (HD + 8) * 2;
-}
-
-template <typename T, int HD>
-int launch_decode_mma(const DecodeParams& p, int B, cudaStream_t st) {
-  constexpr int smem = mma_decode_smem<HD>();
-  static_assert(kMmaDecWarps * kMmaDecTile * HD * 4 + 2 * kMmaDecWarps * kMmaDecTile * 4 <= smem - kMmaDecTile * (HD + 8) * 2,
-                "the merge arrays must fit in the rings");
-  static_assert((kMmaDecMaxGroup * kMaxSplits + kMmaDecMaxGroup) * 4 <= kMmaDecWarps * kMmaDecTile * HD * 4,
-                "the split weights must fit in the value array");
-  auto kern = attn_decode_mma_kernel<T, HD>;
-  static std::atomic<unsigned long long> attr_set{0};  // per template instantiation, one bit per device
-  LRI_ONCE_PER_DEVICE(attr_set, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  dim3 grid(p.num_splits, p.n_kv, B);
-  LRI_CUDA(launch_pdl(kern, grid, dim3(kMmaDecThreads), static_cast<size_t>(smem), st, p));
-  LRI_LAUNCH_CHECK("attn_decode_mma_kernel");
-  return LRI_OK;
-}
-
 template <typename T, int HD>
 int launch_decode(const DecodeParams& p, int B, cudaStream_t st) {
   const int g = p.n_head / p.n_kv;
@@ -824,12 +517,16 @@ int launch_prefill(const PrefillParams& p, int B, cudaStream_t st) {
   return LRI_OK;
 }
 
-// Which decode kernel: the tensor-core kernel from 128 (sequence, KV head) pairs on (measured on
-// B200 at 8 KV heads, context 1152: batch 16 20.0 vs 24.0 us, batch 64 59 vs 82 us per layer),
-// the latency kernels below that.  LRI_ATTN_MMA=1 / 0 forces / forbids it.
-bool attn_mma_wanted(int B, int n_kv) {
+// Which decode kernel: the stream on tensor cores for many (sequence, KV head) pairs, the latency kernels below that.  Where query heads
+// share a KV head (us a layer, 4 of 128 elements, context 1025, latency kernel / stream): 8 pairs 7.6 / 6.7, but beside the MLP
+// of a ladder block the other's smaller CTAs are the better neighbours; 16 pairs 9.1 / 7.5, 32 11.6 / 9.0, 64 14.3 / 10.2, 128 23.7 / 15.3.
+// With one query head each (24 heads, 128 elements): 72 pairs 12.1 / 11.8, 192 24.2 / 20.6, but 144 pairs of 64 elements at 300 positions 5.1 / 6.6.
+// LRI_ATTN_MMA=1 / 0 forces / forbids the stream.
+constexpr int64_t kStreamPairs = 128;  // from here on callers are asked for scratch memory
+bool attn_stream_wanted(int B, int n_head, int n_kv, int64_t smax, int64_t from_pairs) {
   const int mode = option(OPT_ATTN_MMA);
-  return mode == 1 || (mode == -1 && static_cast<int64_t>(B) * n_kv >= 128);
+  const int64_t pairs = static_cast<int64_t>(B) * n_kv;
+  return (mode == 1 || (mode == -1 && pairs >= from_pairs)) && attn_decode_stream_supports(pairs, n_head / n_kv, smax);
 }
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -865,8 +562,8 @@ extern "C" size_t lri_attn_decode_scratch_bytes(int B, int n_head, int n_kv, int
 // current position.  Up to 8 ranges (a power of two; 16 for a one- or two-cluster launch) run as one
 // thread-block cluster and merge through shared memory; that form is kept as long as a CTA then streams at most ~1 MB of K/V.
 // Longer caches take more ranges (up to 64, at least 64 positions each) and merge through the scratch
-// buffer.  The tensor-core kernel (from 128 (sequence, KV head) pairs on) takes one range per pair,
-// two only while one per pair would leave SMs without work.
+// buffer.  The stream kernel (from 128 (sequence, KV head) pairs on) cuts pairs wherever its CTAs' runs end and uses what parts the
+// scratch buffer has room for; it asks for two while one per pair would leave SMs without work.
 extern "C" int lri_attn_decode_plan(int B, int n_head, int n_kv, int head_dim, int64_t smax, int* num_splits) {
   LRI_REQUIRE(num_splits != nullptr, LRI_ERR_ARG, "attn_decode_plan: NULL output");
   LRI_REQUIRE(B >= 1 && n_head >= 1 && n_kv >= 1 && n_head % n_kv == 0 && head_dim >= 1 && smax >= 1, LRI_ERR_ARG,
@@ -879,7 +576,7 @@ extern "C" int lri_attn_decode_plan(int B, int n_head, int n_kv, int head_dim, i
     return LRI_OK;
   }
   const int g = n_head / n_kv;
-  if (g <= kMmaDecMaxGroup && attn_mma_wanted(B, n_kv)) {
+  if (attn_stream_wanted(B, n_head, n_kv, smax, kStreamPairs)) {
     *num_splits = (static_cast<int64_t>(B) * n_kv < 2 * sms && smax >= 256) ? 2 : 1;
     return LRI_OK;
   }
@@ -917,14 +614,17 @@ extern "C" int lri_attn_decode(int dtype, const void* q, const void* k_cache, co
               num_splits, kMaxSplits);
   LRI_REQUIRE(aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && aligned16(out), LRI_ERR_ALIGN,
               "attn_decode: pointers must be 16-byte aligned");
-  const bool mma = attn_mma_wanted(B, n_kv) && n_head / n_kv <= kMmaDecMaxGroup && scratch != nullptr;
-  if (!mma && attn_decode_cluster_supports(num_splits)) {
+  const float scale_log2 = kLog2e / sqrtf(static_cast<float>(head_dim));
+  const bool many = scratch != nullptr && attn_stream_wanted(B, n_head, n_kv, smax, kStreamPairs);
+  if (!many && attn_decode_cluster_supports(num_splits)) {
     // 1, 2, 4, 8 or 16 splits: the splits are the CTAs of one cluster and merge through distributed
     // shared memory; the scratch buffer is not touched
     if (B == 0) return LRI_OK;
+    if (attn_stream_wanted(B, n_head, n_kv, smax, n_head > n_kv ? 16 : kStreamPairs))
+      return attn_decode_stream_launch(dtype, q, k_cache, v_cache, input_pos, pos_is_i64, out, B, n_head, n_kv, head_dim, smax, scale_log2,
+                                       nullptr, nullptr, 1, static_cast<cudaStream_t>(stream));
     return attn_decode_cluster_launch(dtype, q, k_cache, v_cache, input_pos, pos_is_i64, out, B, n_head, n_kv,
-                                      head_dim, smax, num_splits, kLog2e / sqrtf(static_cast<float>(head_dim)),
-                                      static_cast<cudaStream_t>(stream));
+                                      head_dim, smax, num_splits, scale_log2, static_cast<cudaStream_t>(stream));
   }
   LRI_REQUIRE(scratch && aligned16(scratch) &&
                   scratch_bytes >= lri_attn_decode_scratch_bytes(B, n_head, n_kv, head_dim, num_splits),
@@ -937,17 +637,16 @@ extern "C" int lri_attn_decode(int dtype, const void* q, const void* k_cache, co
   DecodeParams p{};
   p.q = q, p.k_cache = k_cache, p.v_cache = v_cache, p.input_pos = input_pos, p.pos_is_i64 = pos_is_i64, p.out = out;
   p.n_head = n_head, p.n_kv = n_kv, p.smax = smax, p.num_splits = num_splits;
-  p.scale_log2 = kLog2e / sqrtf(static_cast<float>(head_dim));
+  p.scale_log2 = scale_log2;
   uint8_t* s = static_cast<uint8_t*>(scratch);
   p.counters = reinterpret_cast<unsigned int*>(s);
   p.part_ml = reinterpret_cast<float*>(s + kCounterBytes);
   p.part_o = reinterpret_cast<float*>(s + kCounterBytes + align_up(rows * num_splits * 2 * 4, 16));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (mma) {
-    if (dtype == LRI_BF16)
-      return head_dim == 128 ? launch_decode_mma<__nv_bfloat16, 128>(p, B, st)
-                             : launch_decode_mma<__nv_bfloat16, 64>(p, B, st);
-    return head_dim == 128 ? launch_decode_mma<__half, 128>(p, B, st) : launch_decode_mma<__half, 64>(p, B, st);
+  if (many) {
+    const bool two = num_splits > 1 || lri_attn_decode_scratch_bytes(B, n_head, n_kv, head_dim, 2) <= scratch_bytes;
+    return attn_decode_stream_launch(dtype, q, k_cache, v_cache, input_pos, pos_is_i64, out, B, n_head, n_kv, head_dim, smax, scale_log2,
+                                     p.counters, p.part_ml, two ? 2 : 1, st);
   }
   if (dtype == LRI_BF16)
     return head_dim == 128 ? launch_decode<__nv_bfloat16, 128>(p, B, st) : launch_decode<__nv_bfloat16, 64>(p, B, st);

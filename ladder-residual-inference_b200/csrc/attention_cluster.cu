@@ -25,6 +25,9 @@ namespace cg = cooperative_groups;
 
 namespace lri {
 int attn_decode_cluster_head_tile(int B, int n_kv, int g);
+// form for many sequences (attention_stream.cu)
+bool attn_decode_stream_supports(int64_t pairs, int group, int64_t smax);
+int attn_decode_stream_masked_launch(int dtype, const WindowParams& w, int B, cudaStream_t st);
 
 namespace {
 
@@ -357,6 +360,12 @@ int attn_decode_masked_launch(int dtype, const WindowParams& w, int B, cudaStrea
   p.q = w.q, p.k_cache = w.k, p.v_cache = w.v, p.input_pos = w.input_pos, p.pos_is_i64 = w.pos_is_i64, p.out = w.out;
   p.n_head = w.H, p.n_kv = n_kv, p.smax = w.k_rows, p.scale_log2 = w.scale * 1.4426950408889634f;
   p.dim = w.d1, p.vdim = w.dv, p.window = w.window, p.chunk = w.chunk, p.sink = w.sink, p.out_ld = w.out_ld, p.out_scale = w.out_scale;
+  // us a layer, this kernel / the stream, context 1025: 32 heads of 8 KV heads, 16 pairs 14.3 / 8.4, 32 21.5 / 10, 128 36.0 / 16.7; one query head each, 64
+  // pairs 10.6 / 10.5, 72 10.7 / 13, 192 21.5 / 22.5, 960 pairs at 701 positions 72.5 / 72.2
+  const int mode = option(OPT_ATTN_MMA);
+  const int64_t pairs = static_cast<int64_t>(B) * n_kv;
+  if ((mode == 1 || (mode == -1 && pairs >= (w.group > 1 ? 16 : 512))) && attn_decode_stream_supports(pairs, w.group, w.k_rows))
+    return attn_decode_stream_masked_launch(dtype, w, B, st);
   int64_t visible = w.k_rows < w.window ? w.k_rows : w.window;
   if (w.chunk > 0 && w.chunk < visible) visible = w.chunk;
   const int gt = attn_decode_cluster_head_tile(B, n_kv, w.group);

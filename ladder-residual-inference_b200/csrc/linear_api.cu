@@ -18,6 +18,7 @@ int gemm_tcgen05_status_read_and_clear(int* status_out);
 int gemm_pair_status_read_and_clear(int* status_out);
 int attn_prefill_tc_status_read_and_clear(int* status_out);
 int window_attention_tc_status_read_and_clear(int* status_out);
+int attn_decode_stream_status_read_and_clear(int* status_out);
 int state_scan_status_read_and_clear(int* status_out);
 bool gemm_tcgen05_fused_supports(int epi, const LinearParams& p, int64_t m);
 int gemm_tcgen05_fused_launch(int dtype, int epi, const LinearParams& p, int64_t m, cudaStream_t st);
@@ -351,6 +352,10 @@ extern "C" int lri_gemm_status(void) {
     rc = window_attention_tc_status_read_and_clear(&v3);
     if (rc != LRI_OK) return rc;
   }
+  int v6 = 0;
+  rc = attn_decode_stream_status_read_and_clear(&v6);
+  if (rc != LRI_OK) return rc;
+  if (v6 != 0) return fail(LRI_ERR_TIMEOUT, "decode attention: a bounded mbarrier wait gave up (site %d)", v6);
   int v4 = 0;
   rc = state_scan_status_read_and_clear(&v4);
   if (rc != LRI_OK) return rc;
