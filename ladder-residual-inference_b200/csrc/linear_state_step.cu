@@ -12,6 +12,7 @@
 #include <cooperative_groups.h>
 
 #include "linear_state.cuh"
+#include "mma.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -48,7 +49,34 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
 }
 
-// y[row] = w[row] . x for n rows: 8 lanes a row, 4 rows a warp
+// 16-bit weights that are staged take the tensor cores, 16 rows of one of the two matrices a warp at a time, the vector in one of the
+// product's eight columns.  Staged rows are `rank` elements and 8 of zeros apart: no bank conflicts, and a rank that is an odd
+// multiple of 8 ends in zeros.  On the FMA pipe, 8 lanes a row, the two 128 x 128 products of a CTA were 4.1 us of its 19.
+__host__ __device__ constexpr int staged_pitch(int rank) { return rank + 8; }
+__host__ __device__ constexpr int staged_rows(int rows) { return (rows + 15) / 16 * 16; }
+template <typename T>
+__device__ __forceinline__ void rows_mma(const T* w, int rank, const T* x, int tile, int rows, float* y) {
+  const int lane = threadIdx.x & 31, pitch = staged_pitch(rank);
+  float acc[2][4] = {};
+  const T* at = w + (tile * 16 + (lane & 15)) * pitch + (lane >> 4) * 8;
+  for (int k = 0, i = 0; k < rank; k += 16, i ^= 1) {
+    uint32_t a0, a1, a2, a3;
+    ldmatrix_x4(at + k, a0, a1, a2, a3);
+    const uint32_t b0 = lane < 4 ? *reinterpret_cast<const uint32_t*>(x + k + lane * 2) : 0u;
+    const uint32_t b1 = lane < 4 ? *reinterpret_cast<const uint32_t*>(x + k + 8 + lane * 2) : 0u;
+    if (i == 0)
+      mma16816<T>(acc[0], a0, a1, a2, a3, b0, b1);
+    else
+      mma16816<T>(acc[1], a0, a1, a2, a3, b0, b1);
+  }
+  const int r = tile * 16 + (lane >> 2);
+  if ((lane & 3) == 0) {
+    if (r < rows) y[r] = acc[0][0] + acc[1][0];
+    if (r + 8 < rows) y[r + 8] = acc[0][2] + acc[1][2];
+  }
+}
+
+// The same in general, y[row] = w[row] . x for n rows: 8 lanes a row, 4 rows a warp
 template <typename T>
 __device__ __forceinline__ void rows_dot(const T* w, int rank, const float* x, int n, float* y) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = (lane & 7) * 8;
@@ -81,15 +109,17 @@ struct StepConv {
     for (int j = 0; j < kRegTaps; ++j) w[j] = live && taps <= kRegTaps && j < taps ? Num<T>::to_f(taps_w[taps - 1 - j]) : 0.f;
   }
   // slot: pos % taps
+  float old[kRegTaps];
+  __device__ __forceinline__ void past(const float* ring, int64_t channels, int taps, int pos, int slot, bool live) {
+#pragma unroll
+    for (int j = 1; j < kRegTaps; ++j) {
+      const int at = slot >= j ? slot - j : slot - j + taps;
+      old[j] = live && taps <= kRegTaps && j < taps && pos >= j ? ring[at * channels] : 0.f;
+    }
+  }
   __device__ __forceinline__ float run(float x, float* ring, int64_t channels, int taps, int pos, int slot, bool keep) const {
     float y = w[0] * x;
     if (taps <= kRegTaps) {
-      float old[kRegTaps];
-#pragma unroll
-      for (int j = 1; j < kRegTaps; ++j) {
-        const int at = slot >= j ? slot - j : slot - j + taps;
-        old[j] = j < taps && pos >= j ? ring[at * channels] : 0.f;
-      }
 #pragma unroll
       for (int j = 1; j < kRegTaps; ++j) y = fmaf(w[j], old[j], y);
     } else {
@@ -120,17 +150,35 @@ __global__ void __launch_bounds__(kThreads, RV <= 4 ? 2 : 1) state_step_kernel(c
   const int cols = E - col0 < kCols ? E - col0 : kCols;
   float* x_a = reinterpret_cast<float*>(step_smem);  // input of the decay's second projection
   float* x_g = x_a + p.a_rank;
-  T* w_smem = reinterpret_cast<T*>(x_g + (DELTA ? p.g_rank : 0));
+  constexpr bool kMma = sizeof(T) == 2;
+  T* t_a = reinterpret_cast<T*>(x_g + (DELTA ? p.g_rank : 0));  // kMma: the same in the storage type, behind them 8 zeros
+  T* t_g = t_a + (kMma ? staged_pitch(p.a_rank) : 0);
+  T* w_smem = t_g + (kMma && DELTA ? staged_pitch(p.g_rank) : 0);
   const T* a2 = static_cast<const T*>(p.a2) + static_cast<int64_t>(h) * C * p.a_rank;
   const T* g2 = DELTA ? static_cast<const T*>(p.g2) + (static_cast<int64_t>(h) * E + col0) * p.g_rank : nullptr;
   float* st_base = p.state + (b * H + h) * static_cast<int64_t>(C) * E;
   if (p.staged) {  // constants of the model
     constexpr int kPer = 16 / sizeof(T);
-    const int na = C * p.a_rank / kPer, ng = DELTA ? cols * p.g_rank / kPer : 0;
-    for (int i = tid; i < na; i += kThreads) cp_async16(w_smem + i * kPer, a2 + i * kPer);
-    for (int i = tid; i < ng; i += kThreads) cp_async16(w_smem + (na + i) * kPer, g2 + i * kPer);
+    auto stage = [&](T* dst, const T* src, int rows, int rank) {
+      const int row_units = rank / kPer, pitch = kMma ? staged_pitch(rank) : rank;
+      for (int i = tid; i < rows * row_units; i += kThreads) {
+        const int r = i / row_units, c = (i - r * row_units) * kPer;
+        cp_async16(dst + r * pitch + c, src + r * rank + c);
+      }
+      if (kMma && rank % 16)
+        for (int r = tid; r < rows; r += kThreads) *reinterpret_cast<uint4*>(dst + r * pitch + rank) = make_uint4(0u, 0u, 0u, 0u);
+    };
+    T* w_gate = w_smem + (kMma ? staged_rows(C) * staged_pitch(p.a_rank) : C * p.a_rank);
+    stage(w_smem, a2, C, p.a_rank);
     a2 = w_smem;
-    if (DELTA) g2 = w_smem + na * kPer;
+    if (DELTA) {
+      stage(w_gate, g2, cols, p.g_rank);
+      g2 = w_gate;
+    }
+    if (kMma && tid < 8) {
+      t_a[p.a_rank + tid] = Num<T>::from_f(0.f);
+      if (DELTA) t_g[p.g_rank + tid] = Num<T>::from_f(0.f);
+    }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
   for (int i = tid; i < C * NC; i += kThreads)  // one request per 128-byte line
@@ -140,12 +188,24 @@ __global__ void __launch_bounds__(kThreads, RV <= 4 ? 2 : 1) state_step_kernel(c
   const int e_mine = tid - (kThreads - kCols);
   const bool has_k = tid < C, has_v = e_mine >= 0 && e_mine < cols;
   const int64_t ch_v = static_cast<int64_t>(h) * E + col0 + e_mine;
+  constexpr bool kApart = CP + kCols <= kThreads;  // no thread has both: the value channel takes the registers of the query's
   [[maybe_unused]] StepConv<T> conv_q, conv_k, conv_v;
   float a = 0.f;
   if constexpr (DELTA) {
-    conv_q.load(p.conv_q, ch_k, p.taps, has_k);
+    if (kApart)
+      conv_q.load(has_k ? p.conv_q : p.conv_v, has_k ? ch_k : ch_v, p.taps, has_k || has_v);
+    else
+      conv_q.load(p.conv_q, ch_k, p.taps, has_k), conv_v.load(p.conv_v, ch_v, p.taps, has_v);
     conv_k.load(p.conv_k, ch_k, p.taps, has_k);
-    conv_v.load(p.conv_v, ch_v, p.taps, has_v);
+    // the rings' lines, whichever slots this position reads
+    const float* ring_all = p.ring + b * p.taps * (2ll * G * C + static_cast<int64_t>(H) * E);
+    for (int i = tid; i < p.taps * 3 * 8; i += kThreads) {
+      const int tap = i / 24, part = i % 24 >> 3, at = (i & 7) * 32;
+      const int64_t channels = 2ll * G * C + static_cast<int64_t>(H) * E;
+      if (at < (part < 2 ? C : cols))
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(ring_all + tap * channels + at + (part == 0 ? static_cast<int64_t>(hk) * C
+                     : part == 1 ? static_cast<int64_t>(G) * C + static_cast<int64_t>(hk) * C : 2ll * G * C + static_cast<int64_t>(h) * E + col0)));
+    }
     a = expf(Num<T>::to_f(static_cast<const T*>(p.a_log)[h]));
   }
   if (has_k) sbias[tid] = Num<T>::to_f(static_cast<const T*>(p.bias)[h * C + tid]);
@@ -157,6 +217,24 @@ __global__ void __launch_bounds__(kThreads, RV <= 4 ? 2 : 1) state_step_kernel(c
 
   // ---- state, and what the columns share -------------------------------------------------------------------
   const int pos = static_cast<int>(load_pos(p.input_pos, p.pos_is_i64, 0));
+  const float* in = p.proj + b * p.ld;
+  const int64_t channels = 2ll * G * C + static_cast<int64_t>(H) * E;
+  float* ring = DELTA ? p.ring + b * p.taps * channels : nullptr;
+  const int slot = DELTA ? (pos < 0 ? 0 : pos) % p.taps : 0;
+  float* ring_k = DELTA ? ring + static_cast<int64_t>(G) * C + ch_k : nullptr;
+  float* ring_v = DELTA ? ring + 2ll * G * C + ch_v : nullptr;
+  // The inputs and the rings are asked for ahead of the state, whose 64 KB would hold them up.
+  float q = has_k ? in[p.q_off + ch_k] : 0.f, k = has_k ? in[p.k_off + ch_k] : 0.f;
+  float v = has_v ? in[p.v_off + ch_v] : 0.f;
+  const float beta_in = DELTA ? in[p.b_off + h] : 0.f;
+  const float gate_in = !DELTA && has_v ? in[p.gate_off + ch_v] : 0.f;
+  if constexpr (DELTA) {
+    if (kApart)
+      conv_q.past(has_k ? ring + ch_k : ring_v, channels, p.taps, pos, slot, has_k || has_v);
+    else
+      conv_q.past(ring + ch_k, channels, p.taps, pos, slot, has_k), conv_v.past(ring_v, channels, p.taps, pos, slot, has_v);
+    conv_k.past(ring_k, channels, p.taps, pos, slot, has_k);
+  }
   float st[RV][4][NC];
   float* st_mine = st_base + 4 * rg * E + e0;
 #pragma unroll
@@ -171,19 +249,13 @@ __global__ void __launch_bounds__(kThreads, RV <= 4 ? 2 : 1) state_step_kernel(c
         st[i][r][0] = pos > 0 && live ? st_mine[(32 * i + r) * E] : 0.f;
       }
     }
-  const float* in = p.proj + b * p.ld;
-  const int64_t channels = 2ll * G * C + static_cast<int64_t>(H) * E;
-  float* ring = DELTA ? p.ring + b * p.taps * channels : nullptr;
-  const float beta = DELTA ? sigmoid_f(in[p.b_off + h]) : 0.f;
-  const int slot = DELTA ? (pos < 0 ? 0 : pos) % p.taps : 0;
-  float q = 0.f, k = 0.f;
+  const float beta = DELTA ? sigmoid_f(beta_in) : 0.f;
   if (tid < CP) {
     if (has_k) {
-      q = in[p.q_off + ch_k], k = in[p.k_off + ch_k];
       if constexpr (DELTA) {
         const bool keep = blockIdx.x == 0 && h % (H / G) == 0;  // the first CTA of a group keeps the shared channels
         q = conv_q.run(q, ring + ch_k, channels, p.taps, pos, slot, keep);
-        k = conv_k.run(k, ring + static_cast<int64_t>(G) * C + ch_k, channels, p.taps, pos, slot, keep);
+        k = conv_k.run(k, ring_k, channels, p.taps, pos, slot, keep);
       }
     } else {
       sg[tid] = 1.f;
@@ -191,18 +263,22 @@ __global__ void __launch_bounds__(kThreads, RV <= 4 ? 2 : 1) state_step_kernel(c
     sq[tid] = q, sk[tid] = k;
   }
   if (e_mine >= 0) {
-    float v = 0.f;
-    if (has_v) {
-      v = in[p.v_off + ch_v];
-      if constexpr (DELTA)
-        v = conv_v.run(v, ring + 2ll * G * C + ch_v, channels, p.taps, pos, slot, true);
-    }
+    if constexpr (DELTA)
+      if (has_v) v = (kApart ? conv_q : conv_v).run(v, ring_v, channels, p.taps, pos, slot, true);
     sv[e_mine] = v;
-    if (!DELTA) sgate[e_mine] = has_v ? silu_f(in[p.gate_off + ch_v]) : 0.f;
+    if (!DELTA) sgate[e_mine] = has_v ? silu_f(gate_in) : 0.f;
   }
-  for (int i = tid; i < p.a_rank; i += kThreads) x_a[i] = rnd<T>(in[p.a_off + i]);
+  for (int i = tid; i < p.a_rank; i += kThreads) {
+    const float f = in[p.a_off + i];
+    x_a[i] = rnd<T>(f);
+    if (kMma) t_a[i] = Num<T>::from_f(f);
+  }
   if (DELTA)
-    for (int i = tid; i < p.g_rank; i += kThreads) x_g[i] = rnd<T>(in[p.gate_off + i]);
+    for (int i = tid; i < p.g_rank; i += kThreads) {
+      const float f = in[p.gate_off + i];
+      x_g[i] = rnd<T>(f);
+      if (kMma) t_g[i] = Num<T>::from_f(f);
+    }
   if constexpr (DELTA) {
     const float qq = warp_sum(q * q), kk = warp_sum(k * k), kq = warp_sum(k * q);
     if (lane == 0) part_qk[warp][0] = qq, part_qk[warp][1] = kk, part_qk[warp][2] = kq;
@@ -210,8 +286,23 @@ __global__ void __launch_bounds__(kThreads, RV <= 4 ? 2 : 1) state_step_kernel(c
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
 
-  rows_dot<T>(a2, p.a_rank, x_a, C, sg);
-  if constexpr (DELTA) rows_dot<T>(g2, p.g_rank, x_g, cols, sgate);
+  bool dots = true;
+  if constexpr (kMma) {
+    if (p.staged) {
+      const int ta = (C + 15) / 16, tg = DELTA ? (cols + 15) / 16 : 0;
+      for (int t = warp; t < ta + tg; t += kThreads / 32) {
+        if (t < ta)
+          rows_mma<T>(w_smem, p.a_rank, t_a, t, C, sg);
+        else
+          rows_mma<T>(g2, p.g_rank, t_g, t - ta, cols, sgate);
+      }
+      dots = false;
+    }
+  }
+  if (dots) {
+    rows_dot<T>(a2, p.a_rank, x_a, C, sg);
+    if constexpr (DELTA) rows_dot<T>(g2, p.g_rank, x_g, cols, sgate);
+  }
   float qs = 1.0f / sqrtf(static_cast<float>(C)), ks = 1.f, kq = 0.f;
   if constexpr (DELTA) {
     float qq = 0.f, kk = 0.f;
@@ -321,8 +412,12 @@ __global__ void __launch_bounds__(kThreads, RV <= 4 ? 2 : 1) state_step_kernel(c
 template <typename T, bool DELTA, int RV, int NC>
 int launch(const StepParams& p, int B, cudaStream_t st) {
   constexpr int kCols = 32 * NC;
-  const size_t x_bytes = (static_cast<size_t>(p.a_rank) + (DELTA ? p.g_rank : 0)) * 4;
-  const size_t w_bytes = (static_cast<size_t>(p.C) * p.a_rank + (DELTA ? static_cast<size_t>(kCols) * p.g_rank : 0)) * sizeof(T);
+  constexpr bool kMma = sizeof(T) == 2;
+  const size_t x_bytes = (static_cast<size_t>(p.a_rank) + (DELTA ? p.g_rank : 0)) * 4 +
+                         (kMma ? static_cast<size_t>(staged_pitch(p.a_rank) + (DELTA ? staged_pitch(p.g_rank) : 0)) * 2 : 0);
+  const size_t w_bytes = kMma ? (static_cast<size_t>(staged_rows(p.C)) * staged_pitch(p.a_rank) +
+                                 (DELTA ? static_cast<size_t>(kCols) * staged_pitch(p.g_rank) : 0)) * 2
+                              : (static_cast<size_t>(p.C) * p.a_rank + (DELTA ? static_cast<size_t>(kCols) * p.g_rank : 0)) * sizeof(T);
   const unsigned cs = (p.E + kCols - 1) / kCols;
   StepParams q = p;
   q.staged = w_bytes <= kStageBytes;
