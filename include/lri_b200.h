@@ -57,7 +57,7 @@ int lri_set_gemm_backend(int backend);
 /* Tuning options: one table per process, each entry initialised from an LRI_* environment variable
  * at first use and changeable at run time; a change applies from the next launch on.  Names (initial
  * value from): stream_rows (LRI_STREAM_ROWS, 1..16, token rows up to which the weight-streaming
- * kernels run), gemv_simt (LRI_GEMV_SMALL=simt), gemv_rows_per_cta (LRI_GEMV_R: 0, 2, 4, 8),
+ * kernels run; large projections take the stream-K kernel from 2 rows on), gemv_simt (LRI_GEMV_SMALL=simt), gemv_rows_per_cta (LRI_GEMV_R: 0, 2, 4, 8),
  * gemv_depth (LRI_GEMV_U: 0, 2), gemv_mma_tiles (LRI_GEMV_MT: 0, 1, 2, 4), gemm_group
  * (LRI_GEMM_GROUP), fused_prefill (LRI_FUSED_PREFILL: 0, 1), pdl (LRI_PDL: 0, 1), attn_cluster
  * (LRI_ATTN_CLUSTER: 0, 1), attn_mma (LRI_ATTN_MMA: -1 choose, 0, 1), decode_splits

@@ -49,7 +49,7 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // first use of any option) and can be changed at run time through lri_set_option(); the kernels'
 // launch code reads the table on every call, so a change takes effect on the next launch.
 enum Option {
-  OPT_STREAM_ROWS = 0,  // LRI_STREAM_ROWS    token rows up to which the weight-streaming kernels run (1..16, default 8)
+  OPT_STREAM_ROWS = 0,  // LRI_STREAM_ROWS    token rows up to which the weight-streaming kernels run (1..16, default 8; large projections from 2 rows on: stream-K)
   OPT_GEMV_SIMT,        // LRI_GEMV_SMALL=simt  keep the SIMT streaming kernel for 2..8 rows (default 0)
   OPT_GEMV_R,           // LRI_GEMV_R         weight rows per CTA of the SIMT streaming kernel: 2, 4 or 8 (0 = choose)
   OPT_GEMV_U,           // LRI_GEMV_U         2 halves the loads in flight per thread of that kernel (0 = default)

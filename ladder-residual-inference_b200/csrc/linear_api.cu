@@ -265,6 +265,19 @@ static bool streamk_rows(int64_t M) {
 static size_t streamk_bytes(int epi, int64_t M, int64_t n) {
   return (M > streaming_rows() && M <= kSplitKMaxRows && n < (1ll << 31)) ? gemm_streamk_workspace_bytes(epi, M, static_cast<int>(n)) : 0;
 }
+// 2 .. streaming_rows() token rows of a large projection go there too.  The streaming kernel reads all token rows in every CTA of 16 weight
+// rows, which is what it waits for behind the kernel that wrote them; the stream-K kernel reads them once an SM and has its ring full of
+// weights by then, but costs a second launch.  Measured on B200, streaming / stream-K, a whole decode step of 4 sequences: 8B (k 4096 and
+// 14336, all projections from 33 MB on) 4399 / 3265 us dense, 3516 / 2811 ladder; Migosun 8B 5051 / 4053.  One projection alone: gated
+// 16384 x 2048 (67 MB) 19.0 / 15.1 us, 16384 x 3072 25.6 / 21.2, 2048 x 8192 (34 MB) 13.0 / 10.4, 3072 x 8192 14.5 / 12.8; but 9216 x 3072 11.0 / 13.7,
+// 8192 x 2048 7.3 / 9.6, 2048 x 2048 4.3 / 6.3.  Vocabulary projections keep the kernel whose logits do not depend on which rows are
+// computed together (greedy decoding on slices).
+static bool streamk_few_rows(int epi, const LinearParams& p, const void* workspace, size_t workspace_bytes) {
+  const bool glu = epi == EPI_SWIGLU || epi == EPI_GLU;
+  const int64_t rows = glu ? 2ll * p.n : p.n;
+  if (p.m < 2 || p.n > 65536 || rows * p.k < (15ll << 20) || (!glu && p.k < 4096)) return false;
+  return !prefer_simt_gemv() && current_gemm_backend() != LRI_GEMM_SIMT && gemm_streamk_supports(epi, p, workspace, workspace_bytes);
+}
 static size_t max_size(size_t a, size_t b) { return a > b ? a : b; }
 
 int swiglu_rows_launch(int dtype, const void* ug, void* h, int64_t m, int n, cudaStream_t st) {
@@ -389,6 +402,8 @@ extern "C" int lri_linear(int dtype, const void* x, const void* w, const void* a
   if (M <= streaming_rows()) {
     LinearParams p{};
     p.x = x, p.w = w, p.y = y, p.addend = addend, p.m = static_cast<int>(M), p.n = N, p.k = K;
+    if (streamk_few_rows(EPI_PLAIN, p, workspace, workspace_bytes))
+      return gemm_streamk_launch(dtype, EPI_PLAIN, p, workspace, workspace_bytes, st);
     return streaming_launch(dtype, EPI_PLAIN, p, st, prefer_simt_gemv());
   }
   if (streamk_rows(M)) {
@@ -424,8 +439,9 @@ extern "C" int lri_linear_f32(int dtype, const void* x, const void* w, float* y,
     return gemm_generic_launch(dtype, x, w, nullptr, y, true, M, N, K, st);
   LinearParams p{};
   p.x = x, p.w = w, p.y = y, p.m = static_cast<int>(M), p.n = N, p.k = K;
-  if (M <= streaming_rows()) return streaming_launch(dtype, EPI_F32, p, st, prefer_simt_gemv());
-  if (streamk_rows(M) && gemm_streamk_supports(EPI_F32, p, workspace, workspace_bytes))
+  if (M <= streaming_rows() && !streamk_few_rows(EPI_F32, p, workspace, workspace_bytes))
+    return streaming_launch(dtype, EPI_F32, p, st, prefer_simt_gemv());
+  if ((M <= streaming_rows() || streamk_rows(M)) && gemm_streamk_supports(EPI_F32, p, workspace, workspace_bytes))
     return gemm_streamk_launch(dtype, EPI_F32, p, workspace, workspace_bytes, st);
   if (M <= kGemvMmaMaxRows) return streaming_launch(dtype, EPI_F32, p, st, prefer_simt_gemv());
   if (current_gemm_backend() != LRI_GEMM_SIMT && N % 8 == 0 && aligned16(y))
@@ -460,8 +476,9 @@ extern "C" int lri_gateup_swiglu(int dtype, const void* x, const void* w1, void*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LinearParams p{};
   p.x = x, p.w = w1, p.y = h, p.m = static_cast<int>(M), p.n = I, p.k = K;
-  if (M <= streaming_rows()) return streaming_launch(dtype, EPI_SWIGLU, p, st, prefer_simt_gemv());
-  if (streamk_rows(M) && gemm_streamk_supports(EPI_SWIGLU, p, workspace, workspace_bytes))
+  if (M <= streaming_rows() && !streamk_few_rows(EPI_SWIGLU, p, workspace, workspace_bytes))
+    return streaming_launch(dtype, EPI_SWIGLU, p, st, prefer_simt_gemv());
+  if ((M <= streaming_rows() || streamk_rows(M)) && gemm_streamk_supports(EPI_SWIGLU, p, workspace, workspace_bytes))
     return gemm_streamk_launch(dtype, EPI_SWIGLU, p, workspace, workspace_bytes, st);
   // no usable workspace: the streaming kernel takes up to 16 rows
   if (M <= kGemvMmaMaxRows) return streaming_launch(dtype, EPI_SWIGLU, p, st, prefer_simt_gemv());
@@ -504,8 +521,8 @@ extern "C" int lri_gateup_glu(int dtype, const void* x, const void* w1, void* h,
   p.ex.glu = GluParams{alpha, limit, offset};
   if (dtype != LRI_FP32 && K % 8 == 0 && aligned16(x) && aligned16(w1)) {
     if (M == 1) return gemv_launch(dtype, EPI_GLU, p, st);
-    if (M <= streaming_rows()) return gemv_mma_launch(dtype, EPI_GLU, p, st);
-    if (streamk_rows(M) && gemm_streamk_supports(EPI_GLU, p, workspace, workspace_bytes))
+    if (M <= streaming_rows() && !streamk_few_rows(EPI_GLU, p, workspace, workspace_bytes)) return gemv_mma_launch(dtype, EPI_GLU, p, st);
+    if ((M <= streaming_rows() || streamk_rows(M)) && gemm_streamk_supports(EPI_GLU, p, workspace, workspace_bytes))
       return gemm_streamk_launch(dtype, EPI_GLU, p, workspace, workspace_bytes, st);
     if (M <= kGemvMmaMaxRows) return gemv_mma_launch(dtype, EPI_GLU, p, st);
     if (current_gemm_backend() != LRI_GEMM_SIMT && gemm_tcgen05_fused_supports(EPI_GLU, p, M))
@@ -551,8 +568,9 @@ extern "C" int lri_qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, 
   p.rope_table = rope_table, p.input_pos = input_pos, p.pos_is_i64 = pos_is_i64;
   p.q_out = q_out, p.k_cache = k_cache, p.v_cache = v_cache;
   p.S = S, p.n_head = n_head, p.n_kv = n_kv, p.head_dim = head_dim, p.smax = smax, p.table_rows = table_rows, p.table_gathered = table_gathered;
-  if (M <= streaming_rows()) return streaming_launch(dtype, EPI_QKV, p, st, prefer_simt_gemv());
-  if (streamk_rows(M) && gemm_streamk_supports(EPI_QKV, p, workspace, workspace_bytes))
+  if (M <= streaming_rows() && !streamk_few_rows(EPI_QKV, p, workspace, workspace_bytes))
+    return streaming_launch(dtype, EPI_QKV, p, st, prefer_simt_gemv());
+  if ((M <= streaming_rows() || streamk_rows(M)) && gemm_streamk_supports(EPI_QKV, p, workspace, workspace_bytes))
     return gemm_streamk_launch(dtype, EPI_QKV, p, workspace, workspace_bytes, st);
   // no usable workspace: the streaming kernel takes up to 16 rows
   if (M <= kGemvMmaMaxRows) return streaming_launch(dtype, EPI_QKV, p, st, prefer_simt_gemv());
