@@ -463,6 +463,26 @@ int lri_head_norm_gate(int dtype, const float* o, const void* norm_weight, float
 /* y [rows, n] = x[row, off .. off + n) rounded to `dtype`. */
 int lri_round_columns(int dtype, const float* x, int64_t ld, int64_t off, int n, void* y, int64_t rows, lri_stream_t stream);
 
+/* ---- the layers of one forward pass on one GPU -------------------------------------------------
+ * From the embedded rows in `resid` to the normed rows in `normed`, by the entry points above in the order of one of the
+ * schedules.  layers: for each layer attention norm, QKV, wo, MLP norm, w1, w2, K cache, V cache; reduces (desync): for each
+ * layer whether attention and MLP fold their partial into the residual.  Buffers hold B S rows.  Nothing is kept of it. */
+enum lri_schedule { LRI_DENSE = 0, LRI_LADDER = 1, LRI_LADDER_TWO_STREAMS = 2, LRI_PARALLEL = 3, LRI_DESYNC = 4 };
+typedef struct {
+  int dtype, schedule, n_layer, B, S, n_head, n_kv, head_dim, dim, inter, pos_is_i64, splits;
+  float eps;
+  int64_t smax, table_rows;
+  const void* const* layers;
+  const unsigned char* reduces;
+  const void *rope_table, *input_pos, *final_norm;
+  void *resid, *normed, *normed_m, *part_a, *part_m, *q, *y, *h;
+  void *ws_qkv, *ws_wo, *ws_ug, *ws_w2, *scratch;
+  size_t ws_qkv_bytes, ws_wo_bytes, ws_ug_bytes, ws_w2_bytes, scratch_bytes;
+  lri_stream_t stream, side;
+  void* const* events; /* two streams: 2 n_layer + 2 cudaEvent_t */
+} lri_llama_pass;
+int lri_llama_run(const lri_llama_pass* pass);
+
 /* Reads (and clears) the device status word: LRI_OK or LRI_ERR_TIMEOUT.  Synchronises `stream`. */
 int lri_comm_status(lri_comm* comm, lri_stream_t stream);
 int lri_comm_destroy(lri_comm* comm);

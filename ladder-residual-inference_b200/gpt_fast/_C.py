@@ -21,6 +21,18 @@ lib = ctypes.CDLL(LIB_PATH)
 
 c_void_p, c_int, c_int64, c_float, c_size_t = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_float, ctypes.c_size_t
 
+class LlamaPass(ctypes.Structure):
+    """lri_llama_pass: what one call of lri_llama_run works on."""
+    _fields_ = ([(k, c_int) for k in ("dtype", "schedule", "n_layer", "B", "S", "n_head", "n_kv", "head_dim", "dim", "inter", "pos_is_i64", "splits")]
+                + [("eps", c_float), ("smax", c_int64), ("table_rows", c_int64)]
+                + [(k, c_void_p) for k in ("layers", "reduces", "rope_table", "input_pos", "final_norm", "resid", "normed", "normed_m", "part_a",
+                                           "part_m", "q", "y", "h", "ws_qkv", "ws_wo", "ws_ug", "ws_w2", "scratch")]
+                + [(k, c_size_t) for k in ("ws_qkv_bytes", "ws_wo_bytes", "ws_ug_bytes", "ws_w2_bytes", "scratch_bytes")]
+                + [(k, c_void_p) for k in ("stream", "side", "events")])
+
+
+DENSE, LADDER, LADDER_TWO_STREAMS, PARALLEL, DESYNC = range(5)
+
 # name -> (restype, argtypes); the order of arguments is that of include/lri_b200.h
 _SIGNATURES = {
     "lri_last_error": (ctypes.c_char_p, []),
@@ -132,6 +144,7 @@ _SIGNATURES = {
     "lri_head_norm_gate": (c_int, [c_int, c_void_p, c_void_p, c_float, c_void_p, c_int64, c_int, c_float, c_void_p, c_int64,
                                    c_int64, c_int, c_int, c_void_p]),
     "lri_round_columns": (c_int, [c_int, c_void_p, c_int64, c_int64, c_int, c_void_p, c_int64, c_void_p]),
+    "lri_llama_run": (c_int, [ctypes.POINTER(LlamaPass)]),
     "lri_comm_status": (c_int, [c_void_p, c_void_p]),
     "lri_comm_destroy": (c_int, [c_void_p]),
 }
@@ -171,7 +184,8 @@ def ptr(t):
 
 
 def stream_handle() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the stream object of torch.cuda.current_stream() costs a microsecond a launch
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def require_cuda(*tensors) -> None:

@@ -26,7 +26,8 @@ import os
 
 import torch
 
-from .comm import make_comm
+from ._C import DENSE, DESYNC, LADDER, LADDER_TWO_STREAMS, PARALLEL, dtype_code
+from .comm import NoComm, make_comm
 from .ops import decode_splits
 
 _MAX_SPLITS = 64
@@ -86,6 +87,8 @@ class Engine:
             # priority was measured slower on B200, 2.80 against 2.58 ms per 8B step)
             self.side_stream = torch.cuda.Stream()
             self._events = [torch.cuda.Event() for _ in range(2 * cfg.n_layer + 2)]
+            for e in self._events:
+                e.record()  # an event has a handle from its first recording on
         self.ready = True
 
     def _setup_head(self, max_batch, device, dtype):
@@ -179,7 +182,46 @@ class Engine:
         """Embedding, layers and final norm; leaves the normalised hidden states in self.normed."""
         self._splits = decode_splits(B, self.nh, self.nkv, self.model.max_seq_length, self.hd) if S == 1 else 1
         self.ops.embedding(self.model.tok_embeddings.weight, idx, self.resid)
-        getattr(self, "_run_" + self.family)(rows, B, S, input_pos)
+        if not self._run_native(B, S, input_pos):
+            getattr(self, "_run_" + self.family)(rows, B, S, input_pos)
+
+    def _run_native(self, B, S, pos):
+        """The schedule's kernels in one native call, on one GPU; False where it has to run from here: with communication, another ops object,
+        blocks of both kinds."""
+        if type(self.comm) is not NoComm or not hasattr(self.ops, "run_layers") or self.model.norm.weight is None:
+            return False
+        m, family = self.model, self.family
+        mixed = getattr(self.cfg, "ladder_layers", None)
+        if family == "ladder" and mixed is not None and len(set(mixed)) != self.cfg.n_layer:
+            return False
+        two = family == "ladder" and S == 1 and self.overlap_sublayers
+        weights, caches, reduces = [], [], [] if family == "desync" else None
+        for layer in m.layers:
+            sub = layer._modules
+            att = sub["attention"]._modules
+            cache = att["kv_cache"]
+            caches += (cache.k_cache, cache.v_cache)
+            if family == "parallel":
+                norm, w = sub["attention_norm"].weight, att["wqkv1"].weight
+                weights += (norm, w, att["wo"].weight, norm, (w, sub["attention"].qkv_rows), att["w2"].weight)
+                continue
+            mlp = sub["feed_forward"]._modules
+            weights += (sub["attention_norm"].weight, att["wqkv"].weight, att["wo"].weight, sub["ffn_norm"].weight, mlp["w1"].weight, mlp["w2"].weight)
+            if reduces is not None:
+                reduces += (int(layer.do_attention_all_reduce), int(layer.do_mlp_all_reduce))
+        main = torch.cuda.current_stream()
+        tensors = dict(rope_table=m.freqs_cis, input_pos=pos, final_norm=m.norm.weight, resid=self.resid, normed=self.normed, part_a=self.part_a,
+                       part_m=self.part_m, q=self.q, y=self.y, h=self.h)
+        if two:
+            tensors["normed_m"] = self.normed_m
+        sizes = dict(dtype=dtype_code(self.dtype), n_layer=len(m.layers), B=B, S=S, n_head=self.nh, n_kv=self.nkv, head_dim=self.hd, dim=self.d,
+                     inter=self.inter, pos_is_i64=int(pos.dtype == torch.int64), splits=self._splits, smax=caches[0].shape[2],
+                     table_rows=m.freqs_cis.shape[0])
+        schedule = {"dense": DENSE, "ladder": LADDER_TWO_STREAMS if two else LADDER, "parallel": PARALLEL, "desync": DESYNC}[family]
+        self.ops.run_layers(schedule, weights, caches, reduces, self._events if two else None, main.cuda_stream,
+                            self.side_stream.cuda_stream if two else None, sizes, self.cfg.norm_eps,
+                            dict(ws_qkv=self.ws_qkv, ws_wo=self.ws_wo, ws_ug=self.ws_ug, ws_w2=self.ws_w2, scratch=self.scratch), **tensors)
+        return True
 
     @torch.no_grad()
     def forward(self, idx, input_pos):

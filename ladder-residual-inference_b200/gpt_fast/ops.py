@@ -119,6 +119,37 @@ class CudaOps:
                                              smax, _C.stream_handle()))
 
 
+    # ---- all layers of a pass ------------------------------------------------------------------------
+    @staticmethod
+    def run_layers(schedule, weights, caches, reduces, events, main, side, sizes, eps, workspaces, **tensors):
+        """lri_llama_run: `weights` six a layer (attention norm, QKV, wo, MLP norm, w1, w2; (tensor, first row) for a slice), `caches` two a layer,
+        `sizes` the integers of lri_llama_pass, `workspaces` and `tensors` by its names."""
+        _C.require_cuda(*tensors.values(), *caches)
+        pointers = []
+        for i, w in enumerate(weights):
+            row = 0
+            if type(w) is tuple:
+                w, row = w
+            if not w.is_cuda:
+                _C.require_cuda(w)
+            pointers.append(w.data_ptr() + row * w.stride(0) * w.element_size() if row else w.data_ptr())
+            if i % 6 == 5:
+                at = i // 6 * 2
+                pointers += (caches[at].data_ptr(), caches[at + 1].data_ptr())
+        layers = (ctypes.c_void_p * len(pointers))(*pointers)
+        p = _C.LlamaPass(schedule=schedule, eps=float(eps), stream=main, side=side, layers=ctypes.cast(layers, ctypes.c_void_p), **sizes)
+        for k, t in tensors.items():
+            setattr(p, k, t.data_ptr())
+        for k, t in workspaces.items():
+            if t is not None:
+                setattr(p, k, t.data_ptr())
+                setattr(p, k + "_bytes", t.numel() * t.element_size())
+        flags = bytes(reduces) if reduces is not None else None
+        p.reduces = ctypes.cast(ctypes.c_char_p(flags), ctypes.c_void_p) if flags is not None else None
+        handles = (ctypes.c_void_p * len(events))(*[e.cuda_event for e in events]) if events is not None else None
+        p.events = ctypes.cast(handles, ctypes.c_void_p) if handles is not None else None
+        _C.check(_C.lib.lri_llama_run(ctypes.byref(p)))
+
     # ---- layers with an fp32 residual stream ---------------------------------------------------------
     @staticmethod
     def linear_f32(x, w, out, rows, workspace=None):
