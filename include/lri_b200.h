@@ -101,7 +101,8 @@ int lri_embedding(int dtype, const void* table, const void* idx, int idx_is_i64,
 /* ---- F5 / F7: linear layer y = x W^T (+ addend) ------------------------------------------
  * x [M, K], w [N, K], y [M, N].  addend (may be NULL) is added after y's own rounding and the
  * sum rounded again (the parallel block's `w2(...) + y`, gpt_fast/utils.py:385).  M <= 8 runs
- * the weight-streaming kernels (SIMT for one row, mma.sync for 2..8); larger M the tcgen05 GEMM.
+ * the weight-streaming kernels (SIMT for one row, mma.sync for 2..8; 2..8 rows of a large projection the stream-K kernel where
+ * the workspace has room for it); larger M the tcgen05 GEMM.
  * For 8 < M <= 64 a workspace of lri_linear_workspace_bytes(M, N) bytes (16-byte aligned) selects
  * the tcgen05 stream-K kernel: all SMs stream equal shares of the weight, fp32 partial tiles go
  * to the workspace and the CTA that completes a tile sums them and applies the addend.  With

@@ -288,7 +288,8 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 // Finishing kernel: grid (tile, group of tokens), one thread per token and output pair (PLAIN /
 // QKV: 4 tokens per CTA) or output (SWIGLU: 2 tokens per CTA).  Tiles that the GEMM kernel
 // completed itself are skipped; for the others the segments are summed in slot order and the
-// epilogue is applied.
+// epilogue is applied.  All segments are asked for before the first is added: one after the other they were a chain of up
+// to eight L2 round trips.
 template <int EPI>
 struct FinishShape {
   static constexpr int kTokens = EPI == EPI_SWIGLU || EPI == EPI_GLU ? 2 : 4;
@@ -310,11 +311,15 @@ __global__ void __launch_bounds__(256) streamk_finish_kernel(const StreamKParams
     const int c = threadIdx.x & 127;
     const int64_t j = static_cast<int64_t>(tile) * kBM + c;
     if (tok >= p.lin.m || j >= p.lin.n) return;
-    float up = 0.f, gate = 0.f;
-    for (int z = 0; z < nseg; ++z) {
-      up += tile_partial[z * kSlot + tok * kBM + c];
-      gate += tile_partial[z * kSlot + (BN + tok) * kBM + c];
+    float us[kMaxSplitK], gs[kMaxSplitK], up = 0.f, gate = 0.f;
+#pragma unroll
+    for (int z = 0; z < kMaxSplitK; ++z) {
+      us[z] = z < nseg ? tile_partial[z * kSlot + tok * kBM + c] : 0.f;
+      gs[z] = z < nseg ? tile_partial[z * kSlot + (BN + tok) * kBM + c] : 0.f;
     }
+#pragma unroll
+    for (int z = 0; z < kMaxSplitK; ++z)
+      if (z < nseg) up += us[z], gate += gs[z];
     static_cast<T*>(p.lin.y)[static_cast<int64_t>(tok) * p.lin.n + j] =
         EPI == EPI_GLU ? Num<T>::from_f(clamped_glu(gate, up, p.lin.ex.glu)) : swiglu_rounded<T>(rnd<T>(up), rnd<T>(gate));
     return;
@@ -323,28 +328,33 @@ __global__ void __launch_bounds__(256) streamk_finish_kernel(const StreamKParams
   const int c = 2 * (threadIdx.x & 63);
   const int64_t n = static_cast<int64_t>(tile) * kBM + c;
   if (tok >= p.lin.m || n >= p.lin.n) return;
+  float2 v[kMaxSplitK];
   float s0 = 0.f, s1 = 0.f;
-  for (int z = 0; z < nseg; ++z) {
-    const float2 v = *reinterpret_cast<const float2*>(tile_partial + z * kSlot + tok * kBM + c);
-    s0 += v.x;
-    s1 += v.y;
+#pragma unroll
+  for (int z = 0; z < kMaxSplitK; ++z)
+    v[z] = z < nseg ? *reinterpret_cast<const float2*>(tile_partial + z * kSlot + tok * kBM + c) : make_float2(0.f, 0.f);
+  if constexpr (EPI == EPI_QKV) {
+    const QkvPlace<T> place(p.lin, tok, static_cast<int>(n));
+#pragma unroll
+    for (int z = 0; z < kMaxSplitK; ++z)
+      if (z < nseg) s0 += v[z].x, s1 += v[z].y;
+    place.store(rnd<T>(s0), rnd<T>(s1));
+    return;
   }
+#pragma unroll
+  for (int z = 0; z < kMaxSplitK; ++z)
+    if (z < nseg) s0 += v[z].x, s1 += v[z].y;
   if (EPI == EPI_F32) {
     *reinterpret_cast<float2*>(static_cast<float*>(p.lin.y) + static_cast<int64_t>(tok) * p.lin.n + n) = make_float2(s0, s1);
     return;
   }
-  const float v0 = rnd<T>(s0), v1 = rnd<T>(s1);
-  if (EPI == EPI_PLAIN) {
-    float o0 = v0, o1 = v1;
-    if (p.lin.addend) {
-      const T* add = static_cast<const T*>(p.lin.addend) + static_cast<int64_t>(tok) * p.lin.n + n;
-      o0 = rnd<T>(v0 + Num<T>::to_f(add[0]));
-      o1 = rnd<T>(v1 + Num<T>::to_f(add[1]));
-    }
-    *reinterpret_cast<uint32_t*>(static_cast<T*>(p.lin.y) + static_cast<int64_t>(tok) * p.lin.n + n) = pack2<T>(o0, o1);
-  } else {
-    qkv_epilogue_pair<T>(p.lin, tok, n, v0, v1);
+  float o0 = rnd<T>(s0), o1 = rnd<T>(s1);
+  if (p.lin.addend) {
+    const T* add = static_cast<const T*>(p.lin.addend) + static_cast<int64_t>(tok) * p.lin.n + n;
+    o0 = rnd<T>(o0 + Num<T>::to_f(add[0]));
+    o1 = rnd<T>(o1 + Num<T>::to_f(add[1]));
   }
+  *reinterpret_cast<uint32_t*>(static_cast<T*>(p.lin.y) + static_cast<int64_t>(tok) * p.lin.n + n) = pack2<T>(o0, o1);
 }
 
 int tiles_of(int n) { return (n + kBM - 1) / kBM; }

@@ -57,41 +57,45 @@ struct LinearParams {
   ArgmaxArgs am;       // ARGMAX epilogue of the SIMT kernel: greedy choice instead of stored logits
 };
 
+// Where a pair of the projection's outputs goes, and how it is turned: apart from the values, so that the loads of position and
+// table can run beside those of the values.
+template <typename T>
+struct QkvPlace {
+  T* dst;  // NULL: outside the cache or the table
+  float c, s;
+  bool turned;
+  __device__ __forceinline__ QkvPlace(const LinearParams& p, int m, int n) : dst(nullptr), c(1.f), s(0.f), turned(false) {
+    const int hd = p.head_dim, nq = p.n_head * hd, nk = p.n_kv * hd;
+    const int b = m / p.S, row = m - b * p.S;
+    const int64_t pos = load_pos(p.input_pos, p.pos_is_i64, row);
+    const int64_t trow = p.table_gathered ? row : pos;
+    if (pos < 0 || pos >= p.smax || trow >= p.table_rows) return;
+    const int part = n < nq ? n : (n < nq + nk ? n - nq : n - nq - nk);
+    const int h = part / hd, e = part - h * hd;
+    const int64_t cache_row = (static_cast<int64_t>(b) * p.n_kv + h) * p.smax + pos;
+    if (n < nq)
+      dst = static_cast<T*>(p.q_out) + static_cast<int64_t>(m) * nq + n;
+    else
+      dst = static_cast<T*>(n < nq + nk ? p.k_cache : p.v_cache) + cache_row * hd + e;
+    turned = n < nq + nk;
+    if (turned) {
+      const T* cs = static_cast<const T*>(p.rope_table) + (trow * (hd >> 1) + (e >> 1)) * 2;
+      Num<T>::unpack2(*reinterpret_cast<const uint32_t*>(cs), c, s);
+    }
+  }
+  __device__ __forceinline__ void store(float v0, float v1) const {
+    if (!dst) return;
+    float o0 = v0, o1 = v1;
+    if (turned) rope_pair(v0, v1, c, s, o0, o1);
+    *reinterpret_cast<uint32_t*>(dst) = pack2<T>(o0, o1);
+  }
+};
 // Epilogue of the QKV projection for token row `m` and the adjacent output pair (n, n+1),
 // n even, values already rounded to T: rotate q / k pairs with the table row of the token's
 // position and scatter to q_out / k_cache / v_cache.
 template <typename T>
 __device__ __forceinline__ void qkv_epilogue_pair(const LinearParams& p, int64_t m, int64_t n, float v0, float v1) {
-  const int hd = p.head_dim;
-  const int64_t nq = static_cast<int64_t>(p.n_head) * hd;
-  const int64_t nk = static_cast<int64_t>(p.n_kv) * hd;
-  const int64_t b = m / p.S;
-  const int64_t s = m - b * p.S;
-  const int64_t pos = load_pos(p.input_pos, p.pos_is_i64, s);
-  const int64_t trow = p.table_gathered ? s : pos;
-  if (pos < 0 || pos >= p.smax || trow >= p.table_rows) return;
-  const T* table = static_cast<const T*>(p.rope_table);
-  if (n < nq + nk) {
-    const int64_t nn = n < nq ? n : n - nq;
-    const int e = static_cast<int>(nn % hd);
-    const T* cs = table + (trow * (hd >> 1) + (e >> 1)) * 2;
-    float o0, o1;
-    rope_pair(v0, v1, Num<T>::to_f(cs[0]), Num<T>::to_f(cs[1]), o0, o1);
-    T* dst;
-    if (n < nq) {
-      dst = static_cast<T*>(p.q_out) + m * nq + n;
-    } else {
-      const int64_t h = nn / hd;
-      dst = static_cast<T*>(p.k_cache) + ((b * p.n_kv + h) * p.smax + pos) * hd + e;
-    }
-    *reinterpret_cast<uint32_t*>(dst) = pack2<T>(o0, o1);
-  } else {
-    const int64_t nn = n - nq - nk;
-    const int64_t h = nn / hd;
-    const int e = static_cast<int>(nn % hd);
-    T* dst = static_cast<T*>(p.v_cache) + ((b * p.n_kv + h) * p.smax + pos) * hd + e;
-    *reinterpret_cast<uint32_t*>(dst) = pack2<T>(v0, v1);
-  }
+  QkvPlace<T>(p, static_cast<int>(m), static_cast<int>(n)).store(v0, v1);
 }
 
 // decode path, 1 <= p.m <= 8 (SIMT FMA)

@@ -52,3 +52,27 @@ def test_gated(dtype, rows, n, k, with_workspace):
     ops.gateup_glu(x, w, h, rows, (1.702, 7.0, 1.0), workspace=ws)
     g = g.clamp(max=7.0)
     assert _rel(h, g * torch.sigmoid(1.702 * g) * (u.clamp(-7, 7) + 1)) < 3 * TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", list(TOL))
+@pytest.mark.parametrize("B,pos", [(2, 0), (8, 37), (16, 62), (40, 63)])
+@pytest.mark.parametrize("k", [4096, 4088])
+def test_qkv(dtype, B, pos, k):
+    """Rotation and cache rows behind stream-K products (4096: from 2 rows on) and streaming ones, at the cache's first and last position."""
+    from gpt_fast.ops import CudaOps as ops
+    nh, nkv, hd, smax = 32, 8, 128, 64
+    x, w = _randn(B, k, dtype=dtype), (_randn((nh + 2 * nkv) * hd, k, dtype=dtype) * k ** -0.5).to(dtype)
+    ang = torch.outer(torch.arange(smax, device="cuda").double(), 1e4 ** (-torch.arange(0, hd, 2, device="cuda").double() / hd))
+    table = torch.stack([ang.cos(), ang.sin()], dim=-1).to(dtype).contiguous()
+    q, kc, vc = (torch.zeros(*s, dtype=dtype, device="cuda") for s in ((B, nh, hd), (B, nkv, smax, hd), (B, nkv, smax, hd)))
+    ws = torch.empty(ops.qkv_workspace_bytes(64, nh, nkv, hd), dtype=torch.uint8, device="cuda")
+    ops.qkv_rope_kvcache(x, w, table, False, torch.tensor([pos], device="cuda"), q, kc, vc, B, 1, nh, nkv, hd, ws)
+    y = (x.double() @ w.double().T).view(B, nh + 2 * nkv, hd)
+    c, s = table[pos].double().unbind(-1)
+    a, b = y[..., 0::2], y[..., 1::2]
+    turned = torch.stack([a * c - b * s, b * c + a * s], dim=-1).flatten(-2)
+    # rounded after the product and after the rotation
+    assert _rel(q, turned[:, :nh]) < 2 * TOL[dtype] and _rel(kc[:, :, pos], turned[:, nh:nh + nkv]) < 2 * TOL[dtype]
+    assert _rel(vc[:, :, pos], y[:, nh + nkv:]) < TOL[dtype]
+    others = [p for p in range(smax) if p != pos]
+    assert not kc[:, :, others].any() and not vc[:, :, others].any()
