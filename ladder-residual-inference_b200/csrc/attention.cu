@@ -518,8 +518,8 @@ int launch_prefill(const PrefillParams& p, int B, cudaStream_t st) {
 }
 
 // Which decode kernel: the stream on tensor cores for many (sequence, KV head) pairs, the latency kernels below that.  Where query heads
-// share a KV head (us a layer, 4 of 128 elements, context 1025, latency kernel / stream): 8 pairs 7.6 / 6.7, but beside the MLP
-// of a ladder block the other's smaller CTAs are the better neighbours; 16 pairs 9.1 / 7.5, 32 11.6 / 9.0, 64 14.3 / 10.2, 128 23.7 / 15.3.
+// share a KV head (us a layer, 4 of 128 elements, context 1025, latency kernel / stream): 8 pairs 7.6 / 6.7 (alone; a single
+// sequence keeps the kernel that was tuned beside the MLP of a ladder block), 16 pairs 9.1 / 7.5, 32 11.6 / 9.0, 64 14.3 / 10.2, 128 23.7 / 15.3.
 // With one query head each (24 heads, 128 elements): 72 pairs 12.1 / 11.8, 192 24.2 / 20.6, but 144 pairs of 64 elements at 300 positions 5.1 / 6.6.
 // LRI_ATTN_MMA=1 / 0 forces / forbids the stream.
 constexpr int64_t kStreamPairs = 128;  // from here on callers are asked for scratch memory
