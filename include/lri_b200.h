@@ -35,6 +35,10 @@ typedef void* lri_stream_t; /* a cudaStream_t */
 
 /* LRI_FP32 is taken by the entry points that say so (every product and sum a true 32-bit operation). */
 enum lri_dtype { LRI_BF16 = 0, LRI_FP16 = 1, LRI_FP32 = 2 };
+/* Added to `dtype` of lri_linear, lri_linear_f32 or lri_gateup_glu: a prompt projection (more than 128 token rows) stays on the kernel
+ * that gives a tile to one SM.  For passes that run kernels of theirs on a second stream beside their projections (see
+ * csrc/gemm_pair.cu). */
+enum { LRI_ONE_SM = 0x100 };
 
 enum lri_status {
   LRI_OK = 0,

@@ -9,8 +9,8 @@
 // tile to the next; tcgen05.commit releases a stage.  Two accumulator buffers in TMEM let the
 // epilogue of one tile overlap the main loop of the next.
 //
-// More than 128 rows go to the kernel on pairs of SMs (gemm_pair.cu); this one runs 65..128 rows, expert tiles and, where there is
-// no workspace for the stream-K kernel, fewer.
+// More than 128 rows go to the kernel on pairs of SMs (gemm_pair.cu); this one runs 65..128 rows, expert tiles, calls with LRI_ONE_SM
+// and, where there is no workspace for the stream-K kernel, fewer.
 // The 128-row operand of the instruction is the activation tile for prefill-sized m; for
 // m <= 64 the operands are swapped (weights take the 128 rows, tokens the N side) so that
 // small decode batches do not waste seven eighths of the tensor-core tile.
@@ -322,11 +322,11 @@ int launch_tile(int dtype, const void* a, const void* w, void* c, int64_t m, int
 }
 
 template <typename T>
-int launch_typed(int dtype, const void* a, const void* w, void* c, int64_t m, int n, int k, cudaStream_t st) {
+int launch_typed(int dtype, const void* a, const void* w, void* c, int64_t m, int n, int k, bool one_sm, cudaStream_t st) {
   if (m <= 16) return launch_tile<T, 16, true>(dtype, a, w, c, m, n, k, st);
   if (m <= 32) return launch_tile<T, 32, true>(dtype, a, w, c, m, n, k, st);
   if (m <= 64) return launch_tile<T, 64, true>(dtype, a, w, c, m, n, k, st);
-  if (const int bn = gemm_pair_bn(m, n)) {
+  if (const int bn = one_sm ? 0 : gemm_pair_bn(m, n)) {
     LinearParams p{};
     p.x = a, p.w = w, p.y = c, p.n = n, p.k = k;
     return gemm_pair_launch(dtype, EPI_PLAIN, p, m, n, bn, st);
@@ -342,13 +342,13 @@ int launch_typed(int dtype, const void* a, const void* w, void* c, int64_t m, in
 }
 
 template <typename T>
-int launch_f32(int dtype, const void* a, const void* w, float* c, int64_t m, int n, int k, cudaStream_t st) {
+int launch_f32(int dtype, const void* a, const void* w, float* c, int64_t m, int n, int k, bool one_sm, cudaStream_t st) {
   LinearParams p{};
   p.y = c;
   if (m <= 16) return launch_tile<T, 16, true, EPI_F32>(dtype, a, w, nullptr, m, n, k, st, &p);
   if (m <= 32) return launch_tile<T, 32, true, EPI_F32>(dtype, a, w, nullptr, m, n, k, st, &p);
   if (m <= 64) return launch_tile<T, 64, true, EPI_F32>(dtype, a, w, nullptr, m, n, k, st, &p);
-  if (const int bn = gemm_pair_bn(m, n)) {
+  if (const int bn = one_sm ? 0 : gemm_pair_bn(m, n)) {
     p.x = a, p.w = w, p.n = n, p.k = k;
     return gemm_pair_launch(dtype, EPI_F32, p, m, n, bn, st);
   }
@@ -378,7 +378,7 @@ template <typename T, int EPI>
 int launch_fused(int dtype, const LinearParams& p, int64_t m, cudaStream_t st) {
   constexpr bool kGlu = EPI == EPI_SWIGLU || EPI == EPI_GLU;
   const int n_rows = kGlu ? 2 * p.n : p.n;       // rows of the weight
-  if (const int bn = gemm_pair_bn(m, n_rows)) return gemm_pair_launch(dtype, EPI, p, m, n_rows, bn, st);
+  if (const int bn = p.one_sm ? 0 : gemm_pair_bn(m, n_rows)) return gemm_pair_launch(dtype, EPI, p, m, n_rows, bn, st);
   const int64_t mt = (m + kBM - 1) / kBM;
   const int w256 = kGlu ? 128 : 256, w128 = kGlu ? 64 : 128;  // outputs per Q tile
   const int64_t t256 = mt * ((p.n + w256 - 1) / w256), t128 = mt * ((p.n + w128 - 1) / w128);
@@ -418,9 +418,9 @@ bool gemm_tcgen05_supports(int64_t m, int n, int k) {
   return m >= 1 && m < (1ll << 31) && n >= 8 && n % 8 == 0 && k >= 8 && k % 8 == 0;
 }
 
-int gemm_tcgen05_f32_launch(int dtype, const void* a, const void* w, float* c, int64_t m, int n, int k, cudaStream_t st) {
-  return dtype == LRI_BF16 ? launch_f32<__nv_bfloat16>(dtype, a, w, c, m, n, k, st)
-                           : launch_f32<__half>(dtype, a, w, c, m, n, k, st);
+int gemm_tcgen05_f32_launch(int dtype, const void* a, const void* w, float* c, int64_t m, int n, int k, bool one_sm, cudaStream_t st) {
+  return dtype == LRI_BF16 ? launch_f32<__nv_bfloat16>(dtype, a, w, c, m, n, k, one_sm, st)
+                           : launch_f32<__half>(dtype, a, w, c, m, n, k, one_sm, st);
 }
 
 bool gemm_tcgen05_experts_supports(int epi, const LinearParams& p) {
@@ -438,9 +438,9 @@ int gemm_tcgen05_experts_launch(int dtype, int epi, const LinearParams& p, int m
                            : launch_experts<__half, EPI_PLAIN>(dtype, p, max_tiles, st);
 }
 
-int gemm_tcgen05_launch(int dtype, const void* a, const void* w, void* c, int64_t m, int n, int k, cudaStream_t st) {
-  return dtype == LRI_BF16 ? launch_typed<__nv_bfloat16>(dtype, a, w, c, m, n, k, st)
-                           : launch_typed<__half>(dtype, a, w, c, m, n, k, st);
+int gemm_tcgen05_launch(int dtype, const void* a, const void* w, void* c, int64_t m, int n, int k, bool one_sm, cudaStream_t st) {
+  return dtype == LRI_BF16 ? launch_typed<__nv_bfloat16>(dtype, a, w, c, m, n, k, one_sm, st)
+                           : launch_typed<__half>(dtype, a, w, c, m, n, k, one_sm, st);
 }
 
 int gemm_tcgen05_status_read_and_clear(int* status_out) {

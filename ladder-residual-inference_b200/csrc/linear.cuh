@@ -54,6 +54,7 @@ struct LinearParams {
   int table_gathered;  // rope_table row s belongs to token s (rows already gathered by position)
   PushArgs push;       // PLAIN epilogue of the SIMT kernel only
   ExpertArgs ex;       // expert weights chosen on the device
+  bool one_sm;         // prompt projections: not the kernel on pairs of SMs (LRI_ONE_SM)
   ArgmaxArgs am;       // ARGMAX epilogue of the SIMT kernel: greedy choice instead of stored logits
 };
 
@@ -126,10 +127,10 @@ int gemm_tcgen05_experts_launch(int dtype, int epi, const LinearParams& p, int m
 int gemm_pair_bn(int64_t m, int64_t cols);
 int gemm_pair_launch(int dtype, int epi, const LinearParams& p, int64_t m, int n_rows, int bn, cudaStream_t st);
 // fp32 output of the plain tcgen05 GEMM
-int gemm_tcgen05_f32_launch(int dtype, const void* a, const void* w, float* c, int64_t m, int n, int k, cudaStream_t st);
+int gemm_tcgen05_f32_launch(int dtype, const void* a, const void* w, float* c, int64_t m, int n, int k, bool one_sm, cudaStream_t st);
 
 // C[m, n] = A[m, k] * W[n, k]^T, C in `dtype`, any m.  backend: lri_gemm_backend.
-int gemm_launch(int dtype, const void* a, const void* w, void* c, int64_t m, int n, int k, cudaStream_t st);
+int gemm_launch(int dtype, const void* a, const void* w, void* c, int64_t m, int n, int k, cudaStream_t st, bool one_sm = false);
 
 // Small-batch decode above the streaming kernels (up to kSplitKMaxRows token rows): a tcgen05
 // stream-K GEMM with the weights as the 128-row operand, fp32 partial tiles in a workspace and

@@ -13,7 +13,7 @@
 namespace lri {
 
 bool gemm_tcgen05_supports(int64_t m, int n, int k);
-int gemm_tcgen05_launch(int dtype, const void* a, const void* w, void* c, int64_t m, int n, int k, cudaStream_t st);
+int gemm_tcgen05_launch(int dtype, const void* a, const void* w, void* c, int64_t m, int n, int k, bool one_sm, cudaStream_t st);
 int gemm_tcgen05_status_read_and_clear(int* status_out);
 int gemm_pair_status_read_and_clear(int* status_out);
 int attn_prefill_tc_status_read_and_clear(int* status_out);
@@ -248,12 +248,12 @@ unsigned blocks_for(int64_t items, int threads) { return static_cast<unsigned>((
 
 }  // namespace
 
-int gemm_launch(int dtype, const void* a, const void* w, void* c, int64_t m, int n, int k, cudaStream_t st) {
+int gemm_launch(int dtype, const void* a, const void* w, void* c, int64_t m, int n, int k, cudaStream_t st, bool one_sm) {
   const int backend = current_gemm_backend();
   const bool tc_ok = gemm_tcgen05_supports(m, n, k) && aligned16(a) && aligned16(w) && aligned16(c);
   if (backend == LRI_GEMM_TCGEN05 && !tc_ok)
     return fail(LRI_ERR_UNSUPPORTED, "gemm: tcgen05 back end needs n %% 8 == 0, k %% 8 == 0 and 16-byte aligned pointers");
-  if (backend != LRI_GEMM_SIMT && tc_ok) return gemm_tcgen05_launch(dtype, a, w, c, m, n, k, st);
+  if (backend != LRI_GEMM_SIMT && tc_ok) return gemm_tcgen05_launch(dtype, a, w, c, m, n, k, one_sm, st);
   return dtype == LRI_BF16 ? launch_simt<__nv_bfloat16>(a, w, c, m, n, k, st)
                            : launch_simt<__half>(a, w, c, m, n, k, st);
 }
@@ -377,6 +377,13 @@ extern "C" int lri_gemm_status(void) {
   return LRI_OK;
 }
 
+// takes LRI_ONE_SM out of `dtype`
+static bool take_one_sm(int& dtype) {
+  const bool one_sm = dtype >= 0 && (dtype & LRI_ONE_SM) != 0;
+  if (one_sm) dtype &= ~LRI_ONE_SM;
+  return one_sm;
+}
+
 static int check_common(const char* who, int dtype, const void* x, const void* w, int64_t M, int K) {
   LRI_REQUIRE(dtype == LRI_BF16 || dtype == LRI_FP16, LRI_ERR_UNSUPPORTED, "%s: dtype %d", who, dtype);
   LRI_REQUIRE(x && w, LRI_ERR_ARG, "%s: NULL input", who);
@@ -388,6 +395,7 @@ static int check_common(const char* who, int dtype, const void* x, const void* w
 
 extern "C" int lri_linear(int dtype, const void* x, const void* w, const void* addend, void* y, int64_t M, int N,
                           int K, void* workspace, size_t workspace_bytes, lri_stream_t stream) {
+  const bool one_sm = take_one_sm(dtype);
   if (dtype == LRI_FP32 || (K > 0 && K % 8 != 0)) {
     LRI_REQUIRE(dtype >= LRI_BF16 && dtype <= LRI_FP32, LRI_ERR_UNSUPPORTED, "linear: dtype %d", dtype);
     LRI_REQUIRE(x && w && y, LRI_ERR_ARG, "linear: NULL pointer");
@@ -417,7 +425,7 @@ extern "C" int lri_linear(int dtype, const void* x, const void* w, const void* a
     p.x = x, p.w = w, p.y = y, p.addend = addend, p.m = static_cast<int>(M), p.n = N, p.k = K;
     return streaming_launch(dtype, EPI_PLAIN, p, st, prefer_simt_gemv());
   }
-  rc = gemm_launch(dtype, x, w, y, M, N, K, st);
+  rc = gemm_launch(dtype, x, w, y, M, N, K, st, one_sm);
   if (rc != LRI_OK || addend == nullptr) return rc;
   LRI_REQUIRE((M * N) % 8 == 0 && aligned16(y) && aligned16(addend), LRI_ERR_ALIGN,
               "linear: addend path needs M*N %% 8 == 0 and 16-byte aligned y, addend");
@@ -430,6 +438,7 @@ extern "C" size_t lri_linear_f32_workspace_bytes(int64_t M, int N) {
 
 extern "C" int lri_linear_f32(int dtype, const void* x, const void* w, float* y, int64_t M, int N, int K, void* workspace,
                               size_t workspace_bytes, lri_stream_t stream) {
+  const bool one_sm = take_one_sm(dtype);
   LRI_REQUIRE(dtype >= LRI_BF16 && dtype <= LRI_FP32, LRI_ERR_UNSUPPORTED, "linear_f32: dtype %d", dtype);
   LRI_REQUIRE(x && w && y, LRI_ERR_ARG, "linear_f32: NULL pointer");
   LRI_REQUIRE(M >= 0 && M < (1ll << 31) && N > 0 && K > 0, LRI_ERR_ARG, "linear_f32: M=%lld N=%d K=%d", (long long)M, N, K);
@@ -445,7 +454,7 @@ extern "C" int lri_linear_f32(int dtype, const void* x, const void* w, float* y,
     return gemm_streamk_launch(dtype, EPI_F32, p, workspace, workspace_bytes, st);
   if (M <= kGemvMmaMaxRows) return streaming_launch(dtype, EPI_F32, p, st, prefer_simt_gemv());
   if (current_gemm_backend() != LRI_GEMM_SIMT && N % 8 == 0 && aligned16(y))
-    return gemm_tcgen05_f32_launch(dtype, x, w, y, M, N, K, st);
+    return gemm_tcgen05_f32_launch(dtype, x, w, y, M, N, K, one_sm, st);
   return gemm_generic_launch(dtype, x, w, nullptr, y, true, M, N, K, st);
 }
 
@@ -511,6 +520,7 @@ extern "C" size_t lri_gateup_glu_workspace_bytes(int dtype, int64_t M, int I, in
 
 extern "C" int lri_gateup_glu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K, float alpha,
                               float limit, float offset, void* workspace, size_t workspace_bytes, lri_stream_t stream) {
+  const bool one_sm = take_one_sm(dtype);
   LRI_REQUIRE(dtype >= LRI_BF16 && dtype <= LRI_FP32, LRI_ERR_UNSUPPORTED, "gateup_glu: dtype %d", dtype);
   LRI_REQUIRE(x && w1 && h, LRI_ERR_ARG, "gateup_glu: NULL pointer");
   LRI_REQUIRE(M >= 0 && M < (1ll << 31) && I > 0 && K > 0, LRI_ERR_ARG, "gateup_glu: M=%lld I=%d K=%d", (long long)M, I, K);
@@ -518,7 +528,7 @@ extern "C" int lri_gateup_glu(int dtype, const void* x, const void* w1, void* h,
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LinearParams p{};
   p.x = x, p.w = w1, p.y = h, p.m = static_cast<int>(M), p.n = I, p.k = K;
-  p.ex.glu = GluParams{alpha, limit, offset};
+  p.ex.glu = GluParams{alpha, limit, offset}, p.one_sm = one_sm;
   if (dtype != LRI_FP32 && K % 8 == 0 && aligned16(x) && aligned16(w1)) {
     if (M == 1) return gemv_launch(dtype, EPI_GLU, p, st);
     if (M <= streaming_rows() && !streamk_few_rows(EPI_GLU, p, workspace, workspace_bytes)) return gemv_mma_launch(dtype, EPI_GLU, p, st);
@@ -531,7 +541,7 @@ extern "C" int lri_gateup_glu(int dtype, const void* x, const void* w1, void* h,
   const size_t need = static_cast<size_t>(M) * 2 * static_cast<size_t>(I) * sizeof(float);
   LRI_REQUIRE(workspace && workspace_bytes >= need && aligned16(workspace), LRI_ERR_WORKSPACE,
               "gateup_glu: workspace of %zu bytes (16-byte aligned) required", need);
-  int rc = lri_linear_f32(dtype, x, w1, static_cast<float*>(workspace), M, 2 * I, K, nullptr, 0, stream);
+  int rc = lri_linear_f32(one_sm ? dtype | LRI_ONE_SM : dtype, x, w1, static_cast<float*>(workspace), M, 2 * I, K, nullptr, 0, stream);
   if (rc != LRI_OK) return rc;
   return glu_rows_launch(dtype, static_cast<const float*>(workspace), h, M, I, p.ex.glu, st);
 }

@@ -31,6 +31,7 @@ class LlamaPass(ctypes.Structure):
                 + [(k, c_void_p) for k in ("stream", "side", "events")])
 
 
+ONE_SM = 0x100  # LRI_ONE_SM
 DENSE, LADDER, LADDER_TWO_STREAMS, PARALLEL, DESYNC = range(5)
 
 # name -> (restype, argtypes); the order of arguments is that of include/lri_b200.h

@@ -21,6 +21,7 @@ import torch.distributed as dist
 
 from .engine import Engine
 from .mixers import LatentAttention, StreamBranch, _offsets
+from .ops import CudaOps, OneSmOps
 
 
 class LayerEngine(Engine):
@@ -29,7 +30,6 @@ class LayerEngine(Engine):
         self.d, self.dtype = cfg.dim, dtype
         self.max_batch, self.max_seq = max_batch, max_seq
         rows = self.max_rows = max_batch * max_seq
-        ops = self.ops
 
         def buf(n, cols, dt=dtype):
             return torch.empty(n, cols, dtype=dt, device=device)
@@ -40,6 +40,12 @@ class LayerEngine(Engine):
 
         def of(kind):
             return [m for m in subs if m.kind == kind]
+
+        if of("chunked_attention") and self.ops is CudaOps:
+            # Designs with side-by-side mixers run a tensor-memory kernel on a second stream.  Prompt passes of theirs that followed one
+            # another without a wait stopped for good once their projections ran on pairs of SMs; they never did on single SMs.
+            self.ops = OneSmOps
+        ops = self.ops
 
         def most(ms, f):
             return max((f(m) for m in ms), default=0)
@@ -115,7 +121,7 @@ class LayerEngine(Engine):
                 self.moe_packed = buf(128 * tiles, self.d)
                 self.moe_scale = torch.zeros(128 * tiles, dtype=torch.float32, device=device)
         self.side_stream = None
-        if of("chunked_attention") and self.comm.world == 1 and self.resid.is_cuda and os.environ.get("LRI_SIDE_STREAM", "1") != "0":
+        if of("chunked_attention") and self.comm.world == 1 and self.ops is OneSmOps and self.resid.is_cuda and os.environ.get("LRI_SIDE_STREAM", "1") != "0":
             self.side_stream = torch.cuda.Stream()
             self._fork, self._join_event = torch.cuda.Event(), torch.cuda.Event()
         self._setup_head(max_batch, device, dtype)

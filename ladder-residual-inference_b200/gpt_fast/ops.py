@@ -5,6 +5,7 @@ tensors and raises otherwise.  The engine takes the ops object as a parameter so
 schedule logic can be exercised by tests with a stand-in.
 """
 import ctypes
+from functools import partial
 
 import torch
 
@@ -36,11 +37,12 @@ class CudaOps:
 
     # ---- linear family -----------------------------------------------------------------------
     @staticmethod
-    def linear(x, w, out, rows, addend=None, workspace=None):
+    def linear(x, w, out, rows, addend=None, workspace=None, flags=0):
+        """flags: 0 or _C.ONE_SM."""
         _C.require_cuda(x, w, out)
         n, k = w.shape
         ws_ptr, ws_bytes = (workspace.data_ptr(), workspace.numel() * workspace.element_size()) if workspace is not None else (None, 0)
-        _C.check(_C.lib.lri_linear(_C.dtype_code_any(x.dtype), x.data_ptr(), w.data_ptr(), _C.ptr(addend), out.data_ptr(),
+        _C.check(_C.lib.lri_linear(_C.dtype_code_any(x.dtype) | flags, x.data_ptr(), w.data_ptr(), _C.ptr(addend), out.data_ptr(),
                                    rows, n, k, ws_ptr, ws_bytes, _C.stream_handle()))
 
     @staticmethod
@@ -152,12 +154,12 @@ class CudaOps:
 
     # ---- layers with an fp32 residual stream ---------------------------------------------------------
     @staticmethod
-    def linear_f32(x, w, out, rows, workspace=None):
+    def linear_f32(x, w, out, rows, workspace=None, flags=0):
         """out (fp32) = x w^T, unrounded."""
         _C.require_cuda(x, w, out)
         n, k = w.shape
         ws_ptr, ws_bytes = (workspace.data_ptr(), workspace.numel() * workspace.element_size()) if workspace is not None else (None, 0)
-        _C.check(_C.lib.lri_linear_f32(_C.dtype_code_any(x.dtype), x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, n, k,
+        _C.check(_C.lib.lri_linear_f32(_C.dtype_code_any(x.dtype) | flags, x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, n, k,
                                        ws_ptr, ws_bytes, _C.stream_handle()))
 
     @staticmethod
@@ -318,12 +320,12 @@ class CudaOps:
         return _C.lib.lri_gateup_glu_workspace_bytes(_C.dtype_code_any(dtype), rows, inter, k)
 
     @staticmethod
-    def gateup_glu(x, w1, h, rows, glu, workspace=None):
+    def gateup_glu(x, w1, h, rows, glu, workspace=None, flags=0):
         """w1 [2 ff, dim] = [up | gate]; glu = (alpha, limit, offset)."""
         _C.require_cuda(x, w1, h)
         two_i, k = w1.shape
         ws_ptr, ws_bytes = (workspace.data_ptr(), workspace.numel() * workspace.element_size()) if workspace is not None else (None, 0)
-        _C.check(_C.lib.lri_gateup_glu(_C.dtype_code_any(x.dtype), x.data_ptr(), w1.data_ptr(), h.data_ptr(), rows, two_i // 2, k,
+        _C.check(_C.lib.lri_gateup_glu(_C.dtype_code_any(x.dtype) | flags, x.data_ptr(), w1.data_ptr(), h.data_ptr(), rows, two_i // 2, k,
                                        *[float(g) for g in glu], ws_ptr, ws_bytes, _C.stream_handle()))
 
     # ---- grouped attention on a cache ------------------------------------------------------------------------
@@ -430,6 +432,13 @@ class CudaOps:
     def round_columns(x, ld, off, n, y, rows):
         _C.require_cuda(x, y)
         _C.check(_C.lib.lri_round_columns(_C.dtype_code_any(y.dtype), x.data_ptr(), ld, off, n, y.data_ptr(), rows, _C.stream_handle()))
+
+
+class OneSmOps(CudaOps):
+    """CudaOps whose prompt projections stay on the kernel that gives a tile to one SM (LRI_ONE_SM)."""
+    linear = staticmethod(partial(CudaOps.linear, flags=_C.ONE_SM))
+    linear_f32 = staticmethod(partial(CudaOps.linear_f32, flags=_C.ONE_SM))
+    gateup_glu = staticmethod(partial(CudaOps.gateup_glu, flags=_C.ONE_SM))
 
 
 def decode_splits(B, n_head, n_kv, smax, head_dim=128):
