@@ -13,8 +13,15 @@
 // Roles per CTA: warp 0 fetches (TMA, no multicast), warp 1 owns the tensor memory and, in the first CTA, issues the products,
 // warps 2-5 store.  The first CTA's `full` barriers count the bytes of both CTAs' copies; commits free a stage, and hand over
 // an accumulator, in both CTAs at once; the stores of both CTAs hand the accumulator back to the first.
-// Every wait on an mbarrier is bounded (device status word, see lri_gemm_status); the cluster barrier at the end is reached by
-// both CTAs in every case, because no other wait is unbounded.
+// Every wait on an mbarrier is bounded (device status word, see lri_gemm_status).  Not bounded are the allocation of tensor memory, the
+// cluster barriers and the wait for the preceding kernel.  The allocation is one operation of both CTAs, so each first waits until
+// the other runs, and it finds the tensor memory of its SMs free: no tensor-memory kernel of this library fits on an SM beside
+// kOwnSmem.  The barriers are reached by both CTAs in every case.
+//
+// Beside a tensor-memory kernel of another stream: prompt passes that ran the prompt attention of latent_attention_tc.cu on a second
+// stream while products of one K step ran here stopped for good (the form that allocated before the other CTA was known to run).
+// Whether that was the cause is not known, and the engines do not bring the two together: designs with side-by-side mixers
+// ask for single SMs (LRI_ONE_SM).  Option gemm_pair = 0 does the same for a program that runs passes on several streams at a time.
 #include "gemm_tile.cuh"
 
 namespace lri {
@@ -29,6 +36,7 @@ constexpr int kTile = kBM * kBK * 2;    // bytes of 128 operand rows
 constexpr int kAccCols = 256;           // TMEM columns of one of the two accumulators
 constexpr int kMaxBn = 256;
 constexpr int kSmemLimit = 226 * 1024;  // of the 227 KB of an SM; the barriers take the rest
+constexpr int kOwnSmem = 181 * 1024;    // the smallest other tensor-memory kernel (prompt attention, heads of 64) takes 49 KB
 
 __device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {
   uint32_t r;
@@ -87,6 +95,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const uint32_t acc_full0 = smem_u32(&bars[2 * kMaxStages]);       // products -> stores, one per accumulator
   const uint32_t acc_empty0 = smem_u32(&bars[2 * kMaxStages + 2]);  // stores -> products (first CTA)
 
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (uint32_t s = 0; s < stages; ++s) {
@@ -100,6 +109,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // the other CTA runs
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
                  "r"(2 * kAccCols)
@@ -253,7 +264,8 @@ int launch(int dtype, const LinearParams& lin, int64_t m, int n_rows, int bn, cu
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(2 * clusters));
   cfg.blockDim = dim3(kGemmThreads);
-  cfg.dynamicSmemBytes = static_cast<size_t>(stages) * stage_bytes + 1024;
+  const int smem = stages * stage_bytes + 1024;
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem > kOwnSmem ? smem : kOwnSmem);
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
