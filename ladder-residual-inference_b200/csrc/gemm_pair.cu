@@ -297,11 +297,17 @@ int launch_epi(int dtype, int epi, const LinearParams& lin, int64_t m, int n_row
 // The width: a step costs about bn + 64 columns' worth (337, 382, 436, 505, 563 cycles at 128 .. 256 by 32), so the narrower tile
 // wins where it fills the last round: 999 x 2048 x 8192 takes 29.4 us at 128 and 44.1 at 256, 2048 x 5120 x 2048 37.9 at 192 and 42.6 at
 // 256, 2048 x 28672 x 4096 363 at 224 and at 256 and 405 at 128.
-int gemm_pair_bn(int64_t m, int64_t cols) {
+// Short sums: a launch costs about a microsecond more here.  Wide tiles do not make up for it below a depth of 512 (us, one SM a tile / here:
+// 2048 x 4096 x 256 10.1 / 11.5, 4096 x 4096 x 384 19.6 / 21.5, 2048 x 4096 x 1024 17.6 / 16.9), narrow ones, which fill a last round, do
+// (1000 x 3072 x 256 8.3 / 7.7).  One or two K steps stay with one SM in any case (2048 x 4096 x 128 9.4 / 10.6, 1000 x 3072 x 128 7.5 / 7.1): they are
+// what ran when passes stopped, see the head of this file.
+constexpr int kMinDepth = 2 * kBK, kMinWideDepth = 512, kWide = 224;
+
+int gemm_pair_bn(int64_t m, int64_t cols, int k) {
   const int forced = option(OPT_GEMM_PAIR);
   if (forced == 0) return 0;
   if (forced > 1) return forced / 32 * 32;
-  if (m <= kBM) return 0;
+  if (m <= kBM || k <= kMinDepth) return 0;
   const int pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   int best = kMaxBn;
   int64_t cost = 0;
@@ -309,7 +315,7 @@ int gemm_pair_bn(int64_t m, int64_t cols) {
     const int64_t c = waves(m, cols, bn, pairs) * (bn + 64);
     if (bn == kMaxBn || c < cost) best = bn, cost = c;
   }
-  return best;
+  return best >= kWide && k < kMinWideDepth ? 0 : best;
 }
 
 // lin.x [m, k], lin.w [n_rows, k]; lin.n outputs where the epilogue counts them

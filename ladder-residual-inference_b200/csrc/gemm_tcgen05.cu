@@ -326,7 +326,7 @@ int launch_typed(int dtype, const void* a, const void* w, void* c, int64_t m, in
   if (m <= 16) return launch_tile<T, 16, true>(dtype, a, w, c, m, n, k, st);
   if (m <= 32) return launch_tile<T, 32, true>(dtype, a, w, c, m, n, k, st);
   if (m <= 64) return launch_tile<T, 64, true>(dtype, a, w, c, m, n, k, st);
-  if (const int bn = one_sm ? 0 : gemm_pair_bn(m, n)) {
+  if (const int bn = one_sm ? 0 : gemm_pair_bn(m, n, k)) {
     LinearParams p{};
     p.x = a, p.w = w, p.y = c, p.n = n, p.k = k;
     return gemm_pair_launch(dtype, EPI_PLAIN, p, m, n, bn, st);
@@ -348,7 +348,7 @@ int launch_f32(int dtype, const void* a, const void* w, float* c, int64_t m, int
   if (m <= 16) return launch_tile<T, 16, true, EPI_F32>(dtype, a, w, nullptr, m, n, k, st, &p);
   if (m <= 32) return launch_tile<T, 32, true, EPI_F32>(dtype, a, w, nullptr, m, n, k, st, &p);
   if (m <= 64) return launch_tile<T, 64, true, EPI_F32>(dtype, a, w, nullptr, m, n, k, st, &p);
-  if (const int bn = one_sm ? 0 : gemm_pair_bn(m, n)) {
+  if (const int bn = one_sm ? 0 : gemm_pair_bn(m, n, k)) {
     p.x = a, p.w = w, p.n = n, p.k = k;
     return gemm_pair_launch(dtype, EPI_F32, p, m, n, bn, st);
   }
@@ -378,7 +378,7 @@ template <typename T, int EPI>
 int launch_fused(int dtype, const LinearParams& p, int64_t m, cudaStream_t st) {
   constexpr bool kGlu = EPI == EPI_SWIGLU || EPI == EPI_GLU;
   const int n_rows = kGlu ? 2 * p.n : p.n;       // rows of the weight
-  if (const int bn = p.one_sm ? 0 : gemm_pair_bn(m, n_rows)) return gemm_pair_launch(dtype, EPI, p, m, n_rows, bn, st);
+  if (const int bn = p.one_sm ? 0 : gemm_pair_bn(m, n_rows, p.k)) return gemm_pair_launch(dtype, EPI, p, m, n_rows, bn, st);
   const int64_t mt = (m + kBM - 1) / kBM;
   const int w256 = kGlu ? 128 : 256, w128 = kGlu ? 64 : 128;  // outputs per Q tile
   const int64_t t256 = mt * ((p.n + w256 - 1) / w256), t128 = mt * ((p.n + w128 - 1) / w128);

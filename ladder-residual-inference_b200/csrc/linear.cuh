@@ -122,9 +122,9 @@ int gemm_generic_launch(int dtype, const void* x, const void* w, const void* add
 // of 128), p.n outputs (GLU: hidden size), p.ex.tiles set, max_tiles = upper bound of tiles[0].
 bool gemm_tcgen05_experts_supports(int epi, const LinearParams& p);
 int gemm_tcgen05_experts_launch(int dtype, int epi, const LinearParams& p, int max_tiles, cudaStream_t st);
-// tcgen05 GEMM on pairs of SMs (gemm_pair.cu): tile width it would take for m token rows and `cols` weight rows, 0 where the
+// tcgen05 GEMM on pairs of SMs (gemm_pair.cu): tile width it would take for m token rows and `cols` weight rows of depth k, 0 where the
 // single-CTA kernel is the better one; p.x, p.w [n_rows, k], p.y and what the epilogue needs are set
-int gemm_pair_bn(int64_t m, int64_t cols);
+int gemm_pair_bn(int64_t m, int64_t cols, int k);
 int gemm_pair_launch(int dtype, int epi, const LinearParams& p, int64_t m, int n_rows, int bn, cudaStream_t st);
 // fp32 output of the plain tcgen05 GEMM
 int gemm_tcgen05_f32_launch(int dtype, const void* a, const void* w, float* c, int64_t m, int n, int k, bool one_sm, cudaStream_t st);

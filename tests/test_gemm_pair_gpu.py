@@ -113,3 +113,25 @@ def test_option_values():
         assert C.lib.lri_set_option(b"gemm_pair", bad) == -1
     C.check(C.lib.lri_get_option(b"gemm_pair", ctypes.byref(v)))
     assert v.value == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,flag,pairs", [(128, 4096, 1024, False, False), (129, 4096, 1024, False, True), (129, 4096, 1024, True, False),
+                                              (300, 1024, 128, False, False), (300, 1024, 136, False, True), (2048, 4096, 504, False, False),
+                                              (2048, 4096, 512, False, True)])
+def test_which_products_take_pairs(m, n, k, flag, pairs):
+    """By rows, depth and width, and by what the caller says; either kernel gives the same products."""
+    from gpt_fast.ops import CudaOps as ops
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    x, w = (torch.randn(r, k, generator=g, device="cuda").bfloat16() for r in (m, n))
+    y, f, h = torch.empty(m, n, dtype=torch.bfloat16, device="cuda"), torch.empty(m, n, device="cuda"), torch.empty(m, n // 2, dtype=torch.bfloat16, device="cuda")
+    flags = _lib().ONE_SM if flag else 0
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        ops.linear(x, w, y, m, flags=flags)
+        ops.linear_f32(x, w, f, m, flags=flags)
+        ops.gateup_glu(x, w, h, m, (1.702, 1.2, 1.0), flags=flags)
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if "gemm" in e.name and e.device_type == torch.autograd.DeviceType.CUDA]
+    assert len(names) == 3 and all(("gemm_pair" in name) == pairs for name in names), names
+    _close(y, (x.double() @ w.double().T).float().cpu(), torch.bfloat16, k)
+    assert torch.equal(f.bfloat16(), y)
