@@ -174,6 +174,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_con
 #pragma unroll 1
       for (int cc = 0; cc < BN; cc += 32) {
         uint32_t r[32];
+        __syncwarp();  // the load is warp-collective, and rows past the end leave the stores early
         tmem_ld32(tacc + cc, r);  // BN == 16: only the first 16 columns are valid (32 are allocated)
         constexpr int kValid = BN < 32 ? BN : 32;
         const int64_t n = static_cast<int64_t>(w.tile_p) * kBM + i;
