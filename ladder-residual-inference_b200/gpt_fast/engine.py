@@ -187,35 +187,56 @@ class Engine:
 
     def _run_native(self, B, S, pos):
         """The schedule's kernels in one native call, on one GPU; False where it has to run from here: with communication, another ops object,
-        blocks of both kinds."""
+        blocks of both kinds, layers of unequal sizes."""
         if type(self.comm) is not NoComm or not hasattr(self.ops, "run_layers") or self.model.norm.weight is None:
             return False
         m, family = self.model, self.family
         mixed = getattr(self.cfg, "ladder_layers", None)
-        if family == "ladder" and mixed is not None and len(set(mixed)) != self.cfg.n_layer:
+        if family == "ladder" and mixed is not None and len(set(mixed)) != self.cfg.n_layer or len(m.layers) != self.cfg.n_layer:
             return False
         two = family == "ladder" and S == 1 and self.overlap_sublayers
+        # The call passes one set of sizes for all layers; the Python form reads each weight's.  A layer that was given others, or whose weights
+        # are not plain parameters, runs there.  (nn.Module's attribute access costs as much as a comparison of sizes: 100 to 150 ns.)
+        nqkv = (self.nh + 2 * self.nkv) * self.hd
+        want_qkv, want_wo, want_w1, want_w2 = (nqkv, self.d), (self.d, self.nh * self.hd), (2 * self.inter, self.d), (self.d, self.inter)
+        want_both = (nqkv + 2 * self.inter, self.d)
+        smax = None
         weights, caches, reduces = [], [], [] if family == "desync" else None
-        for layer in m.layers:
-            sub = layer._modules
-            att = sub["attention"]._modules
-            cache = att["kv_cache"]
-            caches += (cache.k_cache, cache.v_cache)
-            if family == "parallel":
-                norm, w = sub["attention_norm"].weight, att["wqkv1"].weight
-                weights += (norm, w, att["wo"].weight, norm, (w, sub["attention"].qkv_rows), att["w2"].weight)
-                continue
-            mlp = sub["feed_forward"]._modules
-            weights += (sub["attention_norm"].weight, att["wqkv"].weight, att["wo"].weight, sub["ffn_norm"].weight, mlp["w1"].weight, mlp["w2"].weight)
-            if reduces is not None:
-                reduces += (int(layer.do_attention_all_reduce), int(layer.do_mlp_all_reduce))
+        try:
+            for layer in m.layers:
+                sub = layer._modules
+                att = sub["attention"]._modules
+                cache = att["kv_cache"]._buffers
+                k_cache, wo = cache["k_cache"], att["wo"]._parameters["weight"]
+                length = k_cache.shape[2]
+                if smax is None:
+                    smax = length
+                if length != smax or wo.shape != want_wo:
+                    return False
+                caches += (k_cache, cache["v_cache"])
+                norm = sub["attention_norm"]._parameters["weight"]
+                if family == "parallel":
+                    w, w2 = att["wqkv1"]._parameters["weight"], att["w2"]._parameters["weight"]
+                    if w.shape != want_both or w2.shape != want_w2 or sub["attention"].qkv_rows != nqkv:
+                        return False
+                    weights += (norm, w, wo, norm, (w, nqkv), w2)
+                    continue
+                mlp = sub["feed_forward"]._modules
+                w, w1, w2 = att["wqkv"]._parameters["weight"], mlp["w1"]._parameters["weight"], mlp["w2"]._parameters["weight"]
+                if w.shape != want_qkv or w1.shape != want_w1 or w2.shape != want_w2:
+                    return False
+                weights += (norm, w, wo, sub["ffn_norm"]._parameters["weight"], w1, w2)
+                if reduces is not None:
+                    reduces += (int(layer.do_attention_all_reduce), int(layer.do_mlp_all_reduce))
+        except KeyError:
+            return False
         main = torch.cuda.current_stream()
         tensors = dict(rope_table=m.freqs_cis, input_pos=pos, final_norm=m.norm.weight, resid=self.resid, normed=self.normed, part_a=self.part_a,
                        part_m=self.part_m, q=self.q, y=self.y, h=self.h)
         if two:
             tensors["normed_m"] = self.normed_m
         sizes = dict(dtype=dtype_code(self.dtype), n_layer=len(m.layers), B=B, S=S, n_head=self.nh, n_kv=self.nkv, head_dim=self.hd, dim=self.d,
-                     inter=self.inter, pos_is_i64=int(pos.dtype == torch.int64), splits=self._splits, smax=caches[0].shape[2],
+                     inter=self.inter, pos_is_i64=int(pos.dtype == torch.int64), splits=self._splits, smax=smax,
                      table_rows=m.freqs_cis.shape[0])
         schedule = {"dense": DENSE, "ladder": LADDER_TWO_STREAMS if two else LADDER, "parallel": PARALLEL, "desync": DESYNC}[family]
         self.ops.run_layers(schedule, weights, caches, reduces, self._events if two else None, main.cuda_stream,

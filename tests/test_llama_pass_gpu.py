@@ -65,3 +65,28 @@ def test_weights_are_read_for_every_pass_and_errors_arrive():
         with pytest.raises(RuntimeError, match="CUDA"):
             model(tok, pos)
     torch.cuda.synchronize()
+
+
+def test_layers_of_unequal_sizes_run_as_before():
+    """A narrower feed-forward in one layer and a shorter cache in another: read at their own sizes."""
+    results = []
+    for native in (True, False):
+        model = _model("dense", torch.bfloat16, 2)
+        engine = model._engine
+        if not native:
+            engine._run_native = lambda *a: False
+        ff, cache = model.layers[1].feed_forward, model.layers[2].attention.kv_cache
+        up, gate = ff.w1.weight.detach().chunk(2)
+        ff.w1.weight = torch.nn.Parameter(torch.cat([up[:384], gate[:384]]))
+        ff.w2.weight = torch.nn.Parameter(ff.w2.weight.detach()[:, :384].contiguous())
+        cache.k_cache, cache.v_cache = cache.k_cache[:, :, :96].contiguous(), cache.v_cache[:, :, :96].contiguous()
+        ids = torch.randint(0, SHAPE["vocab_size"], (2, 80), generator=torch.Generator().manual_seed(2)).cuda()
+        out = []
+        with torch.no_grad():
+            out.append(model(ids, torch.arange(80, device="cuda")))
+            for i in range(3):
+                out.append(model(ids[:, i:i + 1].to(torch.int32), torch.tensor([80 + i], dtype=torch.int32, device="cuda")))
+        results.append(out)
+    torch.cuda.synchronize()
+    for a, b in zip(*results):
+        assert torch.isfinite(a.float()).all() and torch.equal(a, b)
