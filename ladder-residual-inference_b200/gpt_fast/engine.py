@@ -28,7 +28,7 @@ import torch
 
 from ._C import DENSE, DESYNC, LADDER, LADDER_TWO_STREAMS, PARALLEL, dtype_code
 from .comm import NoComm, make_comm
-from .ops import decode_splits
+from .ops import CudaOps, decode_splits
 
 _MAX_SPLITS = 64
 
@@ -38,10 +38,7 @@ class Engine:
         self.model = model
         self.family = family
         self.cfg = model.config
-        if ops is None:
-            from .ops import CudaOps
-            ops = CudaOps
-        self.ops = ops
+        self.ops = ops if ops is not None else CudaOps
         self.comm = comm if comm is not None else make_comm()
         self.ready = False
         self._norm_pushes = False  # set per step by _reduce_plan
@@ -188,7 +185,7 @@ class Engine:
     def _run_native(self, B, S, pos):
         """The schedule's kernels in one native call, on one GPU; False where it has to run from here: with communication, another ops object,
         blocks of both kinds, layers of unequal sizes."""
-        if type(self.comm) is not NoComm or not hasattr(self.ops, "run_layers") or self.model.norm.weight is None:
+        if type(self.comm) is not NoComm or self.ops is not CudaOps or self.model.norm.weight is None:
             return False
         m, family = self.model, self.family
         mixed = getattr(self.cfg, "ladder_layers", None)

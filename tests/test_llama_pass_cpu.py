@@ -80,3 +80,15 @@ def test_another_number_of_layers_stays_in_python(family, monkeypatch):
     engine._splits = 1
     model.layers = model.layers[:2]
     assert engine._run_native(1, 1, torch.zeros(1, dtype=torch.int32)) is False
+
+
+def test_ops_of_the_callers_own_are_called(monkeypatch):
+    """An ops object derived from the package's own may replace any of its calls: it is not passed by."""
+    from gpt_fast.ops import CudaOps
+
+    class Own(CudaOps):
+        pass
+
+    engine = _model("dense", monkeypatch)._engine
+    engine._splits, engine.ops = 1, Own
+    assert engine._run_native(1, 1, torch.zeros(1, dtype=torch.int32)) is False
