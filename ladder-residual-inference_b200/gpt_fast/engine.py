@@ -189,7 +189,7 @@ class Engine:
             return False
         m, family = self.model, self.family
         mixed = getattr(self.cfg, "ladder_layers", None)
-        if family == "ladder" and mixed is not None and len(set(mixed)) != self.cfg.n_layer or len(m.layers) != self.cfg.n_layer:
+        if family == "ladder" and mixed is not None and len(set(mixed)) != self.cfg.n_layer or not 0 < len(m.layers) == self.cfg.n_layer:
             return False
         two = family == "ladder" and S == 1 and self.overlap_sublayers
         # The call passes one set of sizes for all layers; the Python form reads each weight's.  A layer that was given others, or whose weights
