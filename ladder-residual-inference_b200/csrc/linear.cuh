@@ -99,6 +99,7 @@ __device__ __forceinline__ void qkv_epilogue_pair(const LinearParams& p, int64_t
   QkvPlace<T>(p, static_cast<int>(m), static_cast<int>(n)).store(v0, v1);
 }
 
+int streaming_rows();  // token rows up to which the streaming kernels run (option stream_rows)
 // decode path, 1 <= p.m <= 8 (SIMT FMA)
 int gemv_launch(int dtype, int epi, const LinearParams& p, cudaStream_t st);
 // decode path, 1 <= p.m <= 16 (same streaming, tensor-core FMA)

@@ -270,12 +270,11 @@ static size_t streamk_bytes(int epi, int64_t M, int64_t n) {
 // weights by then, but costs a second launch.  Measured on B200, streaming / stream-K, a whole decode step of 4 sequences: 8B (k 4096 and
 // 14336, all projections from 33 MB on) 4399 / 3265 us dense, 3516 / 2811 ladder; Migosun 8B 5051 / 4053.  One projection alone: gated
 // 16384 x 2048 (67 MB) 19.0 / 15.1 us, 16384 x 3072 25.6 / 21.2, 2048 x 8192 (34 MB) 13.0 / 10.4, 3072 x 8192 14.5 / 12.8; but 9216 x 3072 11.0 / 13.7,
-// 8192 x 2048 7.3 / 9.6, 2048 x 2048 4.3 / 6.3.  Vocabulary projections keep the kernel whose logits do not depend on which rows are
-// computed together (greedy decoding on slices).
+// 8192 x 2048 7.3 / 9.6, 2048 x 2048 4.3 / 6.3.  (Vocabulary projections are called without a workspace, see Engine._head_workspace.)
 static bool streamk_few_rows(int epi, const LinearParams& p, const void* workspace, size_t workspace_bytes) {
   const bool glu = epi == EPI_SWIGLU || epi == EPI_GLU;
   const int64_t rows = glu ? 2ll * p.n : p.n;
-  if (p.m < 2 || p.n > 65536 || rows * p.k < (15ll << 20) || (!glu && p.k < 4096)) return false;
+  if (p.m < 2 || rows * p.k < (15ll << 20) || (!glu && p.k < 4096)) return false;
   return !prefer_simt_gemv() && current_gemm_backend() != LRI_GEMM_SIMT && gemm_streamk_supports(epi, p, workspace, workspace_bytes);
 }
 static size_t max_size(size_t a, size_t b) { return a > b ? a : b; }

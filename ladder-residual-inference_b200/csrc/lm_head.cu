@@ -126,7 +126,8 @@ extern "C" int lri_lm_head_argmax(lri_comm* comm, int dtype, const void* x, cons
     LRI_REQUIRE(logits_ws != nullptr && aligned16(logits_ws) && logits_ws_bytes >= static_cast<size_t>(M) * N * 2,
                 LRI_ERR_WORKSPACE, "lm_head_argmax: M=%lld > %d needs a logits buffer of %zu bytes (16-byte aligned)",
                 (long long)M, kGemvMaxRows, static_cast<size_t>(M) * N * 2);
-    rc = lri_linear(dtype, x, w, nullptr, logits_ws, M, N, K, workspace, workspace_bytes, stream);
+    const bool few = M <= streaming_rows();  // these stay on the streaming kernel, as the logits of a whole vocabulary do
+    rc = lri_linear(dtype, x, w, nullptr, logits_ws, M, N, K, few ? nullptr : workspace, few ? 0 : workspace_bytes, stream);
     if (rc != LRI_OK) return rc;
   }
   const dim3 grid(static_cast<unsigned>(N > 0 ? (N + kRowChunk - 1) / kRowChunk : 1), static_cast<unsigned>(M));

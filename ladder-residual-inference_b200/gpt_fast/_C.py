@@ -180,6 +180,12 @@ def check(status: int) -> None:
         raise RuntimeError(f"lri_b200 error {status}: {lib.lri_last_error().decode()}")
 
 
+def option(name: str) -> int:
+    value = c_int(0)
+    check(lib.lri_get_option(name.encode(), ctypes.byref(value)))
+    return value.value
+
+
 def ptr(t):
     return None if t is None else t.data_ptr()
 

@@ -26,7 +26,7 @@ import os
 
 import torch
 
-from ._C import DENSE, DESYNC, LADDER, LADDER_TWO_STREAMS, PARALLEL, dtype_code
+from ._C import DENSE, DESYNC, LADDER, LADDER_TWO_STREAMS, PARALLEL, dtype_code, option
 from .comm import NoComm, make_comm
 from .ops import CudaOps, decode_splits
 
@@ -108,6 +108,12 @@ class Engine:
             (t == 1 or getattr(self.comm, "handle", None) is not None)
         if self.fused_head:
             self.head_scratch = torch.zeros(self.ops.lm_head_argmax_scratch_bytes(), dtype=torch.uint8, device=device)
+
+    def _head_workspace(self, rows):
+        """Few rows of the output projection stay on the streaming kernel, whose sums hardly depend on how many vocabulary rows are
+        computed together (slices of greedy and sampled heads); with a workspace large projections take the stream-K kernel from 2
+        rows on, which cuts the sums by the number of output tiles."""
+        return self.ws_head if rows > option("stream_rows") else None
 
     # ------------------------------------------------------------------------------------------
     def _attention(self, att, w_qkv, rows, B, S, pos, out, push=0):
@@ -245,7 +251,7 @@ class Engine:
     def forward(self, idx, input_pos):
         B, S, rows = self._trunk(idx, input_pos)
         logits = torch.empty(B, S, self.cfg.vocab_size, dtype=self.dtype, device=self.resid.device)
-        self.ops.linear(self.normed, self.model.output.weight, logits, rows, workspace=self.ws_head)
+        self.ops.linear(self.normed, self.model.output.weight, logits, rows, workspace=self._head_workspace(rows))
         return logits
 
     @torch.no_grad()
@@ -257,7 +263,7 @@ class Engine:
         B, S, rows = self._trunk(idx, input_pos)
         last = self.normed[:rows].view(B, S, self.d)[:, -1].contiguous()
         logits = torch.empty(B, 1, self.cfg.vocab_size, dtype=self.dtype, device=self.resid.device)
-        self.ops.linear(last, self.model.output.weight, logits, B, workspace=self.ws_head)
+        self.ops.linear(last, self.model.output.weight, logits, B, workspace=self._head_workspace(B))
         return logits
 
     @torch.no_grad()
@@ -267,12 +273,12 @@ class Engine:
         The output projection is replicated on every rank (reference gpt_fast/gpt_ladder_TP.py:218, 283),
         and streaming all of it is the largest single item of a decode step at high TP.  Here rank r
         multiplies only rows [r V/t, (r+1) V/t) of its copy, takes the arg-max of its slice, and the
-        ranks exchange one (value, index) pair per sequence.  Up to 8 sequences the streaming kernels
-        compute every logit with a fixed K order whatever other rows are computed, so the token is
-        exactly the one `forward(...).argmax(-1)` gives (lowest index on ties), on every rank.  From 9
-        sequences on the stream-K kernel cuts K per tile by the number of tiles, which differs between
-        the full and the sliced head: logits agree to one rounding of the storage type and a near-tie
-        may resolve differently.
+        ranks exchange one (value, index) pair per sequence.  Logits are compared as the projection would
+        store them, lowest index on ties.  The order in which a logit is summed depends on the kernel: the fused
+        head's differs from that of `forward` from 2 sequences on, the streaming kernel's split of K has
+        three forms by the number of vocabulary rows, and from 9 sequences on the stream-K kernel cuts K by the
+        number of output tiles.  So logits agree with `forward(...)` to one rounding of the storage type, and
+        a near-tie may resolve differently.
         """
         import torch.distributed as dist
         B, S, rows = self._trunk(idx, input_pos)
@@ -289,7 +295,7 @@ class Engine:
         if n > 0:
             local = self.head_logits[: B * n].view(B, n)
             self.ops.linear(self.normed, self.model.output.weight[self.vocab_lo:self.vocab_hi], local, B,
-                            workspace=self.ws_head)
+                            workspace=self._head_workspace(B))
             val, ix = local.float().max(dim=-1)
             mine[:, 0] = val
             mine[:, 1] = ix + self.vocab_lo  # exact in fp32: vocabularies are far below 2**24
@@ -327,7 +333,7 @@ class Engine:
         local = self.head_logits[: B * max(n, 1)].view(B, max(n, 1))
         if n > 0:
             self.ops.linear(self.normed, self.model.output.weight[self.vocab_lo:self.vocab_hi], local, B,
-                            workspace=self.ws_head)
+                            workspace=self._head_workspace(B))
             x = local / max(temperature, 1e-5)
         else:
             x = torch.full((B, 1), float("-inf"), dtype=dtype, device=dev)
