@@ -21,7 +21,8 @@ namespace {
 
 constexpr int kThreads = 256, kMaxCluster = 8;
 constexpr int kRegTaps = 4;  // convolution weights up to this many taps are held in registers
-constexpr int kStageBytes = 96 * 1024;  // second projections up to this size are staged in shared memory
+constexpr int kStageBytes = 96 * 1024;  // second projections up to this size are staged in shared memory (16-bit rows with their padding: 6 KB
+                                        // more at most, and two CTAs still share an SM)
 
 struct StepParams {
   const float* proj;  // [B, ld]
@@ -53,12 +54,12 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 // product's eight columns.  Staged rows are `rank` elements and 8 of zeros apart: no bank conflicts, and a rank that is an odd
 // multiple of 8 ends in zeros.  On the FMA pipe, 8 lanes a row, the two 128 x 128 products of a CTA were 4.1 us of its 19.
 __host__ __device__ constexpr int staged_pitch(int rank) { return rank + 8; }
-__host__ __device__ constexpr int staged_rows(int rows) { return (rows + 15) / 16 * 16; }
 template <typename T>
 __device__ __forceinline__ void rows_mma(const T* w, int rank, const T* x, int tile, int rows, float* y) {
   const int lane = threadIdx.x & 31, pitch = staged_pitch(rank);
   float acc[2][4] = {};
-  const T* at = w + (tile * 16 + (lane & 15)) * pitch + (lane >> 4) * 8;
+  const int row = tile * 16 + (lane & 15);  // rows past the end repeat the last one, and are not stored
+  const T* at = w + (row < rows ? row : rows - 1) * pitch + (lane >> 4) * 8;
   for (int k = 0, i = 0; k < rank; k += 16, i ^= 1) {
     uint32_t a0, a1, a2, a3;
     ldmatrix_x4(at + k, a0, a1, a2, a3);
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(kThreads, RV <= 4 ? 2 : 1) state_step_kernel(c
       if (kMma && rank % 16)
         for (int r = tid; r < rows; r += kThreads) *reinterpret_cast<uint4*>(dst + r * pitch + rank) = make_uint4(0u, 0u, 0u, 0u);
     };
-    T* w_gate = w_smem + (kMma ? staged_rows(C) * staged_pitch(p.a_rank) : C * p.a_rank);
+    T* w_gate = w_smem + C * (kMma ? staged_pitch(p.a_rank) : p.a_rank);
     stage(w_smem, a2, C, p.a_rank);
     a2 = w_smem;
     if (DELTA) {
@@ -415,12 +416,12 @@ int launch(const StepParams& p, int B, cudaStream_t st) {
   constexpr bool kMma = sizeof(T) == 2;
   const size_t x_bytes = (static_cast<size_t>(p.a_rank) + (DELTA ? p.g_rank : 0)) * 4 +
                          (kMma ? static_cast<size_t>(staged_pitch(p.a_rank) + (DELTA ? staged_pitch(p.g_rank) : 0)) * 2 : 0);
-  const size_t w_bytes = kMma ? (static_cast<size_t>(staged_rows(p.C)) * staged_pitch(p.a_rank) +
-                                 (DELTA ? static_cast<size_t>(kCols) * staged_pitch(p.g_rank) : 0)) * 2
-                              : (static_cast<size_t>(p.C) * p.a_rank + (DELTA ? static_cast<size_t>(kCols) * p.g_rank : 0)) * sizeof(T);
+  const size_t rows = static_cast<size_t>(p.C) + (DELTA ? kCols : 0);
+  const size_t bare = (static_cast<size_t>(p.C) * p.a_rank + (DELTA ? static_cast<size_t>(kCols) * p.g_rank : 0)) * sizeof(T);
+  const size_t w_bytes = bare + (kMma ? rows * staged_pitch(0) * sizeof(T) : 0);
   const unsigned cs = (p.E + kCols - 1) / kCols;
   StepParams q = p;
-  q.staged = w_bytes <= kStageBytes;
+  q.staged = bare <= kStageBytes;
   auto kern = state_step_kernel<T, DELTA, RV, NC>;
   static std::atomic<unsigned long long> attr_set{0};
   LRI_ONCE_PER_DEVICE(attr_set, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kStageBytes));

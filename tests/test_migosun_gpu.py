@@ -327,6 +327,18 @@ def test_gated_delta_steps(dtype, size):
             assert _rel(got[b], gated[start:]) < max(EPS[dtype], 5e-6) and _rel(c.state[b], st) < 3e-6
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,C,E,ranks", [(1, 128, 32, (304, 304)), (10, 128, 128, (184, 192)), (10, 128, 128, (192, 192)), (10, 128, 128, (192, 200)),
+                                         (1, 100, 40, (360, 344)), (1, 1, 9, (96, 8))])
+def test_gated_delta_steps_at_the_limit_of_staged_rows(B, C, E, ranks, dtype):
+    """Second projections around the size up to which they are staged (96 KB without padding), rows that do not fill a product's tile."""
+    c = _Delta(dtype, B, 3, 8, 8, C, E, 4, *ranks, -1.0)
+    got = torch.stack([c.step(s) for s in range(3)], 1)
+    for b in (0, B - 1):
+        _, st, gated = c.oracle(b)
+        assert _rel(got[b], gated) < max(EPS[dtype], 5e-6) and _rel(c.state[b], st) < 3e-6
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("B,n,H,C,E,rank,tau,bias", [(1, 41, 2, 12, 20, 5, 7.0, 0.0), (2, 50, 3, 64, 128, 16, 16.0, 2.0), (1, 66, 2, 128, 200, 24, 1.0, -8.0),
                                                      (1, 30, 1, 9, 7, 1, 4.0, 0.0), (1, 23, 1, 256, 256, 8, 16.0, 5.0), (1, 21, 2, 400, 300, 8, 2.0, 0.0)])
