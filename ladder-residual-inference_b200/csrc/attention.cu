@@ -18,7 +18,7 @@ int attn_decode_cluster_launch(int dtype, const void* q, const void* k_cache, co
 bool attn_decode_stream_supports(int64_t pairs, int group, int64_t smax);
 int attn_decode_stream_launch(int dtype, const void* q, const void* k_cache, const void* v_cache, const void* input_pos, int pos_is_i64,
                               void* out, int B, int n_head, int n_kv, int head_dim, int64_t smax, float scale_log2, unsigned int* counters,
-                              float* parts, int64_t part_slots, cudaStream_t st);
+                              float* parts, int64_t part_slots, bool two_term, cudaStream_t st);
 // tcgen05 / TMEM form of the prefill kernel (attention_tc.cu)
 bool attn_prefill_tc_supports(int B, int S, int n_head, int n_kv, int head_dim, int64_t smax);
 int attn_prefill_tc_launch(int dtype, const void* q, const void* k_cache, const void* v_cache, const void* input_pos,
@@ -518,8 +518,8 @@ int launch_prefill(const PrefillParams& p, int B, cudaStream_t st) {
 }
 
 // Which decode kernel: the stream on tensor cores for many (sequence, KV head) pairs, the latency kernels below that.  Where query heads
-// share a KV head (us a layer, 4 of 128 elements, context 1025, latency kernel / stream): 8 pairs 7.6 / 6.7 (alone; a single
-// sequence keeps the kernel that was tuned beside the MLP of a ladder block), 16 pairs 9.1 / 7.5, 32 11.6 / 9.0, 64 14.3 / 10.2, 128 23.7 / 15.3.
+// share a KV head (us a layer, 4 of 128 elements, context 1025, latency kernel / stream): 8 pairs 7.6 / 7.0 (alone; a single
+// sequence keeps the kernel that was tuned beside the MLP of a ladder block), 16 pairs 9.1 / 7.7, 32 12.1 / 9.2, 64 14.1 / 10.5, 120 22.3 / 15.0.
 // With one query head each (24 heads, 128 elements): 72 pairs 12.1 / 11.8, 192 24.2 / 20.6, but 144 pairs of 64 elements at 300 positions 5.1 / 6.6.
 // LRI_ATTN_MMA=1 / 0 forces / forbids the stream.
 constexpr int64_t kStreamPairs = 128;  // from here on callers are asked for scratch memory
@@ -622,7 +622,7 @@ extern "C" int lri_attn_decode(int dtype, const void* q, const void* k_cache, co
     if (B == 0) return LRI_OK;
     if (attn_stream_wanted(B, n_head, n_kv, smax, n_head > n_kv ? 16 : kStreamPairs))
       return attn_decode_stream_launch(dtype, q, k_cache, v_cache, input_pos, pos_is_i64, out, B, n_head, n_kv, head_dim, smax, scale_log2,
-                                       nullptr, nullptr, 1, static_cast<cudaStream_t>(stream));
+                                       nullptr, nullptr, 1, true, static_cast<cudaStream_t>(stream));
     return attn_decode_cluster_launch(dtype, q, k_cache, v_cache, input_pos, pos_is_i64, out, B, n_head, n_kv,
                                       head_dim, smax, num_splits, scale_log2, static_cast<cudaStream_t>(stream));
   }
@@ -646,7 +646,7 @@ extern "C" int lri_attn_decode(int dtype, const void* q, const void* k_cache, co
   if (many) {
     const bool two = num_splits > 1 || lri_attn_decode_scratch_bytes(B, n_head, n_kv, head_dim, 2) <= scratch_bytes;
     return attn_decode_stream_launch(dtype, q, k_cache, v_cache, input_pos, pos_is_i64, out, B, n_head, n_kv, head_dim, smax, scale_log2,
-                                     p.counters, p.part_ml, two ? 2 : 1, st);
+                                     p.counters, p.part_ml, two ? 2 : 1, false, st);
   }
   if (dtype == LRI_BF16)
     return head_dim == 128 ? launch_decode<__nv_bfloat16, 128>(p, B, st) : launch_decode<__nv_bfloat16, 64>(p, B, st);

@@ -12,8 +12,11 @@
 //                        them merges these.  Without scratch memory one CTA a pair.
 //
 // MASKED: key and value widths below HD, a window or chunk that bounds the visible positions from below, a sink in the
-// denominator, row pitch and factor of the output; probabilities enter the product as the sum of two 16-bit numbers, because the
-// kernel that small batches take keeps them in 32 bits.
+// denominator, row pitch and factor of the output.
+// TWO_TERM: probabilities enter the product as the sum of two 16-bit numbers, where the kernel that smaller batches take keeps them in
+// 32 bits (masked form, and plain below 128 pairs or without scratch memory): rounded once, they add an error of the size of the result's own
+// rounding (8B, 2 sequences at 1025 positions, bf16: 1.98e-3 against 64 bits for 1.66e-3, which is the rounding alone).  The second product
+// costs 2 to 4 % of a layer's attention: 16 pairs 7.3 -> 7.65 us, 64 pairs 10.2 -> 10.5, 120 pairs 14.6 -> 15.0.
 //
 // Bound by HBM, from some 100 MB on at 85 to 92 % of a plain copy's rate; below, by a chain of about 4.5 us (position, descriptors, first tile,
 // merge).  Measured on B200, us a layer: 40 sequences x 24 heads of 128, 701 positions (344 MB) 58.0 (77 with one 4-warp CTA a pair), 16 sequences
@@ -106,7 +109,7 @@ __device__ __forceinline__ Deal deal(const StreamParams& p, int64_t pos, bool ma
   return d;
 }
 
-template <typename T, int HD, bool MASKED>
+template <typename T, int HD, bool MASKED, bool TWO_TERM>
 __global__ void __launch_bounds__(kThreads, 2)
 attn_decode_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const StreamParams p) {
   constexpr int KB = HD / 16;
@@ -336,7 +339,7 @@ attn_decode_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             pa[nb * 2 + r] = pack2<T>(pv[2 * r], pv[2 * r + 1]);
-            if (MASKED) {
+            if (TWO_TERM) {
               float h0, h1;
               Num<T>::unpack2(pa[nb * 2 + r], h0, h1);
               pl[nb * 2 + r] = pack2<T>(pv[2 * r] - h0, pv[2 * r + 1] - h1);
@@ -365,7 +368,7 @@ attn_decode_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
             load_matrix_trans(at + (ob2 >> 2) * kChunkBytes + ((unit ^ (row & 7)) << 4), bf);
             mma16816<T>(o[2 * ob2], pa[0], pa[1], pa[2], pa[3], bf[0], bf[1]);
             mma16816<T>(o[2 * ob2 + 1], pa[0], pa[1], pa[2], pa[3], bf[2], bf[3]);
-            if (MASKED) {
+            if (TWO_TERM) {
               mma16816<T>(o[2 * ob2], pl[0], pl[1], pl[2], pl[3], bf[0], bf[1]);
               mma16816<T>(o[2 * ob2 + 1], pl[0], pl[1], pl[2], pl[3], bf[2], bf[3]);
             }
@@ -471,7 +474,7 @@ attn_decode_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   __syncthreads();
 }
 
-template <typename T, int HD, bool MASKED>
+template <typename T, int HD, bool MASKED, bool TWO_TERM>
 int launch(int dtype, const StreamParams& p, int64_t grid, cudaStream_t st) {
   CUtensorMap tk, tv;
   int rc = make_tmap(&tk, dtype, p.k, p.pairs * p.smax, p.dim, kUnit);
@@ -479,7 +482,7 @@ int launch(int dtype, const StreamParams& p, int64_t grid, cudaStream_t st) {
   rc = make_tmap(&tv, dtype, p.v, p.pairs * p.smax, p.vdim, kUnit);
   if (rc != LRI_OK) return rc;
   const int smem = 1024 + kRingBytes + kWarps * p.group * HD * 4 + p.cluster * p.group * (HD + 2) * 4;
-  auto kern = attn_decode_stream_kernel<T, HD, MASKED>;
+  auto kern = attn_decode_stream_kernel<T, HD, MASKED, TWO_TERM>;
   static std::atomic<unsigned long long> attr_set{0};  // per template instantiation, one bit per device
   LRI_ONCE_PER_DEVICE(attr_set, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      1024 + kRingBytes + kWarps * kMaxGroup * HD * 4 + kMaxGathered * (HD + 2) * 4));
@@ -505,7 +508,7 @@ int launch(int dtype, const StreamParams& p, int64_t grid, cudaStream_t st) {
 // CTAs: two of them share an SM.  A pair gets as many (a power of two) as fit at once; clusters of 2 and 4 find room for 7 of 8 CTAs that
 // would fit singly, of 8 for half of them (72 pairs at 1025 positions: 17.1 us in 288 CTAs, 11.8 in 144; 32 pairs: 13.1 in 256, 9.0 in 128).
 // From more pairs than fit on, and with room for their parts, all CTAs get equal runs, each at least a pair long.
-template <bool MASKED>
+template <bool MASKED, bool TWO_TERM>
 int dispatch(int dtype, StreamParams& p, int forced, cudaStream_t st) {
   const int64_t room = 2ll * device_sm_count();
   p.cluster = 1;
@@ -516,8 +519,8 @@ int dispatch(int dtype, StreamParams& p, int forced, cudaStream_t st) {
   const int64_t grid = p.slots > 1 ? room : static_cast<int64_t>(p.pairs) * p.cluster;
   const bool narrow = p.dim <= 64 && p.vdim <= 64;
   if (dtype == LRI_BF16)
-    return narrow ? launch<__nv_bfloat16, 64, MASKED>(dtype, p, grid, st) : launch<__nv_bfloat16, 128, MASKED>(dtype, p, grid, st);
-  return narrow ? launch<__half, 64, MASKED>(dtype, p, grid, st) : launch<__half, 128, MASKED>(dtype, p, grid, st);
+    return narrow ? launch<__nv_bfloat16, 64, MASKED, TWO_TERM>(dtype, p, grid, st) : launch<__nv_bfloat16, 128, MASKED, TWO_TERM>(dtype, p, grid, st);
+  return narrow ? launch<__half, 64, MASKED, TWO_TERM>(dtype, p, grid, st) : launch<__half, 128, MASKED, TWO_TERM>(dtype, p, grid, st);
 }
 
 }  // namespace
@@ -527,10 +530,10 @@ bool attn_decode_stream_supports(int64_t pairs, int group, int64_t smax) {
   return group <= kMaxGroup && pairs * smax + kUnit < (1ll << 31) && pairs < (1 << 24);
 }
 
-// counters: zero, and left zero; parts: room for part_slots parts of every pair
+// counters: zero, and left zero; parts: room for part_slots parts of every pair; two_term: probabilities of more than 16 bits
 int attn_decode_stream_launch(int dtype, const void* q, const void* k_cache, const void* v_cache, const void* input_pos, int pos_is_i64,
                               void* out, int B, int n_head, int n_kv, int head_dim, int64_t smax, float scale_log2, unsigned int* counters,
-                              float* parts, int64_t part_slots, cudaStream_t st) {
+                              float* parts, int64_t part_slots, bool two_term, cudaStream_t st) {
   StreamParams p{};
   p.q = q, p.k = k_cache, p.v = v_cache, p.input_pos = input_pos, p.pos_is_i64 = pos_is_i64, p.out = out, p.out_ld = static_cast<int64_t>(n_head) * head_dim;
   p.pairs = B * n_kv, p.n_head = n_head, p.n_kv = n_kv, p.group = n_head / n_kv, p.smax = smax, p.scale_log2 = scale_log2;
@@ -539,7 +542,7 @@ int attn_decode_stream_launch(int dtype, const void* q, const void* k_cache, con
   p.counters = counters;
   p.part_ml = parts;
   p.part_o = parts + (static_cast<int64_t>(B) * n_head * p.slots * 2 + 3) / 4 * 4;
-  return dispatch<false>(dtype, p, option(OPT_DECODE_SPLITS), st);
+  return two_term ? dispatch<false, true>(dtype, p, option(OPT_DECODE_SPLITS), st) : dispatch<false, false>(dtype, p, option(OPT_DECODE_SPLITS), st);
 }
 
 int attn_decode_stream_masked_launch(int dtype, const WindowParams& w, int B, cudaStream_t st) {
@@ -549,7 +552,7 @@ int attn_decode_stream_masked_launch(int dtype, const WindowParams& w, int B, cu
   p.scale_log2 = w.scale * 1.4426950408889634f;
   p.slots = 1;
   p.dim = w.d1, p.vdim = w.dv, p.window = w.window, p.chunk = w.chunk, p.sink = w.sink, p.out_scale = w.out_scale;
-  return dispatch<true>(dtype, p, option(OPT_DECODE_SPLITS), st);
+  return dispatch<true, true>(dtype, p, option(OPT_DECODE_SPLITS), st);
 }
 
 int attn_decode_stream_status_read_and_clear(int* status_out) {

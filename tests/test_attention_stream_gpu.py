@@ -77,3 +77,22 @@ def test_stream_masked(dtype, B, nh, nkv, dim, vdim, window, chunk, pos):
         # probabilities keep 16 bits and more here: the result is rounded once
         assert ((got.double() - want).norm() / want.norm()).item() < TOL[dtype] / 2
         assert out[:, nh * vdim:].isnan().all()
+
+
+@pytest.mark.parametrize("dtype", list(TOL))
+@pytest.mark.parametrize("B,nh,nkv,hd,pos", [(1, 32, 8, 128, 1022), (2, 32, 8, 128, 1022), (15, 32, 8, 128, 700), (5, 20, 4, 64, 527), (31, 24, 4, 64, 995)])
+def test_probabilities_keep_more_than_the_storage_type(dtype, B, nh, nkv, hd, pos):
+    """Below 128 pairs of a sequence and a KV head, in whichever kernel, rounding the result is all the error there is: a sequence loses no
+    bits when others join it.  Probabilities rounded to the storage type would add an error of the same size (1.2 to 1.4 times in all); as two
+    numbers of it they add 2^-8 of that (bf16), and the fp32 sums less than 1 % (fp16)."""
+    from gpt_fast import _C
+    from gpt_fast.ops import CudaOps as ops, decode_splits
+    _C.check(_C.lib.lri_set_option(b"attn_mma", -1))
+    q, kc, vc, ipos = _case(dtype, B, nh, nkv, hd, hd, 1023, pos)
+    want = _want(q, kc, vc, 0, pos, hd ** -0.5)
+    splits = decode_splits(B, nh, nkv, 1023, hd)
+    scratch = torch.zeros(ops.attn_decode_scratch_bytes(B, nh, nkv, hd, splits), dtype=torch.uint8, device="cuda")
+    out = torch.full((B, nh, hd), float("nan"), dtype=dtype, device="cuda")
+    ops.attention(q, kc, vc, ipos, out, B, 1, nh, nkv, hd, scratch, splits)
+    rounding = (want.to(dtype).double() - want).norm()
+    assert ((out.double() - want).norm() / rounding).item() < 1.02
