@@ -109,8 +109,8 @@ __device__ __forceinline__ Deal deal(const StreamParams& p, int64_t pos, bool ma
   return d;
 }
 
-template <typename T, int HD, bool MASKED, bool TWO_TERM>
-__global__ void __launch_bounds__(kThreads, 2)
+template <typename T, int HD, bool MASKED, bool TWO_TERM, int PER_SM>
+__global__ void __launch_bounds__(kThreads, PER_SM)
 attn_decode_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const StreamParams p) {
   constexpr int KB = HD / 16;
   constexpr int OB = HD / 8;
@@ -474,7 +474,7 @@ attn_decode_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   __syncthreads();
 }
 
-template <typename T, int HD, bool MASKED, bool TWO_TERM>
+template <typename T, int HD, bool MASKED, bool TWO_TERM, int PER_SM>
 int launch(int dtype, const StreamParams& p, int64_t grid, cudaStream_t st) {
   CUtensorMap tk, tv;
   int rc = make_tmap(&tk, dtype, p.k, p.pairs * p.smax, p.dim, kUnit);
@@ -482,7 +482,7 @@ int launch(int dtype, const StreamParams& p, int64_t grid, cudaStream_t st) {
   rc = make_tmap(&tv, dtype, p.v, p.pairs * p.smax, p.vdim, kUnit);
   if (rc != LRI_OK) return rc;
   const int smem = 1024 + kRingBytes + kWarps * p.group * HD * 4 + p.cluster * p.group * (HD + 2) * 4;
-  auto kern = attn_decode_stream_kernel<T, HD, MASKED, TWO_TERM>;
+  auto kern = attn_decode_stream_kernel<T, HD, MASKED, TWO_TERM, PER_SM>;
   static std::atomic<unsigned long long> attr_set{0};  // per template instantiation, one bit per device
   LRI_ONCE_PER_DEVICE(attr_set, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      1024 + kRingBytes + kWarps * kMaxGroup * HD * 4 + kMaxGathered * (HD + 2) * 4));
@@ -505,22 +505,44 @@ int launch(int dtype, const StreamParams& p, int64_t grid, cudaStream_t st) {
   return LRI_OK;
 }
 
-// CTAs: two of them share an SM.  A pair gets as many (a power of two) as fit at once; clusters of 2 and 4 find room for 7 of 8 CTAs that
-// would fit singly, of 8 for half of them (72 pairs at 1025 positions: 17.1 us in 288 CTAs, 11.8 in 144; 32 pairs: 13.1 in 256, 9.0 in 128).
+// CTAs of a cluster that share a pair, with `room` CTAs on the GPU: as many (a power of two) as fit at once.  Clusters of 2 and 4 find room
+// for 7 of 8 CTAs that would fit singly, of 8 for half of them (72 pairs at 1025 positions: 17.1 us in 288 CTAs, 11.8 in 144; 32 pairs: 13.1 in
+// 256, 9.0 in 128).
+int cluster_size(const StreamParams& p, int64_t room, int forced) {
+  int size = 1;
+  for (int c = 2; c <= kMaxCluster; c *= 2)
+    if (static_cast<int64_t>(p.pairs) * c <= (c < 8 ? room / 8 * 7 : room / 2) && p.group * c <= kMaxGathered && (forced == 0 || c <= forced)) size = c;
+  return size;
+}
+
+// CTAs: two of them share an SM.  Rows of 64 elements, whose tiles are half as large, take three where that gives a pair more CTAs or shortens
+// the run of a CTA (us a layer, two / three, 1025 positions: 144 pairs 16.6 / 11.8, 384 26.3 / 19.9, 768 43.6 / 38.7).  Where it does not, two have
+// the registers of three, and a third does not fit: CTAs would come to lie three on one SM and one on another (40 pairs 7.6 / 8.4, 240 pairs
+// 16.9 / 18.5).
 // From more pairs than fit on, and with room for their parts, all CTAs get equal runs, each at least a pair long.
 template <bool MASKED, bool TWO_TERM>
 int dispatch(int dtype, StreamParams& p, int forced, cudaStream_t st) {
-  const int64_t room = 2ll * device_sm_count();
-  p.cluster = 1;
-  for (int c = 2; c <= kMaxCluster; c *= 2)
-    if (static_cast<int64_t>(p.pairs) * c <= (c < 8 ? room / 8 * 7 : room / 2) && p.group * c <= kMaxGathered && (forced == 0 || c <= forced))
-      p.cluster = c;
+  const int64_t sms = device_sm_count();
+  const bool narrow = p.dim <= 64 && p.vdim <= 64;
+  int per_sm = 2;
+  p.cluster = cluster_size(p, 2 * sms, forced);
+  if (narrow && p.group <= 4) {  // more heads take more shared memory than a third of an SM's
+    const int of_three = cluster_size(p, 3 * sms, forced);
+    // pairs of a CTA, times its neighbours, if pairs are not cut
+    const int64_t two_deep = (p.pairs + 2 * sms - 1) / (2 * sms) * 2, three_deep = (p.pairs + 3 * sms - 1) / (3 * sms) * 3;
+    const bool cut = p.slots > 1 && p.smax >= kMinCut * kUnit;
+    if (of_three > p.cluster || (p.pairs > 2 * sms && (cut || three_deep < two_deep))) per_sm = 3;
+    if (of_three > p.cluster) p.cluster = of_three;
+  }
+  const int64_t room = per_sm * sms;
   if (p.cluster > 1 || p.pairs <= room) p.slots = 1;
   const int64_t grid = p.slots > 1 ? room : static_cast<int64_t>(p.pairs) * p.cluster;
-  const bool narrow = p.dim <= 64 && p.vdim <= 64;
-  if (dtype == LRI_BF16)
-    return narrow ? launch<__nv_bfloat16, 64, MASKED, TWO_TERM>(dtype, p, grid, st) : launch<__nv_bfloat16, 128, MASKED, TWO_TERM>(dtype, p, grid, st);
-  return narrow ? launch<__half, 64, MASKED, TWO_TERM>(dtype, p, grid, st) : launch<__half, 128, MASKED, TWO_TERM>(dtype, p, grid, st);
+  if (dtype == LRI_BF16) {
+    if (!narrow) return launch<__nv_bfloat16, 128, MASKED, TWO_TERM, 2>(dtype, p, grid, st);
+    return per_sm == 3 ? launch<__nv_bfloat16, 64, MASKED, TWO_TERM, 3>(dtype, p, grid, st) : launch<__nv_bfloat16, 64, MASKED, TWO_TERM, 2>(dtype, p, grid, st);
+  }
+  if (!narrow) return launch<__half, 128, MASKED, TWO_TERM, 2>(dtype, p, grid, st);
+  return per_sm == 3 ? launch<__half, 64, MASKED, TWO_TERM, 3>(dtype, p, grid, st) : launch<__half, 64, MASKED, TWO_TERM, 2>(dtype, p, grid, st);
 }
 
 }  // namespace

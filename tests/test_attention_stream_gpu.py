@@ -44,7 +44,8 @@ TOL = {torch.bfloat16: 2 * 2 ** -8, torch.float16: 2 * 2 ** -11}
 
 
 @pytest.mark.parametrize("dtype", list(TOL))
-@pytest.mark.parametrize("B,nh,nkv,hd", [(1, 1, 1, 128), (3, 32, 2, 128), (5, 20, 4, 64), (20, 32, 8, 64), (13, 24, 24, 128), (41, 24, 8, 64)])
+@pytest.mark.parametrize("B,nh,nkv,hd", [(1, 1, 1, 128), (3, 32, 2, 128), (5, 20, 4, 64), (20, 32, 8, 64), (13, 24, 24, 128), (41, 24, 8, 64),
+                                             (6, 16, 4, 64), (38, 12, 12, 64)])
 @pytest.mark.parametrize("pos", [0, 31, 32, 479, 480, 481, 527, 995, 1022])
 def test_stream(dtype, B, nh, nkv, hd, pos):
     from gpt_fast.ops import CudaOps as ops, decode_splits
