@@ -28,6 +28,17 @@ def _model(family, dtype, batch, overlap=True, **extra):
     return model
 
 
+def _only(engine, native):
+    """Passes of this engine run in the native call alone, or never there."""
+    if not native:
+        engine._run_native = lambda *a: False
+        return
+
+    def refuse(*a):
+        raise AssertionError("the Python schedule ran")
+    engine._run_dense = engine._run_ladder = engine._run_parallel = engine._run_desync = refuse
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("batch", [1, 3, 20])
 @pytest.mark.parametrize("family,extra", [("dense", {}), ("ladder", {}), ("ladder", {"overlap": False}), ("parallel", {}), ("desync", {}),
@@ -36,9 +47,7 @@ def test_native_pass_equals_calls(dtype, batch, family, extra):
     results = []
     for native in (True, False):
         model = _model(family, dtype, batch, **extra)
-        engine = model._engine
-        if not native:
-            engine._run_native = lambda *a: False
+        _only(model._engine, native)
         ids = torch.randint(0, SHAPE["vocab_size"], (batch, 70), generator=torch.Generator().manual_seed(1)).cuda()
         out = []
         with torch.no_grad():
@@ -52,6 +61,7 @@ def test_native_pass_equals_calls(dtype, batch, family, extra):
 
 def test_weights_are_read_for_every_pass_and_errors_arrive():
     model = _model("dense", torch.bfloat16, 1)
+    _only(model._engine, True)
     tok, pos = torch.tensor([[3]], dtype=torch.int32, device="cuda"), torch.tensor([0], dtype=torch.int32, device="cuda")
     with torch.no_grad():
         first = model(tok, pos)
