@@ -562,8 +562,10 @@ extern "C" size_t lri_attn_decode_scratch_bytes(int B, int n_head, int n_kv, int
 // current position.  Up to 8 ranges (a power of two; 16 for a one- or two-cluster launch) run as one
 // thread-block cluster and merge through shared memory; that form is kept as long as a CTA then streams at most ~1 MB of K/V.
 // Longer caches take more ranges (up to 64, at least 64 positions each) and merge through the scratch
-// buffer.  The stream kernel (from 128 (sequence, KV head) pairs on) cuts pairs wherever its CTAs' runs end and uses what parts the
-// scratch buffer has room for; it asks for two while one per pair would leave SMs without work.
+// buffer.  From 128 (sequence, KV head) pairs on the stream kernel runs, for which the number only says how much scratch memory the caller
+// will have: it needs two parts a pair where there are more pairs than CTAs fit at once, to cut pairs where its CTAs' runs end, and none below.
+// The plan keeps the numbers that callers know (two below 2 pairs an SM, one above); with memory for one part a CTA takes whole pairs.  The
+// engine has memory for 64 and always gets the cut.
 extern "C" int lri_attn_decode_plan(int B, int n_head, int n_kv, int head_dim, int64_t smax, int* num_splits) {
   LRI_REQUIRE(num_splits != nullptr, LRI_ERR_ARG, "attn_decode_plan: NULL output");
   LRI_REQUIRE(B >= 1 && n_head >= 1 && n_kv >= 1 && n_head % n_kv == 0 && head_dim >= 1 && smax >= 1, LRI_ERR_ARG,
