@@ -505,13 +505,14 @@ int launch(int dtype, const StreamParams& p, int64_t grid, cudaStream_t st) {
   return LRI_OK;
 }
 
-// CTAs of a cluster that share a pair, with `room` CTAs on the GPU: as many (a power of two) as fit at once.  Clusters of 2 and 4 find room
-// for 7 of 8 CTAs that would fit singly, of 8 for half of them (72 pairs at 1025 positions: 17.1 us in 288 CTAs, 11.8 in 144; 32 pairs: 13.1 in
-// 256, 9.0 in 128).
+// CTAs of a cluster that share a pair, with `room` CTAs on the GPU: as many (a power of two) as fit at once.  Clusters of 2 find room for all
+// CTAs that would fit singly (8 KV heads, 1025 positions, 136 and 144 pairs: 18.8 and 18.9 us singly, 15.7 and 16.3 in clusters; of 64
+// elements, three CTAs an SM, 216 pairs: 17.1 and 12.8), of 4 for 7 of 8, of 8 for half of them (72 pairs: 17.1 us in 288 CTAs, 11.8 in 144; 32 pairs:
+// 13.1 in 256, 9.0 in 128).
 int cluster_size(const StreamParams& p, int64_t room, int forced) {
   int size = 1;
   for (int c = 2; c <= kMaxCluster; c *= 2)
-    if (static_cast<int64_t>(p.pairs) * c <= (c < 8 ? room / 8 * 7 : room / 2) && p.group * c <= kMaxGathered && (forced == 0 || c <= forced)) size = c;
+    if (static_cast<int64_t>(p.pairs) * c <= (c == 2 ? room : c == 4 ? room / 8 * 7 : room / 2) && p.group * c <= kMaxGathered && (forced == 0 || c <= forced)) size = c;
   return size;
 }
 
