@@ -360,14 +360,17 @@ int attn_decode_masked_launch(int dtype, const WindowParams& w, int B, cudaStrea
   p.q = w.q, p.k_cache = w.k, p.v_cache = w.v, p.input_pos = w.input_pos, p.pos_is_i64 = w.pos_is_i64, p.out = w.out;
   p.n_head = w.H, p.n_kv = n_kv, p.smax = w.k_rows, p.scale_log2 = w.scale * 1.4426950408889634f;
   p.dim = w.d1, p.vdim = w.dv, p.window = w.window, p.chunk = w.chunk, p.sink = w.sink, p.out_ld = w.out_ld, p.out_scale = w.out_scale;
-  // us a layer, this kernel / the stream, context 1025: 32 heads of 8 KV heads, 16 pairs 14.3 / 8.4, 32 21.5 / 10, 128 36.0 / 16.7; one query head each, 64
-  // pairs 10.6 / 10.5, 72 10.7 / 13, 192 21.5 / 22.5, 960 pairs at 701 positions 72.5 / 72.2
-  const int mode = option(OPT_ATTN_MMA);
-  const int64_t pairs = static_cast<int64_t>(B) * n_kv;
-  if ((mode == 1 || (mode == -1 && pairs >= (w.group > 1 ? 16 : 512))) && attn_decode_stream_supports(pairs, w.group, w.k_rows))
-    return attn_decode_stream_masked_launch(dtype, w, B, st);
   int64_t visible = w.k_rows < w.window ? w.k_rows : w.window;
   if (w.chunk > 0 && w.chunk < visible) visible = w.chunk;
+  // us a layer, this kernel / the stream, context 1025: 32 heads of 8 KV heads, 16 pairs 14.3 / 8.4, 32 21.5 / 10, 128 36.0 / 16.7; one query head each, 64
+  // pairs 10.6 / 10.5, 72 10.7 / 13, 192 21.5 / 22.5.  From some 500 pairs of one query head on it is the length that decides: 1536 pairs at 300
+  // positions 50.9 / 62.4, 960 at 701 71.4 / 70.7, 768 at 1025 79.7 / 72.9, 1536 at 2000 321 / 252.  The position is not known here: a cache of 1536
+  // is half full at about the length where the two are equal.  Heads of 64 elements stay (768 pairs at 1025 positions 41.1 / 52.5).
+  const int mode = option(OPT_ATTN_MMA);
+  const int64_t pairs = static_cast<int64_t>(B) * n_kv;
+  const bool many = w.group > 1 ? pairs >= 16 : pairs >= 512 && visible >= 1536 && (w.d1 > 64 || w.dv > 64);
+  if ((mode == 1 || (mode == -1 && many)) && attn_decode_stream_supports(pairs, w.group, w.k_rows))
+    return attn_decode_stream_masked_launch(dtype, w, B, st);
   const int gt = attn_decode_cluster_head_tile(B, n_kv, w.group);
   const int64_t base = static_cast<int64_t>(B) * n_kv * (w.group / gt), want = (2 * device_sm_count() + base - 1) / base;
   const int64_t lim = want < 8 ? want : (base <= 4 ? 16 : 8);
