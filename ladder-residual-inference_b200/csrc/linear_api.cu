@@ -268,7 +268,8 @@ static size_t streamk_bytes(int epi, int64_t M, int64_t n) {
 // 2 .. streaming_rows() token rows of a large projection go there too.  The streaming kernel reads all token rows in every CTA of 16 weight
 // rows, which is what it waits for behind the kernel that wrote them; the stream-K kernel reads them once an SM and has its ring full of
 // weights by then, but costs a second launch.  Measured on B200, streaming / stream-K, a whole decode step of 4 sequences: 8B (k 4096 and
-// 14336, all projections from 33 MB on) 4574 / 3305 us dense, 3567 / 2850 ladder; Migosun 8B 5060 / 4051.  One projection alone: gated
+// 14336, all projections from 33 MB on) 4574 / 3305 us dense (3819 / 3213 with
+// the latency attention kernel), 3567 / 2850 ladder; Migosun 8B 5060 / 4051.  One projection alone: gated
 // 16384 x 2048 (67 MB) 19.0 / 15.1 us, 16384 x 3072 25.6 / 21.2, 2048 x 8192 (34 MB) 13.0 / 10.4, 3072 x 8192 14.5 / 12.8; but 9216 x 3072 11.0 / 13.7,
 // 8192 x 2048 7.3 / 9.6, 2048 x 2048 4.3 / 6.3.  (Vocabulary projections are called without a workspace, see Engine._head_workspace.)
 static bool streamk_few_rows(int epi, const LinearParams& p, const void* workspace, size_t workspace_bytes) {
