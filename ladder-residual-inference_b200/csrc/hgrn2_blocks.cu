@@ -27,11 +27,11 @@ namespace lri {
 namespace {
 
 constexpr int kBlock = 16;
-constexpr int kThreads = 512, kWarps = 16;
 constexpr int kTerms = 3;
 constexpr int kMaxSegments = 8;
 constexpr int kMinSegment = 64;  // tokens
 constexpr int kMaxE = 128;
+constexpr int kNarrow = 64;  // channels and values up to which a CTA has 256 threads, otherwise 512
 
 using bf16 = __nv_bfloat16;
 
@@ -84,19 +84,19 @@ __device__ __forceinline__ float gate(float raw, float bias, float low) {
 }
 __device__ __forceinline__ float silu(float x) { return x * __fdividef(1.0f, 1.0f + __expf(-x)); }
 
-template <int CP>
+template <int CP, int ME>
 struct Smem {
   static constexpr int kPitchC = CP + 8;      // bf16 rows of q", k"
-  static constexpr int kPitchE = kMaxE + 8;   // bf16 rows of v
+  static constexpr int kPitchE = ME + 8;      // bf16 rows of v
   static constexpr int kPitchA = kBlock + 8;  // bf16 rows of A
-  alignas(16) float raw[2][kBlock * (2 * CP + kMaxE)];    // q, f, v of a block as they arrive
+  alignas(16) float raw[2][kBlock * (2 * CP + ME)];    // q, f, v of a block as they arrive
   alignas(16) float q[kBlock][CP];
   alignas(16) float f[kBlock][CP];
   alignas(16) float bias[CP];
   alignas(16) float low[CP];
   alignas(16) float F[2][CP];
-  alignas(16) float w[kMaxE];
-  float o[2][kBlock][kMaxE + 4];  // per half of the channels
+  alignas(16) float w[ME];
+  float o[2][kBlock][ME + 4];  // per half of the channels
   alignas(16) bf16 qd[2][kTerms][kBlock * kPitchC];
   alignas(16) bf16 kd[2][kTerms][kBlock * kPitchC];
   alignas(16) bf16 v[2][2][kBlock * kPitchE];
@@ -104,18 +104,24 @@ struct Smem {
 };
 
 // Grid (segments, heads, sequences).  FULL: outputs and the sequence's final state; otherwise the segment's contribution.
-template <typename T, int CP, bool FULL>
-__global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Params p, const Segments sg) {
+//
+// THREADS 512: a warp takes one token of a block, up to 128 channels and values.  THREADS 256, heads of up to 64 channels and values: a warp
+// takes two tokens, half of its lanes each, and two CTAs share an SM.  With 512 threads half of the lanes of such heads had nothing to do:
+// 32 heads of 64 x 64, 2048 tokens of one sequence, first and second pass: 49 and 108 us with 512 threads and 4 segments, 31 and 83 with 256 and 8.
+template <typename T, int CP, bool FULL, int THREADS>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) hgrn2_blocks_kernel(const Hgrn2Params p, const Segments sg) {
+  constexpr int kThreads = THREADS, kWarps = THREADS / 32, ME = THREADS == 256 ? kNarrow : kMaxE;
+  using Sm = Smem<CP, ME>;
   constexpr int kTiles = CP / 16;  // 8-column tiles of S^T of a warp
   constexpr int kVTerms = sizeof(T) == 2 && std::is_same<T, bf16>::value ? 1 : 2;
   extern __shared__ __align__(16) uint8_t hb_smem[];
-  Smem<CP>& sm = *reinterpret_cast<Smem<CP>*>(hb_smem);
+  Sm& sm = *reinterpret_cast<Sm*>(hb_smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int seg = blockIdx.x, h = blockIdx.y, b = blockIdx.z, H = p.H, C = p.C, E = p.E;
   const int64_t bh = static_cast<int64_t>(b) * H + h, all_bh = static_cast<int64_t>(gridDim.z) * H;
   const int s_begin = seg * sg.tokens;
   const int s_end = seg == sg.count - 1 ? p.S : s_begin + sg.tokens;
-  const int e0 = (warp & 7) * 16, half = warp >> 3, c0 = half * (CP / 2);
+  const int e0 = warp % (kWarps / 2) * 16, half = warp / (kWarps / 2), c0 = half * (CP / 2);
   const bool live = e0 < E;
   const int er = e0 + (lane >> 2), cc = 2 * (lane & 3);  // this thread's first row and column in a tile of S^T
 
@@ -124,22 +130,24 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
     sm.low[c] = c < C ? Num<T>::to_f(static_cast<const T*>(p.lower)[h * C + c]) : 0.f;
   }
   for (int e = tid; e < E; e += kThreads) sm.w[e] = Num<T>::to_f(static_cast<const T*>(p.norm_w)[e]);
-  static_assert(kWarps == kBlock && kThreads == 4 * 128, "work is dealt to warps by token and to threads by channel");
+  constexpr int kPerWarp = kBlock / kWarps;  // tokens of a warp, each on 32 / kPerWarp lanes
+  constexpr int kChannelThreads = kThreads / 4;
+  static_assert(32 / kPerWarp * 4 == ME && CP <= kChannelThreads && CP <= ME, "work is dealt to lanes by token and to threads by channel");
   // channels past C stay zero in the arrays that the products read
   if (C < CP)
-    for (int i = tid; i < 2 * kTerms * kBlock * Smem<CP>::kPitchC; i += kThreads) {
+    for (int i = tid; i < 2 * kTerms * kBlock * Sm::kPitchC; i += kThreads) {
       (&sm.qd[0][0][0])[i] = __float2bfloat16_rn(0.f);
       (&sm.kd[0][0][0])[i] = __float2bfloat16_rn(0.f);
     }
   pdl_launch_dependents();
   pdl_wait();
 
-  // warp t works on token t of a block, a lane on 4 consecutive channels (or values)
-  const int x4 = lane * 4;
+  // a lane works on 4 consecutive channels (or values) of its token of a block
+  const int tok = warp * kPerWarp + lane / (32 / kPerWarp), x4 = lane % (32 / kPerWarp) * 4;
   auto fetch = [&](int s0, int buf) {
-    if (s0 + warp < s_end) {
-      const float* row = p.proj + (static_cast<int64_t>(b) * p.S + s0 + warp) * p.ld + x4;
-      float* dst = sm.raw[buf] + warp * (2 * CP + kMaxE) + x4;
+    if (s0 + tok < s_end) {
+      const float* row = p.proj + (static_cast<int64_t>(b) * p.S + s0 + tok) * p.ld + x4;
+      float* dst = sm.raw[buf] + tok * (2 * CP + ME) + x4;
       if (x4 < C) {
         if (FULL) cp_async16(dst, row + p.q_off + h * C);
         cp_async16(dst + CP, row + p.f_off + h * C);
@@ -186,8 +194,8 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
   // ---- steps of a block; buf = parity of the block ----
   // gates, activations, v terms (each thread reads what it fetched itself)
   auto gates = [&](int s0, int buf) {
-    const bool in = s0 + warp < s_end;
-    const float* rw = sm.raw[buf] + warp * (2 * CP + kMaxE) + x4;
+    const bool in = s0 + tok < s_end;
+    const float* rw = sm.raw[buf] + tok * (2 * CP + ME) + x4;
     if (x4 < CP) {
       float4 f = make_float4(1.f, 1.f, 1.f, 1.f), q = make_float4(0.f, 0.f, 0.f, 0.f);
       if (in && x4 < C) {
@@ -199,8 +207,8 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
           q = make_float4(silu(qr.x), silu(qr.y), silu(qr.z), silu(qr.w));
         }
       }
-      *reinterpret_cast<float4*>(&sm.f[warp][x4]) = f;
-      if (FULL) *reinterpret_cast<float4*>(&sm.q[warp][x4]) = q;
+      *reinterpret_cast<float4*>(&sm.f[tok][x4]) = f;
+      if (FULL) *reinterpret_cast<float4*>(&sm.q[tok][x4]) = q;
     }
     if (x4 < E) {
       const float4 x = in ? *reinterpret_cast<const float4*>(rw + 2 * CP) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -209,14 +217,14 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
       split2(rnd<T>(x.z), rnd<T>(x.w), hi);
 #pragma unroll
       for (int i = 0; i < kVTerms; ++i)
-        *reinterpret_cast<uint2*>(&sm.v[buf][i][warp * Smem<CP>::kPitchE + x4]) = make_uint2(lo[i], hi[i]);
+        *reinterpret_cast<uint2*>(&sm.v[buf][i][tok * Sm::kPitchE + x4]) = make_uint2(lo[i], hi[i]);
     }
   };
   auto products = [&](int buf) {
     // running products: thread (channel, k" or q", first or last 8 tokens)
     {
       constexpr int kH = kBlock / 2;
-      const int c = tid & 127, part = tid >> 7, t0 = (part & 1) * kH;
+      const int c = tid % kChannelThreads, part = tid / kChannelThreads, t0 = (part & 1) * kH;
       if (part < 2) {
         if (c < C) {
           float r = 1.f;
@@ -226,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
 #pragma unroll
           for (int i = kH - 1; i >= 0; --i) {
             const float f = sm.f[t0 + i][c];
-            split_store(&sm.kd[buf][0][(t0 + i) * Smem<CP>::kPitchC + c], kBlock * Smem<CP>::kPitchC, (1.f - f) * r);
+            split_store(&sm.kd[buf][0][(t0 + i) * Sm::kPitchC + c], kBlock * Sm::kPitchC, (1.f - f) * r);
             r *= f;
           }
           if (t0 == 0) {
@@ -244,45 +252,48 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
 #pragma unroll
         for (int i = 0; i < kH; ++i) {
           r *= sm.f[t0 + i][c];
-          split_store(&sm.qd[buf][0][(t0 + i) * Smem<CP>::kPitchC + c], kBlock * Smem<CP>::kPitchC, sm.q[t0 + i][c] * r);
+          split_store(&sm.qd[buf][0][(t0 + i) * Sm::kPitchC + c], kBlock * Sm::kPitchC, sm.q[t0 + i][c] * r);
         }
       }
     }
     if (!FULL) return;
-    // A[t, s]: warp s, lanes over channels
+    // A[t, s]: a warp per s (or a short and a long one), lanes over channels
     constexpr int kPer = CP / 32;
-    const int s = warp;
-    float d[kPer] = {}, a[kBlock];
+#pragma unroll 1
+    for (int turn = 0; turn < kPerWarp; ++turn) {
+      const int s = turn ? kBlock - 1 - warp : warp;
+      float d[kPer] = {}, a[kBlock];
 #pragma unroll
-    for (int t = 0; t < kBlock; ++t) {
-      float x = 0.f;
-      if (t >= s) {
+      for (int t = 0; t < kBlock; ++t) {
+        float x = 0.f;
+        if (t >= s) {
 #pragma unroll
-        for (int j = 0; j < kPer; j += 2) {
-          const float2 f = *reinterpret_cast<const float2*>(&sm.f[t][lane * kPer + j]);
-          const float2 q = *reinterpret_cast<const float2*>(&sm.q[t][lane * kPer + j]);
-          d[j] = t == s ? 1.f - f.x : d[j] * f.x;
-          d[j + 1] = t == s ? 1.f - f.y : d[j + 1] * f.y;
-          x = fmaf(q.x, d[j], x);
-          x = fmaf(q.y, d[j + 1], x);
+          for (int j = 0; j < kPer; j += 2) {
+            const float2 f = *reinterpret_cast<const float2*>(&sm.f[t][lane * kPer + j]);
+            const float2 q = *reinterpret_cast<const float2*>(&sm.q[t][lane * kPer + j]);
+            d[j] = t == s ? 1.f - f.x : d[j] * f.x;
+            d[j + 1] = t == s ? 1.f - f.y : d[j + 1] * f.y;
+            x = fmaf(q.x, d[j], x);
+            x = fmaf(q.y, d[j + 1], x);
+          }
         }
+        a[t] = x;
       }
-      a[t] = x;
-    }
-    // sums over the lanes: each exchange halves the values a lane holds
-    int t_mine = 0;
+      // sums over the lanes: each exchange halves the values a lane holds
+      int t_mine = 0;
 #pragma unroll
-    for (int n = kBlock / 2, o = 16; n >= 1; n >>= 1, o >>= 1) {
-      const bool up = lane & o;
+      for (int n = kBlock / 2, o = 16; n >= 1; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
 #pragma unroll
-      for (int i = 0; i < n; ++i) {
-        const float give = up ? a[i] : a[i + n];
-        a[i] = (up ? a[i + n] : a[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+        for (int i = 0; i < n; ++i) {
+          const float give = up ? a[i] : a[i + n];
+          a[i] = (up ? a[i + n] : a[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+        t_mine = t_mine * 2 + (up ? 1 : 0);
       }
-      t_mine = t_mine * 2 + (up ? 1 : 0);
+      a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+      if ((lane & 1) == 0) split_store(&sm.a[buf][0][t_mine * Sm::kPitchA + s], kBlock * Sm::kPitchA, a[0]);
     }
-    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
-    if ((lane & 1) == 0) split_store(&sm.a[buf][0][t_mine * Smem<CP>::kPitchA + s], kBlock * Smem<CP>::kPitchA, a[0]);
   };
   auto tensor = [&](int buf) {
     if (live) {
@@ -290,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
       uint32_t va[kVTerms][4];
 #pragma unroll
       for (int i = 0; i < kVTerms; ++i)
-        ldmatrix_x4_trans(&sm.v[buf][i][((lane & 7) + ((lane >> 4) & 1) * 8) * Smem<CP>::kPitchE + e0 + ((lane >> 3) & 1) * 8], va[i][0],
+        ldmatrix_x4_trans(&sm.v[buf][i][((lane & 7) + ((lane >> 4) & 1) * 8) * Sm::kPitchE + e0 + ((lane >> 3) & 1) * 8], va[i][0],
                           va[i][1], va[i][2], va[i][3]);
       if (FULL) {
         float o[2][4] = {};
@@ -307,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
           uint32_t b[kTerms][4];  // tokens 0-7: [0], [1]; tokens 8-15: [2], [3]
 #pragma unroll
           for (int i = 0; i < kTerms; ++i)
-            ldmatrix_x4(&sm.qd[buf][i][((lane & 7) + (lane >> 4) * 8) * Smem<CP>::kPitchC + c0 + k * 16 + ((lane >> 3) & 1) * 8], b[i][0], b[i][1],
+            ldmatrix_x4(&sm.qd[buf][i][((lane & 7) + (lane >> 4) * 8) * Sm::kPitchC + c0 + k * 16 + ((lane >> 3) & 1) * 8], b[i][0], b[i][1],
                         b[i][2], b[i][3]);
 #pragma unroll
           for (int n = 0; n < 2; ++n) {
@@ -321,7 +332,7 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
           uint32_t b[kTerms][4];
 #pragma unroll
           for (int i = 0; i < kTerms; ++i)
-            ldmatrix_x4(&sm.a[buf][i][((lane & 7) + (lane >> 4) * 8) * Smem<CP>::kPitchA + ((lane >> 3) & 1) * 8], b[i][0], b[i][1], b[i][2],
+            ldmatrix_x4(&sm.a[buf][i][((lane & 7) + (lane >> 4) * 8) * Sm::kPitchA + ((lane >> 3) & 1) * 8], b[i][0], b[i][1], b[i][2],
                         b[i][3]);
           // each half of the channels adds this product for half of the tokens
           uint32_t b0[kTerms], b1[kTerms];
@@ -343,7 +354,7 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
         uint32_t b[kTerms][4];  // channels c0 + 16 k .. + 7: [0], [1]; + 8 ..: [2], [3]
 #pragma unroll
         for (int i = 0; i < kTerms; ++i)
-          ldmatrix_x4_trans(&sm.kd[buf][i][(lane & 15) * Smem<CP>::kPitchC + c0 + k * 16 + (lane >> 4) * 8], b[i][0], b[i][1], b[i][2], b[i][3]);
+          ldmatrix_x4_trans(&sm.kd[buf][i][(lane & 15) * Sm::kPitchC + c0 + k * 16 + (lane >> 4) * 8], b[i][0], b[i][1], b[i][2], b[i][3]);
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
           const float2 F = *reinterpret_cast<const float2*>(&sm.F[buf][c0 + k * 16 + n * 8 + cc]);
@@ -357,20 +368,21 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
       }
     }
   };
-  // RMSNorm over E, one token per warp
+  // RMSNorm over E, on the lanes of a token
   auto norm = [&](int s0) {
-        const int t = warp;
-    if (s0 + t < s_end) {
-      float x[4], ss = 0.f;
+    float x[4], ss = 0.f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int e = lane * 4 + j;
-        x[j] = e < E ? sm.o[0][t][e] + sm.o[1][t][e] : 0.f;
-        ss += x[j] * x[j];
-      }
-      const float inv = 1.0f / sqrtf(warp_sum(ss) / static_cast<float>(E) + p.eps);
-      if (lane * 4 < E) {
-        T* dst = static_cast<T*>(p.out) + ((static_cast<int64_t>(b) * p.S + s0 + t) * H + h) * E + lane * 4;
+    for (int j = 0; j < 4; ++j) {
+      const int e = x4 + j;
+      x[j] = e < E ? sm.o[0][tok][e] + sm.o[1][tok][e] : 0.f;
+      ss += x[j] * x[j];
+    }
+#pragma unroll
+    for (int o = 16 / kPerWarp; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float inv = 1.0f / sqrtf(ss / static_cast<float>(E) + p.eps);
+    if (s0 + tok < s_end) {
+      if (x4 < E) {
+        T* dst = static_cast<T*>(p.out) + ((static_cast<int64_t>(b) * p.S + s0 + tok) * H + h) * E + x4;
         uint2 v;
         v.x = pack2<T>(x[0] * inv * sm.w[x4], x[1] * inv * sm.w[x4 + 1]);
         v.y = pack2<T>(x[2] * inv * sm.w[x4 + 2], x[3] * inv * sm.w[x4 + 3]);
@@ -413,21 +425,23 @@ __global__ void __launch_bounds__(kThreads, 1) hgrn2_blocks_kernel(const Hgrn2Pa
       each([&](float& x, int c, int row) { p.state[bh * mat + static_cast<int64_t>(c) * E + row] = x; });
   } else {
     each([&](float& x, int c, int row) { sg.part[(seg * all_bh + bh) * mat + static_cast<int64_t>(c) * E + row] = x; });
-    if (tid < C) sg.decay[(seg * all_bh + bh) * C + tid] = decay;  // (part 0: threads of the first 8 tokens)
+    if (tid < kChannelThreads && tid < C) sg.decay[(seg * all_bh + bh) * C + tid] = decay;  // (part 0: threads of the first 8 tokens)
   }
 }
 
-// Segments wanted: as many CTAs as SMs.  Grows with S, so that the workspace of a longer call serves a shorter one.
-int64_t wanted_segments(int B, int S, int H) {
-  int64_t n = device_sm_count() / (static_cast<int64_t>(B) * H);
+bool narrow(int C, int E) { return C <= kNarrow && E <= kNarrow; }
+
+// Segments wanted: as many CTAs as the SMs hold.  Grows with S, so that the workspace of a longer call serves a shorter one.
+int64_t wanted_segments(int B, int S, int H, int C, int E) {
+  int64_t n = device_sm_count() * (narrow(C, E) ? 2ll : 1ll) / (static_cast<int64_t>(B) * H);
   n = n > kMaxSegments ? kMaxSegments : n;
   n = n > S / kMinSegment ? S / kMinSegment : n;
   return n < 1 ? 1 : n;
 }
 
-Segments plan(int B, int S, int H) {
+Segments plan(int B, int S, int H, int C, int E) {
   Segments s{};
-  const int64_t n = wanted_segments(B, S, H);
+  const int64_t n = wanted_segments(B, S, H, C, E);
   int tokens = static_cast<int>((S + n - 1) / n);
   tokens = (tokens + kBlock - 1) / kBlock * kBlock;
   s.tokens = tokens;
@@ -435,21 +449,27 @@ Segments plan(int B, int S, int H) {
   return s;
 }
 
-template <typename T, int CP>
+template <typename T, int CP, int THREADS>
 int launch(const Hgrn2Params& p, const Segments& sg, int B, cudaStream_t st) {
-  constexpr int smem = static_cast<int>(sizeof(Smem<CP>));
-  auto full = hgrn2_blocks_kernel<T, CP, true>;
-  auto part = hgrn2_blocks_kernel<T, CP, false>;
+  constexpr int smem = static_cast<int>(sizeof(Smem<CP, THREADS == 256 ? kNarrow : kMaxE>));
+  auto full = hgrn2_blocks_kernel<T, CP, true, THREADS>;
+  auto part = hgrn2_blocks_kernel<T, CP, false, THREADS>;
   static std::atomic<unsigned long long> full_set{0}, part_set{0};
   LRI_ONCE_PER_DEVICE(full_set, cudaFuncSetAttribute(full, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   LRI_ONCE_PER_DEVICE(part_set, cudaFuncSetAttribute(part, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   if (sg.count > 1) {
-    LRI_CUDA(launch_pdl(part, dim3(sg.count - 1, p.H, B), dim3(kThreads), static_cast<size_t>(smem), st, p, sg));
+    LRI_CUDA(launch_pdl(part, dim3(sg.count - 1, p.H, B), dim3(THREADS), static_cast<size_t>(smem), st, p, sg));
     LRI_LAUNCH_CHECK("hgrn2_blocks_kernel<part>");
   }
-  LRI_CUDA(launch_pdl(full, dim3(sg.count, p.H, B), dim3(kThreads), static_cast<size_t>(smem), st, p, sg));
+  LRI_CUDA(launch_pdl(full, dim3(sg.count, p.H, B), dim3(THREADS), static_cast<size_t>(smem), st, p, sg));
   LRI_LAUNCH_CHECK("hgrn2_blocks_kernel");
   return LRI_OK;
+}
+
+template <typename T>
+int launch_shape(const Hgrn2Params& p, const Segments& sg, int B, cudaStream_t st) {
+  if (narrow(p.C, p.E)) return launch<T, 64, 256>(p, sg, B, st);
+  return p.C <= 64 ? launch<T, 64, 512>(p, sg, B, st) : launch<T, 128, 512>(p, sg, B, st);
 }
 
 }  // namespace
@@ -461,20 +481,18 @@ bool hgrn2_blocks_supports(int dtype, const Hgrn2Params& p, int B) {
 }
 
 size_t hgrn2_blocks_workspace_bytes(int B, int S, int H, int C, int E) {
-  const int64_t n = wanted_segments(B, S, H);
+  const int64_t n = wanted_segments(B, S, H, C, E);
   if (n < 2) return 0;
   return static_cast<size_t>(B) * H * C * (static_cast<size_t>(n) * E + n - 1) * sizeof(float);
 }
 
 int hgrn2_blocks_launch(int dtype, const Hgrn2Params& p, int B, void* workspace, cudaStream_t st) {
-  Segments sg = plan(B, p.S, p.H);
+  Segments sg = plan(B, p.S, p.H, p.C, p.E);
   const size_t mat = static_cast<size_t>(B) * p.H * p.C * p.E;
   sg.init = static_cast<float*>(workspace);
   sg.part = sg.init + mat;
   sg.decay = sg.part + mat * (sg.count - 1);
-  const bool bf = dtype == LRI_BF16;
-  if (p.C <= 64) return bf ? launch<bf16, 64>(p, sg, B, st) : launch<__half, 64>(p, sg, B, st);
-  return bf ? launch<bf16, 128>(p, sg, B, st) : launch<__half, 128>(p, sg, B, st);
+  return dtype == LRI_BF16 ? launch_shape<bf16>(p, sg, B, st) : launch_shape<__half>(p, sg, B, st);
 }
 
 }  // namespace lri
