@@ -73,7 +73,8 @@ int lri_set_gemm_backend(int backend);
  * window_tc (LRI_WINDOW_TC: 0 keeps sliding-window attention on the plain kernel), hgrn2_blocks
  * (LRI_HGRN2_BLOCKS: 0 keeps the HGRN2 recurrence token by token), scan_columns (LRI_SCAN_COLUMNS: state columns per
  * lane of the matrix-state recurrences, 0 choose, 1, 2, 4), scan_warps (LRI_SCAN_WARPS: their warps per CTA, 0 choose, 1, 2, 4),
- * scan_lanes (LRI_SCAN_LANES: lanes per state column, 0 choose, 8, 16).  Unknown
+ * scan_lanes (LRI_SCAN_LANES: lanes per state column, 0 choose, 8, 16), scan_segments (LRI_SCAN_SEGMENTS: segments of a sequence
+ * that run side by side, 0 choose, 1..16).  Unknown
  * names and values an option does not take return LRI_ERR_ARG.  No counterpart in the reference
  * (its only switches are benchmark.py's command-line flags). */
 int lri_set_option(const char* name, int value);
@@ -445,6 +446,12 @@ int lri_gla_blocks(int dtype, const float* proj, int64_t ld, int64_t q_off, int6
 int lri_state_scan(const float* qd, const float* kd, const float* ku, const float* decay, const float* coef, const float* v,
                    int64_t v_row, float* state, const void* input_pos, int pos_is_i64, float* o, int B, int S, int heads,
                    int dim, int vdim, lri_stream_t stream);
+/* The same with room for the states between segments of a sequence, which then run side by side: calls of few sequences and many
+ * tokens leave most of the chip idle otherwise.  workspace NULL or smaller than lri_state_scan_workspace_bytes(...): one segment. */
+size_t lri_state_scan_workspace_bytes(int B, int S, int heads, int dim, int vdim, int delta);
+int lri_state_scan_segments(const float* qd, const float* kd, const float* ku, const float* decay, const float* coef, const float* v,
+                            int64_t v_row, float* state, const void* input_pos, int pos_is_i64, float* o, int B, int S, int heads,
+                            int dim, int vdim, void* workspace, size_t workspace_bytes, lri_stream_t stream);
 /* One token per sequence, everything between the input projections and the output projection's rows in one kernel; inputs
  * as above, the low-rank second projections included: a2 [heads dim, a_rank] and g2 [heads vdim, g_rank] in `dtype` multiply
  * the columns at a_off and g_off rounded to `dtype` (ranks multiples of 8, zero padded).  out (pitch out_ld) = factor *

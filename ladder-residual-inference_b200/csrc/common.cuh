@@ -70,6 +70,7 @@ enum Option {
   OPT_SCAN_COLUMNS,     // LRI_SCAN_COLUMNS   state columns per lane of the recurrence kernel: 1, 2, 4 (0 = choose)
   OPT_SCAN_WARPS,       // LRI_SCAN_WARPS     warps per CTA of that kernel: 1, 2, 4 (0 = choose)
   OPT_SCAN_LANES,       // LRI_SCAN_LANES     lanes per state column of that kernel: 8, 16 (0 = choose)
+  OPT_SCAN_SEGMENTS,    // LRI_SCAN_SEGMENTS  segments of a sequence that run side by side: 1..16 (0 = choose)
   OPT_COUNT
 };
 int option(int which);

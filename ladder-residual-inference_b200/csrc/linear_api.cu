@@ -56,6 +56,7 @@ const OptionSpec kOptionSpecs[OPT_COUNT] = {
     {"scan_columns", "LRI_SCAN_COLUMNS", 0, 0, 4},
     {"scan_warps", "LRI_SCAN_WARPS", 0, 0, 4},
     {"scan_lanes", "LRI_SCAN_LANES", 0, 0, 16},
+    {"scan_segments", "LRI_SCAN_SEGMENTS", 0, 0, 16},
 };
 
 bool option_value_ok(int which, int v) {

@@ -97,6 +97,12 @@ class LayerEngine(Engine):
             vectors = buf(4 * blocks, hc, torch.float32), buf(4 * blocks if delta else 0, hc, torch.float32), buf(4 * blocks, hc, torch.float32)
             self.scan_blocks = vectors + (buf(blocks, hc, torch.float32), buf(blocks, 32 * most(scans, lambda m: m.heads), torch.float32))
             self.ws_low = workspace(ops.linear_f32_workspace_bytes, *[m.a2.shape[0] for m in scans], *[m.g2.shape[0] for m in delta])
+            self.ws_scan = None
+            if hasattr(ops, "state_scan_workspace_bytes"):
+                # fewer sequences are cut into more segments: the largest batch is not the largest workspace
+                size = max(ops.state_scan_workspace_bytes(b, max_seq, m.heads, m.dim, m.vdim, m in delta)
+                           for m in scans for b in range(1, max_batch + 1))
+                self.ws_scan = torch.empty(size, dtype=torch.uint8, device=device) if size else None
         if delta:
             self.scan_v = buf(rows, most(delta, lambda m: m.out_width), torch.float32)
             self.scan_gate = buf(rows, most(delta, lambda m: m.out_width), torch.float32)
@@ -171,6 +177,10 @@ class LayerEngine(Engine):
         self.ops.round_columns(self.proj, self.ld, off, w.shape[1], self.low, rows)
         self.ops.linear_f32(self.low, w, out, rows, workspace=self.ws_low)
 
+    def _scan(self, delta, v, v_row, m, pos, B, S):
+        kw = {} if self.ws_scan is None else dict(workspace=self.ws_scan)
+        self.ops.state_scan(self.scan_blocks, delta, v, v_row, m.kv_cache.state, pos, self.scan_o, B, S, **kw)
+
     def _gla(self, m, rows, B, S, pos, eps):
         ops, at, proj = self.ops, _offsets(m.parts(), self.off), self.proj.view(-1)
         if S == 1 and ops.state_step_supports(m.dim, m.vdim, m.a2.shape[1], 0):
@@ -179,7 +189,7 @@ class LayerEngine(Engine):
             return
         self._low_rank(at["a1"], m.a2, self.scan_z, rows)
         ops.gla_blocks(self.proj, self.ld, (at["q"], at["k"]), self.scan_z, m.a2_bias, m.tau, self.scan_blocks, B, S, m.heads, m.dim)
-        ops.state_scan(self.scan_blocks, False, proj[at["v"]:], self.ld, m.kv_cache.state, pos, self.scan_o, B, S)
+        self._scan(False, proj[at["v"]:], self.ld, m, pos, B, S)
         ops.head_norm_gate(self.scan_o, m.norm, eps, proj[at["g"]:], self.ld, "silu", 1.0, self.y, m.out_width, rows, m.heads)
 
     def _grouped(self, m, at, y, y_ld, factor, rows, B, S, pos, eps):
@@ -204,7 +214,7 @@ class LayerEngine(Engine):
         v = m.out_width
         ops.delta_blocks(self.proj, self.ld, (at["q"], at["k"], at["v"], at["b"]), convs, ring, self.scan_z, m.a_log, m.dt_bias,
                          pos, self.scan_blocks, self.scan_v, B, S, m.heads, m.kv_heads, m.dim, m.vdim)
-        ops.state_scan(self.scan_blocks, True, self.scan_v, v, m.kv_cache.state, pos, self.scan_o, B, S)
+        self._scan(True, self.scan_v, v, m, pos, B, S)
         ops.head_norm_gate(self.scan_o, m.norm, eps, self.scan_gate, v, "sigmoid", factor, y, y_ld, rows, m.heads)
 
     def _parallel(self, m, rows, B, S, pos, eps):

@@ -384,15 +384,22 @@ class CudaOps:
                                        _C.stream_handle()))
 
     @staticmethod
-    def state_scan(blocks, delta, v, v_row, state, input_pos, o, B, S):
-        """v starts at its first column."""
+    def state_scan_workspace_bytes(B, S, heads, dim, vdim, delta):
+        return _C.lib.lri_state_scan_workspace_bytes(B, S, heads, dim, vdim, int(delta))
+
+    @staticmethod
+    def state_scan(blocks, delta, v, v_row, state, input_pos, o, B, S, workspace=None):
+        """v starts at its first column.  With a workspace long calls run in segments side by side."""
         _C.require_cuda(*[x for x in blocks if x is not None], v, state, input_pos, o)
         qd, kd, ku, decay, coef = blocks
         _, heads, dim, vdim = state.shape
-        _C.check(_C.lib.lri_state_scan(qd.data_ptr(), kd.data_ptr() if delta else None, ku.data_ptr(), decay.data_ptr(),
-                                       coef.data_ptr(), v.data_ptr(), v_row, state.data_ptr(), input_pos.data_ptr(),
-                                       int(input_pos.dtype == torch.int64), o.data_ptr(), B, S, heads, dim, vdim,
-                                       _C.stream_handle()))
+        if workspace is not None:
+            _C.require_cuda(workspace)
+        _C.check(_C.lib.lri_state_scan_segments(qd.data_ptr(), kd.data_ptr() if delta else None, ku.data_ptr(), decay.data_ptr(),
+                                                coef.data_ptr(), v.data_ptr(), v_row, state.data_ptr(), input_pos.data_ptr(),
+                                                int(input_pos.dtype == torch.int64), o.data_ptr(), B, S, heads, dim, vdim,
+                                                None if workspace is None else workspace.data_ptr(),
+                                                0 if workspace is None else workspace.numel(), _C.stream_handle()))
 
     @staticmethod
     def state_step_supports(dim, vdim, decay_rank, gate_rank):
