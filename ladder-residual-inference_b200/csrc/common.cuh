@@ -71,6 +71,7 @@ enum Option {
   OPT_SCAN_WARPS,       // LRI_SCAN_WARPS     warps per CTA of that kernel: 1, 2, 4 (0 = choose)
   OPT_SCAN_LANES,       // LRI_SCAN_LANES     lanes per state column of that kernel: 8, 16 (0 = choose)
   OPT_SCAN_SEGMENTS,    // LRI_SCAN_SEGMENTS  segments of a sequence that run side by side: 1..16 (0 = choose)
+  OPT_FOLD_NORM,        // LRI_FOLD_NORM      0: decode steps of one sequence take their norms in kernels of their own
   OPT_COUNT
 };
 int option(int which);

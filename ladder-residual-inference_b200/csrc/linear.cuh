@@ -36,6 +36,13 @@ struct ExpertArgs {
   GluParams glu;
 };
 
+// Add and RMSNorm in front of a projection of one row: x = norm(res + add1 + add2) * weight, each sum rounded (add1, add2 may be NULL).
+struct NormArgs {
+  const void *res, *add1, *add2, *weight;  // [k]; weight NULL: x is given
+  void* res_out;                           // the sum, written once; not `res`, which every CTA reads; may be NULL
+  float eps;
+};
+
 struct LinearParams {
   const void* x;  // [m, k]
   const void* w;  // PLAIN/QKV: [n, k]; SWIGLU: [2n, k] = [up rows | gate rows]
@@ -55,6 +62,7 @@ struct LinearParams {
   PushArgs push;       // PLAIN epilogue of the SIMT kernel only
   ExpertArgs ex;       // expert weights chosen on the device
   bool one_sm;         // prompt projections: not the kernel on pairs of SMs (LRI_ONE_SM)
+  NormArgs nm;         // one-row QKV and SWIGLU forms of the SIMT kernel
   ArgmaxArgs am;       // ARGMAX epilogue of the SIMT kernel: greedy choice instead of stored logits
 };
 
@@ -102,6 +110,14 @@ __device__ __forceinline__ void qkv_epilogue_pair(const LinearParams& p, int64_t
 int streaming_rows();  // token rows up to which the streaming kernels run (option stream_rows)
 // decode path, 1 <= p.m <= 8 (SIMT FMA)
 int gemv_launch(int dtype, int epi, const LinearParams& p, cudaStream_t st);
+// one row whose norm is taken on the way (p.nm): EPI_QKV and EPI_SWIGLU
+bool gemv_norm_supports(int64_t m, int k);
+int gemv_norm_launch(int dtype, int epi, const LinearParams& p, cudaStream_t st);
+// The projections of linear_api.cu with that norm in front; one row, no workspace
+int norm_qkv_rope_kvcache(int dtype, const NormArgs& nm, const void* wqkv, const void* rope_table, const void* input_pos, int pos_is_i64,
+                          void* q_out, void* k_cache, void* v_cache, int K, int n_head, int n_kv, int head_dim, int64_t smax,
+                          int64_t table_rows, cudaStream_t st);
+int norm_gateup_swiglu(int dtype, const NormArgs& nm, const void* w1, void* h, int I, int K, cudaStream_t st);
 // decode path, 1 <= p.m <= 16 (same streaming, tensor-core FMA)
 constexpr int kGemvMmaMaxRows = 16;
 int gemv_mma_launch(int dtype, int epi, const LinearParams& p, cudaStream_t st);

@@ -57,6 +57,7 @@ const OptionSpec kOptionSpecs[OPT_COUNT] = {
     {"scan_warps", "LRI_SCAN_WARPS", 0, 0, 4},
     {"scan_lanes", "LRI_SCAN_LANES", 0, 0, 16},
     {"scan_segments", "LRI_SCAN_SEGMENTS", 0, 0, 16},
+    {"fold_norm", "LRI_FOLD_NORM", 1, 0, 1},
 };
 
 bool option_value_ok(int which, int v) {
@@ -477,6 +478,22 @@ extern "C" size_t lri_gateup_workspace_bytes(int64_t M, int I) {
   return max_size(gateup_raw_bytes(M, I), streamk_bytes(EPI_SWIGLU, M, I));
 }
 
+static int check_norm(const char* who, int dtype, const NormArgs& nm, const void* w, int K) {
+  int rc = check_common(who, dtype, nm.res, w, 1, K);
+  if (rc != LRI_OK) return rc;
+  LRI_REQUIRE(nm.weight && nm.res_out != nm.res, LRI_ERR_ARG, "%s: norm without a weight, or in place", who);
+  LRI_REQUIRE(aligned16(nm.add1) && aligned16(nm.add2) && aligned16(nm.weight) && aligned16(nm.res_out), LRI_ERR_ALIGN,
+              "%s: pointers must be 16-byte aligned", who);
+  return LRI_OK;
+}
+int lri::norm_gateup_swiglu(int dtype, const NormArgs& nm, const void* w1, void* h, int I, int K, cudaStream_t st) {
+  int rc = check_norm("gateup_swiglu", dtype, nm, w1, K);
+  if (rc != LRI_OK) return rc;
+  LRI_REQUIRE(h != nullptr && I > 0, LRI_ERR_ARG, "gateup_swiglu: h is NULL or I=%d", I);
+  LinearParams p{};
+  p.nm = nm, p.x = nm.res, p.w = w1, p.y = h, p.m = 1, p.n = I, p.k = K;
+  return gemv_norm_launch(dtype, EPI_SWIGLU, p, st);
+}
 extern "C" int lri_gateup_swiglu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K,
                                  void* workspace, size_t workspace_bytes, lri_stream_t stream) {
   int rc = check_common("gateup_swiglu", dtype, x, w1, M, K);
@@ -555,6 +572,32 @@ extern "C" size_t lri_qkv_workspace_bytes(int64_t M, int n_head, int n_kv, int h
                   streamk_bytes(EPI_QKV, M, static_cast<int64_t>(n_head + 2 * n_kv) * head_dim));
 }
 
+static int check_qkv(const void* rope_table, const void* input_pos, const void* q_out, const void* k_cache, const void* v_cache, int n_head,
+                     int n_kv, int head_dim, int64_t smax, int64_t table_rows) {
+  LRI_REQUIRE(rope_table && input_pos && q_out && k_cache && v_cache, LRI_ERR_ARG, "qkv_rope_kvcache: NULL pointer");
+  LRI_REQUIRE(n_head > 0 && n_kv > 0 && head_dim > 0 && head_dim % 8 == 0, LRI_ERR_UNSUPPORTED,
+              "qkv_rope_kvcache: n_head=%d n_kv=%d head_dim=%d (head_dim must be a multiple of 8)", n_head, n_kv,
+              head_dim);
+  LRI_REQUIRE(smax > 0 && table_rows > 0, LRI_ERR_ARG, "qkv_rope_kvcache: smax=%lld table_rows=%lld", (long long)smax,
+              (long long)table_rows);
+  LRI_REQUIRE(aligned16(q_out) && aligned16(k_cache) && aligned16(v_cache) && aligned16(rope_table), LRI_ERR_ALIGN,
+              "qkv_rope_kvcache: outputs and table must be 16-byte aligned");
+  return LRI_OK;
+}
+int lri::norm_qkv_rope_kvcache(int dtype, const NormArgs& nm, const void* wqkv, const void* rope_table, const void* input_pos, int pos_is_i64,
+                               void* q_out, void* k_cache, void* v_cache, int K, int n_head, int n_kv, int head_dim, int64_t smax,
+                               int64_t table_rows, cudaStream_t st) {
+  int rc = check_norm("qkv_rope_kvcache", dtype, nm, wqkv, K);
+  if (rc != LRI_OK) return rc;
+  rc = check_qkv(rope_table, input_pos, q_out, k_cache, v_cache, n_head, n_kv, head_dim, smax, table_rows);
+  if (rc != LRI_OK) return rc;
+  LinearParams p{};
+  p.nm = nm, p.x = nm.res, p.w = wqkv, p.m = 1, p.n = (n_head + 2 * n_kv) * head_dim, p.k = K;
+  p.rope_table = rope_table, p.input_pos = input_pos, p.pos_is_i64 = pos_is_i64;
+  p.q_out = q_out, p.k_cache = k_cache, p.v_cache = v_cache;
+  p.S = 1, p.n_head = n_head, p.n_kv = n_kv, p.head_dim = head_dim, p.smax = smax, p.table_rows = table_rows;
+  return gemv_norm_launch(dtype, EPI_QKV, p, st);
+}
 extern "C" int lri_qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, const void* rope_table,
                                     const void* input_pos, int pos_is_i64, void* q_out, void* k_cache, void* v_cache,
                                     int B, int S, int K, int n_head, int n_kv, int head_dim, int64_t smax,
@@ -564,14 +607,8 @@ extern "C" int lri_qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, 
   const int64_t M = static_cast<int64_t>(B) * S;
   int rc = check_common("qkv_rope_kvcache", dtype, x, wqkv, M, K);
   if (rc != LRI_OK) return rc;
-  LRI_REQUIRE(rope_table && input_pos && q_out && k_cache && v_cache, LRI_ERR_ARG, "qkv_rope_kvcache: NULL pointer");
-  LRI_REQUIRE(n_head > 0 && n_kv > 0 && head_dim > 0 && head_dim % 8 == 0, LRI_ERR_UNSUPPORTED,
-              "qkv_rope_kvcache: n_head=%d n_kv=%d head_dim=%d (head_dim must be a multiple of 8)", n_head, n_kv,
-              head_dim);
-  LRI_REQUIRE(smax > 0 && table_rows > 0, LRI_ERR_ARG, "qkv_rope_kvcache: smax=%lld table_rows=%lld", (long long)smax,
-              (long long)table_rows);
-  LRI_REQUIRE(aligned16(q_out) && aligned16(k_cache) && aligned16(v_cache) && aligned16(rope_table), LRI_ERR_ALIGN,
-              "qkv_rope_kvcache: outputs and table must be 16-byte aligned");
+  rc = check_qkv(rope_table, input_pos, q_out, k_cache, v_cache, n_head, n_kv, head_dim, smax, table_rows);
+  if (rc != LRI_OK) return rc;
   if (M == 0) return LRI_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LinearParams p{};

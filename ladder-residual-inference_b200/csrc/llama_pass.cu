@@ -4,7 +4,7 @@
 // A decode step of a small model is a chain of 2 to 4 us kernels; called one by one from Python each costs 8 us of host time (stories110M,
 // 125 launches: 1004 us a step for 290 us of device time).  One call per pass leaves the launches themselves.  Nothing is kept between
 // calls: every pointer comes from the caller, who reads it from the model's tensors for this pass.
-#include "common.cuh"
+#include "linear.cuh"
 
 using namespace lri;
 
@@ -31,9 +31,13 @@ struct Pass {
   }
   bool attention(int l) {
     void *kc = const_cast<void*>(at(l, kKCache)), *vc = const_cast<void*>(at(l, kVCache));
-    if (!ok(lri_qkv_rope_kvcache(p.dtype, p.normed, at(l, kQkv), p.rope_table, p.input_pos, p.pos_is_i64, p.q, kc, vc, p.B, p.S, p.dim, p.n_head,
-                                 p.n_kv, p.head_dim, p.smax, p.table_rows, 0, p.ws_qkv, p.ws_qkv_bytes, p.stream)))
-      return false;
+    return ok(lri_qkv_rope_kvcache(p.dtype, p.normed, at(l, kQkv), p.rope_table, p.input_pos, p.pos_is_i64, p.q, kc, vc, p.B, p.S, p.dim, p.n_head,
+                                   p.n_kv, p.head_dim, p.smax, p.table_rows, 0, p.ws_qkv, p.ws_qkv_bytes, p.stream)) &&
+           attend(l);
+  }
+  // from the queries and the caches to the output projection
+  bool attend(int l) {
+    void *kc = const_cast<void*>(at(l, kKCache)), *vc = const_cast<void*>(at(l, kVCache));
     const bool done =
         p.S == 1 ? ok(lri_attn_decode(p.dtype, p.q, kc, vc, p.input_pos, p.pos_is_i64, p.y, p.B, p.n_head, p.n_kv, p.head_dim, p.smax, p.splits,
                                       p.scratch, p.scratch_bytes, p.stream))
@@ -87,27 +91,70 @@ struct Pass {
     }
     return norm(p.final_norm, pending, nullptr, false, p.normed, p.stream);
   }
-  // where a sublayer reduces, its partial is added to the residual first, and the sum (here: itself) is the new residual
-  bool fold(const void* partial) {
-    return ok(lri_add_rmsnorm(p.dtype, p.resid, partial, nullptr, 1.0f, nullptr, p.eps, p.resid, nullptr, rows, p.dim, p.stream));
+
+  // ---- one row, called eagerly: norms taken by the projections behind them ----------------------------------------
+  // Small models called eagerly are bound by the host, 2.3 us a launch: five launches a layer instead of seven take 49 of the 195 us that the
+  // launches of a stories110M step take (step 302 -> 250 us).  On the device the chain gets no shorter, because each of a projection's CTAs
+  // works out the norm after the wait (captured: 196 us with kernels for the norms, 209 without; Ladder-Llama 1B 457 and 623).  So captured
+  // steps and wider models keep them.  The results are the same bits.
+  const void* cur = nullptr;  // the residual, and where the next sum goes: every CTA of a projection reads the one, so it is not written
+  void* other = nullptr;
+  bool folds() {
+    if (!option(OPT_FOLD_NORM) || p.n_layer < 1 || !p.row_ws || rows != 1 || !gemv_norm_supports(1, p.dim)) return false;
+    cudaStreamCaptureStatus status;
+    return cudaStreamIsCapturing(static_cast<cudaStream_t>(p.stream), &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
   }
-  bool desync() {
+  bool folded_qkv(int l, const void* add1, bool write) {
+    void *kc = const_cast<void*>(at(l, kKCache)), *vc = const_cast<void*>(at(l, kVCache));
+    const NormArgs nm{cur, add1, nullptr, at(l, kAttentionNorm), write ? other : nullptr, p.eps};
+    return ok(norm_qkv_rope_kvcache(p.dtype, nm, at(l, kQkv), p.rope_table, p.input_pos, p.pos_is_i64, p.q, kc, vc, p.dim, p.n_head, p.n_kv,
+                                    p.head_dim, p.smax, p.table_rows, static_cast<cudaStream_t>(p.stream)));
+  }
+  bool folded_up(int l, const void* add1, const void* add2, bool write) {
+    const NormArgs nm{cur, add1, add2, at(l, kMlpNorm), write ? other : nullptr, p.eps};
+    return ok(norm_gateup_swiglu(p.dtype, nm, at(l, kW1), p.h, p.inter, p.dim, static_cast<cudaStream_t>(p.stream)));
+  }
+  bool down(int l, const void* addend) {
+    return ok(lri_linear(p.dtype, p.h, at(l, kW2), addend, p.part_m, rows, p.dim, p.inter, p.ws_w2, p.ws_w2_bytes, p.stream));
+  }
+  void written() {
+    void* was = const_cast<void*>(cur);
+    cur = other, other = was;
+  }
+  bool last_norm(const void* add1, const void* add2) {
+    return ok(lri_add_rmsnorm(p.dtype, cur, add1, add2, 1.0f, p.final_norm, p.eps, nullptr, p.normed, rows, p.dim, p.stream));
+  }
+  bool folded_dense() {
     const void* pending = nullptr;
     for (int l = 0; l < p.n_layer; ++l) {
-      if (!norm(at(l, kAttentionNorm), pending, nullptr, true, p.normed, p.stream) || !attention(l)) return false;
-      pending = p.part_a;
-      if (p.reduces[2 * l]) {
-        if (!fold(pending)) return false;
-        pending = nullptr;
-      }
-      if (!norm(at(l, kMlpNorm), pending, nullptr, true, p.normed, p.stream) || !mlp(l, p.normed, nullptr, p.stream)) return false;
+      if (!folded_qkv(l, pending, pending)) return false;
+      if (pending) written();
+      if (!attend(l) || !folded_up(l, p.part_a, nullptr, true)) return false;
+      written();
+      if (!down(l, nullptr)) return false;
       pending = p.part_m;
-      if (p.reduces[2 * l + 1]) {
-        if (!fold(pending)) return false;
-        pending = nullptr;
-      }
     }
-    return norm(p.final_norm, pending, nullptr, false, p.normed, p.stream);
+    return last_norm(pending, nullptr);
+  }
+  // both sublayers start from the residual before the layer; the MLP's projection adds the results of the layer before and writes the sum
+  bool folded_ladder() {
+    for (int l = 0; l < p.n_layer; ++l) {
+      const void *add1 = l ? p.part_a : nullptr, *add2 = l ? p.part_m : nullptr;
+      if (!folded_qkv(l, add1, false) || !folded_up(l, add1, add2, l > 0)) return false;
+      if (l) written();
+      if (!attend(l) || !down(l, nullptr)) return false;
+    }
+    return last_norm(p.part_a, p.part_m);
+  }
+  bool folded_parallel() {
+    const void* pending = nullptr;
+    for (int l = 0; l < p.n_layer; ++l) {
+      if (!folded_qkv(l, pending, false) || !attend(l) || !folded_up(l, pending, nullptr, pending != nullptr)) return false;
+      if (pending) written();
+      if (!down(l, p.part_a)) return false;
+      pending = p.part_m;
+    }
+    return last_norm(pending, nullptr);
   }
 };
 
@@ -120,12 +167,23 @@ extern "C" int lri_llama_run(const lri_llama_pass* pass) {
               "llama_pass: two streams need events and a second buffer");
   LRI_REQUIRE(pass->schedule != LRI_DESYNC || pass->reduces != nullptr, LRI_ERR_ARG, "llama_pass: NULL flags");
   Pass run{*pass, static_cast<int64_t>(pass->B) * pass->S};
+  if (run.folds()) {
+    run.cur = pass->resid, run.other = pass->row_ws;
+    switch (pass->schedule) {
+      case LRI_DENSE:
+      case LRI_DESYNC: run.folded_dense(); return run.rc;
+      case LRI_LADDER:
+      case LRI_LADDER_TWO_STREAMS: run.folded_ladder(); return run.rc;
+      case LRI_PARALLEL: run.folded_parallel(); return run.rc;
+    }
+  }
   switch (pass->schedule) {
-    case LRI_DENSE: run.dense(); break;
+    case LRI_DENSE:
+    // on one GPU a partial that is reduced at once and one that is added by the next norm are the same sums
+    case LRI_DESYNC: run.dense(); break;
     case LRI_LADDER: run.ladder(); break;
     case LRI_LADDER_TWO_STREAMS: run.ladder_two_streams(); break;
     case LRI_PARALLEL: run.parallel(); break;
-    case LRI_DESYNC: run.desync(); break;
     default: return fail(LRI_ERR_ARG, "llama_pass: schedule %d", pass->schedule);
   }
   return run.rc;

@@ -28,7 +28,7 @@ class LlamaPass(ctypes.Structure):
                 + [(k, c_void_p) for k in ("layers", "reduces", "rope_table", "input_pos", "final_norm", "resid", "normed", "normed_m", "part_a",
                                            "part_m", "q", "y", "h", "ws_qkv", "ws_wo", "ws_ug", "ws_w2", "scratch")]
                 + [(k, c_size_t) for k in ("ws_qkv_bytes", "ws_wo_bytes", "ws_ug_bytes", "ws_w2_bytes", "scratch_bytes")]
-                + [(k, c_void_p) for k in ("stream", "side", "events")])
+                + [(k, c_void_p) for k in ("stream", "side", "events", "row_ws")])
 
 
 ONE_SM = 0x100  # LRI_ONE_SM

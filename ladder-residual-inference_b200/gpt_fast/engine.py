@@ -53,8 +53,8 @@ class Engine:
         rows = max_batch * max_seq
         self.max_rows = rows
 
-        def buf(cols):
-            return torch.empty(rows, cols, dtype=dtype, device=device)
+        def buf(cols, n=rows):
+            return torch.empty(n, cols, dtype=dtype, device=device)
 
         self.resid, self.normed = buf(self.d), buf(self.d)
         self.part_a, self.part_m = buf(self.d), buf(self.d)
@@ -74,6 +74,8 @@ class Engine:
         self.ws_w2 = workspace(self.ops.linear_workspace_bytes, self.d)
         nbytes = self.ops.attn_decode_scratch_bytes(max_batch, self.nh, self.nkv, self.hd, _MAX_SPLITS)
         self.scratch = torch.zeros(max(nbytes, 16), dtype=torch.uint8, device=device)
+        # one sequence: the second residual of passes whose projections take the norms
+        self.row_ws = buf(self.d, 1)
         self._setup_head(max_batch, device, dtype)
         # ladder decode runs the attention and MLP chains of a layer on two streams (LRI_LADDER_OVERLAP=0: one)
         self.overlap_sublayers = (self.family == "ladder" and self.resid.is_cuda and
@@ -235,7 +237,7 @@ class Engine:
             return False
         main = torch.cuda.current_stream()
         tensors = dict(rope_table=m.freqs_cis, input_pos=pos, final_norm=m.norm.weight, resid=self.resid, normed=self.normed, part_a=self.part_a,
-                       part_m=self.part_m, q=self.q, y=self.y, h=self.h)
+                       part_m=self.part_m, q=self.q, y=self.y, h=self.h, row_ws=self.row_ws)
         if two:
             tensors["normed_m"] = self.normed_m
         sizes = dict(dtype=dtype_code(self.dtype), n_layer=len(m.layers), B=B, S=S, n_head=self.nh, n_kv=self.nkv, head_dim=self.hd, dim=self.d,
