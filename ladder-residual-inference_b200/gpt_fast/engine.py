@@ -201,12 +201,14 @@ class Engine:
             return False
         two = family == "ladder" and S == 1 and self.overlap_sublayers
         # The call passes one set of sizes for all layers; the Python form reads each weight's.  A layer that was given others, or whose weights
-        # are not plain parameters, runs there.  (nn.Module's attribute access costs as much as a comparison of sizes: 100 to 150 ns.)
+        # are not plain parameters, runs there.  (nn.Module's attribute access costs as much as a comparison of sizes: 100 to 150 ns.  A step of
+        # a small model is bound by this and by the launches.)
         nqkv = (self.nh + 2 * self.nkv) * self.hd
         want_qkv, want_wo, want_w1, want_w2 = (nqkv, self.d), (self.d, self.nh * self.hd), (2 * self.inter, self.d), (self.d, self.inter)
         want_both = (nqkv + 2 * self.inter, self.d)
         smax = None
-        weights, caches, reduces = [], [], [] if family == "desync" else None
+        # a layer's attention norm, QKV, wo, MLP norm, w1, w2, K cache, V cache; where w1 is the lower part of a tensor, the bytes above it
+        tensors, above, reduces = [], [], [] if family == "desync" else None
         try:
             for layer in m.layers:
                 sub = layer._modules
@@ -218,35 +220,35 @@ class Engine:
                     smax = length
                 if length != smax or wo.shape != want_wo:
                     return False
-                caches += (k_cache, cache["v_cache"])
                 norm = sub["attention_norm"]._parameters["weight"]
                 if family == "parallel":
                     w, w2 = att["wqkv1"]._parameters["weight"], att["w2"]._parameters["weight"]
                     if w.shape != want_both or w2.shape != want_w2 or sub["attention"].qkv_rows != nqkv:
                         return False
-                    weights += (norm, w, wo, norm, (w, nqkv), w2)
+                    tensors += (norm, w, wo, norm, w, w2, k_cache, cache["v_cache"])
+                    above.append(nqkv * w.stride(0) * w.element_size())
                     continue
                 mlp = sub["feed_forward"]._modules
                 w, w1, w2 = att["wqkv"]._parameters["weight"], mlp["w1"]._parameters["weight"], mlp["w2"]._parameters["weight"]
                 if w.shape != want_qkv or w1.shape != want_w1 or w2.shape != want_w2:
                     return False
-                weights += (norm, w, wo, sub["ffn_norm"]._parameters["weight"], w1, w2)
+                tensors += (norm, w, wo, sub["ffn_norm"]._parameters["weight"], w1, w2, k_cache, cache["v_cache"])
                 if reduces is not None:
                     reduces += (int(layer.do_attention_all_reduce), int(layer.do_mlp_all_reduce))
         except KeyError:
             return False
         main = torch.cuda.current_stream()
-        tensors = dict(rope_table=m.freqs_cis, input_pos=pos, final_norm=m.norm.weight, resid=self.resid, normed=self.normed, part_a=self.part_a,
+        buffers = dict(rope_table=m.freqs_cis, input_pos=pos, final_norm=m.norm.weight, resid=self.resid, normed=self.normed, part_a=self.part_a,
                        part_m=self.part_m, q=self.q, y=self.y, h=self.h, row_ws=self.row_ws)
         if two:
-            tensors["normed_m"] = self.normed_m
+            buffers["normed_m"] = self.normed_m
         sizes = dict(dtype=dtype_code(self.dtype), n_layer=len(m.layers), B=B, S=S, n_head=self.nh, n_kv=self.nkv, head_dim=self.hd, dim=self.d,
                      inter=self.inter, pos_is_i64=int(pos.dtype == torch.int64), splits=self._splits, smax=smax,
                      table_rows=m.freqs_cis.shape[0])
         schedule = {"dense": DENSE, "ladder": LADDER_TWO_STREAMS if two else LADDER, "parallel": PARALLEL, "desync": DESYNC}[family]
-        self.ops.run_layers(schedule, weights, caches, reduces, self._events if two else None, main.cuda_stream,
+        self.ops.run_layers(schedule, tensors, above, reduces, self._events if two else None, main.cuda_stream,
                             self.side_stream.cuda_stream if two else None, sizes, self.cfg.norm_eps,
-                            dict(ws_qkv=self.ws_qkv, ws_wo=self.ws_wo, ws_ug=self.ws_ug, ws_w2=self.ws_w2, scratch=self.scratch), **tensors)
+                            dict(ws_qkv=self.ws_qkv, ws_wo=self.ws_wo, ws_ug=self.ws_ug, ws_w2=self.ws_w2, scratch=self.scratch), **buffers)
         return True
 
     @torch.no_grad()

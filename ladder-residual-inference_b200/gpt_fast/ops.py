@@ -5,6 +5,7 @@ tensors and raises otherwise.  The engine takes the ops object as a parameter so
 schedule logic can be exercised by tests with a stand-in.
 """
 import ctypes
+from array import array
 from functools import partial
 
 import torch
@@ -123,23 +124,14 @@ class CudaOps:
 
     # ---- all layers of a pass ------------------------------------------------------------------------
     @staticmethod
-    def run_layers(schedule, weights, caches, reduces, events, main, side, sizes, eps, workspaces, **tensors):
-        """lri_llama_run: `weights` six a layer (attention norm, QKV, wo, MLP norm, w1, w2; (tensor, first row) for a slice), `caches` two a layer,
-        `sizes` the integers of lri_llama_pass, `workspaces` and `tensors` by its names."""
-        _C.require_cuda(*tensors.values(), *caches)
-        pointers = []
-        for i, w in enumerate(weights):
-            row = 0
-            if type(w) is tuple:
-                w, row = w
-            if not w.is_cuda:
-                _C.require_cuda(w)
-            pointers.append(w.data_ptr() + row * w.stride(0) * w.element_size() if row else w.data_ptr())
-            if i % 6 == 5:
-                at = i // 6 * 2
-                pointers += (caches[at].data_ptr(), caches[at + 1].data_ptr())
-        layers = (ctypes.c_void_p * len(pointers))(*pointers)
-        p = _C.LlamaPass(schedule=schedule, eps=float(eps), stream=main, side=side, layers=ctypes.cast(layers, ctypes.c_void_p), **sizes)
+    def run_layers(schedule, layers, above, reduces, events, main, side, sizes, eps, workspaces, **tensors):
+        """lri_llama_run: `layers` eight tensors a layer as there, `above` the bytes in front of each layer's w1 (empty: none), `sizes` the
+        integers of lri_llama_pass, `workspaces` and `tensors` by its names."""
+        _C.require_cuda(*tensors.values(), *layers)
+        pointers = array("Q", [t.data_ptr() for t in layers])
+        for i, n in enumerate(above):
+            pointers[8 * i + 4] += n
+        p = _C.LlamaPass(schedule=schedule, eps=float(eps), stream=main, side=side, layers=pointers.buffer_info()[0], **sizes)
         for k, t in tensors.items():
             setattr(p, k, t.data_ptr())
         for k, t in workspaces.items():
