@@ -39,6 +39,9 @@ enum lri_dtype { LRI_BF16 = 0, LRI_FP16 = 1, LRI_FP32 = 2 };
  * that gives a tile to one SM.  For passes that run kernels of theirs on a second stream beside their projections (see
  * csrc/gemm_pair.cu). */
 enum { LRI_ONE_SM = 0x100 };
+/* The same for lri_qkv_rope_kvcache, lri_gateup_swiglu and lri_linear: another stream's projections run beside this one, so small batches
+ * take shared memory that leaves room for them.  The results are the same bits. */
+enum { LRI_BESIDE = 0x200 };
 
 enum lri_status {
   LRI_OK = 0,

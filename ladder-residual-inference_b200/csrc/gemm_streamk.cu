@@ -378,6 +378,22 @@ int plan_ctas(int tiles, int total_kt, int max_seg) {
   return static_cast<int>(ctas);
 }
 
+// Stages of the ring: all the shared memory an SM has to give, up to eight.  Beside another stream's projections (the two chains of a ladder
+// layer) half of it, so that two CTAs share an SM: one's weights arrive while the other waits for its token rows or finishes.  A whole step, us,
+// whole ring / half: 8B, 2, 4, 8, 16, 24, 40, 64 sequences 2783 / 2664, 2822 / 2660, 2898 / 2802, 2998 / 2923, 3346 / 3187, 3897 / 3707, 4467 /
+// 4356; 1B, 2, 4, 16, 24, 40, 64 651 / 635, 679 / 650, 748 / 715, 822 / 791, 931 / 861, 1126 / 1087.  Alone on the GPU the half ring is the
+// slower one (8B dense, 16 sequences 3528 / 3639).  With 5 to 8 rows only the other projections of a narrow model are on the streaming kernel, whose
+// CTAs want the room themselves: gated ones keep four stages (1B, 6 and 8 sequences 691, 715 whole, 707, 756 half, 682, 712 with four).
+int ring_stages(const LinearParams& lin, int stage_bytes, int accumulators) {
+  constexpr int kHalf = 108 * 1024;
+  int stages = kSmemBudget / stage_bytes;
+  if (lin.beside) {
+    stages = kHalf / stage_bytes;
+    if (accumulators == 2 && lin.m > 4 && lin.m <= 8 && lin.k < 4096) stages = 4;
+  }
+  return stages > 8 ? 8 : stages;
+}
+
 template <typename T, int BN, int EPI>
 int launch(int dtype, const LinearParams& lin, float* partial, cudaStream_t st) {
   constexpr int kAcc = Acc<EPI>::kCount;
@@ -394,8 +410,7 @@ int launch(int dtype, const LinearParams& lin, float* partial, cudaStream_t st) 
   rc = make_tmap(&tx, dtype, lin.x, lin.m, lin.k, BN);
   if (rc != LRI_OK) return rc;
   constexpr int kStageBytes = (kAcc * kBM + BN) * kBK * 2;
-  const int stages = kSmemBudget / kStageBytes;
-  p.stages = stages > 8 ? 8 : stages;
+  p.stages = ring_stages(lin, kStageBytes, kAcc);
   const int smem = p.stages * kStageBytes + 1024;
   auto kern = gemm_streamk_kernel<T, BN, EPI>;
   static std::atomic<unsigned long long> attr_set{0};  // per template instantiation, one bit per device

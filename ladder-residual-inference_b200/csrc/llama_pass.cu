@@ -16,6 +16,7 @@ struct Pass {
   const lri_llama_pass& p;
   int64_t rows;
   int rc = LRI_OK;
+  int beside = 0;  // LRI_BESIDE where two streams run
 
   const void* at(int layer, int which) const { return p.layers[static_cast<int64_t>(layer) * kPointers + which]; }
   bool ok(int r) { return (rc = r) == LRI_OK; }
@@ -31,7 +32,7 @@ struct Pass {
   }
   bool attention(int l) {
     void *kc = const_cast<void*>(at(l, kKCache)), *vc = const_cast<void*>(at(l, kVCache));
-    return ok(lri_qkv_rope_kvcache(p.dtype, p.normed, at(l, kQkv), p.rope_table, p.input_pos, p.pos_is_i64, p.q, kc, vc, p.B, p.S, p.dim, p.n_head,
+    return ok(lri_qkv_rope_kvcache(p.dtype | beside, p.normed, at(l, kQkv), p.rope_table, p.input_pos, p.pos_is_i64, p.q, kc, vc, p.B, p.S, p.dim, p.n_head,
                                    p.n_kv, p.head_dim, p.smax, p.table_rows, 0, p.ws_qkv, p.ws_qkv_bytes, p.stream)) &&
            attend(l);
   }
@@ -42,11 +43,11 @@ struct Pass {
         p.S == 1 ? ok(lri_attn_decode(p.dtype, p.q, kc, vc, p.input_pos, p.pos_is_i64, p.y, p.B, p.n_head, p.n_kv, p.head_dim, p.smax, p.splits,
                                       p.scratch, p.scratch_bytes, p.stream))
                  : ok(lri_attn_prefill(p.dtype, p.q, kc, vc, p.input_pos, p.pos_is_i64, p.y, p.B, p.S, p.n_head, p.n_kv, p.head_dim, p.smax, p.stream));
-    return done && ok(lri_linear(p.dtype, p.y, at(l, kWo), nullptr, p.part_a, rows, p.dim, p.n_head * p.head_dim, p.ws_wo, p.ws_wo_bytes, p.stream));
+    return done && ok(lri_linear(p.dtype | beside, p.y, at(l, kWo), nullptr, p.part_a, rows, p.dim, p.n_head * p.head_dim, p.ws_wo, p.ws_wo_bytes, p.stream));
   }
   bool mlp(int l, const void* normed, const void* addend, lri_stream_t st) {
-    return ok(lri_gateup_swiglu(p.dtype, normed, at(l, kW1), p.h, rows, p.inter, p.dim, p.ws_ug, p.ws_ug_bytes, st)) &&
-           ok(lri_linear(p.dtype, p.h, at(l, kW2), addend, p.part_m, rows, p.dim, p.inter, p.ws_w2, p.ws_w2_bytes, st));
+    return ok(lri_gateup_swiglu(p.dtype | beside, normed, at(l, kW1), p.h, rows, p.inter, p.dim, p.ws_ug, p.ws_ug_bytes, st)) &&
+           ok(lri_linear(p.dtype | beside, p.h, at(l, kW2), addend, p.part_m, rows, p.dim, p.inter, p.ws_w2, p.ws_w2_bytes, st));
   }
   bool record(int i, lri_stream_t st) {
     return cuda(cudaEventRecord(static_cast<cudaEvent_t>(p.events[i]), static_cast<cudaStream_t>(st)), "cudaEventRecord");
@@ -74,6 +75,7 @@ struct Pass {
   // the attention chain of a layer on `stream`, its MLP chain on `side`: see Engine._run_ladder_two_streams
   bool ladder_two_streams() {
     if (!record(0, p.stream) || !wait(0, p.side)) return false;
+    beside = LRI_BESIDE;
     int n = 1;
     for (int l = 0; l < p.n_layer; ++l, n += 2) {
       if (!norm(at(l, kAttentionNorm), l ? p.part_a : nullptr, nullptr, true, p.normed, p.stream) || !record(n, p.stream) || !attention(l)) return false;
