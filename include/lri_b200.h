@@ -494,7 +494,7 @@ typedef struct {
   void *ws_qkv, *ws_wo, *ws_ug, *ws_w2, *scratch;
   size_t ws_qkv_bytes, ws_wo_bytes, ws_ug_bytes, ws_w2_bytes, scratch_bytes;
   lri_stream_t stream, side;
-  void* const* events; /* two streams: 2 n_layer + 2 cudaEvent_t */
+  void* const* events; /* two streams: 2 n_layer + 2 cudaEvent_t; LRI_PARALLEL with events runs gate/up on `side` beside the attention chain */
   void* row_ws; /* one row: dim elements; with them small models called eagerly leave norms to the projections behind.  NULL: never */
 } lri_llama_pass;
 int lri_llama_run(const lri_llama_pass* pass);

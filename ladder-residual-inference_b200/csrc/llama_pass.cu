@@ -94,6 +94,22 @@ struct Pass {
     return norm(p.final_norm, pending, nullptr, false, p.normed, p.stream);
   }
 
+  // the gate/up projection beside the attention chain: both read the norm
+  bool parallel_two_streams() {
+    const void* pending = nullptr;
+    beside = rows > 8 ? LRI_BESIDE : 0;  // (3B, whole / half ring: 2 sequences 1677 / 1779 us, 4 1785 / 1903, 16 2445 / 2390, 40 3499 / 3495)
+    for (int l = 0; l < p.n_layer; ++l) {
+      if (!norm(at(l, kAttentionNorm), pending, nullptr, true, p.normed, p.stream) || !record(2 * l, p.stream) || !wait(2 * l, p.side)) return false;
+      if (!attention(l) ||
+          !ok(lri_gateup_swiglu(p.dtype | beside, p.normed, at(l, kW1), p.h, rows, p.inter, p.dim, p.ws_ug, p.ws_ug_bytes, p.side)) ||
+          !record(2 * l + 1, p.side) || !wait(2 * l + 1, p.stream) ||
+          !ok(lri_linear(p.dtype | beside, p.h, at(l, kW2), p.part_a, p.part_m, rows, p.dim, p.inter, p.ws_w2, p.ws_w2_bytes, p.stream)))
+        return false;
+      pending = p.part_m;
+    }
+    return norm(p.final_norm, pending, nullptr, false, p.normed, p.stream);
+  }
+
   // ---- one row, called eagerly: norms taken by the projections behind them ----------------------------------------
   // Small models called eagerly are bound by the host, 2.3 us a launch: five launches a layer instead of seven take 49 of the 195 us that the
   // launches of a stories110M step take (step 302 -> 250 us).  On the device the chain gets no shorter, because each of a projection's CTAs
@@ -185,7 +201,7 @@ extern "C" int lri_llama_run(const lri_llama_pass* pass) {
     case LRI_DESYNC: run.dense(); break;
     case LRI_LADDER: run.ladder(); break;
     case LRI_LADDER_TWO_STREAMS: run.ladder_two_streams(); break;
-    case LRI_PARALLEL: run.parallel(); break;
+    case LRI_PARALLEL: pass->events ? run.parallel_two_streams() : run.parallel(); break;
     default: return fail(LRI_ERR_ARG, "llama_pass: schedule %d", pass->schedule);
   }
   return run.rc;

@@ -77,14 +77,16 @@ class Engine:
         # one sequence: the second residual of passes whose projections take the norms
         self.row_ws = buf(self.d, 1)
         self._setup_head(max_batch, device, dtype)
-        # ladder decode runs the attention and MLP chains of a layer on two streams (LRI_LADDER_OVERLAP=0: one)
-        self.overlap_sublayers = (self.family == "ladder" and self.resid.is_cuda and
+        # ladder and parallel decode run the two sides of a layer on two streams (LRI_LADDER_OVERLAP=0: one); parallel in native passes only
+        self.overlap_sublayers = (self.family in ("ladder", "parallel") and self.resid.is_cuda and
                                   os.environ.get("LRI_LADDER_OVERLAP", "1") != "0")
         if self.overlap_sublayers:
-            self.normed_m = buf(self.d)
+            if self.family == "ladder":
+                self.normed_m = buf(self.d)
             # (same priority as the main stream: giving the MLP chain, four fifths of a layer's bytes, the higher
             # priority was measured slower on B200, 2.80 against 2.58 ms per 8B step)
             self.side_stream = torch.cuda.Stream()
+            self.sms = torch.cuda.get_device_properties(self.resid.device).multi_processor_count
             self._events = [torch.cuda.Event() for _ in range(2 * cfg.n_layer + 2)]
             for e in self._events:
                 e.record()  # an event has a handle from its first recording on
@@ -190,6 +192,20 @@ class Engine:
         if not self._run_native(B, S, input_pos):
             getattr(self, "_run_" + self.family)(rows, B, S, input_pos)
 
+    def _two_streams(self, B):
+        """Whether a native decode pass runs the two sides of a layer on two streams (ladder: attention and MLP chain, parallel: the attention
+        chain and gate/up).  Not a small model called eagerly, which is bound by the host (stories110M ladder, 4 sequences 301 us on one
+        stream, 322 on two, parallel 268 and 303), nor one sequence of parallel blocks called so (3B 1496 and 1510, captured 1467 and 1400).
+        And not parallel blocks of 128-wide heads with about one (sequence, KV head) pair an SM: their attention fills the chip for one
+        pair's length, and gate/up in between only delays it (3B, 6 and 7 sequences 1974 and 2045 us on one stream, 2010 and 2074 on two;
+        5, 8 and 12 2055, 2091 and 2326 to 1872, 2081 and 2072)."""
+        if not self.overlap_sublayers:
+            return False
+        parallel = self.family == "parallel"
+        if (self.d < 1024 or (parallel and B == 1)) and not torch.cuda.is_current_stream_capturing():
+            return False
+        return not parallel or self.hd != 128 or not 7 * self.sms <= 8 * B * self.nkv <= 10 * self.sms
+
     def _run_native(self, B, S, pos):
         """The schedule's kernels in one native call, on one GPU; False where it has to run from here: with communication, another ops object,
         blocks of both kinds, layers of unequal sizes."""
@@ -199,7 +215,7 @@ class Engine:
         mixed = getattr(self.cfg, "ladder_layers", None)
         if family == "ladder" and mixed is not None and len(set(mixed)) != self.cfg.n_layer or not 0 < len(m.layers) == self.cfg.n_layer:
             return False
-        two = family == "ladder" and S == 1 and self.overlap_sublayers
+        two = S == 1 and self._two_streams(B)
         # The call passes one set of sizes for all layers; the Python form reads each weight's.  A layer that was given others, or whose weights
         # are not plain parameters, runs there.  (nn.Module's attribute access costs as much as a comparison of sizes: 100 to 150 ns.  A step of
         # a small model is bound by this and by the launches.)
@@ -240,7 +256,7 @@ class Engine:
         main = torch.cuda.current_stream()
         buffers = dict(rope_table=m.freqs_cis, input_pos=pos, final_norm=m.norm.weight, resid=self.resid, normed=self.normed, part_a=self.part_a,
                        part_m=self.part_m, q=self.q, y=self.y, h=self.h, row_ws=self.row_ws)
-        if two:
+        if two and family == "ladder":
             buffers["normed_m"] = self.normed_m
         sizes = dict(dtype=dtype_code(self.dtype), n_layer=len(m.layers), B=B, S=S, n_head=self.nh, n_kv=self.nkv, head_dim=self.hd, dim=self.d,
                      inter=self.inter, pos_is_i64=int(pos.dtype == torch.int64), splits=self._splits, smax=smax,

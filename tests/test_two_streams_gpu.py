@@ -1,0 +1,52 @@
+"""Decode passes whose layers run on two streams: captured steps (two streams, half of the ring in the small-batch projections) against eager ones of the same
+small model (one stream, whole ring), bit for bit, many replays behind one another; and the rule that chooses."""
+import pytest
+import torch
+
+from test_llama_pass_gpu import _model, _only
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("batch", [1, 2, 5, 8, 9, 16, 17, 33, 64])
+@pytest.mark.parametrize("family", ["ladder", "parallel"])
+@pytest.mark.parametrize("sizes", [{}, dict(dim=960, n_head=15, n_local_heads=5, intermediate_size=2056)], ids=["256", "960"])
+def test_captured_steps_on_two_streams(family, batch, dtype, sizes):
+    model = _model(family, dtype, batch, **sizes)
+    engine = model._engine
+    _only(engine, True)
+    tok = torch.randint(0, 512, (batch, 1), generator=torch.Generator().manual_seed(1)).to(torch.int32).cuda()
+    pos = torch.tensor([0], dtype=torch.int32, device="cuda")
+    assert engine.overlap_sublayers and not engine._two_streams(batch)
+    with torch.no_grad():
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            model(tok, pos)
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            assert engine._two_streams(batch)
+            logits = model(tok, pos)
+        for p in (1, 2, 40, 150):
+            pos.fill_(p)
+            for _ in range(5):
+                graph.replay()
+            captured = logits.clone()
+            assert torch.isfinite(captured.float()).all() and torch.equal(captured, model(tok, pos))
+    torch.cuda.synchronize()
+    from gpt_fast import _C
+    assert _C.lib.lri_gemm_status() == 0
+
+
+def test_choice_of_streams():
+    """Wide models take two streams eagerly too; parallel blocks not where attention has about one 128-wide pair an SM."""
+    engine = _model("parallel", torch.bfloat16, 2, dim=2048, n_head=16, n_local_heads=16, intermediate_size=512)._engine
+    engine.sms = 148
+    assert [b for b in range(1, 65) if not engine._two_streams(b)] == [1, 9, 10, 11]
+    engine.hd = 64
+    assert [b for b in range(1, 65) if not engine._two_streams(b)] == [1]
+    engine = _model("ladder", torch.bfloat16, 2, dim=2048, n_head=16, n_local_heads=16, intermediate_size=512)._engine
+    assert all(engine._two_streams(b) for b in range(1, 65))
+    assert not _model("dense", torch.bfloat16, 2)._engine._two_streams(1)
