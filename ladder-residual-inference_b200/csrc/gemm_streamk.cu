@@ -302,8 +302,13 @@ __global__ void __launch_bounds__(256) streamk_finish_kernel(const StreamKParams
   const int tile = blockIdx.x;
   int first_cta, nseg;
   tile_segments(tile, p, first_cta, nseg);
+  // The kernel behind may come as soon as the projection's CTAs leave their SMs: its weights, which nothing here writes, arrive beside the sums
+  // below.  us a step, let in behind the wait / before: 8B dense, 16 sequences 3549 / 3510; 1B, 16 925 / 868; stories110M, 16 400 / 355; Migosun
+  // 1B, 24 1282 / 1175, 8B, 16 4690 / 4640.  Not where another stream's kernels wait for the same SMs, which it would keep out (8B ladder, 16
+  // sequences 3103 / 3310).
+  if (!p.lin.beside) pdl_launch_dependents();
   pdl_wait();
-  pdl_launch_dependents();
+  if (p.lin.beside) pdl_launch_dependents();
   if (nseg == 1 && EPI != EPI_QKV) return;
   const float* tile_partial = p.partial + static_cast<int64_t>(tile) * p.max_seg * kSlot;
   if (EPI == EPI_SWIGLU || EPI == EPI_GLU) {
@@ -387,7 +392,7 @@ int plan_ctas(int tiles, int total_kt, int max_seg) {
 int ring_stages(const LinearParams& lin, int stage_bytes, int accumulators) {
   constexpr int kHalf = 108 * 1024;
   int stages = kSmemBudget / stage_bytes;
-  if (lin.beside) {
+  if (lin.half_ring) {
     stages = kHalf / stage_bytes;
     if (accumulators == 2 && lin.m > 4 && lin.m <= 8 && lin.k < 4096) stages = 4;
   }

@@ -62,7 +62,7 @@ struct LinearParams {
   PushArgs push;       // PLAIN epilogue of the SIMT kernel only
   ExpertArgs ex;       // expert weights chosen on the device
   bool one_sm;         // prompt projections: not the kernel on pairs of SMs (LRI_ONE_SM)
-  bool beside;         // small batches: another stream's projections run beside this one (LRI_BESIDE)
+  bool beside, half_ring;  // small batches: what runs on another stream at the same time (LRI_BESIDE, LRI_HALF_RING)
   NormArgs nm;         // one-row QKV and SWIGLU forms of the SIMT kernel
   ArgmaxArgs am;       // ARGMAX epilogue of the SIMT kernel: greedy choice instead of stored logits
 };

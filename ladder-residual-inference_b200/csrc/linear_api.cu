@@ -379,7 +379,7 @@ extern "C" int lri_gemm_status(void) {
   return LRI_OK;
 }
 
-// takes a flag (LRI_ONE_SM, LRI_BESIDE) out of `dtype`
+// takes a flag (LRI_ONE_SM, LRI_BESIDE, LRI_HALF_RING) out of `dtype`
 static bool take_flag(int& dtype, int flag) {
   const bool set = dtype >= 0 && (dtype & flag) != 0;
   if (set) dtype &= ~flag;
@@ -397,7 +397,7 @@ static int check_common(const char* who, int dtype, const void* x, const void* w
 
 extern "C" int lri_linear(int dtype, const void* x, const void* w, const void* addend, void* y, int64_t M, int N,
                           int K, void* workspace, size_t workspace_bytes, lri_stream_t stream) {
-  const bool one_sm = take_flag(dtype, LRI_ONE_SM), beside = take_flag(dtype, LRI_BESIDE);
+  const bool one_sm = take_flag(dtype, LRI_ONE_SM), beside = take_flag(dtype, LRI_BESIDE), half_ring = take_flag(dtype, LRI_HALF_RING);
   if (dtype == LRI_FP32 || (K > 0 && K % 8 != 0)) {
     LRI_REQUIRE(dtype >= LRI_BF16 && dtype <= LRI_FP32, LRI_ERR_UNSUPPORTED, "linear: dtype %d", dtype);
     LRI_REQUIRE(x && w && y, LRI_ERR_ARG, "linear: NULL pointer");
@@ -411,14 +411,14 @@ extern "C" int lri_linear(int dtype, const void* x, const void* w, const void* a
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (M <= streaming_rows()) {
     LinearParams p{};
-    p.x = x, p.w = w, p.y = y, p.addend = addend, p.m = static_cast<int>(M), p.n = N, p.k = K, p.beside = beside;
+    p.x = x, p.w = w, p.y = y, p.addend = addend, p.m = static_cast<int>(M), p.n = N, p.k = K, p.beside = beside, p.half_ring = half_ring;
     if (streamk_few_rows(EPI_PLAIN, p, workspace, workspace_bytes))
       return gemm_streamk_launch(dtype, EPI_PLAIN, p, workspace, workspace_bytes, st);
     return streaming_launch(dtype, EPI_PLAIN, p, st, prefer_simt_gemv());
   }
   if (streamk_rows(M)) {
     LinearParams p{};
-    p.x = x, p.w = w, p.y = y, p.addend = addend, p.m = static_cast<int>(M), p.n = N, p.k = K, p.beside = beside;
+    p.x = x, p.w = w, p.y = y, p.addend = addend, p.m = static_cast<int>(M), p.n = N, p.k = K, p.beside = beside, p.half_ring = half_ring;
     if (gemm_streamk_supports(EPI_PLAIN, p, workspace, workspace_bytes))
       return gemm_streamk_launch(dtype, EPI_PLAIN, p, workspace, workspace_bytes, st);
   }
@@ -496,14 +496,14 @@ int lri::norm_gateup_swiglu(int dtype, const NormArgs& nm, const void* w1, void*
 }
 extern "C" int lri_gateup_swiglu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K,
                                  void* workspace, size_t workspace_bytes, lri_stream_t stream) {
-  const bool beside = take_flag(dtype, LRI_BESIDE);
+  const bool beside = take_flag(dtype, LRI_BESIDE), half_ring = take_flag(dtype, LRI_HALF_RING);
   int rc = check_common("gateup_swiglu", dtype, x, w1, M, K);
   if (rc != LRI_OK) return rc;
   LRI_REQUIRE(h != nullptr && I > 0, LRI_ERR_ARG, "gateup_swiglu: h is NULL or I=%d", I);
   if (M == 0) return LRI_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LinearParams p{};
-  p.x = x, p.w = w1, p.y = h, p.m = static_cast<int>(M), p.n = I, p.k = K, p.beside = beside;
+  p.x = x, p.w = w1, p.y = h, p.m = static_cast<int>(M), p.n = I, p.k = K, p.beside = beside, p.half_ring = half_ring;
   if (M <= streaming_rows() && !streamk_few_rows(EPI_SWIGLU, p, workspace, workspace_bytes))
     return streaming_launch(dtype, EPI_SWIGLU, p, st, prefer_simt_gemv());
   if ((M <= streaming_rows() || streamk_rows(M)) && gemm_streamk_supports(EPI_SWIGLU, p, workspace, workspace_bytes))
@@ -605,7 +605,7 @@ extern "C" int lri_qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, 
                                     int64_t table_rows, int table_gathered, void* workspace,
                                     size_t workspace_bytes, lri_stream_t stream) {
   LRI_REQUIRE(B >= 0 && S >= 0, LRI_ERR_ARG, "qkv_rope_kvcache: B=%d S=%d", B, S);
-  const bool beside = take_flag(dtype, LRI_BESIDE);
+  const bool beside = take_flag(dtype, LRI_BESIDE), half_ring = take_flag(dtype, LRI_HALF_RING);
   const int64_t M = static_cast<int64_t>(B) * S;
   int rc = check_common("qkv_rope_kvcache", dtype, x, wqkv, M, K);
   if (rc != LRI_OK) return rc;
@@ -614,7 +614,7 @@ extern "C" int lri_qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, 
   if (M == 0) return LRI_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LinearParams p{};
-  p.x = x, p.w = wqkv, p.m = static_cast<int>(M), p.n = (n_head + 2 * n_kv) * head_dim, p.k = K, p.beside = beside;
+  p.x = x, p.w = wqkv, p.m = static_cast<int>(M), p.n = (n_head + 2 * n_kv) * head_dim, p.k = K, p.beside = beside, p.half_ring = half_ring;
   p.rope_table = rope_table, p.input_pos = input_pos, p.pos_is_i64 = pos_is_i64;
   p.q_out = q_out, p.k_cache = k_cache, p.v_cache = v_cache;
   p.S = S, p.n_head = n_head, p.n_kv = n_kv, p.head_dim = head_dim, p.smax = smax, p.table_rows = table_rows, p.table_gathered = table_gathered;

@@ -16,7 +16,7 @@ struct Pass {
   const lri_llama_pass& p;
   int64_t rows;
   int rc = LRI_OK;
-  int beside = 0;  // LRI_BESIDE where two streams run
+  int beside = 0;  // LRI_BESIDE, LRI_HALF_RING where two streams run
 
   const void* at(int layer, int which) const { return p.layers[static_cast<int64_t>(layer) * kPointers + which]; }
   bool ok(int r) { return (rc = r) == LRI_OK; }
@@ -75,7 +75,7 @@ struct Pass {
   // the attention chain of a layer on `stream`, its MLP chain on `side`: see Engine._run_ladder_two_streams
   bool ladder_two_streams() {
     if (!record(0, p.stream) || !wait(0, p.side)) return false;
-    beside = LRI_BESIDE;
+    beside = LRI_BESIDE | LRI_HALF_RING;
     int n = 1;
     for (int l = 0; l < p.n_layer; ++l, n += 2) {
       if (!norm(at(l, kAttentionNorm), l ? p.part_a : nullptr, nullptr, true, p.normed, p.stream) || !record(n, p.stream) || !attention(l)) return false;
@@ -97,7 +97,7 @@ struct Pass {
   // the gate/up projection beside the attention chain: both read the norm
   bool parallel_two_streams() {
     const void* pending = nullptr;
-    beside = rows > 8 ? LRI_BESIDE : 0;  // (3B, whole / half ring: 2 sequences 1677 / 1779 us, 4 1785 / 1903, 16 2445 / 2390, 40 3499 / 3495)
+    beside = LRI_BESIDE | (rows > 8 ? LRI_HALF_RING : 0);  // (3B, whole / half ring: 2 sequences 1677 / 1779 us, 4 1785 / 1903, 16 2445 / 2390, 40 3499 / 3495)
     for (int l = 0; l < p.n_layer; ++l) {
       if (!norm(at(l, kAttentionNorm), pending, nullptr, true, p.normed, p.stream) || !record(2 * l, p.stream) || !wait(2 * l, p.side)) return false;
       if (!attention(l) ||
