@@ -73,12 +73,15 @@ __global__ void __launch_bounds__(THREADS) gated_norm_add_kernel(const GatedNorm
   pdl_launch_dependents();
   pdl_wait();
   float t[NV][VEC];
-  [[maybe_unused]] float res[NV][VEC];
+  [[maybe_unused]] float res[NV][VEC], gate[NV][VEC];
   if constexpr (PRE) {
-    if (p.resid)
 #pragma unroll
-      for (int i = 0; i < NV; ++i)
-        if (threadIdx.x + i * THREADS < nvec) load_v<float, VEC>(p.resid + row * dim + (threadIdx.x + i * THREADS) * VEC, res[i]);
+    for (int i = 0; i < NV; ++i) {
+      const int v = threadIdx.x + i * THREADS;
+      if (v >= nvec) continue;
+      if (p.resid) load_v<float, VEC>(p.resid + row * dim + v * VEC, res[i]);
+      if (p.gate) load_v<float, VEC>(p.gate + row * p.gate_ld + v * VEC, gate[i]);
+    }
   }
   float ss = 0.f;
 #pragma unroll
@@ -87,23 +90,32 @@ __global__ void __launch_bounds__(THREADS) gated_norm_add_kernel(const GatedNorm
     if (v >= nvec) continue;
 #pragma unroll
     for (int e = 0; e < VEC; ++e) t[i][e] = 0.f;
-    for (int s = 0; s < p.n_slots; ++s) {
+    auto slot = [&](int s) {
       int64_t src = row * p.n_slots + s;
       if (p.slots) src = p.slots[src];
       if (p.slots64) src = p.slots64[src];
       src = src < 0 ? 0 : (src >= p.y_rows ? p.y_rows - 1 : src);
-      float f[VEC];
-      load_v<T, VEC>(y + src * dim + v * VEC, f);
+      return y + src * dim + v * VEC;
+    };
+    for (int s = 0; s < p.n_slots; s += 2) {  // two on their way at a time
+      const bool two = s + 1 < p.n_slots;
+      float f[VEC], f2[VEC];
+      load_v<T, VEC>(slot(s), f);
+      if (two) load_v<T, VEC>(slot(s + 1), f2);
 #pragma unroll
       for (int e = 0; e < VEC; ++e) t[i][e] += f[e];
+      if (two) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) t[i][e] += f2[e];
+      }
     }
     if (p.gate) {
       float g[VEC], b[VEC];
-      load_v<float, VEC>(p.gate + row * p.gate_ld + v * VEC, g);
       if constexpr (PRE) {
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) b[e] = cb[i][e];
+        for (int e = 0; e < VEC; ++e) b[e] = cb[i][e], g[e] = gate[i][e];
       } else {
+        load_v<float, VEC>(p.gate + row * p.gate_ld + v * VEC, g);
         load_v<T, VEC>(bias + v * VEC, b);
       }
 #pragma unroll
@@ -193,6 +205,9 @@ int dispatch(const GatedNormParams& p, int64_t rows, cudaStream_t st) {
     return launch<T, 1, 16, 1024>(p, rows, st);
   }
   const int nvec = p.dim / 8;
+  // At most a CTA an SM: latency too, but where rows wait for room the registers of PRE cost more than they save.  Patevik 1B (width 2048), without
+  // / with it: a step of 1, 4, 16, 40 sequences 901 / 858, 1475 / 1435, 2152 / 2106, 2522 / 2493 us, a prompt of 100 2748 / 2693, of 2048 7315 / 7403.
+  if (rows <= device_sm_count() && nvec <= 256) return launch<T, 8, 1, 256, true>(p, rows, st);
   if (rows <= 16 && nvec > 256) {  // few rows: the kernel is one thread's latency chain, spread the row
     if (nvec <= 512) return launch<T, 8, 1, 512, true>(p, rows, st);
     if (nvec <= 1024) return launch<T, 8, 1, 1024, true>(p, rows, st);
