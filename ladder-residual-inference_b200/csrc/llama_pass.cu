@@ -16,7 +16,7 @@ struct Pass {
   const lri_llama_pass& p;
   int64_t rows;
   int rc = LRI_OK;
-  int beside = 0;  // LRI_BESIDE, LRI_HALF_RING where two streams run
+  int beside = 0;  // LRI_BESIDE, LRI_HALF_RING: see late() and where two streams run
 
   const void* at(int layer, int which) const { return p.layers[static_cast<int64_t>(layer) * kPointers + which]; }
   bool ok(int r) { return (rc = r) == LRI_OK; }
@@ -117,11 +117,14 @@ struct Pass {
   // steps and wider models keep them.  The results are the same bits.
   const void* cur = nullptr;  // the residual, and where the next sum goes: every CTA of a projection reads the one, so it is not written
   void* other = nullptr;
-  bool folds() {
-    if (!option(OPT_FOLD_NORM) || p.n_layer < 1 || !p.row_ws || rows != 1 || !gemv_norm_supports(1, p.dim)) return false;
+  bool folds() const { return option(OPT_FOLD_NORM) && p.n_layer > 0 && p.row_ws && rows == 1 && gemv_norm_supports(1, p.dim) && eager(); }
+  bool eager() const {
     cudaStreamCaptureStatus status;
     return cudaStreamIsCapturing(static_cast<cudaStream_t>(p.stream), &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
   }
+  // One stream, 25 to 64 rows: kernels behind small-batch projections come early (gemm_streamk.cu) but for wide models (8B dense, 32, 64 sequences 3612
+  // / 3647, 4225 / 4264 us) and small ones called eagerly (stories110M, 49 476 / 498, captured 462 / 437; 1B, 32 964 / 909).
+  bool late() const { return rows > 24 && rows <= kSplitKMaxRows && (p.dim >= 4096 || (p.dim < 1024 && eager())); }
   bool folded_qkv(int l, const void* add1, bool write) {
     void *kc = const_cast<void*>(at(l, kKCache)), *vc = const_cast<void*>(at(l, kVCache));
     const NormArgs nm{cur, add1, nullptr, at(l, kAttentionNorm), write ? other : nullptr, p.eps};
@@ -195,6 +198,7 @@ extern "C" int lri_llama_run(const lri_llama_pass* pass) {
       case LRI_PARALLEL: run.folded_parallel(); return run.rc;
     }
   }
+  if (run.late()) run.beside = LRI_BESIDE;
   switch (pass->schedule) {
     case LRI_DENSE:
     // on one GPU a partial that is reduced at once and one that is added by the next norm are the same sums
