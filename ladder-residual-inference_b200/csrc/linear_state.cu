@@ -547,10 +547,79 @@ head_norm_gate_kernel(const float* o, const T* w, float eps, const float* gate, 
   }
 }
 
+// The same where a head is a whole number of 16-byte vectors, at most two a lane: LANES lanes an item, everything of it asked for at once.  A warp an
+// item asked for four bytes a lane, and for the gate only behind the sum.  3000 tokens: 16 heads of 64 18.8 -> 7.9 us, 16 of 128 25.9 -> 14.8.
+template <typename T, int ACT, int LANES, int NV>
+__global__ void __launch_bounds__(256)
+head_norm_gate_vec_kernel(const float* o, const T* w, float eps, const float* gate, int64_t gate_ld, float scale, T* out, int64_t out_ld,
+                          int64_t items, int H, int E) {
+  const int lane = threadIdx.x % LANES;
+  float wv[NV][4];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int e = (lane + i * LANES) * 4;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) wv[i][r] = e < E ? Num<T>::to_f(w[e + r]) : 0.f;  // constant of the model
+  }
+  pdl_launch_dependents();
+  pdl_wait();
+  const int64_t item = static_cast<int64_t>(blockIdx.x) * (256 / LANES) + threadIdx.x / LANES;
+  const bool live = item < items;  // (all lanes of a warp take part in the sums)
+  const int64_t row = live ? item / H : 0;
+  const int h = live ? static_cast<int>(item - row * H) : 0;
+  const float* x = o + (live ? item : 0) * E;
+  const float* gt = gate + row * gate_ld + static_cast<int64_t>(h) * E;
+  float4 xv[NV], gv[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int e = (lane + i * LANES) * 4;
+    const bool in = live && e < E;
+    xv[i] = in ? *reinterpret_cast<const float4*>(x + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    gv[i] = in ? *reinterpret_cast<const float4*>(gt + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) ss = fmaf(xv[i].x, xv[i].x, fmaf(xv[i].y, xv[i].y, fmaf(xv[i].z, xv[i].z, fmaf(xv[i].w, xv[i].w, ss))));
+#pragma unroll
+  for (int n = LANES / 2; n > 0; n >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, n);
+  const float inv = scale / sqrtf(ss / static_cast<float>(E) + eps);
+  T* dst = out + row * out_ld + static_cast<int64_t>(h) * E;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int e = (lane + i * LANES) * 4;
+    if (!live || e >= E) continue;
+    auto act = [](float g) { return ACT == 0 ? sigmoid_f(g) : silu_f(g); };
+    const float y[4] = {xv[i].x * inv * wv[i][0] * act(gv[i].x), xv[i].y * inv * wv[i][1] * act(gv[i].y), xv[i].z * inv * wv[i][2] * act(gv[i].z),
+                        xv[i].w * inv * wv[i][3] * act(gv[i].w)};
+    if constexpr (sizeof(T) == 2)
+      *reinterpret_cast<uint2*>(dst + e) = make_uint2(pack2<T>(y[0], y[1]), pack2<T>(y[2], y[3]));
+    else
+      *reinterpret_cast<float4*>(dst + e) = make_float4(y[0], y[1], y[2], y[3]);
+  }
+}
+template <typename T, int LANES, int NV>
+int head_norm_gate_vec(const float* o, const T* w, float eps, const float* gate, int64_t gate_ld, int act, float scale, T* out, int64_t out_ld,
+                       int64_t items, int H, int E, cudaStream_t st) {
+  auto kern = act == 0 ? head_norm_gate_vec_kernel<T, 0, LANES, NV> : head_norm_gate_vec_kernel<T, 1, LANES, NV>;
+  constexpr int kItems = 256 / LANES;
+  LRI_CUDA(launch_pdl(kern, dim3(static_cast<unsigned>((items + kItems - 1) / kItems)), dim3(256), 0, st, o, w, eps, gate, gate_ld, scale, out, out_ld,
+                      items, H, E));
+  LRI_LAUNCH_CHECK("head_norm_gate_kernel");
+  return LRI_OK;
+}
+
 template <typename T>
 int head_norm_gate(const float* o, const void* w, float eps, const float* gate, int64_t gate_ld, int act, float scale, void* out,
                    int64_t out_ld, int64_t rows, int H, int E, cudaStream_t st) {
   const int64_t items = rows * H;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(out);
+  if (E % 4 == 0 && E <= 256 && gate_ld % 4 == 0 && out_ld % 4 == 0 && aligned16(o) && aligned16(gate) && at % (4 * sizeof(T)) == 0) {
+    const T* weight = static_cast<const T*>(w);
+    T* dst = static_cast<T*>(out);
+    if (E <= 64) return head_norm_gate_vec<T, 16, 1>(o, weight, eps, gate, gate_ld, act, scale, dst, out_ld, items, H, E, st);
+    if (E <= 128) return head_norm_gate_vec<T, 32, 1>(o, weight, eps, gate, gate_ld, act, scale, dst, out_ld, items, H, E, st);
+    return head_norm_gate_vec<T, 32, 2>(o, weight, eps, gate, gate_ld, act, scale, dst, out_ld, items, H, E, st);
+  }
   auto kern = act == 0 ? head_norm_gate_kernel<T, 0> : head_norm_gate_kernel<T, 1>;
   LRI_CUDA(launch_pdl(kern, dim3(static_cast<unsigned>((items + 7) / 8)), dim3(256), 0, st, o, static_cast<const T*>(w), eps, gate, gate_ld,
                       scale, static_cast<T*>(out), out_ld, items, H, E));
