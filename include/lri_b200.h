@@ -39,10 +39,6 @@ enum lri_dtype { LRI_BF16 = 0, LRI_FP16 = 1, LRI_FP32 = 2 };
  * that gives a tile to one SM.  For passes that run kernels of theirs on a second stream beside their projections (see
  * csrc/gemm_pair.cu). */
 enum { LRI_ONE_SM = 0x100 };
-/* The same for lri_qkv_rope_kvcache, lri_gateup_swiglu and lri_linear of small batches: another stream's kernels run beside this one (or the
- * caller knows better), so the kernel behind is not let in early; and, LRI_HALF_RING, another stream's projections share the SMs, so half of their shared memory is left.
- * The results are the same bits. */
-enum { LRI_BESIDE = 0x200, LRI_HALF_RING = 0x400 };
 
 enum lri_status {
   LRI_OK = 0,

@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(256) streamk_finish_kernel(const StreamKParams
   // below.  us a step, let in behind the wait / before: 8B dense, 16 sequences 3549 / 3510; 1B, 16 925 / 868; stories110M, 16 400 / 355; Migosun
   // 1B, 24 1282 / 1175, 8B, 16 4690 / 4640.  Not where another stream's kernels wait for the same SMs, which it would keep out (8B ladder, 16
   // sequences 3103 / 3310), and not with up to eight rows, where streaming kernels of thousands of CTAs follow (Patevik 8B, 4 sequences 9180 / 9600).
-  const bool early = !p.lin.beside && p.lin.m > 8;
+  const bool early = !p.lin.share.late && p.lin.m > 8;
   if (early) pdl_launch_dependents();
   pdl_wait();
   if (!early) pdl_launch_dependents();
@@ -393,7 +393,7 @@ int plan_ctas(int tiles, int total_kt, int max_seg) {
 int ring_stages(const LinearParams& lin, int stage_bytes, int accumulators) {
   constexpr int kHalf = 108 * 1024;
   int stages = kSmemBudget / stage_bytes;
-  if (lin.half_ring) {
+  if (lin.share.half_ring) {
     stages = kHalf / stage_bytes;
     if (accumulators == 2 && lin.m > 4 && lin.m <= 8 && lin.k < 4096) stages = 4;
   }

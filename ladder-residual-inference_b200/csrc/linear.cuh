@@ -43,6 +43,11 @@ struct NormArgs {
   float eps;
 };
 
+// Small batches, for a caller who knows what runs around a projection; the results are the same bits.
+struct Share {
+  bool late;       // another stream's kernels run beside it (or it is known to lose): the kernel behind is not let in early
+  bool half_ring;  // another stream's projections share the SMs: half of their shared memory is left to them
+};
 struct LinearParams {
   const void* x;  // [m, k]
   const void* w;  // PLAIN/QKV: [n, k]; SWIGLU: [2n, k] = [up rows | gate rows]
@@ -62,7 +67,7 @@ struct LinearParams {
   PushArgs push;       // PLAIN epilogue of the SIMT kernel only
   ExpertArgs ex;       // expert weights chosen on the device
   bool one_sm;         // prompt projections: not the kernel on pairs of SMs (LRI_ONE_SM)
-  bool beside, half_ring;  // small batches: what runs on another stream at the same time (LRI_BESIDE, LRI_HALF_RING)
+  Share share;
   NormArgs nm;         // one-row QKV and SWIGLU forms of the SIMT kernel
   ArgmaxArgs am;       // ARGMAX epilogue of the SIMT kernel: greedy choice instead of stored logits
 };
@@ -114,7 +119,15 @@ int gemv_launch(int dtype, int epi, const LinearParams& p, cudaStream_t st);
 // one row whose norm is taken on the way (p.nm): EPI_QKV and EPI_SWIGLU
 bool gemv_norm_supports(int64_t m, int k);
 int gemv_norm_launch(int dtype, int epi, const LinearParams& p, cudaStream_t st);
-// The projections of linear_api.cu with that norm in front; one row, no workspace
+// lri_linear, lri_gateup_swiglu, lri_qkv_rope_kvcache
+int linear(int dtype, const void* x, const void* w, const void* addend, void* y, int64_t M, int N, int K, void* workspace, size_t workspace_bytes,
+           Share share, lri_stream_t stream);
+int gateup_swiglu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K, void* workspace, size_t workspace_bytes, Share share,
+                  lri_stream_t stream);
+int qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, const void* rope_table, const void* input_pos, int pos_is_i64, void* q_out,
+                     void* k_cache, void* v_cache, int B, int S, int K, int n_head, int n_kv, int head_dim, int64_t smax, int64_t table_rows,
+                     int table_gathered, void* workspace, size_t workspace_bytes, Share share, lri_stream_t stream);
+// The latter two with that norm in front; one row, no workspace
 int norm_qkv_rope_kvcache(int dtype, const NormArgs& nm, const void* wqkv, const void* rope_table, const void* input_pos, int pos_is_i64,
                           void* q_out, void* k_cache, void* v_cache, int K, int n_head, int n_kv, int head_dim, int64_t smax,
                           int64_t table_rows, cudaStream_t st);

@@ -379,11 +379,11 @@ extern "C" int lri_gemm_status(void) {
   return LRI_OK;
 }
 
-// takes a flag (LRI_ONE_SM, LRI_BESIDE, LRI_HALF_RING) out of `dtype`
-static bool take_flag(int& dtype, int flag) {
-  const bool set = dtype >= 0 && (dtype & flag) != 0;
-  if (set) dtype &= ~flag;
-  return set;
+// takes LRI_ONE_SM out of `dtype`
+static bool take_one_sm(int& dtype) {
+  const bool one_sm = dtype >= 0 && (dtype & LRI_ONE_SM) != 0;
+  if (one_sm) dtype &= ~LRI_ONE_SM;
+  return one_sm;
 }
 
 static int check_common(const char* who, int dtype, const void* x, const void* w, int64_t M, int K) {
@@ -395,9 +395,9 @@ static int check_common(const char* who, int dtype, const void* x, const void* w
   return LRI_OK;
 }
 
-extern "C" int lri_linear(int dtype, const void* x, const void* w, const void* addend, void* y, int64_t M, int N,
-                          int K, void* workspace, size_t workspace_bytes, lri_stream_t stream) {
-  const bool one_sm = take_flag(dtype, LRI_ONE_SM), beside = take_flag(dtype, LRI_BESIDE), half_ring = take_flag(dtype, LRI_HALF_RING);
+int lri::linear(int dtype, const void* x, const void* w, const void* addend, void* y, int64_t M, int N, int K, void* workspace,
+                size_t workspace_bytes, Share share, lri_stream_t stream) {
+  const bool one_sm = take_one_sm(dtype);
   if (dtype == LRI_FP32 || (K > 0 && K % 8 != 0)) {
     LRI_REQUIRE(dtype >= LRI_BF16 && dtype <= LRI_FP32, LRI_ERR_UNSUPPORTED, "linear: dtype %d", dtype);
     LRI_REQUIRE(x && w && y, LRI_ERR_ARG, "linear: NULL pointer");
@@ -411,14 +411,14 @@ extern "C" int lri_linear(int dtype, const void* x, const void* w, const void* a
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (M <= streaming_rows()) {
     LinearParams p{};
-    p.x = x, p.w = w, p.y = y, p.addend = addend, p.m = static_cast<int>(M), p.n = N, p.k = K, p.beside = beside, p.half_ring = half_ring;
+    p.x = x, p.w = w, p.y = y, p.addend = addend, p.m = static_cast<int>(M), p.n = N, p.k = K, p.share = share;
     if (streamk_few_rows(EPI_PLAIN, p, workspace, workspace_bytes))
       return gemm_streamk_launch(dtype, EPI_PLAIN, p, workspace, workspace_bytes, st);
     return streaming_launch(dtype, EPI_PLAIN, p, st, prefer_simt_gemv());
   }
   if (streamk_rows(M)) {
     LinearParams p{};
-    p.x = x, p.w = w, p.y = y, p.addend = addend, p.m = static_cast<int>(M), p.n = N, p.k = K, p.beside = beside, p.half_ring = half_ring;
+    p.x = x, p.w = w, p.y = y, p.addend = addend, p.m = static_cast<int>(M), p.n = N, p.k = K, p.share = share;
     if (gemm_streamk_supports(EPI_PLAIN, p, workspace, workspace_bytes))
       return gemm_streamk_launch(dtype, EPI_PLAIN, p, workspace, workspace_bytes, st);
   }
@@ -433,6 +433,10 @@ extern "C" int lri_linear(int dtype, const void* x, const void* w, const void* a
               "linear: addend path needs M*N %% 8 == 0 and 16-byte aligned y, addend");
   return add_rows_launch(dtype, y, addend, M * N, st);
 }
+extern "C" int lri_linear(int dtype, const void* x, const void* w, const void* addend, void* y, int64_t M, int N, int K, void* workspace,
+                          size_t workspace_bytes, lri_stream_t stream) {
+  return lri::linear(dtype, x, w, addend, y, M, N, K, workspace, workspace_bytes, {}, stream);
+}
 
 extern "C" size_t lri_linear_f32_workspace_bytes(int64_t M, int N) {
   return M < 0 || N <= 0 ? 0 : streamk_bytes(EPI_F32, M, N);
@@ -440,7 +444,7 @@ extern "C" size_t lri_linear_f32_workspace_bytes(int64_t M, int N) {
 
 extern "C" int lri_linear_f32(int dtype, const void* x, const void* w, float* y, int64_t M, int N, int K, void* workspace,
                               size_t workspace_bytes, lri_stream_t stream) {
-  const bool one_sm = take_flag(dtype, LRI_ONE_SM);
+  const bool one_sm = take_one_sm(dtype);
   LRI_REQUIRE(dtype >= LRI_BF16 && dtype <= LRI_FP32, LRI_ERR_UNSUPPORTED, "linear_f32: dtype %d", dtype);
   LRI_REQUIRE(x && w && y, LRI_ERR_ARG, "linear_f32: NULL pointer");
   LRI_REQUIRE(M >= 0 && M < (1ll << 31) && N > 0 && K > 0, LRI_ERR_ARG, "linear_f32: M=%lld N=%d K=%d", (long long)M, N, K);
@@ -494,16 +498,15 @@ int lri::norm_gateup_swiglu(int dtype, const NormArgs& nm, const void* w1, void*
   p.nm = nm, p.x = nm.res, p.w = w1, p.y = h, p.m = 1, p.n = I, p.k = K;
   return gemv_norm_launch(dtype, EPI_SWIGLU, p, st);
 }
-extern "C" int lri_gateup_swiglu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K,
-                                 void* workspace, size_t workspace_bytes, lri_stream_t stream) {
-  const bool beside = take_flag(dtype, LRI_BESIDE), half_ring = take_flag(dtype, LRI_HALF_RING);
+int lri::gateup_swiglu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K, void* workspace, size_t workspace_bytes,
+                       Share share, lri_stream_t stream) {
   int rc = check_common("gateup_swiglu", dtype, x, w1, M, K);
   if (rc != LRI_OK) return rc;
   LRI_REQUIRE(h != nullptr && I > 0, LRI_ERR_ARG, "gateup_swiglu: h is NULL or I=%d", I);
   if (M == 0) return LRI_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LinearParams p{};
-  p.x = x, p.w = w1, p.y = h, p.m = static_cast<int>(M), p.n = I, p.k = K, p.beside = beside, p.half_ring = half_ring;
+  p.x = x, p.w = w1, p.y = h, p.m = static_cast<int>(M), p.n = I, p.k = K, p.share = share;
   if (M <= streaming_rows() && !streamk_few_rows(EPI_SWIGLU, p, workspace, workspace_bytes))
     return streaming_launch(dtype, EPI_SWIGLU, p, st, prefer_simt_gemv());
   if ((M <= streaming_rows() || streamk_rows(M)) && gemm_streamk_supports(EPI_SWIGLU, p, workspace, workspace_bytes))
@@ -522,6 +525,10 @@ extern "C" int lri_gateup_swiglu(int dtype, const void* x, const void* w1, void*
   if (rc != LRI_OK) return rc;
   return swiglu_rows_launch(dtype, workspace, h, M, I, st);
 }
+extern "C" int lri_gateup_swiglu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K, void* workspace, size_t workspace_bytes,
+                                 lri_stream_t stream) {
+  return lri::gateup_swiglu(dtype, x, w1, h, M, I, K, workspace, workspace_bytes, {}, stream);
+}
 
 // The fused forms need K in 16-byte steps; everything else goes through fp32 products and an elementwise kernel.
 static bool glu_fused(int dtype, int64_t M, int I, int K) {
@@ -539,7 +546,7 @@ extern "C" size_t lri_gateup_glu_workspace_bytes(int dtype, int64_t M, int I, in
 
 extern "C" int lri_gateup_glu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K, float alpha,
                               float limit, float offset, void* workspace, size_t workspace_bytes, lri_stream_t stream) {
-  const bool one_sm = take_flag(dtype, LRI_ONE_SM);
+  const bool one_sm = take_one_sm(dtype);
   LRI_REQUIRE(dtype >= LRI_BF16 && dtype <= LRI_FP32, LRI_ERR_UNSUPPORTED, "gateup_glu: dtype %d", dtype);
   LRI_REQUIRE(x && w1 && h, LRI_ERR_ARG, "gateup_glu: NULL pointer");
   LRI_REQUIRE(M >= 0 && M < (1ll << 31) && I > 0 && K > 0, LRI_ERR_ARG, "gateup_glu: M=%lld I=%d K=%d", (long long)M, I, K);
@@ -599,13 +606,10 @@ int lri::norm_qkv_rope_kvcache(int dtype, const NormArgs& nm, const void* wqkv, 
   p.S = 1, p.n_head = n_head, p.n_kv = n_kv, p.head_dim = head_dim, p.smax = smax, p.table_rows = table_rows;
   return gemv_norm_launch(dtype, EPI_QKV, p, st);
 }
-extern "C" int lri_qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, const void* rope_table,
-                                    const void* input_pos, int pos_is_i64, void* q_out, void* k_cache, void* v_cache,
-                                    int B, int S, int K, int n_head, int n_kv, int head_dim, int64_t smax,
-                                    int64_t table_rows, int table_gathered, void* workspace,
-                                    size_t workspace_bytes, lri_stream_t stream) {
+int lri::qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, const void* rope_table, const void* input_pos, int pos_is_i64, void* q_out,
+                          void* k_cache, void* v_cache, int B, int S, int K, int n_head, int n_kv, int head_dim, int64_t smax, int64_t table_rows,
+                          int table_gathered, void* workspace, size_t workspace_bytes, Share share, lri_stream_t stream) {
   LRI_REQUIRE(B >= 0 && S >= 0, LRI_ERR_ARG, "qkv_rope_kvcache: B=%d S=%d", B, S);
-  const bool beside = take_flag(dtype, LRI_BESIDE), half_ring = take_flag(dtype, LRI_HALF_RING);
   const int64_t M = static_cast<int64_t>(B) * S;
   int rc = check_common("qkv_rope_kvcache", dtype, x, wqkv, M, K);
   if (rc != LRI_OK) return rc;
@@ -614,7 +618,7 @@ extern "C" int lri_qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, 
   if (M == 0) return LRI_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LinearParams p{};
-  p.x = x, p.w = wqkv, p.m = static_cast<int>(M), p.n = (n_head + 2 * n_kv) * head_dim, p.k = K, p.beside = beside, p.half_ring = half_ring;
+  p.x = x, p.w = wqkv, p.m = static_cast<int>(M), p.n = (n_head + 2 * n_kv) * head_dim, p.k = K, p.share = share;
   p.rope_table = rope_table, p.input_pos = input_pos, p.pos_is_i64 = pos_is_i64;
   p.q_out = q_out, p.k_cache = k_cache, p.v_cache = v_cache;
   p.S = S, p.n_head = n_head, p.n_kv = n_kv, p.head_dim = head_dim, p.smax = smax, p.table_rows = table_rows, p.table_gathered = table_gathered;
@@ -634,4 +638,10 @@ extern "C" int lri_qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, 
   rc = gemm_launch(dtype, x, wqkv, workspace, M, p.n, K, st);
   if (rc != LRI_OK) return rc;
   return qkv_scatter_launch(dtype, workspace, p, st);
+}
+extern "C" int lri_qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, const void* rope_table, const void* input_pos, int pos_is_i64,
+                                    void* q_out, void* k_cache, void* v_cache, int B, int S, int K, int n_head, int n_kv, int head_dim, int64_t smax,
+                                    int64_t table_rows, int table_gathered, void* workspace, size_t workspace_bytes, lri_stream_t stream) {
+  return lri::qkv_rope_kvcache(dtype, x, wqkv, rope_table, input_pos, pos_is_i64, q_out, k_cache, v_cache, B, S, K, n_head, n_kv, head_dim, smax,
+                               table_rows, table_gathered, workspace, workspace_bytes, {}, stream);
 }

@@ -16,7 +16,7 @@ struct Pass {
   const lri_llama_pass& p;
   int64_t rows;
   int rc = LRI_OK;
-  int beside = 0;  // LRI_BESIDE, LRI_HALF_RING: see late() and where two streams run
+  Share share{};  // see late() and where two streams run
 
   const void* at(int layer, int which) const { return p.layers[static_cast<int64_t>(layer) * kPointers + which]; }
   bool ok(int r) { return (rc = r) == LRI_OK; }
@@ -32,8 +32,8 @@ struct Pass {
   }
   bool attention(int l) {
     void *kc = const_cast<void*>(at(l, kKCache)), *vc = const_cast<void*>(at(l, kVCache));
-    return ok(lri_qkv_rope_kvcache(p.dtype | beside, p.normed, at(l, kQkv), p.rope_table, p.input_pos, p.pos_is_i64, p.q, kc, vc, p.B, p.S, p.dim, p.n_head,
-                                   p.n_kv, p.head_dim, p.smax, p.table_rows, 0, p.ws_qkv, p.ws_qkv_bytes, p.stream)) &&
+    return ok(lri::qkv_rope_kvcache(p.dtype, p.normed, at(l, kQkv), p.rope_table, p.input_pos, p.pos_is_i64, p.q, kc, vc, p.B, p.S, p.dim, p.n_head,
+                                   p.n_kv, p.head_dim, p.smax, p.table_rows, 0, p.ws_qkv, p.ws_qkv_bytes, share, p.stream)) &&
            attend(l);
   }
   // from the queries and the caches to the output projection
@@ -43,11 +43,11 @@ struct Pass {
         p.S == 1 ? ok(lri_attn_decode(p.dtype, p.q, kc, vc, p.input_pos, p.pos_is_i64, p.y, p.B, p.n_head, p.n_kv, p.head_dim, p.smax, p.splits,
                                       p.scratch, p.scratch_bytes, p.stream))
                  : ok(lri_attn_prefill(p.dtype, p.q, kc, vc, p.input_pos, p.pos_is_i64, p.y, p.B, p.S, p.n_head, p.n_kv, p.head_dim, p.smax, p.stream));
-    return done && ok(lri_linear(p.dtype | beside, p.y, at(l, kWo), nullptr, p.part_a, rows, p.dim, p.n_head * p.head_dim, p.ws_wo, p.ws_wo_bytes, p.stream));
+    return done && ok(lri::linear(p.dtype, p.y, at(l, kWo), nullptr, p.part_a, rows, p.dim, p.n_head * p.head_dim, p.ws_wo, p.ws_wo_bytes, share, p.stream));
   }
   bool mlp(int l, const void* normed, const void* addend, lri_stream_t st) {
-    return ok(lri_gateup_swiglu(p.dtype | beside, normed, at(l, kW1), p.h, rows, p.inter, p.dim, p.ws_ug, p.ws_ug_bytes, st)) &&
-           ok(lri_linear(p.dtype | beside, p.h, at(l, kW2), addend, p.part_m, rows, p.dim, p.inter, p.ws_w2, p.ws_w2_bytes, st));
+    return ok(lri::gateup_swiglu(p.dtype, normed, at(l, kW1), p.h, rows, p.inter, p.dim, p.ws_ug, p.ws_ug_bytes, share, st)) &&
+           ok(lri::linear(p.dtype, p.h, at(l, kW2), addend, p.part_m, rows, p.dim, p.inter, p.ws_w2, p.ws_w2_bytes, share, st));
   }
   bool record(int i, lri_stream_t st) {
     return cuda(cudaEventRecord(static_cast<cudaEvent_t>(p.events[i]), static_cast<cudaStream_t>(st)), "cudaEventRecord");
@@ -75,7 +75,7 @@ struct Pass {
   // the attention chain of a layer on `stream`, its MLP chain on `side`: see Engine._run_ladder_two_streams
   bool ladder_two_streams() {
     if (!record(0, p.stream) || !wait(0, p.side)) return false;
-    beside = LRI_BESIDE | LRI_HALF_RING;
+    share = {true, true};
     int n = 1;
     for (int l = 0; l < p.n_layer; ++l, n += 2) {
       if (!norm(at(l, kAttentionNorm), l ? p.part_a : nullptr, nullptr, true, p.normed, p.stream) || !record(n, p.stream) || !attention(l)) return false;
@@ -97,13 +97,13 @@ struct Pass {
   // the gate/up projection beside the attention chain: both read the norm
   bool parallel_two_streams() {
     const void* pending = nullptr;
-    beside = LRI_BESIDE | (rows > 8 ? LRI_HALF_RING : 0);  // (3B, whole / half ring: 2 sequences 1677 / 1779 us, 4 1785 / 1903, 16 2445 / 2390, 40 3499 / 3495)
+    share = {true, rows > 8};  // (3B, whole / half ring: 2 sequences 1677 / 1779 us, 4 1785 / 1903, 16 2445 / 2390, 40 3499 / 3495)
     for (int l = 0; l < p.n_layer; ++l) {
       if (!norm(at(l, kAttentionNorm), pending, nullptr, true, p.normed, p.stream) || !record(2 * l, p.stream) || !wait(2 * l, p.side)) return false;
       if (!attention(l) ||
-          !ok(lri_gateup_swiglu(p.dtype | beside, p.normed, at(l, kW1), p.h, rows, p.inter, p.dim, p.ws_ug, p.ws_ug_bytes, p.side)) ||
+          !ok(lri::gateup_swiglu(p.dtype, p.normed, at(l, kW1), p.h, rows, p.inter, p.dim, p.ws_ug, p.ws_ug_bytes, share, p.side)) ||
           !record(2 * l + 1, p.side) || !wait(2 * l + 1, p.stream) ||
-          !ok(lri_linear(p.dtype | beside, p.h, at(l, kW2), p.part_a, p.part_m, rows, p.dim, p.inter, p.ws_w2, p.ws_w2_bytes, p.stream)))
+          !ok(lri::linear(p.dtype, p.h, at(l, kW2), p.part_a, p.part_m, rows, p.dim, p.inter, p.ws_w2, p.ws_w2_bytes, share, p.stream)))
         return false;
       pending = p.part_m;
     }
@@ -198,7 +198,7 @@ extern "C" int lri_llama_run(const lri_llama_pass* pass) {
       case LRI_PARALLEL: run.folded_parallel(); return run.rc;
     }
   }
-  if (run.late()) run.beside = LRI_BESIDE;
+  if (run.late()) run.share.late = true;
   switch (pass->schedule) {
     case LRI_DENSE:
     // on one GPU a partial that is reduced at once and one that is added by the next norm are the same sums
