@@ -14,8 +14,9 @@
 //         the identity for the delta rule (C more columns beside the E of the state)
 //   join  state before each segment, one after the other:  S_{g+1} = M_g S_g + S0_g
 //   scan  every segment from its own first state, with results
-// All of it in fp32, and the delta rule's M is a product of contractions, so errors do not grow: 2 x 1500 tokens of 16 heads of 64 x 64 against 64
-// bits, results 7.53e-7 in one segment, 7.58e-7 in eight (state 1.026e-6, 1.028e-6), gated linear attention 1.762e-7 and 1.763e-7.
+// All of it in fp32, and the delta rule's M is a product of contractions, so errors do not grow.  Errors against 64 bits, segments over one segment: 45
+// calls of 1300 to 4000 tokens, one and two sequences of 16 heads of 64 x 64, three ranges of decays, results 0.9998 on average (0.993 to 1.005),
+// states 1.002 (0.992 to 1.017); gated linear attention, 22 calls, 1.0006 and 1.0005 (at most 1.001 and 1.005).
 #include "linear_state.cuh"
 #include "tcgen05.cuh"
 
@@ -327,7 +328,9 @@ __global__ void __launch_bounds__(128, 1) state_scan_kernel(const __grid_constan
 constexpr int kJoinCols = 16, kJoinThreads = 256;
 
 // Delta rule: one CTA per 16 columns of a head, one thread per column and every 16th row; M of the next segment is copied in while
-// this one's product runs (5 to 7 us for 8 segments of 64 x 64).
+// this one's product runs.  The product has sums of its own, four a thread, and joins S0 in one rounding: added to S0 term by term each of the C
+// roundings had the size of the state (1300 tokens in ten segments, 128 x 96, error of the state 1.34e-7 in one segment, 1.82e-7 so, 1.37e-7 now;
+// the whole recurrence of 2 x 1500 tokens, 16 heads of 64 x 64, 144 us so, 136 now).
 __global__ void __launch_bounds__(kJoinThreads) state_join_kernel(const ScanParams p) {
   extern __shared__ __align__(16) float join_smem[];
   const int C = p.C, E = p.E, H = p.H, h = blockIdx.y, segs = p.segs;
@@ -354,11 +357,13 @@ __global__ void __launch_bounds__(kJoinThreads) state_join_kernel(const ScanPara
     s[c * kJoinCols + col] = mine ? slot(1)[static_cast<int64_t>(c) * E] : 0.f;
   }
   for (int g = 1; g < segs - 1; ++g) {
-    float part[kRows];
+    float part[kRows], acc[kRows][4];
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
       const int c = row + i * (kJoinThreads / kJoinCols);
       part[i] = mine && c < C ? slot(g + 1)[static_cast<int64_t>(c) * E] : 0.f;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) acc[i][r] = 0.f;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -373,7 +378,10 @@ __global__ void __launch_bounds__(kJoinThreads) state_join_kernel(const ScanPara
         const int c = row + i * (kJoinThreads / kJoinCols);
         if (c < C) {
           const float4 w = *reinterpret_cast<const float4*>(mg + c * C + k);
-          part[i] = fmaf(w.x, x[0], fmaf(w.y, x[1], fmaf(w.z, x[2], fmaf(w.w, x[3], part[i]))));
+          acc[i][0] = fmaf(w.x, x[0], acc[i][0]);
+          acc[i][1] = fmaf(w.y, x[1], acc[i][1]);
+          acc[i][2] = fmaf(w.z, x[2], acc[i][2]);
+          acc[i][3] = fmaf(w.w, x[3], acc[i][3]);
         }
       }
     }
@@ -382,6 +390,7 @@ __global__ void __launch_bounds__(kJoinThreads) state_join_kernel(const ScanPara
     for (int i = 0; i < kRows; ++i) {
       const int c = row + i * (kJoinThreads / kJoinCols);
       if (c < C) {
+        part[i] += (acc[i][0] + acc[i][1]) + (acc[i][2] + acc[i][3]);
         s[c * kJoinCols + col] = part[i];
         if (mine) slot(g + 1)[static_cast<int64_t>(c) * E] = part[i];
       }
