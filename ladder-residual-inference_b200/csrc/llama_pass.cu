@@ -199,13 +199,16 @@ extern "C" int lri_llama_run(const lri_llama_pass* pass) {
     }
   }
   if (run.late()) run.share.late = true;
+  // From 129 rows on (or 65, where the option forces it) the projections of two streams would run on pairs of SMs beside each other, which is not
+  // done (gemm_pair.cu): such a pass runs on one stream, with the same results.
+  const bool two = run.rows <= (option(OPT_GEMM_PAIR) > 1 ? kSplitKMaxRows : 128);
   switch (pass->schedule) {
     case LRI_DENSE:
     // on one GPU a partial that is reduced at once and one that is added by the next norm are the same sums
     case LRI_DESYNC: run.dense(); break;
     case LRI_LADDER: run.ladder(); break;
-    case LRI_LADDER_TWO_STREAMS: run.ladder_two_streams(); break;
-    case LRI_PARALLEL: pass->events ? run.parallel_two_streams() : run.parallel(); break;
+    case LRI_LADDER_TWO_STREAMS: two ? run.ladder_two_streams() : run.ladder(); break;
+    case LRI_PARALLEL: two && pass->events ? run.parallel_two_streams() : run.parallel(); break;
     default: return fail(LRI_ERR_ARG, "llama_pass: schedule %d", pass->schedule);
   }
   return run.rc;

@@ -31,6 +31,10 @@ from .comm import NoComm, make_comm
 from .ops import CudaOps, decode_splits
 
 _MAX_SPLITS = 64
+# Token rows up to which a decode step runs on two streams.  More would bring the kernel on pairs of SMs beside another stream's tensor-memory
+# kernel, which the engines keep apart (csrc/gemm_pair.cu).  us a captured step, one stream / two: 8B ladder, 80, 96, 128 sequences 5991 / 4288,
+# 6045 / 4430, 6349 / 6394; 8B parallel 5929 / 5387, 5977 / 5400, 6266 / 5900; 1B ladder 1674 / 1112, 1688 / 1150, 1803 / 1300.
+_TWO_STREAM_ROWS = 128
 
 
 class Engine:
@@ -199,7 +203,7 @@ class Engine:
         And not parallel blocks of 128-wide heads with about one (sequence, KV head) pair an SM: their attention fills the chip for one
         pair's length, and gate/up in between only delays it (3B, 6 and 7 sequences 1974 and 2045 us on one stream, 2010 and 2074 on two;
         5, 8 and 12 2055, 2091 and 2326 to 1872, 2081 and 2072)."""
-        if not self.overlap_sublayers:
+        if not self.overlap_sublayers or B > _TWO_STREAM_ROWS:
             return False
         parallel = self.family == "parallel"
         if (self.d < 1024 or (parallel and B == 1)) and not torch.cuda.is_current_stream_capturing():
@@ -392,7 +396,7 @@ class Engine:
         mixed = getattr(self.cfg, "ladder_layers", None)
         if mixed is not None and len(set(mixed)) != self.cfg.n_layer:
             return self._run_hybrid(rows, B, S, pos, set(mixed))
-        if S == 1 and self.overlap_sublayers:
+        if S == 1 and self.overlap_sublayers and rows <= _TWO_STREAM_ROWS:
             return self._run_ladder_two_streams(rows, B, S, pos)
         comm, m = self.comm, self.model
         ca, cm, pa, pm, split = self._reduce_plan(rows, hidden=True)

@@ -1,0 +1,39 @@
+"""How many token rows a decode step may have on two streams: the kernel on pairs of SMs, which takes projections of more than 128 rows, never runs
+beside another stream's tensor-memory kernel."""
+import pytest
+import torch
+
+SHAPE = dict(block_size=64, vocab_size=64, n_layer=2, n_head=4, n_local_heads=4, dim=1024, intermediate_size=96)
+
+
+def _engine(family, monkeypatch, batch):
+    import gpt_fast
+    from gpt_fast import gpt_ladder_TP, gpt_parallel_TP
+    mod, cls = {"ladder": (gpt_ladder_TP, gpt_fast.GPTLadder), "parallel": (gpt_parallel_TP, gpt_fast.GPTParallel)}[family]
+    monkeypatch.setitem(mod.transformer_configs, "two-streams-rows", dict(SHAPE))
+    model = cls.from_name("two-streams-rows").to(torch.bfloat16).eval()
+    model.setup_caches(max_batch_size=batch, max_seq_length=8)
+    engine = model._engine
+    engine.overlap_sublayers, engine.sms = True, 148
+    return engine
+
+
+@pytest.mark.parametrize("capturing", [False, True])
+@pytest.mark.parametrize("family", ["ladder", "parallel"])
+def test_rows_of_native_passes(family, capturing, monkeypatch):
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
+    engine = _engine(family, monkeypatch, 130)
+    assert [b for b in (64, 65, 128, 129, 130) if engine._two_streams(b)] == [64, 65, 128]
+
+
+def test_rows_of_the_python_schedule(monkeypatch):
+    engine = _engine("ladder", monkeypatch, 130)
+    ran = []
+    monkeypatch.setattr(engine, "_run_ladder_two_streams", lambda rows, *a: ran.append(rows))
+    monkeypatch.setattr(engine, "_norm", lambda *a, **k: None)
+    monkeypatch.setattr(engine, "_attention", lambda *a, **k: None)
+    monkeypatch.setattr(engine, "_mlp", lambda *a, **k: None)
+    monkeypatch.setattr(engine, "_issue", lambda *a: None)
+    for b in (1, 64, 65, 128, 129, 130):
+        engine._run_ladder(b, b, 1, torch.zeros(1, dtype=torch.int32))
+    assert ran == [1, 64, 65, 128]

@@ -50,3 +50,19 @@ def test_choice_of_streams():
     engine = _model("ladder", torch.bfloat16, 2, dim=2048, n_head=16, n_local_heads=16, intermediate_size=512)._engine
     assert all(engine._two_streams(b) for b in range(1, 65))
     assert not _model("dense", torch.bfloat16, 2)._engine._two_streams(1)
+
+
+@pytest.mark.parametrize("family", ["ladder", "parallel"])
+def test_more_rows_run_on_one_stream(family):
+    """Whoever asks for two streams with more rows than they are made for gets one: no event is recorded, and the results are those of one stream."""
+    results = []
+    for asked in (False, True):
+        model = _model(family, torch.bfloat16, 129)
+        engine = model._engine
+        _only(engine, True)
+        engine._two_streams = lambda B: asked
+        engine._events = [type("", (), {"cuda_event": None})()] * 8
+        tok = torch.arange(129, dtype=torch.int32, device="cuda").view(129, 1)
+        with torch.no_grad():
+            results.append(model(tok, torch.tensor([0], dtype=torch.int32, device="cuda")))
+    assert torch.isfinite(results[0].float()).all() and torch.equal(*results)
