@@ -479,7 +479,8 @@ int lri_round_columns(int dtype, const float* x, int64_t ld, int64_t off, int n,
  * From the embedded rows in `resid` to the normed rows in `normed`, by the entry points above in the order of one of the
  * schedules.  layers: for each layer attention norm, QKV, wo, MLP norm, w1, w2, K cache, V cache; reduces (desync): for each
  * layer whether attention and MLP fold their partial into the residual.  Buffers hold B S rows.  Nothing is kept of it. */
-enum lri_schedule { LRI_DENSE = 0, LRI_LADDER = 1, LRI_LADDER_TWO_STREAMS = 2, LRI_PARALLEL = 3, LRI_DESYNC = 4 };
+enum lri_schedule { LRI_DENSE = 0, LRI_LADDER = 1, LRI_LADDER_TWO_STREAMS = 2, LRI_PARALLEL = 3, LRI_DESYNC = 4,
+                    LRI_PARALLEL_TWO_STREAMS = 5 /* gate/up on `side` beside the attention chain; needs `side` and `events` */ };
 typedef struct {
   int dtype, schedule, n_layer, B, S, n_head, n_kv, head_dim, dim, inter, pos_is_i64, splits;
   float eps;
@@ -491,7 +492,7 @@ typedef struct {
   void *ws_qkv, *ws_wo, *ws_ug, *ws_w2, *scratch;
   size_t ws_qkv_bytes, ws_wo_bytes, ws_ug_bytes, ws_w2_bytes, scratch_bytes;
   lri_stream_t stream, side;
-  void* const* events; /* two streams: 2 n_layer + 2 cudaEvent_t; LRI_PARALLEL with events runs gate/up on `side` beside the attention chain */
+  void* const* events; /* two streams: 2 n_layer + 2 cudaEvent_t */
   void* row_ws; /* one row: dim elements; with them small models called eagerly leave norms to the projections behind.  NULL: never */
 } lri_llama_pass;
 int lri_llama_run(const lri_llama_pass* pass);

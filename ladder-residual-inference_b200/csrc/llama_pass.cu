@@ -186,6 +186,8 @@ extern "C" int lri_llama_run(const lri_llama_pass* pass) {
   LRI_REQUIRE(pass->n_layer >= 0 && pass->B >= 0 && pass->S >= 0, LRI_ERR_ARG, "llama_pass: n_layer=%d B=%d S=%d", pass->n_layer, pass->B, pass->S);
   LRI_REQUIRE(pass->schedule != LRI_LADDER_TWO_STREAMS || (pass->events != nullptr && pass->normed_m != nullptr), LRI_ERR_ARG,
               "llama_pass: two streams need events and a second buffer");
+  LRI_REQUIRE(pass->schedule != LRI_PARALLEL_TWO_STREAMS || (pass->events != nullptr && pass->side != nullptr), LRI_ERR_ARG,
+              "llama_pass: two streams need events and a second stream");
   LRI_REQUIRE(pass->schedule != LRI_DESYNC || pass->reduces != nullptr, LRI_ERR_ARG, "llama_pass: NULL flags");
   Pass run{*pass, static_cast<int64_t>(pass->B) * pass->S};
   if (run.folds()) {
@@ -195,7 +197,8 @@ extern "C" int lri_llama_run(const lri_llama_pass* pass) {
       case LRI_DESYNC: run.folded_dense(); return run.rc;
       case LRI_LADDER:
       case LRI_LADDER_TWO_STREAMS: run.folded_ladder(); return run.rc;
-      case LRI_PARALLEL: run.folded_parallel(); return run.rc;
+      case LRI_PARALLEL:
+      case LRI_PARALLEL_TWO_STREAMS: run.folded_parallel(); return run.rc;
     }
   }
   if (run.late()) run.share.late = true;
@@ -208,7 +211,8 @@ extern "C" int lri_llama_run(const lri_llama_pass* pass) {
     case LRI_DESYNC: run.dense(); break;
     case LRI_LADDER: run.ladder(); break;
     case LRI_LADDER_TWO_STREAMS: two ? run.ladder_two_streams() : run.ladder(); break;
-    case LRI_PARALLEL: two && pass->events ? run.parallel_two_streams() : run.parallel(); break;
+    case LRI_PARALLEL: run.parallel(); break;
+    case LRI_PARALLEL_TWO_STREAMS: two ? run.parallel_two_streams() : run.parallel(); break;
     default: return fail(LRI_ERR_ARG, "llama_pass: schedule %d", pass->schedule);
   }
   return run.rc;

@@ -32,7 +32,7 @@ class LlamaPass(ctypes.Structure):
 
 
 ONE_SM = 0x100  # LRI_ONE_SM
-DENSE, LADDER, LADDER_TWO_STREAMS, PARALLEL, DESYNC = range(5)
+DENSE, LADDER, LADDER_TWO_STREAMS, PARALLEL, DESYNC, PARALLEL_TWO_STREAMS = range(6)
 
 # name -> (restype, argtypes); the order of arguments is that of include/lri_b200.h
 _SIGNATURES = {

@@ -26,7 +26,7 @@ import os
 
 import torch
 
-from ._C import DENSE, DESYNC, LADDER, LADDER_TWO_STREAMS, PARALLEL, dtype_code, option
+from ._C import DENSE, DESYNC, LADDER, LADDER_TWO_STREAMS, PARALLEL, PARALLEL_TWO_STREAMS, dtype_code, option
 from .comm import NoComm, make_comm
 from .ops import CudaOps, decode_splits
 
@@ -265,7 +265,8 @@ class Engine:
         sizes = dict(dtype=dtype_code(self.dtype), n_layer=len(m.layers), B=B, S=S, n_head=self.nh, n_kv=self.nkv, head_dim=self.hd, dim=self.d,
                      inter=self.inter, pos_is_i64=int(pos.dtype == torch.int64), splits=self._splits, smax=smax,
                      table_rows=m.freqs_cis.shape[0])
-        schedule = {"dense": DENSE, "ladder": LADDER_TWO_STREAMS if two else LADDER, "parallel": PARALLEL, "desync": DESYNC}[family]
+        schedule = {"dense": DENSE, "ladder": LADDER_TWO_STREAMS if two else LADDER, "parallel": PARALLEL_TWO_STREAMS if two else PARALLEL,
+                    "desync": DESYNC}[family]
         self.ops.run_layers(schedule, tensors, above, reduces, self._events if two else None, main.cuda_stream,
                             self.side_stream.cuda_stream if two else None, sizes, self.cfg.norm_eps,
                             dict(ws_qkv=self.ws_qkv, ws_wo=self.ws_wo, ws_ug=self.ws_ug, ws_w2=self.ws_w2, scratch=self.scratch), **buffers)

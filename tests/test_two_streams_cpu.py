@@ -37,3 +37,13 @@ def test_rows_of_the_python_schedule(monkeypatch):
     for b in (1, 64, 65, 128, 129, 130):
         engine._run_ladder(b, b, 1, torch.zeros(1, dtype=torch.int32))
     assert ran == [1, 64, 65, 128]
+
+
+def test_two_streams_need_a_second_one():
+    """Without one the kernels would go to the legacy stream, which no capture allows."""
+    import ctypes
+    from gpt_fast import _C
+    some = (ctypes.c_void_p * 8)()
+    for given in ({}, dict(events=ctypes.cast(some, ctypes.c_void_p)), dict(side=ctypes.addressof(some))):
+        p = _C.LlamaPass(schedule=_C.PARALLEL_TWO_STREAMS, layers=ctypes.addressof(some), **given)
+        assert _C.lib.lri_llama_run(ctypes.byref(p)) == -1 and b"second stream" in _C.lib.lri_last_error()

@@ -66,3 +66,22 @@ def test_more_rows_run_on_one_stream(family):
         with torch.no_grad():
             results.append(model(tok, torch.tensor([0], dtype=torch.int32, device="cuda")))
     assert torch.isfinite(results[0].float()).all() and torch.equal(*results)
+
+
+def test_parallel_passes_of_one_stream_read_no_events(monkeypatch):
+    """LRI_PARALLEL with events and without a second stream: one stream, as before there was a schedule of two."""
+    from gpt_fast.ops import CudaOps
+    run, null = CudaOps.run_layers, [type("", (), {"cuda_event": None})()] * 8
+    tok, pos = torch.arange(9, dtype=torch.int32, device="cuda").view(9, 1), torch.tensor([0], dtype=torch.int32, device="cuda")
+    results = []
+    for events in (None, null):
+        model = _model("parallel", torch.bfloat16, 9)
+        _only(model._engine, True)
+
+        def given(schedule, layers, above, reduces, _, main, side, *rest, **kw):
+            assert side is None
+            return run(schedule, layers, above, reduces, events, main, None, *rest, **kw)
+        monkeypatch.setattr(CudaOps, "run_layers", staticmethod(given))
+        with torch.no_grad():
+            results.append(model(tok, pos))
+    assert torch.isfinite(results[0].float()).all() and torch.equal(*results)
