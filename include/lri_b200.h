@@ -74,7 +74,7 @@ int lri_set_gemm_backend(int backend);
  * (LRI_HGRN2_BLOCKS: 0 keeps the HGRN2 recurrence token by token), scan_columns (LRI_SCAN_COLUMNS: state columns per
  * lane of the matrix-state recurrences, 0 choose, 1, 2, 4), scan_warps (LRI_SCAN_WARPS: their warps per CTA, 0 choose, 1, 2, 4),
  * scan_lanes (LRI_SCAN_LANES: lanes per state column, 0 choose, 8, 16), scan_segments (LRI_SCAN_SEGMENTS: segments of a sequence
- * that run side by side, 0 choose, 1..16), fold_norm (LRI_FOLD_NORM: 0 keeps the norms of lri_llama_run in kernels of their own).  Unknown
+ * that run side by side, 0 choose, 1..16), fold_norm (LRI_FOLD_NORM: 0 keeps the norms of lri_llama_run_row in kernels of their own).  Unknown
  * names and values an option does not take return LRI_ERR_ARG.  No counterpart in the reference
  * (its only switches are benchmark.py's command-line flags). */
 int lri_set_option(const char* name, int value);
@@ -493,9 +493,11 @@ typedef struct {
   size_t ws_qkv_bytes, ws_wo_bytes, ws_ug_bytes, ws_w2_bytes, scratch_bytes;
   lri_stream_t stream, side;
   void* const* events; /* two streams: 2 n_layer + 2 cudaEvent_t */
-  void* row_ws; /* one row: dim elements; with them small models called eagerly leave norms to the projections behind.  NULL: never */
 } lri_llama_pass;
 int lri_llama_run(const lri_llama_pass* pass);
+/* The same with room for a second residual of one row (dim elements, 16-byte aligned; NULL: none): an eager pass of one row of a model up to
+ * 1024 wide leaves its norms to the projections behind them, and the last residual may stand in `resid` or in `row_ws` after it.  Same results. */
+int lri_llama_run_row(const lri_llama_pass* pass, void* row_ws);
 
 /* Reads (and clears) the device status word: LRI_OK or LRI_ERR_TIMEOUT.  Synchronises `stream`. */
 int lri_comm_status(lri_comm* comm, lri_stream_t stream);

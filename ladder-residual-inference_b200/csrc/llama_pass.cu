@@ -15,6 +15,7 @@ enum LayerPointer { kAttentionNorm, kQkv, kWo, kMlpNorm, kW1, kW2, kKCache, kVCa
 struct Pass {
   const lri_llama_pass& p;
   int64_t rows;
+  void* row_ws;
   int rc = LRI_OK;
   Share share{};  // see late() and where two streams run
 
@@ -117,7 +118,7 @@ struct Pass {
   // steps and wider models keep them.  The results are the same bits.
   const void* cur = nullptr;  // the residual, and where the next sum goes: every CTA of a projection reads the one, so it is not written
   void* other = nullptr;
-  bool folds() const { return option(OPT_FOLD_NORM) && p.n_layer > 0 && p.row_ws && rows == 1 && gemv_norm_supports(1, p.dim) && eager(); }
+  bool folds() const { return option(OPT_FOLD_NORM) && p.n_layer > 0 && row_ws && rows == 1 && gemv_norm_supports(1, p.dim) && eager(); }
   bool eager() const {
     cudaStreamCaptureStatus status;
     return cudaStreamIsCapturing(static_cast<cudaStream_t>(p.stream), &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
@@ -181,7 +182,9 @@ struct Pass {
 
 }  // namespace
 
-extern "C" int lri_llama_run(const lri_llama_pass* pass) {
+extern "C" int lri_llama_run(const lri_llama_pass* pass) { return lri_llama_run_row(pass, nullptr); }
+
+extern "C" int lri_llama_run_row(const lri_llama_pass* pass, void* row_ws) {
   LRI_REQUIRE(pass != nullptr && pass->layers != nullptr, LRI_ERR_ARG, "llama_pass: NULL pointer");
   LRI_REQUIRE(pass->n_layer >= 0 && pass->B >= 0 && pass->S >= 0, LRI_ERR_ARG, "llama_pass: n_layer=%d B=%d S=%d", pass->n_layer, pass->B, pass->S);
   LRI_REQUIRE(pass->schedule != LRI_LADDER_TWO_STREAMS || (pass->events != nullptr && pass->normed_m != nullptr), LRI_ERR_ARG,
@@ -189,9 +192,9 @@ extern "C" int lri_llama_run(const lri_llama_pass* pass) {
   LRI_REQUIRE(pass->schedule != LRI_PARALLEL_TWO_STREAMS || (pass->events != nullptr && pass->side != nullptr), LRI_ERR_ARG,
               "llama_pass: two streams need events and a second stream");
   LRI_REQUIRE(pass->schedule != LRI_DESYNC || pass->reduces != nullptr, LRI_ERR_ARG, "llama_pass: NULL flags");
-  Pass run{*pass, static_cast<int64_t>(pass->B) * pass->S};
+  Pass run{*pass, static_cast<int64_t>(pass->B) * pass->S, row_ws};
   if (run.folds()) {
-    run.cur = pass->resid, run.other = pass->row_ws;
+    run.cur = pass->resid, run.other = row_ws;
     switch (pass->schedule) {
       case LRI_DENSE:
       case LRI_DESYNC: run.folded_dense(); return run.rc;

@@ -22,13 +22,13 @@ lib = ctypes.CDLL(LIB_PATH)
 c_void_p, c_int, c_int64, c_float, c_size_t = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_float, ctypes.c_size_t
 
 class LlamaPass(ctypes.Structure):
-    """lri_llama_pass: what one call of lri_llama_run works on."""
+    """lri_llama_pass: what one call of lri_llama_run or lri_llama_run_row works on."""
     _fields_ = ([(k, c_int) for k in ("dtype", "schedule", "n_layer", "B", "S", "n_head", "n_kv", "head_dim", "dim", "inter", "pos_is_i64", "splits")]
                 + [("eps", c_float), ("smax", c_int64), ("table_rows", c_int64)]
                 + [(k, c_void_p) for k in ("layers", "reduces", "rope_table", "input_pos", "final_norm", "resid", "normed", "normed_m", "part_a",
                                            "part_m", "q", "y", "h", "ws_qkv", "ws_wo", "ws_ug", "ws_w2", "scratch")]
                 + [(k, c_size_t) for k in ("ws_qkv_bytes", "ws_wo_bytes", "ws_ug_bytes", "ws_w2_bytes", "scratch_bytes")]
-                + [(k, c_void_p) for k in ("stream", "side", "events", "row_ws")])
+                + [(k, c_void_p) for k in ("stream", "side", "events")])
 
 
 ONE_SM = 0x100  # LRI_ONE_SM
@@ -149,6 +149,7 @@ _SIGNATURES = {
                                    c_int64, c_int, c_int, c_void_p]),
     "lri_round_columns": (c_int, [c_int, c_void_p, c_int64, c_int64, c_int, c_void_p, c_int64, c_void_p]),
     "lri_llama_run": (c_int, [ctypes.POINTER(LlamaPass)]),
+    "lri_llama_run_row": (c_int, [ctypes.POINTER(LlamaPass), c_void_p]),
     "lri_comm_status": (c_int, [c_void_p, c_void_p]),
     "lri_comm_destroy": (c_int, [c_void_p]),
 }

@@ -259,7 +259,7 @@ class Engine:
             return False
         main = torch.cuda.current_stream()
         buffers = dict(rope_table=m.freqs_cis, input_pos=pos, final_norm=m.norm.weight, resid=self.resid, normed=self.normed, part_a=self.part_a,
-                       part_m=self.part_m, q=self.q, y=self.y, h=self.h, row_ws=self.row_ws)
+                       part_m=self.part_m, q=self.q, y=self.y, h=self.h)
         if two and family == "ladder":
             buffers["normed_m"] = self.normed_m
         sizes = dict(dtype=dtype_code(self.dtype), n_layer=len(m.layers), B=B, S=S, n_head=self.nh, n_kv=self.nkv, head_dim=self.hd, dim=self.d,
@@ -269,7 +269,7 @@ class Engine:
                     "desync": DESYNC}[family]
         self.ops.run_layers(schedule, tensors, above, reduces, self._events if two else None, main.cuda_stream,
                             self.side_stream.cuda_stream if two else None, sizes, self.cfg.norm_eps,
-                            dict(ws_qkv=self.ws_qkv, ws_wo=self.ws_wo, ws_ug=self.ws_ug, ws_w2=self.ws_w2, scratch=self.scratch), **buffers)
+                            dict(ws_qkv=self.ws_qkv, ws_wo=self.ws_wo, ws_ug=self.ws_ug, ws_w2=self.ws_w2, scratch=self.scratch), self.row_ws, **buffers)
         return True
 
     @torch.no_grad()

@@ -124,10 +124,10 @@ class CudaOps:
 
     # ---- all layers of a pass ------------------------------------------------------------------------
     @staticmethod
-    def run_layers(schedule, layers, above, reduces, events, main, side, sizes, eps, workspaces, **tensors):
-        """lri_llama_run: `layers` eight tensors a layer as there, `above` the bytes in front of each layer's w1 (empty: none), `sizes` the
+    def run_layers(schedule, layers, above, reduces, events, main, side, sizes, eps, workspaces, row_ws, **tensors):
+        """lri_llama_run_row: `layers` eight tensors a layer as there, `above` the bytes in front of each layer's w1 (empty: none), `sizes` the
         integers of lri_llama_pass, `workspaces` and `tensors` by its names."""
-        _C.require_cuda(*tensors.values(), *layers)
+        _C.require_cuda(row_ws, *tensors.values(), *layers)
         pointers = array("Q", [t.data_ptr() for t in layers])
         for i, n in enumerate(above):
             pointers[8 * i + 4] += n
@@ -142,7 +142,7 @@ class CudaOps:
         p.reduces = ctypes.cast(ctypes.c_char_p(flags), ctypes.c_void_p) if flags is not None else None
         handles = (ctypes.c_void_p * len(events))(*[e.cuda_event for e in events]) if events is not None else None
         p.events = ctypes.cast(handles, ctypes.c_void_p) if handles is not None else None
-        _C.check(_C.lib.lri_llama_run(ctypes.byref(p)))
+        _C.check(_C.lib.lri_llama_run_row(ctypes.byref(p), row_ws.data_ptr()))
 
     # ---- layers with an fp32 residual stream ---------------------------------------------------------
     @staticmethod

@@ -93,3 +93,12 @@ def test_ops_of_the_callers_own_are_called(monkeypatch):
     engine = _model("dense", monkeypatch)._engine
     engine._splits, engine.ops = 1, Own
     assert engine._run_native(1, 1, torch.zeros(1, dtype=torch.int32)) is False
+
+
+def test_the_pass_has_the_size_that_callers_know():
+    """It has no field for its size: one more member would be read behind the struct of whoever was compiled without it."""
+    import ctypes
+    from gpt_fast import _C
+    ints, wide, pointers, sizes = 12 + 1, 2, 2 + 3 + 8 + 5 + 3, 5
+    assert ctypes.sizeof(_C.LlamaPass) == 4 * ints + 4 + 8 * (wide + pointers + sizes)
+    assert _C.LlamaPass._fields_[-1][0] == "events"
