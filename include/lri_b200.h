@@ -35,9 +35,9 @@ typedef void* lri_stream_t; /* a cudaStream_t */
 
 /* LRI_FP32 is taken by the entry points that say so (every product and sum a true 32-bit operation). */
 enum lri_dtype { LRI_BF16 = 0, LRI_FP16 = 1, LRI_FP32 = 2 };
-/* Added to `dtype` of lri_linear, lri_linear_f32 or lri_gateup_glu: a prompt projection (more than 128 token rows) stays on the kernel
- * that gives a tile to one SM.  For passes that run kernels of theirs on a second stream beside their projections (see
- * csrc/gemm_pair.cu). */
+/* Added to `dtype` of lri_linear, lri_linear_f32, lri_gateup_glu or their _early forms: a prompt projection (more than 128
+ * token rows) stays on the kernel that gives a tile to one SM.  For passes that run kernels of theirs on a second stream
+ * beside their projections (see csrc/gemm_pair.cu). */
 enum { LRI_ONE_SM = 0x100 };
 
 enum lri_status {
@@ -125,6 +125,15 @@ int lri_streamk_plan(int64_t M, int N, int K, int* tiles, int* k_tiles, int* max
                      int* token_tile);
 int lri_linear(int dtype, const void* x, const void* w, const void* addend, void* y, int64_t M,
                int N, int K, void* workspace, size_t workspace_bytes, lri_stream_t stream);
+/* lri_linear, lri_linear_f32 and lri_gateup_glu for a caller who knows that no other stream's kernels run beside the projection: with 9 to 64
+ * token rows the kernel behind it on `stream` may start before the projection's last sums (it waits for them before it reads; the results are the
+ * same bits).  Beside another stream's kernels that costs more than it gains, so the plain entry points never do it. */
+int lri_linear_early(int dtype, const void* x, const void* w, const void* addend, void* y, int64_t M, int N, int K, void* workspace,
+                     size_t workspace_bytes, lri_stream_t stream);
+int lri_linear_f32_early(int dtype, const void* x, const void* w, float* y, int64_t M, int N, int K, void* workspace,
+                         size_t workspace_bytes, lri_stream_t stream);
+int lri_gateup_glu_early(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K, float alpha, float limit, float offset,
+                         void* workspace, size_t workspace_bytes, lri_stream_t stream);
 /* y = x W^T with y in fp32, no rounding: projections that feed fp32 arithmetic (norms, gates, recurrences,
  * routers).  Kernels and workspace as lri_linear.  Both entry points also take LRI_FP32 (then y is fp32 in
  * either) and any K; those run a plain SIMT kernel.  No counterpart in the reference. */

@@ -302,11 +302,11 @@ __global__ void __launch_bounds__(256) streamk_finish_kernel(const StreamKParams
   const int tile = blockIdx.x;
   int first_cta, nseg;
   tile_segments(tile, p, first_cta, nseg);
-  // The kernel behind may come as soon as the projection's CTAs leave their SMs: its weights, which nothing here writes, arrive beside the sums
-  // below.  us a step, let in behind the wait / before: 8B dense, 16 sequences 3549 / 3510; 1B, 16 925 / 868; stories110M, 16 400 / 355; Migosun
+  // For a caller who says so, the kernel behind may come as soon as the projection's CTAs leave their SMs: its weights, which nothing here writes,
+  // arrive beside the sums below.  us a captured step, let in behind the wait / before: 8B dense, 16 sequences 3549 / 3510; 1B, 16 925 / 868; stories110M, 16 400 / 355; Migosun
   // 1B, 24 1282 / 1175, 8B, 16 4690 / 4640.  Not where another stream's kernels wait for the same SMs, which it would keep out (8B ladder, 16
   // sequences 3103 / 3310), and not with up to eight rows, where streaming kernels of thousands of CTAs follow (Patevik 8B, 4 sequences 9180 / 9600).
-  const bool early = !p.lin.share.late && p.lin.m > 8;
+  const bool early = p.lin.share.early && p.lin.m > 8;
   if (early) pdl_launch_dependents();
   pdl_wait();
   if (!early) pdl_launch_dependents();

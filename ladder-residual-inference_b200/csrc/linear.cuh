@@ -45,7 +45,7 @@ struct NormArgs {
 
 // Small batches, for a caller who knows what runs around a projection; the results are the same bits.
 struct Share {
-  bool late;       // another stream's kernels run beside it (or it is known to lose): the kernel behind is not let in early
+  bool early;      // nothing of another stream runs beside it: the kernel behind may be let in before the sums
   bool half_ring;  // another stream's projections share the SMs: half of their shared memory is left to them
 };
 struct LinearParams {

@@ -437,13 +437,17 @@ extern "C" int lri_linear(int dtype, const void* x, const void* w, const void* a
                           size_t workspace_bytes, lri_stream_t stream) {
   return lri::linear(dtype, x, w, addend, y, M, N, K, workspace, workspace_bytes, {}, stream);
 }
+extern "C" int lri_linear_early(int dtype, const void* x, const void* w, const void* addend, void* y, int64_t M, int N, int K, void* workspace,
+                                size_t workspace_bytes, lri_stream_t stream) {
+  return lri::linear(dtype, x, w, addend, y, M, N, K, workspace, workspace_bytes, Share{true, false}, stream);
+}
 
 extern "C" size_t lri_linear_f32_workspace_bytes(int64_t M, int N) {
   return M < 0 || N <= 0 ? 0 : streamk_bytes(EPI_F32, M, N);
 }
 
-extern "C" int lri_linear_f32(int dtype, const void* x, const void* w, float* y, int64_t M, int N, int K, void* workspace,
-                              size_t workspace_bytes, lri_stream_t stream) {
+static int linear_f32(int dtype, const void* x, const void* w, float* y, int64_t M, int N, int K, void* workspace, size_t workspace_bytes, Share share,
+                      lri_stream_t stream) {
   const bool one_sm = take_one_sm(dtype);
   LRI_REQUIRE(dtype >= LRI_BF16 && dtype <= LRI_FP32, LRI_ERR_UNSUPPORTED, "linear_f32: dtype %d", dtype);
   LRI_REQUIRE(x && w && y, LRI_ERR_ARG, "linear_f32: NULL pointer");
@@ -453,7 +457,7 @@ extern "C" int lri_linear_f32(int dtype, const void* x, const void* w, float* y,
   if (dtype == LRI_FP32 || K % 8 != 0 || !aligned16(x) || !aligned16(w))
     return gemm_generic_launch(dtype, x, w, nullptr, y, true, M, N, K, st);
   LinearParams p{};
-  p.x = x, p.w = w, p.y = y, p.m = static_cast<int>(M), p.n = N, p.k = K;
+  p.x = x, p.w = w, p.y = y, p.m = static_cast<int>(M), p.n = N, p.k = K, p.share = share;
   if (M <= streaming_rows() && !streamk_few_rows(EPI_F32, p, workspace, workspace_bytes))
     return streaming_launch(dtype, EPI_F32, p, st, prefer_simt_gemv());
   if ((M <= streaming_rows() || streamk_rows(M)) && gemm_streamk_supports(EPI_F32, p, workspace, workspace_bytes))
@@ -462,6 +466,14 @@ extern "C" int lri_linear_f32(int dtype, const void* x, const void* w, float* y,
   if (current_gemm_backend() != LRI_GEMM_SIMT && N % 8 == 0 && aligned16(y))
     return gemm_tcgen05_f32_launch(dtype, x, w, y, M, N, K, one_sm, st);
   return gemm_generic_launch(dtype, x, w, nullptr, y, true, M, N, K, st);
+}
+extern "C" int lri_linear_f32(int dtype, const void* x, const void* w, float* y, int64_t M, int N, int K, void* workspace,
+                              size_t workspace_bytes, lri_stream_t stream) {
+  return linear_f32(dtype, x, w, y, M, N, K, workspace, workspace_bytes, {}, stream);
+}
+extern "C" int lri_linear_f32_early(int dtype, const void* x, const void* w, float* y, int64_t M, int N, int K, void* workspace,
+                                    size_t workspace_bytes, lri_stream_t stream) {
+  return linear_f32(dtype, x, w, y, M, N, K, workspace, workspace_bytes, Share{true, false}, stream);
 }
 
 extern "C" int lri_streamk_plan(int64_t M, int N, int K, int* tiles, int* k_tiles, int* max_segments, int* ctas,
@@ -544,8 +556,8 @@ extern "C" size_t lri_gateup_glu_workspace_bytes(int dtype, int64_t M, int I, in
   return max_size(glu_raw_bytes(dtype, M, I, K), sk);
 }
 
-extern "C" int lri_gateup_glu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K, float alpha,
-                              float limit, float offset, void* workspace, size_t workspace_bytes, lri_stream_t stream) {
+static int gateup_glu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K, float alpha, float limit, float offset,
+                      void* workspace, size_t workspace_bytes, Share share, lri_stream_t stream) {
   const bool one_sm = take_one_sm(dtype);
   LRI_REQUIRE(dtype >= LRI_BF16 && dtype <= LRI_FP32, LRI_ERR_UNSUPPORTED, "gateup_glu: dtype %d", dtype);
   LRI_REQUIRE(x && w1 && h, LRI_ERR_ARG, "gateup_glu: NULL pointer");
@@ -554,7 +566,7 @@ extern "C" int lri_gateup_glu(int dtype, const void* x, const void* w1, void* h,
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LinearParams p{};
   p.x = x, p.w = w1, p.y = h, p.m = static_cast<int>(M), p.n = I, p.k = K;
-  p.ex.glu = GluParams{alpha, limit, offset}, p.one_sm = one_sm;
+  p.ex.glu = GluParams{alpha, limit, offset}, p.one_sm = one_sm, p.share = share;
   if (dtype != LRI_FP32 && K % 8 == 0 && aligned16(x) && aligned16(w1)) {
     if (M == 1) return gemv_launch(dtype, EPI_GLU, p, st);
     if (M <= streaming_rows() && !streamk_few_rows(EPI_GLU, p, workspace, workspace_bytes)) return gemv_mma_launch(dtype, EPI_GLU, p, st);
@@ -570,6 +582,14 @@ extern "C" int lri_gateup_glu(int dtype, const void* x, const void* w1, void* h,
   int rc = lri_linear_f32(one_sm ? dtype | LRI_ONE_SM : dtype, x, w1, static_cast<float*>(workspace), M, 2 * I, K, nullptr, 0, stream);
   if (rc != LRI_OK) return rc;
   return glu_rows_launch(dtype, static_cast<const float*>(workspace), h, M, I, p.ex.glu, st);
+}
+extern "C" int lri_gateup_glu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K, float alpha, float limit, float offset,
+                              void* workspace, size_t workspace_bytes, lri_stream_t stream) {
+  return gateup_glu(dtype, x, w1, h, M, I, K, alpha, limit, offset, workspace, workspace_bytes, {}, stream);
+}
+extern "C" int lri_gateup_glu_early(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K, float alpha, float limit,
+                                    float offset, void* workspace, size_t workspace_bytes, lri_stream_t stream) {
+  return gateup_glu(dtype, x, w1, h, M, I, K, alpha, limit, offset, workspace, workspace_bytes, Share{true, false}, stream);
 }
 
 static size_t qkv_raw_bytes(int64_t M, int n_head, int n_kv, int head_dim) {

@@ -17,7 +17,7 @@ struct Pass {
   int64_t rows;
   void* row_ws;
   int rc = LRI_OK;
-  Share share{};  // see late() and where two streams run
+  Share share{};  // see early() and where two streams run
 
   const void* at(int layer, int which) const { return p.layers[static_cast<int64_t>(layer) * kPointers + which]; }
   bool ok(int r) { return (rc = r) == LRI_OK; }
@@ -76,7 +76,7 @@ struct Pass {
   // the attention chain of a layer on `stream`, its MLP chain on `side`: see Engine._run_ladder_two_streams
   bool ladder_two_streams() {
     if (!record(0, p.stream) || !wait(0, p.side)) return false;
-    share = {true, true};
+    share = {false, true};
     int n = 1;
     for (int l = 0; l < p.n_layer; ++l, n += 2) {
       if (!norm(at(l, kAttentionNorm), l ? p.part_a : nullptr, nullptr, true, p.normed, p.stream) || !record(n, p.stream) || !attention(l)) return false;
@@ -98,7 +98,7 @@ struct Pass {
   // the gate/up projection beside the attention chain: both read the norm
   bool parallel_two_streams() {
     const void* pending = nullptr;
-    share = {true, rows > 8};  // (3B, whole / half ring: 2 sequences 1677 / 1779 us, 4 1785 / 1903, 16 2445 / 2390, 40 3499 / 3495)
+    share = {false, rows > 8};  // (3B, whole / half ring: 2 sequences 1677 / 1779 us, 4 1785 / 1903, 16 2445 / 2390, 40 3499 / 3495)
     for (int l = 0; l < p.n_layer; ++l) {
       if (!norm(at(l, kAttentionNorm), pending, nullptr, true, p.normed, p.stream) || !record(2 * l, p.stream) || !wait(2 * l, p.side)) return false;
       if (!attention(l) ||
@@ -123,9 +123,9 @@ struct Pass {
     cudaStreamCaptureStatus status;
     return cudaStreamIsCapturing(static_cast<cudaStream_t>(p.stream), &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
   }
-  // One stream, 25 to 64 rows: kernels behind small-batch projections come early (gemm_streamk.cu) but for wide models (8B dense, 32, 64 sequences 3612
-  // / 3647, 4225 / 4264 us) and small ones called eagerly (stories110M, 49 476 / 498, captured 462 / 437; 1B, 32 964 / 909).
-  bool late() const { return rows > 24 && rows <= kSplitKMaxRows && (p.dim >= 4096 || (p.dim < 1024 && eager())); }
+  // One stream: kernels behind small-batch projections come early (gemm_streamk.cu), from 25 rows on but for wide models (8B dense, 32, 64 sequences
+  // 3612 / 3647, 4225 / 4264 us) and small ones called eagerly (stories110M, 49 476 / 498, captured 462 / 437; 1B, 32 964 / 909).
+  bool early() const { return rows <= 24 || (p.dim < 4096 && (p.dim >= 1024 || !eager())); }
   bool folded_qkv(int l, const void* add1, bool write) {
     void *kc = const_cast<void*>(at(l, kKCache)), *vc = const_cast<void*>(at(l, kVCache));
     const NormArgs nm{cur, add1, nullptr, at(l, kAttentionNorm), write ? other : nullptr, p.eps};
@@ -204,7 +204,7 @@ extern "C" int lri_llama_run_row(const lri_llama_pass* pass, void* row_ws) {
       case LRI_PARALLEL_TWO_STREAMS: run.folded_parallel(); return run.rc;
     }
   }
-  if (run.late()) run.share.late = true;
+  run.share.early = run.early();
   // From 129 rows on (or 65, where the option forces it) the projections of two streams would run on pairs of SMs beside each other, which is not
   // done (gemm_pair.cu): such a pass runs on one stream, with the same results.
   const bool two = run.rows <= (option(OPT_GEMM_PAIR) > 1 ? kSplitKMaxRows : 128);

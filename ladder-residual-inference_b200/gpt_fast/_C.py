@@ -154,6 +154,9 @@ _SIGNATURES = {
     "lri_comm_destroy": (c_int, [c_void_p]),
 }
 
+for _name in ("lri_linear", "lri_linear_f32", "lri_gateup_glu"):
+    _SIGNATURES[_name + "_early"] = _SIGNATURES[_name]
+
 for _name, (_res, _args) in _SIGNATURES.items():
     _fn = getattr(lib, _name)
     _fn.restype = _res

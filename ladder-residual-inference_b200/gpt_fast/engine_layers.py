@@ -126,6 +126,9 @@ class LayerEngine(Engine):
             if packed:
                 self.moe_packed = buf(128 * tiles, self.d)
                 self.moe_scale = torch.zeros(128 * tiles, dtype=torch.float32, device=device)
+        # On one GPU nothing runs beside these projections (low-rank ones are left out: in prompts the side stream's attention does).  An ops
+        # object of the caller's own need not know the word.
+        self.alone = dict(early=True) if self.comm.world == 1 and self.ops in (CudaOps, OneSmOps) else {}
         self.side_stream = None
         if of("chunked_attention") and self.comm.world == 1 and self.ops is OneSmOps and self.resid.is_cuda and os.environ.get("LRI_SIDE_STREAM", "1") != "0":
             self.side_stream = torch.cuda.Stream()
@@ -291,7 +294,7 @@ class LayerEngine(Engine):
         self.off = branch.gate_rows
         if branch.in_proj is not None:
             self.ld = branch.in_proj.weight.shape[0]
-            self.ops.linear_f32(self.normed, branch.in_proj.weight, self.proj, rows, workspace=self.ws_in)
+            self.ops.linear_f32(self.normed, branch.in_proj.weight, self.proj, rows, workspace=self.ws_in, **self.alone)
 
     def _body(self, idx, rows, B, S, pos):
         eps, ops = self.cfg.norm_eps, self.ops
@@ -305,10 +308,10 @@ class LayerEngine(Engine):
                 slots, y_rows = self._experts(sub, rows)
                 self._join(branch, nxt, self.moe_out, rows, sub.top, slots, y_rows)
             elif sub.kind == "glu":
-                ops.gateup_glu(self.normed, sub.w1, self.glu_hidden, rows, sub.glu, workspace=self.ws_glu)
-                ops.linear(self.glu_hidden, sub.w2, self.part, rows, workspace=self.ws_out)
+                ops.gateup_glu(self.normed, sub.w1, self.glu_hidden, rows, sub.glu, workspace=self.ws_glu, **self.alone)
+                ops.linear(self.glu_hidden, sub.w2, self.part, rows, workspace=self.ws_out, **self.alone)
                 self._join(branch, nxt, self.part, rows)
             else:
                 run[sub.kind](sub, rows, B, S, pos, eps)
-                ops.linear(self.y, sub.wo.weight, self.part, rows, workspace=self.ws_out)
+                ops.linear(self.y, sub.wo.weight, self.part, rows, workspace=self.ws_out, **self.alone)
                 self._join(branch, nxt, self.part, rows)

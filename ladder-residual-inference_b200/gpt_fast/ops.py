@@ -38,13 +38,14 @@ class CudaOps:
 
     # ---- linear family -----------------------------------------------------------------------
     @staticmethod
-    def linear(x, w, out, rows, addend=None, workspace=None, flags=0):
-        """flags: 0 or _C.ONE_SM."""
+    def linear(x, w, out, rows, addend=None, workspace=None, flags=0, early=False):
+        """flags: 0 or _C.ONE_SM; early: see lri_linear_early."""
         _C.require_cuda(x, w, out)
         n, k = w.shape
         ws_ptr, ws_bytes = (workspace.data_ptr(), workspace.numel() * workspace.element_size()) if workspace is not None else (None, 0)
-        _C.check(_C.lib.lri_linear(_C.dtype_code_any(x.dtype) | flags, x.data_ptr(), w.data_ptr(), _C.ptr(addend), out.data_ptr(),
-                                   rows, n, k, ws_ptr, ws_bytes, _C.stream_handle()))
+        call = _C.lib.lri_linear_early if early else _C.lib.lri_linear
+        _C.check(call(_C.dtype_code_any(x.dtype) | flags, x.data_ptr(), w.data_ptr(), _C.ptr(addend), out.data_ptr(), rows, n, k, ws_ptr, ws_bytes,
+                      _C.stream_handle()))
 
     @staticmethod
     def linear_workspace_bytes(rows, n):
@@ -146,13 +147,13 @@ class CudaOps:
 
     # ---- layers with an fp32 residual stream ---------------------------------------------------------
     @staticmethod
-    def linear_f32(x, w, out, rows, workspace=None, flags=0):
+    def linear_f32(x, w, out, rows, workspace=None, flags=0, early=False):
         """out (fp32) = x w^T, unrounded."""
         _C.require_cuda(x, w, out)
         n, k = w.shape
         ws_ptr, ws_bytes = (workspace.data_ptr(), workspace.numel() * workspace.element_size()) if workspace is not None else (None, 0)
-        _C.check(_C.lib.lri_linear_f32(_C.dtype_code_any(x.dtype) | flags, x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, n, k,
-                                       ws_ptr, ws_bytes, _C.stream_handle()))
+        call = _C.lib.lri_linear_f32_early if early else _C.lib.lri_linear_f32
+        _C.check(call(_C.dtype_code_any(x.dtype) | flags, x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, n, k, ws_ptr, ws_bytes, _C.stream_handle()))
 
     @staticmethod
     def linear_f32_workspace_bytes(rows, n):
@@ -312,13 +313,14 @@ class CudaOps:
         return _C.lib.lri_gateup_glu_workspace_bytes(_C.dtype_code_any(dtype), rows, inter, k)
 
     @staticmethod
-    def gateup_glu(x, w1, h, rows, glu, workspace=None, flags=0):
+    def gateup_glu(x, w1, h, rows, glu, workspace=None, flags=0, early=False):
         """w1 [2 ff, dim] = [up | gate]; glu = (alpha, limit, offset)."""
         _C.require_cuda(x, w1, h)
         two_i, k = w1.shape
         ws_ptr, ws_bytes = (workspace.data_ptr(), workspace.numel() * workspace.element_size()) if workspace is not None else (None, 0)
-        _C.check(_C.lib.lri_gateup_glu(_C.dtype_code_any(x.dtype) | flags, x.data_ptr(), w1.data_ptr(), h.data_ptr(), rows, two_i // 2, k,
-                                       *[float(g) for g in glu], ws_ptr, ws_bytes, _C.stream_handle()))
+        call = _C.lib.lri_gateup_glu_early if early else _C.lib.lri_gateup_glu
+        _C.check(call(_C.dtype_code_any(x.dtype) | flags, x.data_ptr(), w1.data_ptr(), h.data_ptr(), rows, two_i // 2, k, *[float(g) for g in glu],
+                      ws_ptr, ws_bytes, _C.stream_handle()))
 
     # ---- grouped attention on a cache ------------------------------------------------------------------------
     @staticmethod
