@@ -123,9 +123,18 @@ struct Pass {
     cudaStreamCaptureStatus status;
     return cudaStreamIsCapturing(static_cast<cudaStream_t>(p.stream), &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
   }
-  // One stream: kernels behind small-batch projections come early (gemm_streamk.cu), from 25 rows on but for wide models (8B dense, 32, 64 sequences
-  // 3612 / 3647, 4225 / 4264 us) and small ones called eagerly (stories110M, 49 476 / 498, captured 462 / 437; 1B, 32 964 / 909).
-  bool early() const { return rows <= 24 || (p.dim < 4096 && (p.dim >= 1024 || !eager())); }
+  // One stream: where the kernels behind small-batch projections come early (gemm_streamk.cu).  us, late / early.
+  // Captured steps: 8B dense, 9, 16, 20 sequences 3272 / 3218, 3359 / 3277, 3491 / 3420, 24 the same (0.989 to 1.013 in three comparisons), but 28, 40, 64
+  // 3569 / 3596, 3900 / 3961, 4133 / 4177; 3B dense, 16, 24, 28 2179 / 2167, 2367 / 2338, 2536 / 2513, but 32, 48, 64 2539 / 2560, 2971 / 3007, 3475 / 3511; narrower models at any
+  // number: 1B 16, 32, 64 902 / 833, 963 / 910, 1136 / 1127, stories110M 371 / 351, 409 / 394, 576 / 558.
+  // Eager passes lose by it: 8B dense, 16 and 64 sequences 3402 / 3477, 4293 / 4389, a prompt of 16 tokens 3414 / 3466; 3B 2269 / 2348, 3555 / 3601,
+  // 2081 / 2116; 1B 896 / 917, 1174 / 1227, 896 / 922; stories110M 404 / 425, 603 / 625, 407 / 417.  But not short prompts through parallel blocks: 3B,
+  // 9, 16, 32 tokens 2027 / 1998, 2055 / 2033, 2167 / 2181; 8B 3338 / 3297, 3379 / 3373, 3573 / 3605; 1B, 9, 16, 32, 64 890 / 870, 895 / 884, 943 / 922,
+  // 1061 / 1054.
+  bool early() const {
+    if (eager()) return p.schedule == LRI_PARALLEL && p.S > 1 && rows <= (p.dim > 2048 ? 16 : kSplitKMaxRows);
+    return rows <= (p.dim >= 4096 ? 24 : p.dim > 2048 ? 28 : kSplitKMaxRows);
+  }
   bool folded_qkv(int l, const void* add1, bool write) {
     void *kc = const_cast<void*>(at(l, kKCache)), *vc = const_cast<void*>(at(l, kVCache));
     const NormArgs nm{cur, add1, nullptr, at(l, kAttentionNorm), write ? other : nullptr, p.eps};
@@ -204,7 +213,7 @@ extern "C" int lri_llama_run_row(const lri_llama_pass* pass, void* row_ws) {
       case LRI_PARALLEL_TWO_STREAMS: run.folded_parallel(); return run.rc;
     }
   }
-  run.share.early = run.early();
+  run.share.early = run.rows > 8 && run.early();  // (few rows: see gemm_streamk.cu)
   // From 129 rows on (or 65, where the option forces it) the projections of two streams would run on pairs of SMs beside each other, which is not
   // done (gemm_pair.cu): such a pass runs on one stream, with the same results.
   const bool two = run.rows <= (option(OPT_GEMM_PAIR) > 1 ? kSplitKMaxRows : 128);

@@ -126,15 +126,22 @@ class LayerEngine(Engine):
             if packed:
                 self.moe_packed = buf(128 * tiles, self.d)
                 self.moe_scale = torch.zeros(128 * tiles, dtype=torch.float32, device=device)
-        # On one GPU nothing runs beside these projections (low-rank ones are left out: in prompts the side stream's attention does).  An ops
-        # object of the caller's own need not know the word.
-        self.alone = dict(early=True) if self.comm.world == 1 and self.ops in (CudaOps, OneSmOps) else {}
+        self.early_eagerly = not moes
         self.side_stream = None
         if of("chunked_attention") and self.comm.world == 1 and self.ops is OneSmOps and self.resid.is_cuda and os.environ.get("LRI_SIDE_STREAM", "1") != "0":
             self.side_stream = torch.cuda.Stream()
             self._fork, self._join_event = torch.cuda.Event(), torch.cuda.Event()
         self._setup_head(max_batch, device, dtype)
         self.ready = True
+
+    def _nothing_beside(self):
+        """Whether input and output projections ask for an early start of the kernel behind them (lri_linear_early).  On one GPU nothing runs beside
+        them (beside low-rank ones the side stream's attention does, in prompts); an ops object of the caller's own need not know the word.  Designs
+        with experts only in captures: us, late / early, Patevik 1B with 16 and 32 sequences captured 2216 / 2185, 2371 / 2354, eagerly 2287 / 2319,
+        2455 / 2479, a prompt of 48 tokens 2361 / 2384; Migosun 8B captured 4580 / 4448, 5726 / 5603, eagerly 4907 / 4845, 6060 / 5900."""
+        if self.comm.world > 1 or self.ops not in (CudaOps, OneSmOps):
+            return False
+        return self.early_eagerly or (self.resid.is_cuda and torch.cuda.is_current_stream_capturing())
 
     # ------------------------------------------------------------------------------------------
     # Mixers leave the rows that their output projection reads in self.y.
@@ -299,6 +306,7 @@ class LayerEngine(Engine):
     def _body(self, idx, rows, B, S, pos):
         eps, ops = self.cfg.norm_eps, self.ops
         run = {"latent_attention": self._latent_attention, "hgrn2": self._hgrn2, "gla": self._gla, "parallel": self._parallel}
+        self.alone = dict(early=True) if self._nothing_beside() else {}
         self._start(idx, self.branches[0])
         for i, branch in enumerate(self.branches):
             nxt = self.branches[i + 1] if i + 1 < len(self.branches) else None

@@ -64,19 +64,36 @@ def test_plain_calls_of_the_two_stream_schedule(monkeypatch):
     assert lib.calls.count("lri_linear") == 4 and not [n for n in lib.calls if n.endswith("_early")]
 
 
-def test_which_engines_ask():
+@pytest.mark.parametrize("util,eagerly", [(mu, True), (pu, False)])
+def test_which_layer_engines_ask(util, eagerly):
     from gpt_fast.ops import CudaOps
-    for util in (mu, pu):
-        case = next(iter(util.CONFIGS.values()))
-        model = util.build(case[0] if util is mu else case, util.weights(case), torch.bfloat16, "cpu", 1, 16)
-        engine = model._engine
-        assert engine.alone == {"early": True}
+    case = next(iter(util.CONFIGS.values()))
+    engine = util.build(case[0] if util is mu else case, util.weights(case), torch.bfloat16, "cpu", 1, 16)._engine
+    assert engine._nothing_beside() is eagerly
 
-        class Own(CudaOps):
-            pass
-        engine.ops = Own
-        engine.setup(1, 16, "cpu", torch.bfloat16)
-        assert engine.alone == {}
+    class Own(CudaOps):
+        pass
+    engine.ops = Own
+    assert not engine._nothing_beside()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("util,eagerly", [(mu, {"early": True}), (pu, {})])
+def test_experts_ask_in_captures_alone(util, eagerly):
+    case = next(iter(util.CONFIGS.values()))
+    model = util.build(case[0] if util is mu else case, util.weights(case), torch.bfloat16, "cuda", 16, 16)
+    tok, pos = torch.zeros(16, 1, dtype=torch.int32, device="cuda"), torch.tensor([0], dtype=torch.int32, device="cuda")
+    with torch.no_grad():
+        eager = model(tok, pos)
+        assert model._engine.alone == eagerly
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            logits = model(tok, pos)
+        assert model._engine.alone == {"early": True}
+        graph.replay()
+        assert torch.equal(eager, logits)
+        model(tok, pos)
+        assert model._engine.alone == eagerly
 
 
 @pytest.mark.gpu
