@@ -98,7 +98,10 @@ struct Pass {
   // the gate/up projection beside the attention chain: both read the norm
   bool parallel_two_streams() {
     const void* pending = nullptr;
-    share = {false, rows > 8};  // (3B, whole / half ring: 2 sequences 1677 / 1779 us, 4 1785 / 1903, 16 2445 / 2390, 40 3499 / 3495)
+    // us a captured step, whole / half ring.  8B: 16, 32 sequences 3251 / 3176, 3488 / 3400, but 33, 40, 48, 64 3542 / 3609, 3777 / 3851, 3848 / 3950, 4025 /
+    // 4120; 3B: 2, 4 1677 / 1779, 1785 / 1903, 9, 40, 48 1842 / 1785, 2712 / 2702, 2798 / 2797, 64 3241 / 3258; 1B: 9, 16, 32 787 / 756, 795 / 777, 869 / 845,
+    // 48, 64 943 / 944, 1048 / 1056.
+    share = {false, rows > 8 && rows <= (p.dim >= 4096 ? 32 : 48)};
     for (int l = 0; l < p.n_layer; ++l) {
       if (!norm(at(l, kAttentionNorm), pending, nullptr, true, p.normed, p.stream) || !record(2 * l, p.stream) || !wait(2 * l, p.side)) return false;
       if (!attention(l) ||
