@@ -20,11 +20,16 @@ namespace {
 
 constexpr int kGemvMaxWarps = 8;
 
+// the NORM form alone has that struct among its parameters
+struct NoNorm {};
+template <bool NORM>
+using NormOf = std::conditional_t<NORM, NormArgs, NoNorm>;
+
 // NORM (one row): x is the norm of a sum that every CTA takes for itself; all of K is in flight at once.  One launch less in front of a
 // projection, for about 1.4 us more in it (llama_pass.cu says when that pays).  Sums are taken as in add_rmsnorm_kernel (a chunk of 256
 // elements here is a warp there): the same bits.
 template <typename T, int M, int R, int U, int EPI, bool NORM = false>
-__global__ void __launch_bounds__(kGemvMaxWarps * 32) gemv_kernel(const LinearParams p) {
+__global__ void __launch_bounds__(kGemvMaxWarps * 32) gemv_kernel(const LinearParams p, const NormOf<NORM> nm) {
   static_assert(R % 2 == 0, "epilogues work on pairs of rows");
   static_assert(!NORM || M == 1, "one row");
   const int lane = threadIdx.x & 31;
@@ -91,7 +96,7 @@ __global__ void __launch_bounds__(kGemvMaxWarps * 32) gemv_kernel(const LinearPa
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int k = ((c0 + u * W) << 8) + lane * 8;
-      nw[u] = k < K ? __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.nm.weight) + k)) : make_uint4(0, 0, 0, 0);
+      nw[u] = k < K ? __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(nm.weight) + k)) : make_uint4(0, 0, 0, 0);
     }
   }
   if (!by_pair) {
@@ -106,9 +111,9 @@ __global__ void __launch_bounds__(kGemvMaxWarps * 32) gemv_kernel(const LinearPa
       const int k = ((c0 + u * W) << 8) + lane * 8;
       rv[u] = av[u] = bv[u] = make_uint4(0, 0, 0, 0);
       if (k < K) {
-        rv[u] = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.nm.res) + k);
-        if (p.nm.add1) av[u] = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.nm.add1) + k);
-        if (p.nm.add2) bv[u] = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.nm.add2) + k);
+        rv[u] = *reinterpret_cast<const uint4*>(static_cast<const T*>(nm.res) + k);
+        if (nm.add1) av[u] = *reinterpret_cast<const uint4*>(static_cast<const T*>(nm.add1) + k);
+        if (nm.add2) bv[u] = *reinterpret_cast<const uint4*>(static_cast<const T*>(nm.add2) + k);
       }
     }
     float xs[U][8];
@@ -116,13 +121,13 @@ __global__ void __launch_bounds__(kGemvMaxWarps * 32) gemv_kernel(const LinearPa
     for (int u = 0; u < U; ++u) {
       const int c = c0 + u * W;
       unpack8<T>(rv[u], xs[u]);
-      if (p.nm.add1) {
+      if (nm.add1) {
         float a[8];
         unpack8<T>(av[u], a);
 #pragma unroll
         for (int e = 0; e < 8; ++e) xs[u][e] = rnd<T>(xs[u][e] + a[e]);
       }
-      if (p.nm.add2) {
+      if (nm.add2) {
         float b[8];
         unpack8<T>(bv[u], b);
 #pragma unroll
@@ -133,11 +138,11 @@ __global__ void __launch_bounds__(kGemvMaxWarps * 32) gemv_kernel(const LinearPa
       for (int e = 0; e < 8; ++e) ss += xs[u][e] * xs[u][e];
       ss = warp_sum(ss);
       if (lane == 0 && c < nchunks) squares[c] = ss;
-      if (tile == 0 && p.nm.res_out && c * 256 + lane * 8 < K)
-        *reinterpret_cast<uint4*>(static_cast<T*>(p.nm.res_out) + c * 256 + lane * 8) = pack8<T>(xs[u]);
+      if (tile == 0 && nm.res_out && c * 256 + lane * 8 < K)
+        *reinterpret_cast<uint4*>(static_cast<T*>(nm.res_out) + c * 256 + lane * 8) = pack8<T>(xs[u]);
     }
     __syncthreads();
-    const float inv = rsqrtf(warp_sum(lane < nchunks ? squares[lane] : 0.f) / static_cast<float>(K) + p.nm.eps);
+    const float inv = rsqrtf(warp_sum(lane < nchunks ? squares[lane] : 0.f) / static_cast<float>(K) + nm.eps);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       float nf[8], xf[8];
@@ -279,7 +284,7 @@ __global__ void __launch_bounds__(kGemvMaxWarps * 32) gemv_kernel(const LinearPa
 }
 
 template <typename T, int M, int R, int U, int EPI, bool NORM = false>
-int launch_gemv(const LinearParams& p, cudaStream_t st) {
+int launch_gemv(const LinearParams& p, cudaStream_t st, const NormOf<NORM>& nm = {}) {
   const int nchunks = (p.k + 255) >> 8;
   int W = (nchunks + U - 1) / U;
   W = W < 1 ? 1 : (W > kGemvMaxWarps ? kGemvMaxWarps : W);
@@ -287,7 +292,7 @@ int launch_gemv(const LinearParams& p, cudaStream_t st) {
   const int64_t grid = (p.n + per_cta - 1) / per_cta;
   const unsigned pairs = p.ex.pairs > 0 ? static_cast<unsigned>(p.ex.pairs) : 1u;
   const dim3 dims = p.ex.pairs > 0 ? dim3(pairs, static_cast<unsigned>(grid)) : dim3(static_cast<unsigned>(grid));
-  LRI_CUDA(launch_pdl(gemv_kernel<T, M, R, U, EPI, NORM>, dims, dim3(W * 32), 0, st, p));
+  LRI_CUDA(launch_pdl(gemv_kernel<T, M, R, U, EPI, NORM>, dims, dim3(W * 32), 0, st, p, nm));
   LRI_LAUNCH_CHECK("gemv_kernel");
   return LRI_OK;
 }
@@ -330,10 +335,10 @@ int dispatch_m(const LinearParams& p, cudaStream_t st) {
 constexpr int kNormMaxK = 1024;
 // the forms that dispatch_m takes for one row of at most that width
 template <typename T, int EPI>
-int dispatch_norm(const LinearParams& p, cudaStream_t st) {
+int dispatch_norm(const LinearParams& p, const NormArgs& nm, cudaStream_t st) {
   const int r = rows_per_cta(p);
-  if (r == 2) return launch_gemv<T, 1, 2, 8, EPI, true>(p, st);
-  return r == 8 ? launch_gemv<T, 1, 8, 2, EPI, true>(p, st) : launch_gemv<T, 1, 4, 4, EPI, true>(p, st);
+  if (r == 2) return launch_gemv<T, 1, 2, 8, EPI, true>(p, st, nm);
+  return r == 8 ? launch_gemv<T, 1, 8, 2, EPI, true>(p, st, nm) : launch_gemv<T, 1, 4, 4, EPI, true>(p, st, nm);
 }
 
 template <typename T>
@@ -355,10 +360,10 @@ int dispatch_epi(int epi, const LinearParams& p, cudaStream_t st) {
 
 bool gemv_norm_supports(int64_t m, int k) { return m == 1 && k % 8 == 0 && k <= kNormMaxK; }
 
-int gemv_norm_launch(int dtype, int epi, const LinearParams& p, cudaStream_t st) {
+int gemv_norm_launch(int dtype, int epi, const LinearParams& p, const NormArgs& nm, cudaStream_t st) {
   if (!gemv_norm_supports(p.m, p.k) || (epi != EPI_QKV && epi != EPI_SWIGLU)) return fail(LRI_ERR_ARG, "gemv with norm: m=%d k=%d", p.m, p.k);
-  if (dtype == LRI_BF16) return epi == EPI_QKV ? dispatch_norm<__nv_bfloat16, EPI_QKV>(p, st) : dispatch_norm<__nv_bfloat16, EPI_SWIGLU>(p, st);
-  return epi == EPI_QKV ? dispatch_norm<__half, EPI_QKV>(p, st) : dispatch_norm<__half, EPI_SWIGLU>(p, st);
+  if (dtype == LRI_BF16) return epi == EPI_QKV ? dispatch_norm<__nv_bfloat16, EPI_QKV>(p, nm, st) : dispatch_norm<__nv_bfloat16, EPI_SWIGLU>(p, nm, st);
+  return epi == EPI_QKV ? dispatch_norm<__half, EPI_QKV>(p, nm, st) : dispatch_norm<__half, EPI_SWIGLU>(p, nm, st);
 }
 
 int gemv_launch(int dtype, int epi, const LinearParams& p, cudaStream_t st) {

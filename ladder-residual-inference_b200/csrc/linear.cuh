@@ -68,7 +68,6 @@ struct LinearParams {
   ExpertArgs ex;       // expert weights chosen on the device
   bool one_sm;         // prompt projections: not the kernel on pairs of SMs (LRI_ONE_SM)
   Share share;
-  NormArgs nm;         // one-row QKV and SWIGLU forms of the SIMT kernel
   ArgmaxArgs am;       // ARGMAX epilogue of the SIMT kernel: greedy choice instead of stored logits
 };
 
@@ -116,9 +115,9 @@ __device__ __forceinline__ void qkv_epilogue_pair(const LinearParams& p, int64_t
 int streaming_rows();  // token rows up to which the streaming kernels run (option stream_rows)
 // decode path, 1 <= p.m <= 8 (SIMT FMA)
 int gemv_launch(int dtype, int epi, const LinearParams& p, cudaStream_t st);
-// one row whose norm is taken on the way (p.nm): EPI_QKV and EPI_SWIGLU
+// one row whose norm is taken on the way: EPI_QKV and EPI_SWIGLU
 bool gemv_norm_supports(int64_t m, int k);
-int gemv_norm_launch(int dtype, int epi, const LinearParams& p, cudaStream_t st);
+int gemv_norm_launch(int dtype, int epi, const LinearParams& p, const NormArgs& nm, cudaStream_t st);
 // lri_linear, lri_gateup_swiglu, lri_qkv_rope_kvcache
 int linear(int dtype, const void* x, const void* w, const void* addend, void* y, int64_t M, int N, int K, void* workspace, size_t workspace_bytes,
            Share share, lri_stream_t stream);

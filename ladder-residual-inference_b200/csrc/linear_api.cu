@@ -507,8 +507,8 @@ int lri::norm_gateup_swiglu(int dtype, const NormArgs& nm, const void* w1, void*
   if (rc != LRI_OK) return rc;
   LRI_REQUIRE(h != nullptr && I > 0, LRI_ERR_ARG, "gateup_swiglu: h is NULL or I=%d", I);
   LinearParams p{};
-  p.nm = nm, p.x = nm.res, p.w = w1, p.y = h, p.m = 1, p.n = I, p.k = K;
-  return gemv_norm_launch(dtype, EPI_SWIGLU, p, st);
+  p.x = nm.res, p.w = w1, p.y = h, p.m = 1, p.n = I, p.k = K;
+  return gemv_norm_launch(dtype, EPI_SWIGLU, p, nm, st);
 }
 int lri::gateup_swiglu(int dtype, const void* x, const void* w1, void* h, int64_t M, int I, int K, void* workspace, size_t workspace_bytes,
                        Share share, lri_stream_t stream) {
@@ -620,11 +620,11 @@ int lri::norm_qkv_rope_kvcache(int dtype, const NormArgs& nm, const void* wqkv, 
   rc = check_qkv(rope_table, input_pos, q_out, k_cache, v_cache, n_head, n_kv, head_dim, smax, table_rows);
   if (rc != LRI_OK) return rc;
   LinearParams p{};
-  p.nm = nm, p.x = nm.res, p.w = wqkv, p.m = 1, p.n = (n_head + 2 * n_kv) * head_dim, p.k = K;
+  p.x = nm.res, p.w = wqkv, p.m = 1, p.n = (n_head + 2 * n_kv) * head_dim, p.k = K;
   p.rope_table = rope_table, p.input_pos = input_pos, p.pos_is_i64 = pos_is_i64;
   p.q_out = q_out, p.k_cache = k_cache, p.v_cache = v_cache;
   p.S = 1, p.n_head = n_head, p.n_kv = n_kv, p.head_dim = head_dim, p.smax = smax, p.table_rows = table_rows;
-  return gemv_norm_launch(dtype, EPI_QKV, p, st);
+  return gemv_norm_launch(dtype, EPI_QKV, p, nm, st);
 }
 int lri::qkv_rope_kvcache(int dtype, const void* x, const void* wqkv, const void* rope_table, const void* input_pos, int pos_is_i64, void* q_out,
                           void* k_cache, void* v_cache, int B, int S, int K, int n_head, int n_kv, int head_dim, int64_t smax, int64_t table_rows,
