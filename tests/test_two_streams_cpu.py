@@ -6,11 +6,11 @@ import torch
 SHAPE = dict(block_size=64, vocab_size=64, n_layer=2, n_head=4, n_local_heads=4, dim=1024, intermediate_size=96)
 
 
-def _engine(family, monkeypatch, batch):
+def _engine(family, monkeypatch, batch, dim=1024):
     import gpt_fast
     from gpt_fast import gpt_ladder_TP, gpt_parallel_TP
     mod, cls = {"ladder": (gpt_ladder_TP, gpt_fast.GPTLadder), "parallel": (gpt_parallel_TP, gpt_fast.GPTParallel)}[family]
-    monkeypatch.setitem(mod.transformer_configs, "two-streams-rows", dict(SHAPE))
+    monkeypatch.setitem(mod.transformer_configs, "two-streams-rows", dict(SHAPE, dim=dim))
     model = cls.from_name("two-streams-rows").to(torch.bfloat16).eval()
     model.setup_caches(max_batch_size=batch, max_seq_length=8)
     engine = model._engine
@@ -47,3 +47,15 @@ def test_two_streams_need_a_second_one():
     for given in ({}, dict(events=ctypes.cast(some, ctypes.c_void_p)), dict(side=ctypes.addressof(some))):
         p = _C.LlamaPass(schedule=_C.PARALLEL_TWO_STREAMS, layers=ctypes.addressof(some), **given)
         assert _C.lib.lri_llama_run(ctypes.byref(p)) == -1 and b"second stream" in _C.lib.lri_last_error()
+
+
+@pytest.mark.parametrize("family,few", [("ladder", list(range(1, 9))), ("parallel", list(range(1, 65)))])
+def test_small_models_called_eagerly(family, few, monkeypatch):
+    """One stream where the host is the limit: few sequences of a ladder model, any of parallel blocks; captured steps take two."""
+    engine = _engine(family, monkeypatch, 64, dim=512)
+    capturing = False
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
+    assert [b for b in range(1, 65) if not engine._two_streams(b)] == few
+    capturing = True
+    engine.hd = 64
+    assert all(engine._two_streams(b) for b in range(1, 65))
