@@ -59,3 +59,14 @@ def test_small_models_called_eagerly(family, few, monkeypatch):
     capturing = True
     engine.hd = 64
     assert all(engine._two_streams(b) for b in range(1, 65))
+
+
+@pytest.mark.parametrize("kv_heads,one", [(8, [1, 17, 18, 19, 20, 21, 22, 23]), (4, [1])])
+def test_one_head_an_sm(kv_heads, one, monkeypatch):
+    """Parallel blocks with about one 128-wide (sequence, head) pair an SM stay on one stream, but not where query heads share keys."""
+    monkeypatch.setitem(SHAPE, "n_head", 8)
+    monkeypatch.setitem(SHAPE, "n_local_heads", kv_heads)
+    engine = _engine("parallel", monkeypatch, 64)
+    assert engine.hd == 128
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    assert [b for b in range(1, 65) if not engine._two_streams(b)] == one
