@@ -48,10 +48,13 @@ __device__ __forceinline__ void store_v(T* p, const float (&f)[VEC]) {
   }
 }
 
-// PRE (few rows): the kernel is a chain of load latencies, so everything that can be loaded at once is.
+// PRE (few rows): the kernel is a chain of load latencies, so everything that can be loaded at once is; the gate and a second result only where a
+// thread has registers for them (1024 threads spill with them: 8192 wide, 16 rows, one result 4.79 -> 5.77 us, two 4.92 -> 6.07), and not without
+// PRE (4096 wide, 64 rows, two results 5.88 -> 6.24).
 template <typename T, int VEC, int NV, int THREADS, bool PRE>
 __global__ void __launch_bounds__(THREADS) gated_norm_add_kernel(const GatedNormParams p) {
   __shared__ float part[33];
+  constexpr bool kAhead = PRE && THREADS <= 512;
   const int64_t row = blockIdx.x;
   const int dim = p.dim, nvec = dim / VEC;
   const T* y = static_cast<const T*>(p.y);
@@ -80,7 +83,8 @@ __global__ void __launch_bounds__(THREADS) gated_norm_add_kernel(const GatedNorm
       const int v = threadIdx.x + i * THREADS;
       if (v >= nvec) continue;
       if (p.resid) load_v<float, VEC>(p.resid + row * dim + v * VEC, res[i]);
-      if (p.gate) load_v<float, VEC>(p.gate + row * p.gate_ld + v * VEC, gate[i]);
+      if constexpr (kAhead)
+        if (p.gate) load_v<float, VEC>(p.gate + row * p.gate_ld + v * VEC, gate[i]);
     }
   }
   float ss = 0.f;
@@ -97,26 +101,40 @@ __global__ void __launch_bounds__(THREADS) gated_norm_add_kernel(const GatedNorm
       src = src < 0 ? 0 : (src >= p.y_rows ? p.y_rows - 1 : src);
       return y + src * dim + v * VEC;
     };
-    for (int s = 0; s < p.n_slots; s += 2) {  // two on their way at a time
-      const bool two = s + 1 < p.n_slots;
-      float f[VEC], f2[VEC];
-      load_v<T, VEC>(slot(s), f);
-      if (two) load_v<T, VEC>(slot(s + 1), f2);
+    if constexpr (kAhead) {
+      for (int s = 0; s < p.n_slots; s += 2) {  // two on their way at a time
+        const bool two = s + 1 < p.n_slots;
+        float f[VEC], f2[VEC];
+        load_v<T, VEC>(slot(s), f);
+        if (two) load_v<T, VEC>(slot(s + 1), f2);
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) t[i][e] += f[e];
-      if (two) {
+        for (int e = 0; e < VEC; ++e) t[i][e] += f[e];
+        if (two) {
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) t[i][e] += f2[e];
+          for (int e = 0; e < VEC; ++e) t[i][e] += f2[e];
+        }
+      }
+    } else {
+      for (int s = 0; s < p.n_slots; ++s) {
+        float f[VEC];
+        load_v<T, VEC>(slot(s), f);
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) t[i][e] += f[e];
       }
     }
     if (p.gate) {
       float g[VEC], b[VEC];
       if constexpr (PRE) {
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) b[e] = cb[i][e], g[e] = gate[i][e];
+        for (int e = 0; e < VEC; ++e) b[e] = cb[i][e];
+      } else {
+        load_v<T, VEC>(bias + v * VEC, b);
+      }
+      if constexpr (kAhead) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) g[e] = gate[i][e];
       } else {
         load_v<float, VEC>(p.gate + row * p.gate_ld + v * VEC, g);
-        load_v<T, VEC>(bias + v * VEC, b);
       }
 #pragma unroll
       for (int e = 0; e < VEC; ++e) t[i][e] *= sigmoid_f(g[e] + b[e]);
