@@ -31,7 +31,7 @@ constexpr int kTerms = 3;
 constexpr int kMaxSegments = 8;
 constexpr int kMinSegment = 64;  // tokens
 constexpr int kMaxE = 128;
-constexpr int kNarrow = 64;  // channels and values up to which a CTA has 256 threads, otherwise 512
+constexpr int kNarrow = 64;  // channels and values up to which a CTA may have 256 threads instead of 512
 
 using bf16 = __nv_bfloat16;
 
@@ -106,8 +106,9 @@ struct Smem {
 // Grid (segments, heads, sequences).  FULL: outputs and the sequence's final state; otherwise the segment's contribution.
 //
 // THREADS 512: a warp takes one token of a block, up to 128 channels and values.  THREADS 256, heads of up to 64 channels and values: a warp
-// takes two tokens, half of its lanes each, and two CTAs share an SM.  With 512 threads half of the lanes of such heads had nothing to do:
+// takes two tokens, half of its lanes each, and two CTAs share an SM.  With 512 threads half of the lanes of such heads have nothing to do:
 // 32 heads of 64 x 64, 2048 tokens of one sequence, first and second pass: 49 and 108 us with 512 threads and 4 segments, 31 and 83 with 256 and 8.
+// takes_narrow() chooses.
 template <typename T, int CP, bool FULL, int THREADS>
 __global__ void __launch_bounds__(THREADS, 512 / THREADS) hgrn2_blocks_kernel(const Hgrn2Params p, const Segments sg) {
   constexpr int kThreads = THREADS, kWarps = THREADS / 32, ME = THREADS == 256 ? kNarrow : kMaxE;
@@ -429,24 +430,39 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) hgrn2_blocks_kernel(co
   }
 }
 
-bool narrow(int C, int E) { return C <= kNarrow && E <= kNarrow; }
+bool fits_narrow(int C, int E) { return C <= kNarrow && E <= kNarrow; }
 
 // Segments wanted: as many CTAs as the SMs hold.  Grows with S, so that the workspace of a longer call serves a shorter one.
-int64_t wanted_segments(int B, int S, int H, int C, int E) {
-  int64_t n = device_sm_count() * (narrow(C, E) ? 2ll : 1ll) / (static_cast<int64_t>(B) * H);
+int64_t wanted_segments(int B, int S, int H, bool narrow) {
+  int64_t n = device_sm_count() * (narrow ? 2ll : 1ll) / (static_cast<int64_t>(B) * H);
   n = n > kMaxSegments ? kMaxSegments : n;
   n = n > S / kMinSegment ? S / kMinSegment : n;
   return n < 1 ? 1 : n;
 }
 
-Segments plan(int B, int S, int H, int C, int E) {
+Segments segments(int B, int S, int H, bool narrow) {
   Segments s{};
-  const int64_t n = wanted_segments(B, S, H, C, E);
+  const int64_t n = wanted_segments(B, S, H, narrow);
   int tokens = static_cast<int>((S + n - 1) / n);
   tokens = (tokens + kBlock - 1) / kBlock * kBlock;
   s.tokens = tokens;
   s.count = (S + tokens - 1) / tokens;
   return s;
+}
+
+// Whether a call of narrow heads runs on 256 threads.  A CTA of 512 is the faster one where SMs have no second one to hold: 1 x 300 tokens of 32 heads
+// 28.9 us for 33.8 (four segments either way), 4 x 100 25.3 for 31.2 (one).  With twice the CTAs at work it is not: 1 x 2048 153 and 101, 2 x 300
+// 50.5 and 34.9, 3 x 1000 210 and 126, 8 x 64 30.9 and 20.4, 64 x 50 213 and 136, 4 x 500 107 and 96.  So the two are estimated, in halves of a us
+// from those figures: a block of a CTA takes 7 or 9 in the pass with results, 10 or 13 in both passes, the second launch 6.
+bool takes_narrow(int B, int S, int H, int C, int E) {
+  if (!fits_narrow(C, E)) return false;
+  auto cost = [&](bool narrow) {
+    const Segments s = segments(B, S, H, narrow);
+    const int64_t room = device_sm_count() * (narrow ? 2ll : 1ll), waves = (static_cast<int64_t>(B) * H * s.count + room - 1) / room;
+    const int64_t blocks = waves * ((s.tokens + kBlock - 1) / kBlock);
+    return s.count > 1 ? blocks * (narrow ? 13 : 10) + 6 : blocks * (narrow ? 9 : 7);
+  };
+  return cost(true) < cost(false);
 }
 
 template <typename T, int CP, int THREADS>
@@ -467,8 +483,8 @@ int launch(const Hgrn2Params& p, const Segments& sg, int B, cudaStream_t st) {
 }
 
 template <typename T>
-int launch_shape(const Hgrn2Params& p, const Segments& sg, int B, cudaStream_t st) {
-  if (narrow(p.C, p.E)) return launch<T, 64, 256>(p, sg, B, st);
+int launch_shape(const Hgrn2Params& p, const Segments& sg, bool narrow, int B, cudaStream_t st) {
+  if (narrow) return launch<T, 64, 256>(p, sg, B, st);
   return p.C <= 64 ? launch<T, 64, 512>(p, sg, B, st) : launch<T, 128, 512>(p, sg, B, st);
 }
 
@@ -481,18 +497,20 @@ bool hgrn2_blocks_supports(int dtype, const Hgrn2Params& p, int B) {
 }
 
 size_t hgrn2_blocks_workspace_bytes(int B, int S, int H, int C, int E) {
-  const int64_t n = wanted_segments(B, S, H, C, E);
+  // (room for either form: which one runs does not grow with S)
+  const int64_t n = wanted_segments(B, S, H, fits_narrow(C, E));
   if (n < 2) return 0;
   return static_cast<size_t>(B) * H * C * (static_cast<size_t>(n) * E + n - 1) * sizeof(float);
 }
 
 int hgrn2_blocks_launch(int dtype, const Hgrn2Params& p, int B, void* workspace, cudaStream_t st) {
-  Segments sg = plan(B, p.S, p.H, p.C, p.E);
+  const bool narrow = takes_narrow(B, p.S, p.H, p.C, p.E);
+  Segments sg = segments(B, p.S, p.H, narrow);
   const size_t mat = static_cast<size_t>(B) * p.H * p.C * p.E;
   sg.init = static_cast<float*>(workspace);
   sg.part = sg.init + mat;
   sg.decay = sg.part + mat * (sg.count - 1);
-  return dtype == LRI_BF16 ? launch_shape<bf16>(p, sg, B, st) : launch_shape<__half>(p, sg, B, st);
+  return dtype == LRI_BF16 ? launch_shape<bf16>(p, sg, narrow, B, st) : launch_shape<__half>(p, sg, narrow, B, st);
 }
 
 }  // namespace lri
