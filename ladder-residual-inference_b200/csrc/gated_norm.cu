@@ -50,7 +50,7 @@ __device__ __forceinline__ void store_v(T* p, const float (&f)[VEC]) {
 
 // PRE (few rows): the kernel is a chain of load latencies, so everything that can be loaded at once is; the gate and a second result only where a
 // thread has registers for them (1024 threads spill with them: 8192 wide, 16 rows, one result 4.79 -> 5.77 us, two 4.92 -> 6.07), and not without
-// PRE (4096 wide, 64 rows, two results 5.88 -> 6.24).
+// PRE (4096 wide, 64 and 2048 rows, two results 5.86 -> 6.25, 30.2 -> 32.6, four 6.12 -> 7.19, 35.0 -> 41.0).
 template <typename T, int VEC, int NV, int THREADS, bool PRE>
 __global__ void __launch_bounds__(THREADS) gated_norm_add_kernel(const GatedNormParams p) {
   __shared__ float part[33];
@@ -101,26 +101,22 @@ __global__ void __launch_bounds__(THREADS) gated_norm_add_kernel(const GatedNorm
       src = src < 0 ? 0 : (src >= p.y_rows ? p.y_rows - 1 : src);
       return y + src * dim + v * VEC;
     };
-    if constexpr (kAhead) {
-      for (int s = 0; s < p.n_slots; s += 2) {  // two on their way at a time
-        const bool two = s + 1 < p.n_slots;
-        float f[VEC], f2[VEC];
-        load_v<T, VEC>(slot(s), f);
-        if (two) load_v<T, VEC>(slot(s + 1), f2);
+    int s = 0;
+    if (kAhead && (p.n_slots == 2 || p.n_slots == 3)) {
+      float f[VEC], f2[VEC];
+      load_v<T, VEC>(slot(0), f);
+      load_v<T, VEC>(slot(1), f2);
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) t[i][e] += f[e];
-        if (two) {
+      for (int e = 0; e < VEC; ++e) t[i][e] += f[e];
 #pragma unroll
-          for (int e = 0; e < VEC; ++e) t[i][e] += f2[e];
-        }
-      }
-    } else {
-      for (int s = 0; s < p.n_slots; ++s) {
-        float f[VEC];
-        load_v<T, VEC>(slot(s), f);
+      for (int e = 0; e < VEC; ++e) t[i][e] += f2[e];
+      s = 2;
+    }
+    for (; s < p.n_slots; ++s) {
+      float f[VEC];
+      load_v<T, VEC>(slot(s), f);
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) t[i][e] += f[e];
-      }
+      for (int e = 0; e < VEC; ++e) t[i][e] += f[e];
     }
     if (p.gate) {
       float g[VEC], b[VEC];
@@ -225,7 +221,8 @@ int dispatch(const GatedNormParams& p, int64_t rows, cudaStream_t st) {
   const int nvec = p.dim / 8;
   // At most a CTA an SM: latency too, but where rows wait for room the registers of PRE cost more than they save.  Patevik 1B (width 2048), without
   // / with it: a step of 1, 4, 16, 40 sequences 901 / 858, 1475 / 1435, 2152 / 2106, 2522 / 2493 us, a prompt of 100 2748 / 2693, of 2048 7315 / 7403.
-  if (rows <= device_sm_count() && nvec <= 256) return launch<T, 8, 1, 256, true>(p, rows, st);
+  // Not with more than three results (64 rows, four 3.79 us without PRE, 3.96 with it).
+  if (rows <= device_sm_count() && nvec <= 256 && p.n_slots <= 3) return launch<T, 8, 1, 256, true>(p, rows, st);
   if (rows <= 16 && nvec > 256) {  // few rows: the kernel is one thread's latency chain, spread the row
     if (nvec <= 512) return launch<T, 8, 1, 512, true>(p, rows, st);
     if (nvec <= 1024) return launch<T, 8, 1, 1024, true>(p, rows, st);
