@@ -486,8 +486,8 @@ int lri_round_columns(int dtype, const float* x, int64_t ld, int64_t off, int n,
 
 /* ---- the layers of one forward pass on one GPU -------------------------------------------------
  * From the embedded rows in `resid` to the normed rows in `normed`, by the entry points above in the order of one of the
- * schedules.  layers: for each layer attention norm, QKV, wo, MLP norm, w1, w2, K cache, V cache; reduces (desync): for each
- * layer whether attention and MLP fold their partial into the residual.  Buffers hold B S rows.  Nothing is kept of it. */
+ * schedules.  layers: for each layer attention norm, QKV, wo, MLP norm, w1, w2, K cache, V cache; reduces: not NULL for
+ * LRI_DESYNC, but not read (on one GPU a partial that is reduced at once gives the sums of one that the next norm adds).  Buffers hold B S rows.  Nothing is kept of it. */
 enum lri_schedule { LRI_DENSE = 0, LRI_LADDER = 1, LRI_LADDER_TWO_STREAMS = 2, LRI_PARALLEL = 3, LRI_DESYNC = 4,
                     LRI_PARALLEL_TWO_STREAMS = 5 /* gate/up on `side` beside the attention chain; needs `side` and `events` */ };
 typedef struct {

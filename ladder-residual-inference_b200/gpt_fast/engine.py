@@ -231,7 +231,7 @@ class Engine:
         want_both = (nqkv + 2 * self.inter, self.d)
         smax = None
         # a layer's attention norm, QKV, wo, MLP norm, w1, w2, K cache, V cache; where w1 is the lower part of a tensor, the bytes above it
-        tensors, above, reduces = [], [], [] if family == "desync" else None
+        tensors, above = [], []
         try:
             for layer in m.layers:
                 sub = layer._modules
@@ -256,8 +256,6 @@ class Engine:
                 if w.shape != want_qkv or w1.shape != want_w1 or w2.shape != want_w2:
                     return False
                 tensors += (norm, w, wo, sub["ffn_norm"]._parameters["weight"], w1, w2, k_cache, cache["v_cache"])
-                if reduces is not None:
-                    reduces += (int(layer.do_attention_all_reduce), int(layer.do_mlp_all_reduce))
         except KeyError:
             return False
         main = torch.cuda.current_stream()
@@ -270,7 +268,7 @@ class Engine:
                      table_rows=m.freqs_cis.shape[0])
         schedule = {"dense": DENSE, "ladder": LADDER_TWO_STREAMS if two else LADDER, "parallel": PARALLEL_TWO_STREAMS if two else PARALLEL,
                     "desync": DESYNC}[family]
-        self.ops.run_layers(schedule, tensors, above, reduces, self._events if two else None, main.cuda_stream,
+        self.ops.run_layers(schedule, tensors, above, self._events if two else None, main.cuda_stream,
                             self.side_stream.cuda_stream if two else None, sizes, self.cfg.norm_eps,
                             dict(ws_qkv=self.ws_qkv, ws_wo=self.ws_wo, ws_ug=self.ws_ug, ws_w2=self.ws_w2, scratch=self.scratch), self.row_ws, **buffers)
         return True

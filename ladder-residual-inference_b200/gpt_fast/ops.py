@@ -125,7 +125,7 @@ class CudaOps:
 
     # ---- all layers of a pass ------------------------------------------------------------------------
     @staticmethod
-    def run_layers(schedule, layers, above, reduces, events, main, side, sizes, eps, workspaces, row_ws, **tensors):
+    def run_layers(schedule, layers, above, events, main, side, sizes, eps, workspaces, row_ws, **tensors):
         """lri_llama_run_row: `layers` eight tensors a layer as there, `above` the bytes in front of each layer's w1 (empty: none), `sizes` the
         integers of lri_llama_pass, `workspaces` and `tensors` by its names."""
         _C.require_cuda(row_ws, *tensors.values(), *layers)
@@ -139,8 +139,7 @@ class CudaOps:
             if t is not None:
                 setattr(p, k, t.data_ptr())
                 setattr(p, k + "_bytes", t.numel() * t.element_size())
-        flags = bytes(reduces) if reduces is not None else None
-        p.reduces = ctypes.cast(ctypes.c_char_p(flags), ctypes.c_void_p) if flags is not None else None
+        p.reduces = p.layers  # (what a desync pass wants to be there and does not read)
         handles = (ctypes.c_void_p * len(events))(*[e.cuda_event for e in events]) if events is not None else None
         p.events = ctypes.cast(handles, ctypes.c_void_p) if handles is not None else None
         _C.check(_C.lib.lri_llama_run_row(ctypes.byref(p), row_ws.data_ptr()))

@@ -102,3 +102,19 @@ def test_the_pass_has_the_size_that_callers_know():
     ints, wide, pointers, sizes = 12 + 1, 2, 2 + 3 + 8 + 5 + 3, 5
     assert ctypes.sizeof(_C.LlamaPass) == 4 * ints + 4 + 8 * (wide + pointers + sizes)
     assert _C.LlamaPass._fields_[-1][0] == "events"
+
+
+def test_a_desync_pass_on_one_gpu_asks_no_layer_what_it_reduces(monkeypatch):
+    """Its sums are the same whichever layers do; the walk over the layers bounds a small model's step."""
+    model = _model("desync", monkeypatch)
+    engine = model._engine
+    engine._splits = 1
+    for layer in model.layers:
+        del layer.do_attention_all_reduce, layer.do_mlp_all_reduce
+
+    def called(*args, **kwargs):
+        raise Called
+
+    monkeypatch.setattr(torch.cuda, "current_stream", called)
+    with pytest.raises(Called):
+        engine._run_native(1, 1, torch.zeros(1, dtype=torch.int32))

@@ -78,9 +78,9 @@ def test_parallel_passes_of_one_stream_read_no_events(monkeypatch):
         model = _model("parallel", torch.bfloat16, 9)
         _only(model._engine, True)
 
-        def given(schedule, layers, above, reduces, _, main, side, *rest, **kw):
+        def given(schedule, layers, above, _, main, side, *rest, **kw):
             assert side is None
-            return run(schedule, layers, above, reduces, events, main, None, *rest, **kw)
+            return run(schedule, layers, above, events, main, None, *rest, **kw)
         monkeypatch.setattr(CudaOps, "run_layers", staticmethod(given))
         with torch.no_grad():
             results.append(model(tok, pos))
