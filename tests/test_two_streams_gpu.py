@@ -85,3 +85,41 @@ def test_parallel_passes_of_one_stream_read_no_events(monkeypatch):
         with torch.no_grad():
             results.append(model(tok, pos))
     assert torch.isfinite(results[0].float()).all() and torch.equal(*results)
+
+
+@pytest.mark.parametrize("family,batches", [("ladder", [2, 4, 5, 8, 20]), ("parallel", [2, 8, 9, 20, 33, 40, 49])])
+def test_large_projections_beside_each_other(family, batches):
+    """Projections of 15 M weights and more take the small-batch kernel from two rows on, so that its rings of every length run beside another stream's:
+    eager and captured steps on two streams against one, bit for bit."""
+    from gpt_fast import _C
+    for batch in batches:
+        model = _model(family, torch.bfloat16, batch, n_layer=2, dim=2048, n_head=16, n_local_heads=8, intermediate_size=8192)
+        engine = model._engine
+        _only(engine, True)
+        tok = torch.randint(0, 512, (batch, 1), generator=torch.Generator().manual_seed(1)).to(torch.int32).cuda()
+        pos = torch.tensor([0], dtype=torch.int32, device="cuda")
+
+        def step(overlap):
+            engine.overlap_sublayers = overlap
+            assert engine._two_streams(batch) is overlap
+            return model(tok, pos)
+        with torch.no_grad():
+            for p in range(3):  # (each writes the row that the next ones read)
+                pos.fill_(p)
+                got, want = step(True), step(False)
+                assert torch.isfinite(got.float()).all() and torch.equal(got, want)
+            side = torch.cuda.Stream()
+            side.wait_stream(torch.cuda.current_stream())
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=side):
+                logits = step(True)
+            torch.cuda.current_stream().wait_stream(side)
+            for p in (3, 50):
+                pos.fill_(p)
+                for _ in range(5):
+                    graph.replay()
+                captured = logits.clone()
+                assert torch.equal(captured, step(False))
+        torch.cuda.synchronize()
+        assert _C.lib.lri_gemm_status() == 0
+        del model, graph
