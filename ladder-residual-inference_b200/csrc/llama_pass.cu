@@ -100,8 +100,8 @@ struct Pass {
     const void* pending = nullptr;
     // us a captured step, whole / half ring.  8B: 16, 32 sequences 3251 / 3176, 3488 / 3400, but 33, 40, 48, 64 3542 / 3609, 3777 / 3851, 3848 / 3950, 4025 /
     // 4120; 3B: 2, 4 1677 / 1779, 1785 / 1903, 9, 40, 48 1842 / 1785, 2712 / 2702, 2798 / 2797, 64 3241 / 3258; 1B: 9, 16, 32 787 / 756, 795 / 777, 869 / 845,
-    // 48, 64 943 / 944, 1048 / 1056.
-    share = {false, rows > 8 && rows <= (p.dim >= 4096 ? 32 : 48)};
+    // 48, 64 943 / 944, 1048 / 1056, but called eagerly 1173 / 1118 (on another machine 1162 / 1152).
+    share = {false, rows > 8 && rows <= (p.dim >= 4096 ? 32 : p.dim > 2048 ? 48 : kSplitKMaxRows)};
     for (int l = 0; l < p.n_layer; ++l) {
       if (!norm(at(l, kAttentionNorm), pending, nullptr, true, p.normed, p.stream) || !record(2 * l, p.stream) || !wait(2 * l, p.side)) return false;
       if (!attention(l) ||
