@@ -330,7 +330,8 @@ constexpr int kJoinCols = 16, kJoinThreads = 256;
 // Delta rule: one CTA per 16 columns of a head, one thread per column and every 16th row; M of the next segment is copied in while
 // this one's product runs.  The product has sums of its own, four a thread, and joins S0 in one rounding: added to S0 term by term each of the C
 // roundings had the size of the state (1300 tokens in ten segments, 128 x 96, error of the state 1.34e-7 in one segment, 1.82e-7 so, 1.37e-7 now;
-// the whole recurrence of 2 x 1500 tokens, 16 heads of 64 x 64, 144 us so, 136 now).
+// the whole recurrence of 2 x 1500 tokens, 16 heads of 64 x 64, 144 us so, 136 now).  About 3 us a product of 64 x 64 x 64: 20.5 us
+// for two sequences in eight segments, 25 and 42 for one in ten and sixteen.
 __global__ void __launch_bounds__(kJoinThreads) state_join_kernel(const ScanParams p) {
   extern __shared__ __align__(16) float join_smem[];
   const int C = p.C, E = p.E, H = p.H, h = blockIdx.y, segs = p.segs;
@@ -472,10 +473,12 @@ int launch_scan(const ScanParams& p, int B, int warps, cudaStream_t st) {
 }
 
 // Segments of a sequence, from the elements of all states (more of them fill the chip without) and the tokens.  Measured, us, one segment / this
-// rule: gated linear attention 64 x 128 x 16 heads (131 K elements a sequence), one sequence, 500 tokens 42 / 35, 1000 80 / 46, 2048 159 / 82;
-// 2 x 1500 134 / 106, 3 x 1000 136 / 103, 4 x 800 128 / 111; 128 x 256, 1000 154 / 128, 2048 311 / 225; but 6 x 680 119 / 143 and, 128 x 256, 2 x 1000
-// 200 / 220.  The delta rule runs three columns where one segment has one: 64 x 64 x 16 heads (66 K), one sequence, 1200 tokens 113 / 103, 2048
-// 191 / 136, 4000 369 / 219; 2 x 1500 173 / 146, 2 x 2048 236 / 184; but 800 76 / 81, 4 x 1000 148 / 164 and, 128 x 128, 2048 263 / 281.
+// rule: gated linear attention 64 x 128 x 16 heads (131 K elements a sequence), one sequence, 500 tokens 42 / 33, 1000 82 / 49, 2048 163 / 79;
+// 2 x 1500 178 / 102, 3 x 1000 153 / 103, 4 x 800 129 / 118, 4 x 2000 317 / 235; 128 x 256, 1000 160 / 125, 2048 325 / 227; but 5 x 800 137 / 138 with
+// eight and, 128 x 256, 2 x 1000 198 / 218.  The delta rule runs three columns where one segment has one: 64 x 64 x 16 heads (66 K), one sequence, 1200
+// tokens 117 / 104, 2048 198 / 130, 4000 396 / 213; 2 x 1500 189 / 136, 2 x 2048 256 / 174; but 800 79 / 80 with eight, 4 x 1000 169 / 172, 8 x 500 129 /
+// 193 and, 128 x 128, 2048 261 / 273.  Its line at 128 K elements leaves out three sequences, which six segments would serve (3 x 1000 159 / 121, 3 x 2000
+// 315 / 209), and four long ones (4 x 2000 335 / 300 with four).
 int scan_segments(int B, int S, int heads, int dim, int vdim, bool delta) {
   if (dim > kMaxSegmentChannels || dim % 4 != 0 || vdim % 4 != 0) return 1;
   const int forced = option(OPT_SCAN_SEGMENTS);
