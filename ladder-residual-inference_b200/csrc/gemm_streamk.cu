@@ -391,14 +391,16 @@ int plan_ctas(int tiles, int total_kt, int max_seg) {
 // layer) half of it, so that two CTAs share an SM: one's weights arrive while the other waits for its token rows or finishes.  A whole step, us,
 // whole ring / half: 8B, 2, 4, 8, 16, 24, 40, 64 sequences 2783 / 2664, 2822 / 2660, 2898 / 2802, 2998 / 2923, 3346 / 3187, 3897 / 3707, 4467 /
 // 4356; 1B, 2, 4, 16, 24, 40, 64 651 / 635, 679 / 650, 748 / 715, 822 / 791, 931 / 861, 1126 / 1087.  Alone on the GPU the half ring is the
-// slower one (8B dense, 16 sequences 3528 / 3639).  With 5 to 8 rows only the other projections of a narrow model are on the streaming kernel, whose
-// CTAs want the room themselves: gated ones keep four stages (1B, 6 and 8 sequences 691, 715 whole, 707, 756 half, 682, 712 with four).
+// slower one (8B dense, 16 sequences 3528 / 3639).  With up to 8 rows the other projections of a narrow model are on the streaming kernel, whose
+// CTAs want the room themselves: with 5 to 8 gated ones keep four stages (1B, 6 and 8 sequences 691, 715 whole, 707, 756 half, 682, 712 with four), and
+// three rows the whole ring (1B, 2, 3, 4 sequences 637, 643, 650 whole, 613, 665, 633 half; 8B 2749, 2754, 2757 and 2673, 2691, 2667).
 int ring_stages(const LinearParams& lin, int stage_bytes, int accumulators) {
   constexpr int kHalf = 108 * 1024;
   int stages = kSmemBudget / stage_bytes;
   if (lin.share.half_ring) {
-    stages = kHalf / stage_bytes;
-    if (accumulators == 2 && lin.m > 4 && lin.m <= 8 && lin.k < 4096) stages = 4;
+    const bool narrow = accumulators == 2 ? lin.k < 4096 : lin.n < 4096;
+    if (!(narrow && lin.m == 3)) stages = kHalf / stage_bytes;
+    if (narrow && accumulators == 2 && lin.m > 4 && lin.m <= 8) stages = 4;
   }
   return stages > 8 ? 8 : stages;
 }
