@@ -76,7 +76,11 @@ struct Pass {
   // the attention chain of a layer on `stream`, its MLP chain on `side`: see Engine._run_ladder_two_streams
   bool ladder_two_streams() {
     if (!record(0, p.stream) || !wait(0, p.side)) return false;
-    share = {false, true};
+    // Half of the ring for each (gemm_streamk.cu), but not in wide models where attention over a long cache is what runs beside 9 to 16 rows.  8B, us a
+    // captured step, whole / half: 9 sequences at 1000, 2000, 4000 positions 2967 / 2924, 3200 / 3202, 3648 / 3679; 12 2983 / 2961, 3234 / 3254, 3728 / 3818;
+    // 16 3054 / 3012, 3364 / 3394, 3983 / 4055; but 8 at 7000 3778 / 3738, 24 at 2600 4193 / 4184, 64 at 900 4648 / 4565; 1B, 16 at 1900 852 / 819.  The
+    // position is not known here, the cache's length is.
+    share = {false, !(p.dim >= 4096 && rows > 8 && rows <= 16 && p.smax > 1600)};
     int n = 1;
     for (int l = 0; l < p.n_layer; ++l, n += 2) {
       if (!norm(at(l, kAttentionNorm), l ? p.part_a : nullptr, nullptr, true, p.normed, p.stream) || !record(n, p.stream) || !attention(l)) return false;
