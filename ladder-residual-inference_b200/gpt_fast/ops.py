@@ -386,13 +386,13 @@ class CudaOps:
         _C.require_cuda(*[x for x in blocks if x is not None], v, state, input_pos, o)
         qd, kd, ku, decay, coef = blocks
         _, heads, dim, vdim = state.shape
-        if workspace is not None:
-            _C.require_cuda(workspace)
-        _C.check(_C.lib.lri_state_scan_segments(qd.data_ptr(), kd.data_ptr() if delta else None, ku.data_ptr(), decay.data_ptr(),
-                                                coef.data_ptr(), v.data_ptr(), v_row, state.data_ptr(), input_pos.data_ptr(),
-                                                int(input_pos.dtype == torch.int64), o.data_ptr(), B, S, heads, dim, vdim,
-                                                None if workspace is None else workspace.data_ptr(),
-                                                0 if workspace is None else workspace.numel(), _C.stream_handle()))
+        call = (qd.data_ptr(), kd.data_ptr() if delta else None, ku.data_ptr(), decay.data_ptr(), coef.data_ptr(), v.data_ptr(), v_row,
+                state.data_ptr(), input_pos.data_ptr(), int(input_pos.dtype == torch.int64), o.data_ptr(), B, S, heads, dim, vdim)
+        if workspace is None:
+            _C.check(_C.lib.lri_state_scan(*call, _C.stream_handle()))
+            return
+        _C.require_cuda(workspace)
+        _C.check(_C.lib.lri_state_scan_segments(*call, workspace.data_ptr(), workspace.numel(), _C.stream_handle()))
 
     @staticmethod
     def state_step_supports(dim, vdim, decay_rank, gate_rank):

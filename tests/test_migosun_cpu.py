@@ -145,3 +145,21 @@ def test_entry_points_check_arguments_without_a_gpu():
     assert lib.lri_state_step_supports(128, 128, 16, 16) == 1 and lib.lri_state_step_supports(300, 8, 8, 8) == 0
     assert lib.lri_state_step_supports(64, 64, 12, 8) == 0
     assert lib.lri_head_norm_gate(0, 16, 16, 1e-5, 16, 8, 2, 1.0, 16, 8, 1, 1, 8, None) == -1
+
+
+def test_short_prompts_scan_without_the_workspace(monkeypatch):
+    from gpt_fast import _C
+    case = mu.CONFIGS["tiles"]
+    model = mu.build(case[0], mu.weights(case), torch.bfloat16, "cpu", 1, 1300)
+    engine = model._engine
+    scans = [b.mixer.sublayer.right if b.mixer.sublayer.kind == "parallel" else b.mixer.sublayer for b in model.layers]
+
+    def segments(S):
+        return any(_C.lib.lri_state_scan_workspace_bytes(1, S, m.heads, m.dim, m.vdim, int(m.kind == "gated_delta")) for m in scans)
+    assert engine.ws_scan is not None and segments(engine.scan_from) and not segments(engine.scan_from - 1)
+    given = []
+    monkeypatch.setattr(type(engine.ops) if not isinstance(engine.ops, type) else engine.ops, "state_scan", staticmethod(lambda *a, **kw: given.append(kw)))
+    engine.scan_blocks = None
+    for S in (engine.scan_from - 1, engine.scan_from):
+        engine._scan(False, None, 0, scans[-1], None, 1, S)
+    assert given == [{}, {"workspace": engine.ws_scan}]
