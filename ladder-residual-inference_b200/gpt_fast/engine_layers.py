@@ -100,12 +100,12 @@ class LayerEngine(Engine):
             self.ws_scan = None
             if hasattr(ops, "state_scan_workspace_bytes"):
                 # fewer sequences are cut into more segments: the largest batch is not the largest workspace
-                size = max(ops.state_scan_workspace_bytes(b, max_seq, m.heads, m.dim, m.vdim, m in delta)
-                           for m in scans for b in range(1, max_batch + 1))
+                shapes = {(m.heads, m.dim, m.vdim, m.kind == "gated_delta") for m in scans}
+                size = max(ops.state_scan_workspace_bytes(b, max_seq, *shape) for shape in shapes for b in range(1, max_batch + 1))
                 self.ws_scan = torch.empty(size, dtype=torch.uint8, device=device) if size else None
                 # shorter calls than one sequence's shortest in segments do without it
-                self.scan_from = next((s for s in range(16, max_seq + 1, 16)
-                                       if any(ops.state_scan_workspace_bytes(1, s, m.heads, m.dim, m.vdim, m in delta) for m in scans)), max_seq + 1)
+                self.scan_from = next((s for s in range(16, max_seq + 1, 16) if any(ops.state_scan_workspace_bytes(1, s, *shape) for shape in shapes)),
+                                      max_seq + 1)
         if delta:
             self.scan_v = buf(rows, most(delta, lambda m: m.out_width), torch.float32)
             self.scan_gate = buf(rows, most(delta, lambda m: m.out_width), torch.float32)
