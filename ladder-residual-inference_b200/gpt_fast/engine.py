@@ -198,9 +198,9 @@ class Engine:
 
     def _two_streams(self, B):
         """Whether a native decode pass runs the two sides of a layer on two streams (ladder: attention and MLP chain, parallel: the attention
-        chain and gate/up).  Not few sequences of a small model called eagerly, which is bound by the host (stories110M ladder, us on one stream
-        and two, on two machines: 4 sequences 300 and 288, 299 and 317, 8 306 and 289, 304 and 315, but 9 391 and 372, 441 and 421, 16 397 and 373,
-        445 and 424, 48 504 and 418, 506 and 435; parallel 9, 16 366 and 385, 382 and 390), nor one sequence of parallel blocks called so (3B 1496 and 1510, captured 1467 and 1400).
+        chain and gate/up).  Not a small model called eagerly, which is bound by the host (stories110M, us on one stream and two, on two machines:
+        ladder, 4 sequences 300 and 288, 299 and 317, 8 306 and 289, 304 and 315, parallel 9, 16 366 and 385, 382 and 390; see _many_of_a_small_ladder),
+        nor one sequence of parallel blocks called so (3B 1496 and 1510, captured 1467 and 1400).
         And not parallel blocks of 128-wide heads, each with keys of its own, with about one (sequence, head) pair an SM: their attention fills the
         chip for one pair's length, and gate/up in between only delays it (3B, 6 and 7 sequences 1974 and 2045 us on one stream, 2010 and 2074 on
         two; 5, 8 and 12 2055, 2091 and 2326 to 1872, 2081 and 2072).  Heads that share keys have another kernel there (8B, 8 KV heads, 17, 20, 22,
@@ -208,10 +208,15 @@ class Engine:
         if not self.overlap_sublayers or B > _TWO_STREAM_ROWS:
             return False
         parallel = self.family == "parallel"
-        few = parallel and B == 1 if self.d >= 1024 else parallel or B <= 8
-        if few and not torch.cuda.is_current_stream_capturing():
+        if (self.d < 1024 or (parallel and B == 1)) and not torch.cuda.is_current_stream_capturing():
             return False
         return not parallel or self.hd != 128 or self.nh != self.nkv or not 7 * self.sms <= 8 * B * self.nkv <= 10 * self.sms
+
+    def _many_of_a_small_ladder(self, B):
+        """Two streams for a small ladder model called eagerly after all: with nine sequences and more the projections have two kernels each, and the
+        device is as long as the host (stories110M, us on one stream and two, on two machines: 9 391 and 372, 441 and 421, 16 397 and 373, 445 and
+        424, 48 504 and 418, 506 and 435)."""
+        return self.overlap_sublayers and self.family == "ladder" and self.d < 1024 and 8 < B <= _TWO_STREAM_ROWS
 
     def _run_native(self, B, S, pos):
         """The schedule's kernels in one native call, on one GPU; False where it has to run from here: with communication, another ops object,
@@ -222,7 +227,7 @@ class Engine:
         mixed = getattr(self.cfg, "ladder_layers", None)
         if family == "ladder" and mixed is not None and len(set(mixed)) != self.cfg.n_layer or not 0 < len(m.layers) == self.cfg.n_layer:
             return False
-        two = S == 1 and self._two_streams(B)
+        two = S == 1 and (self._two_streams(B) or self._many_of_a_small_ladder(B))
         # The call passes one set of sizes for all layers; the Python form reads each weight's.  A layer that was given others, or whose weights
         # are not plain parameters, runs there.  (nn.Module's attribute access costs as much as a comparison of sizes: 100 to 150 ns.  A step of
         # a small model is bound by this and by the launches.)

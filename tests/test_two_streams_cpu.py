@@ -24,6 +24,8 @@ def test_rows_of_native_passes(family, capturing, monkeypatch):
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
     engine = _engine(family, monkeypatch, 130)
     assert [b for b in (64, 65, 128, 129, 130) if engine._two_streams(b)] == [64, 65, 128]
+    engine.d = 512
+    assert [b for b in (8, 9, 128, 129, 130) if engine._many_of_a_small_ladder(b)] == ([9, 128] if family == "ladder" else [])
 
 
 def test_rows_of_the_python_schedule(monkeypatch):
@@ -55,7 +57,7 @@ def test_small_models_called_eagerly(family, few, monkeypatch):
     engine = _engine(family, monkeypatch, 64, dim=512)
     capturing = False
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
-    assert [b for b in range(1, 65) if not engine._two_streams(b)] == few
+    assert [b for b in range(1, 65) if not (engine._two_streams(b) or engine._many_of_a_small_ladder(b))] == few
     capturing = True
     engine.hd = 64
     assert all(engine._two_streams(b) for b in range(1, 65))

@@ -1,4 +1,5 @@
-"""Decode passes whose layers run on two streams: captured steps on two streams against eager ones of the same model kept on one, bit for bit, many replays behind one another; and the rule that chooses."""
+"""Decode passes whose layers run on two streams: captured steps (two streams, half of the ring in the small-batch projections) against eager ones of the same
+small model (one stream, whole ring), bit for bit, many replays behind one another; and the rule that chooses."""
 import pytest
 import torch
 
@@ -17,6 +18,7 @@ def test_captured_steps_on_two_streams(family, batch, dtype, sizes):
     _only(engine, True)
     tok = torch.randint(0, 512, (batch, 1), generator=torch.Generator().manual_seed(1)).to(torch.int32).cuda()
     pos = torch.tensor([0], dtype=torch.int32, device="cuda")
+    assert engine.overlap_sublayers and not engine._two_streams(batch)
     with torch.no_grad():
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
@@ -32,9 +34,7 @@ def test_captured_steps_on_two_streams(family, batch, dtype, sizes):
             for _ in range(5):
                 graph.replay()
             captured = logits.clone()
-            engine.overlap_sublayers = False
             assert torch.isfinite(captured.float()).all() and torch.equal(captured, model(tok, pos))
-            engine.overlap_sublayers = True
     torch.cuda.synchronize()
     from gpt_fast import _C
     assert _C.lib.lri_gemm_status() == 0
