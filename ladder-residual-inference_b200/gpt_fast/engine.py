@@ -403,7 +403,8 @@ class Engine:
         mixed = getattr(self.cfg, "ladder_layers", None)
         if mixed is not None and len(set(mixed)) != self.cfg.n_layer:
             return self._run_hybrid(rows, B, S, pos, set(mixed))
-        if S == 1 and self.overlap_sublayers and rows <= _TWO_STREAM_ROWS:
+        # (beyond 64 rows only where the kernel on pairs of SMs is not forced upon every projection, as in lri_llama_run)
+        if S == 1 and self.overlap_sublayers and (rows <= 64 or rows <= _TWO_STREAM_ROWS and option("gemm_pair") <= 1):
             return self._run_ladder_two_streams(rows, B, S, pos)
         comm, m = self.comm, self.model
         ca, cm, pa, pm, split = self._reduce_plan(rows, hidden=True)

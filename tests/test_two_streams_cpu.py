@@ -1,9 +1,22 @@
 """How many token rows a decode step may have on two streams: the kernel on pairs of SMs, which takes projections of more than 128 rows, never runs
 beside another stream's tensor-memory kernel."""
+import contextlib
+
 import pytest
 import torch
 
 SHAPE = dict(block_size=64, vocab_size=64, n_layer=2, n_head=4, n_local_heads=4, dim=1024, intermediate_size=96)
+
+
+@contextlib.contextmanager
+def _option(name, value):
+    from gpt_fast import _C
+    before = _C.option(name)
+    _C.check(_C.lib.lri_set_option(name.encode(), value))
+    try:
+        yield
+    finally:
+        _C.check(_C.lib.lri_set_option(name.encode(), before))
 
 
 def _engine(family, monkeypatch, batch, dim=1024):
@@ -39,6 +52,11 @@ def test_rows_of_the_python_schedule(monkeypatch):
     for b in (1, 64, 65, 128, 129, 130):
         engine._run_ladder(b, b, 1, torch.zeros(1, dtype=torch.int32))
     assert ran == [1, 64, 65, 128]
+    ran.clear()
+    with _option("gemm_pair", 128):
+        for b in (64, 65, 128):
+            engine._run_ladder(b, b, 1, torch.zeros(1, dtype=torch.int32))
+    assert ran == [64]
 
 
 def test_two_streams_need_a_second_one():
