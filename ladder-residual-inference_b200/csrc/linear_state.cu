@@ -14,9 +14,9 @@
 //         the identity for the delta rule (C more columns beside the E of the state)
 //   join  state before each segment, one after the other:  S_{g+1} = M_g S_g + S0_g
 //   scan  every segment from its own first state, with results
-// All of it in fp32, and the delta rule's M is a product of contractions, so errors do not grow.  Errors against 64 bits, segments over one segment: 45
-// calls of 1300 to 4000 tokens, one and two sequences of 16 heads of 64 x 64, three ranges of decays, results 0.9998 on average (0.993 to 1.005),
-// states 1.002 (0.992 to 1.017); gated linear attention, 22 calls, 1.0006 and 1.0005 (at most 1.001 and 1.005).
+// All of it in fp32, and the delta rule's M is a product of contractions.  2 x 1500 tokens of 16 heads of 64 x 64 against 64 bits: results 7.53e-7 in
+// one segment, 7.58e-7 in eight (state 1.026e-6, 1.028e-6), gated linear attention 1.762e-7 and 1.763e-7.  Where a state is all but what the join wrote
+// it is further off (1300 tokens in ten segments, 128 x 96: 1.34e-7 in one, 1.82e-7).
 #include "linear_state.cuh"
 #include "tcgen05.cuh"
 
@@ -328,10 +328,9 @@ __global__ void __launch_bounds__(128, 1) state_scan_kernel(const __grid_constan
 constexpr int kJoinCols = 16, kJoinThreads = 256;
 
 // Delta rule: one CTA per 16 columns of a head, one thread per column and every 16th row; M of the next segment is copied in while
-// this one's product runs.  The product has sums of its own, four a thread, and joins S0 in one rounding: added to S0 term by term each of the C
-// roundings had the size of the state (1300 tokens in ten segments, 128 x 96, error of the state 1.34e-7 in one segment, 1.82e-7 so, 1.37e-7 now;
-// the whole recurrence of 2 x 1500 tokens, 16 heads of 64 x 64, 144 us so, 136 now).  About 3 us a product of 64 x 64 x 64: 20.5 us
-// for two sequences in eight segments, 25 and 42 for one in ten and sixteen.
+// this one's product runs.  3.4 to 4 us a product of 64 x 64 x 64: 25 us for two sequences in eight segments, 30 and 49 for one in ten and sixteen.
+// Each sum goes on from S0 term by term; four sums apart from it are 5 us shorter there and one rounding better, but change the last bits of every
+// state and, through the layers behind, of a prompt.
 __global__ void __launch_bounds__(kJoinThreads) state_join_kernel(const ScanParams p) {
   extern __shared__ __align__(16) float join_smem[];
   const int C = p.C, E = p.E, H = p.H, h = blockIdx.y, segs = p.segs;
@@ -358,13 +357,11 @@ __global__ void __launch_bounds__(kJoinThreads) state_join_kernel(const ScanPara
     s[c * kJoinCols + col] = mine ? slot(1)[static_cast<int64_t>(c) * E] : 0.f;
   }
   for (int g = 1; g < segs - 1; ++g) {
-    float part[kRows], acc[kRows][4];
+    float part[kRows];
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
       const int c = row + i * (kJoinThreads / kJoinCols);
       part[i] = mine && c < C ? slot(g + 1)[static_cast<int64_t>(c) * E] : 0.f;
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[i][r] = 0.f;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -379,10 +376,7 @@ __global__ void __launch_bounds__(kJoinThreads) state_join_kernel(const ScanPara
         const int c = row + i * (kJoinThreads / kJoinCols);
         if (c < C) {
           const float4 w = *reinterpret_cast<const float4*>(mg + c * C + k);
-          acc[i][0] = fmaf(w.x, x[0], acc[i][0]);
-          acc[i][1] = fmaf(w.y, x[1], acc[i][1]);
-          acc[i][2] = fmaf(w.z, x[2], acc[i][2]);
-          acc[i][3] = fmaf(w.w, x[3], acc[i][3]);
+          part[i] = fmaf(w.x, x[0], fmaf(w.y, x[1], fmaf(w.z, x[2], fmaf(w.w, x[3], part[i]))));
         }
       }
     }
@@ -391,7 +385,6 @@ __global__ void __launch_bounds__(kJoinThreads) state_join_kernel(const ScanPara
     for (int i = 0; i < kRows; ++i) {
       const int c = row + i * (kJoinThreads / kJoinCols);
       if (c < C) {
-        part[i] += (acc[i][0] + acc[i][1]) + (acc[i][2] + acc[i][3]);
         s[c * kJoinCols + col] = part[i];
         if (mine) slot(g + 1)[static_cast<int64_t>(c) * E] = part[i];
       }
@@ -476,9 +469,9 @@ int launch_scan(const ScanParams& p, int B, int warps, cudaStream_t st) {
 // rule: gated linear attention 64 x 128 x 16 heads (131 K elements a sequence), one sequence, 500 tokens 42 / 33, 1000 82 / 49, 2048 163 / 79;
 // 2 x 1500 178 / 102, 3 x 1000 153 / 103, 4 x 800 129 / 118, 4 x 2000 317 / 235; 128 x 256, 1000 160 / 125, 2048 325 / 227; but 5 x 800 137 / 138 with
 // eight and, 128 x 256, 2 x 1000 198 / 218.  The delta rule runs three columns where one segment has one: 64 x 64 x 16 heads (66 K), one sequence, 1200
-// tokens 117 / 104, 2048 198 / 130, 4000 396 / 213; 2 x 1500 189 / 136, 2 x 2048 256 / 174; but 800 79 / 80 with eight, 4 x 1000 169 / 172, 8 x 500 129 /
-// 193 and, 128 x 128, 2048 261 / 273.  Its line at 128 K elements leaves out three sequences, which six segments would serve (3 x 1000 159 / 121, 3 x 2000
-// 315 / 209), and four long ones (4 x 2000 335 / 300 with four).
+// tokens 131 / 116, 2048 222 / 135, 4000 433 / 218; 2 x 1500 218 / 145, 2 x 2048 296 / 182; but 800 88 / 87 with eight, 8 x 500 131 / 194 and, 128 x 128,
+// 2048 261 / 279.  Its line at 128 K elements leaves out three and four sequences, which six and four segments would serve (3 x 1000 185 / 127, 3 x 2000
+// 369 / 216, 4 x 1000 199 / 162, 4 x 2000 395 / 303).
 int scan_segments(int B, int S, int heads, int dim, int vdim, bool delta) {
   if (dim > kMaxSegmentChannels || dim % 4 != 0 || vdim % 4 != 0) return 1;
   const int forced = option(OPT_SCAN_SEGMENTS);

@@ -1,7 +1,5 @@
 """Matrix-state recurrences in segments that run side by side, against the recurrence token by token in 64 bits: every number of segments, segments of
 one stage and ragged last ones, from zero and from a state, and calls whose workspace is too small for them."""
-import math
-
 import pytest
 import torch
 
@@ -69,20 +67,6 @@ def test_gated_linear_attention(segments, B, S, H, C, E, n):
             dec = torch.exp(torch.nn.functional.logsigmoid(z.double().view(B, S, H, C)[b] + bias.double().view(H, C)) / 4.0)
             out, st = mo.linear_attention_recurrence(q, k, v, dec, st0[b].double() if pos0 else None)
             assert _rel(o.view(B, S, H, E)[b], out) < BOUND and _rel(state[b], st) < BOUND
-
-
-@pytest.mark.parametrize("size,seed", [((1, 1300, 4, 2, 64, 64), 1), ((1, 1300, 4, 2, 128, 96), 0)], ids=str)
-@pytest.mark.parametrize("bias", [0.0, 1.0])
-def test_joined_states_lose_one_rounding(segments, size, seed, bias):
-    """Ten segments, the last of four tokens: the state is all but the one that the join wrote.  Next to the error of one segment it may have one more
-    rounding of its own size, not one for every product that is summed into it."""
-    errors = []
-    for n in (1, 10):
-        segments(n)
-        c = _Delta(torch.float32, *size, 4, 8, 8, bias, seed)
-        c.blocks(0, size[1])
-        errors.append(_rel(c.state[0], c.oracle(0)[1]))
-    assert errors[1] < math.hypot(errors[0], 2.0 ** -24)
 
 
 def test_chosen_segments_and_small_workspaces(segments):
